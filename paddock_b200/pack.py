@@ -10,6 +10,8 @@ import ctypes as C
 import os
 import re
 
+from . import _launch
+
 PACK_MAGIC = 0x504B4450
 PACK_ABI_VERSION = 2
 TABLE_SLOTS = 953
@@ -146,6 +148,11 @@ class KernelPack:
     def __init__(self, lib, info, table, origin):
         self._lib, self.info, self._table, self.origin = lib, info, table, origin
         self._fns = {}
+        # call(name, *args, stream=0): launch slot `name` (or a named extra) and raise LaunchError on a non-zero
+        # status; status(...) returns the raw status instead.  Pointer arguments may be ints or torch tensors.
+        # Native (host/launch.cc): the argument conversion of a ctypes call costs as much as a launch.
+        self.call = _launch.Caller(self._entry, self._slow_status, LaunchError)
+        self.status = _launch.Caller(self._entry, self._slow_status, None)
 
     @classmethod
     def load(cls, path=None):
@@ -226,13 +233,15 @@ class KernelPack:
         f.restype = C.c_uint
         return f()
 
-    def call(self, name, *args, stream=0):
-        """Launch slot `name` (or a named extra) and raise LaunchError on a
-        non-zero status.  Pointer arguments may be ints or torch tensors."""
+    def _entry(self, name):
+        """The native launch entry of slot `name` or of a named extra; MissingOp when there is none."""
+        fn = self.extra(name) if name in _EXTRA_SIGS else self.fn(name)
+        return _launch.Entry(C.cast(fn, C.c_void_p).value, _EXTRA_SIGS.get(name) or _SIGS[name], name)
+
+    def _slow_status(self, name, *args, stream=0):
+        """status() through ctypes, for arguments the native path does not convert (ctypes arrays)."""
         f = self.extra(name) if name in _EXTRA_SIGS else self.fn(name)
-        rc = f(*[_arg(a) for a in args], stream)
-        if rc != 0:
-            raise LaunchError(name, rc)
+        return f(*[_arg(a) for a in args], stream)
 
     def bind(self, name, *args, stream=0):
         """A zero-argument callable that launches `name` with these arguments (converted once): for
@@ -247,11 +256,6 @@ class KernelPack:
                 raise LaunchError(name, rc)
         launch.keep = args
         return launch
-
-    def status(self, name, *args, stream=0):
-        """Like call() but returns the raw status instead of raising."""
-        f = self.extra(name) if name in _EXTRA_SIGS else self.fn(name)
-        return f(*[_arg(a) for a in args], stream)
 
 
 def _arg(a):

@@ -15,7 +15,9 @@ GGML_Q4_K = 12
 
 
 def _stream():
-    return torch.cuda.current_stream().cuda_stream
+    """Raw handle of the current stream.  torch.cuda.current_stream() builds a Stream object per call: 3.2 us
+    on a B200 host against 0.2 us here, next to 2.4 us for a launch."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 @dataclass
@@ -43,6 +45,7 @@ class GpuExecutor:
     def __init__(self, pack=None, device=None):
         if not torch.cuda.is_available():
             raise RuntimeError("paddock_b200 needs a CUDA device: there is no CPU path")
+        torch.cuda.init()
         self.pack = pack or KernelPack.load()
         self.device = torch.device("cuda", torch.cuda.current_device() if device is None else device)
 
