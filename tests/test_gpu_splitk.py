@@ -1,0 +1,44 @@
+"""The K-split FP8 / NVFP4 GEMM at the edges of its plan: one token, whole and ragged token tiles (32, 64, 128, several
+of 128), one channel to a ragged last 128-row tile, one K step, and splits that do not divide K (f64 matmul of the
+decoded operands; the bounds are those of test_gpu_fp8.py and test_gpu_nvf4.py: exact products, f32 sums)."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import cond_err, dev, dev_f32, rel_l2
+from test_gpu_fp8 import fp8_case
+from test_gpu_nvf4 import check_nvf4_gemm_w4a4
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 1, 256), (1, 127, 2304), (31, 129, 1280), (32, 128, 5120), (33, 640, 256), (64, 1003, 1792), (65, 260, 768),
+          (128, 256, 4096), (129, 384, 2560), (385, 136, 1536), (7, 20000, 512)]
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES + [(3, 64, 16), (5, 72, 2064)])
+@pytest.mark.parametrize("out", ["f32", "bf16"])
+def test_fp8(pack, m, n, k, out):
+    wq, ws, xq, xs, ref, ab = fp8_case(m, n, k, 900 + m + n)
+    d_y = torch.full((m * n,), float("nan"), dtype=torch.float32 if out == "f32" else torch.bfloat16, device="cuda")
+    args = dev(wq), dev_f32(ws), dev(xq), dev_f32(xs), d_y, k, n, m
+    name = "f8row_gemm" if out == "f32" else "pdk_f8row_gemm_bf16"
+    pack.call(name, *args)
+    torch.cuda.synchronize()
+    first = d_y.clone()
+    d_y.fill_(float("nan"))
+    pack.call(name, *args)
+    torch.cuda.synchronize()
+    assert pack.device_error() == 0
+    assert torch.equal(first.view(torch.uint8), d_y.view(torch.uint8))      # the partial sums meet in rank order
+    y = d_y.float().cpu().numpy().reshape(m, n)
+    assert np.isfinite(y).all()
+    if out == "f32":
+        assert cond_err(y, ref, ab) < 1e-5 and rel_l2(y, ref) < 1e-5
+    else:
+        assert rel_l2(y, ref) < 4e-3
+
+
+@pytest.mark.parametrize("m,n,k", SHAPES)
+@pytest.mark.parametrize("out", ["f32", "bf16"])
+def test_nvfp4(pack, m, n, k, out):
+    check_nvf4_gemm_w4a4(pack, m, n, k, out)
