@@ -26,22 +26,6 @@ __device__ __forceinline__ float e2m1_to_f32(uint32_t code) {
     return (code & 8u) ? -m : m;
 }
 
-// RN-even onto {0, .5, 1, 1.5, 2, 3, 4, 6}; ties go to the even mantissa.
-__device__ __forceinline__ uint32_t e2m1_rn(float v) {
-    const uint32_t s = v < 0.0f ? 8u : 0u;
-    const float a = fabsf(v);
-    uint32_t m;
-    if (a <= 0.25f) m = 0u;
-    else if (a < 0.75f) m = 1u;
-    else if (a <= 1.25f) m = 2u;
-    else if (a < 1.75f) m = 3u;
-    else if (a <= 2.5f) m = 4u;
-    else if (a < 3.5f) m = 5u;
-    else if (a <= 5.0f) m = 6u;
-    else m = 7u;
-    return s | m;
-}
-
 // The NVFP4 rule for one 16-element block (packs/cuda/src/quant/e2m1.cuh): scale byte =
 // RN_e4m3(amax / 6), raised to the smallest subnormal when amax > 0 rounds to zero; elements =
 // e2m1_rn(v / decode(scale byte)).  A block whose amax is 0 stores scale 0 and codes 0.
@@ -61,14 +45,25 @@ __device__ __forceinline__ Nvf4BlockScale nvf4_block_scale(float amax) {
 __device__ __forceinline__ float amax4(const float4& v) {
     return fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
 }
-// four values -> four e2m1 codes, first value in the low nibble
+// four values -> four e2m1 codes, first value in the low nibble: the hardware's RN-even conversion onto
+// {0, .5, 1, 1.5, 2, 3, 4, 6}.  The products are rounded on their own, then + 0 turns a product of -0 into +0:
+// a zero has no sign in these planes.
+__device__ __forceinline__ uint32_t e2m1x2(float lo, float hi) {
+    uint32_t d;
+    asm("{\n\t.reg .b8 b;\n\tcvt.rn.satfinite.e2m1x2.f32 b, %1, %2;\n\tcvt.u32.u8 %0, b;\n\t}" : "=r"(d) : "f"(hi), "f"(lo));
+    return d;
+}
 __device__ __forceinline__ uint32_t nvf4_codes4(const float4& v, float recip) {
-    return e2m1_rn(v.x * recip) | e2m1_rn(v.y * recip) << 4 | e2m1_rn(v.z * recip) << 8 | e2m1_rn(v.w * recip) << 12;
+    const float x = __fadd_rn(__fmul_rn(v.x, recip), 0.0f), y = __fadd_rn(__fmul_rn(v.y, recip), 0.0f);
+    const float z = __fadd_rn(__fmul_rn(v.z, recip), 0.0f), w = __fadd_rn(__fmul_rn(v.w, recip), 0.0f);
+    return e2m1x2(x, y) | e2m1x2(z, w) << 8;
 }
 
 // One thread per 8 elements (half a block); the lane pair closes the 16-element amax.
 __global__ void quantize_nvf4_kernel(const float* __restrict__ x, uint8_t* __restrict__ q,
                                      uint8_t* __restrict__ scale, uint32_t n) {
+    pdk_pdl_launch_dependents();
+    pdk_pdl_wait();
     const uint32_t i = (blockIdx.x * 256u + threadIdx.x) * 8u;
     if (i >= n) return;  // n % 32 == 0: lane pairs leave together
     const float4 a = *reinterpret_cast<const float4*>(x + i);
@@ -258,9 +253,8 @@ nvf4_gemv_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict__ s
 PDK_EXPORT int pd_quantize_nvf4(const void* x, void* q, void* scale, uint32_t n, void* stream) {
     if (n == 0) return 0;
     if ((n & 31u) != 0u || !pdk_aligned(x, 16) || !pdk_aligned(q, 4)) return cudaErrorInvalidValue;
-    quantize_nvf4_kernel<<<(n / 8u + 255u) / 256u, 256, 0, (cudaStream_t)stream>>>((const float*)x, (uint8_t*)q,
-                                                                                    (uint8_t*)scale, n);
-    return pdk_launch_status();
+    return pdk_launch_pdl(quantize_nvf4_kernel, dim3((n / 8u + 255u) / 256u), dim3(256), 0, (cudaStream_t)stream, (const float*)x,
+                          (uint8_t*)q, (uint8_t*)scale, n);
 }
 
 // slot 436, packs/cuda/src/quant/nvf4.cuh:545-571: x f32 [batch][n] += proj (proj may be null),
