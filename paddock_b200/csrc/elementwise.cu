@@ -42,7 +42,49 @@ PDK_EXPORT int pd_q8_0_dequant_f32(const void* in, void* out, uint64_t n_blocks,
 }
 
 // ---------------------------------------------------------------- Q8_0 repack
-// Eight threads per block, one 4-byte word of the int8 payload each (read as
+// Planes whose pointers are 16-byte aligned go through shared memory: a CTA takes 512 blocks (17408 contiguous bytes, a
+// whole number of 16-byte vectors), loads them as vectors, four or five in flight per thread, and reads each
+// block's payload back as the two 16-byte halves the plane stores: the payload sits at 34 b + 2, on a word for odd
+// b and half a word off for even b, where neighbouring words are funnelled together.  HBM bound; 4864 x 20246: 76 us with
+// the kernel below (two 2-byte loads per stored word), 34 us now (0.93 of the HBM copy rate).
+constexpr uint32_t kQ8RepackBlocks = 512;
+__global__ void __launch_bounds__(256)
+pdk_q8_0_repack16_kernel(const uint8_t* __restrict__ src, uint4* __restrict__ dst_data, uint16_t* __restrict__ dst_scale,
+                         uint64_t n_blocks) {
+    constexpr uint32_t kVecs = kQ8RepackBlocks * 34u / 16u;
+    __shared__ __align__(16) uint32_t raw[kVecs * 4u + 4u];
+    const uint64_t b0 = (uint64_t)blockIdx.x * kQ8RepackBlocks;
+    const uint32_t n = n_blocks - b0 < kQ8RepackBlocks ? (uint32_t)(n_blocks - b0) : kQ8RepackBlocks;
+    const uint32_t bytes = n * 34u, vecs = bytes >> 4;
+    const uint4* s = reinterpret_cast<const uint4*>(src + b0 * 34u);
+    uint4 v[(kVecs + 255u) / 256u];
+#pragma unroll
+    for (uint32_t i = 0; i < (kVecs + 255u) / 256u; ++i)
+        if (i * 256u + threadIdx.x < vecs) v[i] = pdk_ldg_stream16(s + i * 256u + threadIdx.x);
+#pragma unroll
+    for (uint32_t i = 0; i < (kVecs + 255u) / 256u; ++i)
+        if (i * 256u + threadIdx.x < vecs) reinterpret_cast<uint4*>(raw)[i * 256u + threadIdx.x] = v[i];
+    // the last CTA's bytes behind its last whole vector
+    for (uint32_t i = vecs * 8u + threadIdx.x; i < bytes / 2u; i += 256u)
+        reinterpret_cast<uint16_t*>(raw)[i] = reinterpret_cast<const uint16_t*>(src + b0 * 34u)[i];
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < n * 2u; i += 256u) {
+        const uint32_t b = i >> 1, at = b * 34u + 2u + (i & 1u) * 16u;
+        const uint32_t* w = raw + (at >> 2);
+        uint4 o;
+        if (at & 2u) {
+            const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3], w4 = w[4];
+            o = make_uint4(__funnelshift_r(w0, w1, 16), __funnelshift_r(w1, w2, 16), __funnelshift_r(w2, w3, 16),
+                           __funnelshift_r(w3, w4, 16));
+        } else {
+            o = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+        dst_data[b0 * 2u + i] = o;
+    }
+    for (uint32_t b = threadIdx.x; b < n; b += 256u) dst_scale[b0 + b] = reinterpret_cast<const uint16_t*>(raw)[b * 17u];
+}
+
+// Any alignment the slot takes: eight threads per block, one 4-byte word of the int8 payload each (read as
 // two u16: the payload sits at 34*b + 2, only 2-byte aligned); a warp covers
 // four blocks = 136 contiguous source bytes and writes 128 contiguous bytes.
 __global__ void pdk_q8_0_repack_kernel(const uint8_t* __restrict__ src, uint32_t* __restrict__ dst_data,
@@ -62,6 +104,11 @@ PDK_EXPORT int pd_q8_0_repack(const void* src, void* dst_data, void* dst_scale, 
     if (!pdk_aligned(src, 2) || !pdk_aligned(dst_data, 4) || !pdk_aligned(dst_scale, 2)) return cudaErrorInvalidValue;
     const uint64_t blocks = (n_blocks * 8u + 255u) / 256u;
     if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
+    if (pdk_aligned(src, 16) && pdk_aligned(dst_data, 16)) {
+        pdk_q8_0_repack16_kernel<<<(uint32_t)((n_blocks + kQ8RepackBlocks - 1u) / kQ8RepackBlocks), 256, 0, (cudaStream_t)stream>>>(
+            (const uint8_t*)src, (uint4*)dst_data, (uint16_t*)dst_scale, n_blocks);
+        return pdk_launch_status();
+    }
     pdk_q8_0_repack_kernel<<<(uint32_t)blocks, 256, 0, (cudaStream_t)stream>>>(
         (const uint8_t*)src, (uint32_t*)dst_data, (uint16_t*)dst_scale, n_blocks);
     return pdk_launch_status();
