@@ -120,20 +120,29 @@ static EncodeTiledFn encode_fn() {
     return fn;
 }
 
-int pdk_make_tmap_2d(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t elem_bytes, const void* base,
-                     uint64_t inner, uint64_t rows, uint64_t pitch, uint32_t box_inner, uint32_t box_rows) {
+static int make_tmap_swizzled(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t elem_bytes, const void* base, uint64_t inner,
+                              uint64_t rows, uint64_t pitch, uint32_t box_inner, uint32_t box_rows, CUtensorMapSwizzle swizzle,
+                              uint32_t span) {
     EncodeTiledFn enc = encode_fn();
     if (!enc) return cudaErrorNotSupported;
-    if (((uintptr_t)base & 15u) || (pitch & 15u) || box_inner * elem_bytes > 128u || box_rows > 256u)
+    if (((uintptr_t)base & 15u) || (pitch & 15u) || box_inner * elem_bytes > span || box_rows > 256u)
         return cudaErrorInvalidValue;
     const cuuint64_t gdim[2] = {inner, rows};
     const cuuint64_t gstride[1] = {pitch};
     const cuuint32_t box[2] = {box_inner, box_rows};
     const cuuint32_t estride[2] = {1u, 1u};
     const CUresult r = enc(map, dtype, 2u, const_cast<void*>(base), gdim, gstride, box, estride,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle,
                            CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS ? 0 : cudaErrorInvalidValue;
+}
+int pdk_make_tmap_2d(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t elem_bytes, const void* base,
+                     uint64_t inner, uint64_t rows, uint64_t pitch, uint32_t box_inner, uint32_t box_rows) {
+    return make_tmap_swizzled(map, dtype, elem_bytes, base, inner, rows, pitch, box_inner, box_rows, CU_TENSOR_MAP_SWIZZLE_128B, 128u);
+}
+int pdk_make_tmap_2d_sw64(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t elem_bytes, const void* base,
+                          uint64_t inner, uint64_t rows, uint64_t pitch, uint32_t box_inner, uint32_t box_rows) {
+    return make_tmap_swizzled(map, dtype, elem_bytes, base, inner, rows, pitch, box_inner, box_rows, CU_TENSOR_MAP_SWIZZLE_64B, 64u);
 }
 
 int pdk_make_tmap_2d_dense(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t elem_bytes, const void* base,

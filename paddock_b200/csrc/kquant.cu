@@ -40,12 +40,13 @@ int pdk_iq4xs_gemv_i8(const void* data, const void* scales, const float* x, floa
                       cudaStream_t st);  // gemv_i8.cu
 int pdk_q6k_gemv_i8(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim,
                     uint32_t out_dim, cudaStream_t st);  // gemv_q6k.cu
-// q4k_batch_i8.cu: 1..16 tokens, f32 or int8 activations; -1 = shape outside its plan
+// kq_batch.cu: 1..16 tokens of every format here, f32 or int8 activations; -1 = shape outside its plan
+int pdk_kq_batch(const void* data, const void* scales, const float* x, const int8_t* xq, const float* xq_scale, float* y,
+                 uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t dtype, cudaStream_t st);
+// q4k_batch_i8.cu: 1..8 tokens, same operands and return convention
 int pdk_q4k_batch_i8(const void* data, const void* scales, const float* x, const int8_t* xq, const float* xq_scale,
                      float* y, uint32_t in_dim, uint32_t out_dim, uint32_t batch, cudaStream_t st);
 int pdk_q5k_batch_i8(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim, uint32_t out_dim,
-                     uint32_t batch, cudaStream_t st);
-int pdk_q6k_batch_i8(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim, uint32_t out_dim,
                      uint32_t batch, cudaStream_t st);
 // q4k_tc5.cu: 1..32 tokens on tcgen05 (f16 weights); same operands and return convention
 int pdk_q4k_tc5(const void* data, const void* scales, const float* x, const int8_t* xq, const float* xq_scale, float* y,
@@ -550,10 +551,40 @@ uint32_t tc5_min_tokens() {
     return v;
 }
 
-// 2 <= tokens on the tensor paths: up to 32 tokens per launch on tcgen05 from tc5_min_tokens() on,
-// up to 16 on the int8 path below that.  Activations f32 (x) or int8 with per-32 scales (xq, xs).
-// Returns the number of tokens done (all of them unless a shape is outside both plans), or
-// -(cudaError_t) - 1 on a launch error.
+// Where kq_batch.cu (clusters over K, any width) beats the kernels it shares a format with.
+//
+// Against the integer kernel of q4k_batch_i8.cu (Q4_K, Q5_K up to 8 tokens), whose time hardly falls below that of one round
+// of 64-row CTAs while this one splits K until the chip is full: kq_batch grows with tokens and plane, so the line falls
+// with both.  Measured (us, kq_batch against integer, Q4_K): K = 5120, N = 4096: 9.1 / 9.7 at 2 tokens, 10.7 / 9.8 at 4;
+// N = 2048: 8.7 / 9.6 at 4, 10.5 / 9.8 at 8; N = 1024: 7.9 / 9.5 at 8; N = 25600: 25.4 / 22.1 at 2; K = 1024, N = 9472:
+// 4.8 / 5.7 at 2, 4.9 / 5.5 at 4, 5.7 / 5.7 at 8; N = 13824: 6.3 / 5.6 at 2.
+bool kq_beats_i8(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
+    const uint64_t limit = batch <= 2u ? 30000000u : batch <= 4u ? 20000000u : 10000000u;
+    return (uint64_t)out_dim * (in_dim + 2048u) <= limit;
+}
+// Against the tcgen05 kernel of q4k_tc5.cu (Q4_0 from 4 tokens), which costs the same at 4 and at 16 tokens: K = 5120,
+// N = 25600: 26.4 / 29.2 at 4 tokens; N = 9472: 14.3 / 14.9 at 4, 16.2 / 15.2 at 8; N = 4096: 12.0 / 12.9 at 8.
+bool kq_beats_tc5(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
+    return batch <= 4u || (batch <= 8u && (uint64_t)out_dim * in_dim <= 25000000u);
+}
+
+// Up to 16 tokens of `batch` through kq_batch.cu, in passes of one width (17 tokens are 9 + 8: the weights are read once per
+// pass whatever its width), or fewer where K is so long that their activations do not fit.  The tokens done, or -(cudaError_t) - 1.
+int kq_pass(const void* data, const void* scales, const float* x, const int8_t* xq, const float* xs, float* y, uint32_t in_dim,
+            uint32_t out_dim, uint32_t batch, uint32_t dtype, cudaStream_t st) {
+    const uint32_t passes = (batch + 15u) / 16u;
+    for (uint32_t take = (batch + passes - 1u) / passes; take != 0u; take = take > 8u ? 8u : take / 2u) {
+        const int rc = pdk_kq_batch(data, scales, x, xq, xs, y, in_dim, out_dim, take, dtype, st);
+        if (rc == 0) return (int)take;
+        if (rc != -1) return -rc - 1;
+    }
+    return 0;
+}
+
+// 2 <= tokens of a Q4_K plane on the tensor paths: up to 32 tokens per launch on tcgen05 from tc5_min_tokens() on, up to 8 on
+// the integer kernel where kq_beats_i8 does not say otherwise, and whatever is outside their plans up to 16 on kq_batch.cu.
+// Activations f32 (x) or int8 with per-32 scales (xq, xs).  Returns the number of tokens done (all of them unless a
+// shape is outside every plan), or -(cudaError_t) - 1 on a launch error.
 int small_batch(const void* data, const void* scales, const float* x, const int8_t* xq, const float* xs, float* y,
                 uint32_t in_dim, uint32_t out_dim, uint32_t batch, cudaStream_t st) {
     uint32_t b = 0;
@@ -569,11 +600,44 @@ int small_batch(const void* data, const void* scales, const float* x, const int8
             take = left < 32u ? left : 32u;
             rc = pdk_q4k_tc5(data, scales, xb, qb, sb, yb, in_dim, out_dim, take, st);
         }
-        if (rc == -1) {
-            take = left < 16u ? left : 16u;
+        if (rc == -1 && left <= 8u && !kq_beats_i8(in_dim, out_dim, left)) {
+            take = left;
             rc = pdk_q4k_batch_i8(data, scales, xb, qb, sb, yb, in_dim, out_dim, take, st);
         }
-        if (rc == -1) break;
+        if (rc == -1) {
+            const int done = kq_pass(data, scales, xb, qb, sb, yb, in_dim, out_dim, left, PDK_KQ_Q4K, st);
+            if (done < 0) return done;
+            if (done == 0) break;
+            take = (uint32_t)done;
+            rc = 0;
+        }
+        if (rc != 0) return -rc - 1;
+        b += take;
+    }
+    return (int)b;
+}
+
+// The same for Q4_0 (tcgen05 where kq_beats_tc5 does not say otherwise), Q5_K (the integer kernel up to 8 tokens) and Q6_K.
+int small_batch_more(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim, uint32_t out_dim,
+                     uint32_t batch, uint32_t dtype, cudaStream_t st) {
+    uint32_t b = 0;
+    while (b < batch) {
+        const uint32_t left = batch - b;
+        const float* xb = x + (size_t)b * in_dim;
+        float* yb = y + (size_t)b * out_dim;
+        uint32_t take = left < 32u ? left : 32u;
+        int rc = -1;
+        if (dtype == PDK_KQ_Q4_0 && tc5_min_tokens() != 0u && !kq_beats_tc5(in_dim, out_dim, left))
+            rc = pdk_q4_0_tc5(data, scales, xb, yb, in_dim, out_dim, take, st);
+        if (dtype == PDK_KQ_Q5K && left <= 8u && !kq_beats_i8(in_dim, out_dim, left))
+            rc = pdk_q5k_batch_i8(data, scales, xb, yb, in_dim, out_dim, left, st);
+        if (rc == -1) {
+            const int done = kq_pass(data, scales, xb, nullptr, nullptr, yb, in_dim, out_dim, left, dtype, st);
+            if (done < 0) return done;
+            if (done == 0) break;
+            take = (uint32_t)done;
+            rc = 0;
+        }
         if (rc != 0) return -rc - 1;
         b += take;
     }
@@ -686,48 +750,17 @@ PDK_EXPORT int pdk_kquant_gemm_f32(const void* data, const void* scales, const v
     if (out_dim == 0 || batch == 0) return 0;
     if (batch > 64u) return cudaErrorInvalidValue;
     if (int rc = check_gemv(data, scales, x, y, in_dim, dtype)) return rc;
-    if (dtype == PDK_KQ_Q4_0 && batch >= 4u && !force_plain() && tc5_min_tokens() != 0u) {
-        // Q4_0 shares Q4_K's nibble planes: from four tokens on the tcgen05 kernel (32 us per 32 tokens at K=5120,
-        // N=25600) beats one 17 us decode GEMV per token
-        uint32_t b = 0;
-        int rc = 0;
-        while (b < batch && rc == 0) {
-            const uint32_t take = batch - b < 32u ? batch - b : 32u;
-            rc = pdk_q4_0_tc5(data, scales, (const float*)x + (size_t)b * in_dim, (float*)y + (size_t)b * out_dim, in_dim,
-                              out_dim, take, (cudaStream_t)stream);
-            if (rc == 0) b += take;
-        }
-        if (rc > 0) return rc;
-        if (b == batch) return 0;
-        // -1: the shape is outside the kernel's plan, or this stream has no scratch slice (both hold for
-        // the whole call, so b is 0 here unless slices were released meanwhile): the routes below
-        // take what is left
-        x = (const float*)x + (size_t)b * in_dim;
-        y = (float*)y + (size_t)b * out_dim;
-        batch -= b;
-    }
-    if ((dtype == PDK_KQ_Q5K || dtype == PDK_KQ_Q6K) && batch >= 2u && !force_plain() && pdk_aligned(data, 16)) {
-        // Q5_K: Q4_K's integer batch kernel with the fifth bit ORed into the codes; Q6_K: its sibling with one
-        // product per 16-weight block.  16 tokens per weight pass
-        uint32_t b = 0;
-        int rc = 0;
-        while (b < batch && rc == 0) {
-            const uint32_t take = batch - b < 16u ? batch - b : 16u;
-            rc = (dtype == PDK_KQ_Q5K ? pdk_q5k_batch_i8 : pdk_q6k_batch_i8)(
-                data, scales, (const float*)x + (size_t)b * in_dim, (float*)y + (size_t)b * out_dim, in_dim, out_dim, take,
-                (cudaStream_t)stream);
-            if (rc == 0) b += take;
-        }
-        if (rc > 0) return rc;
-        if (b == batch) return 0;
-        x = (const float*)x + (size_t)b * in_dim;   // -1: outside the kernel's plan, the routes below take what is left
-        y = (float*)y + (size_t)b * out_dim;
-        batch -= b;
+    if ((dtype == PDK_KQ_Q4_0 || dtype == PDK_KQ_Q5K || dtype == PDK_KQ_Q6K) && batch >= 2u && !force_plain()) {
+        const int done = small_batch_more(data, scales, (const float*)x, (float*)y, in_dim, out_dim, batch, dtype, (cudaStream_t)stream);
+        if (done < 0) return -done - 1;
+        if ((uint32_t)done == batch) return 0;
+        x = (const float*)x + (size_t)done * in_dim;   // outside every plan: the routes below take what is left
+        y = (float*)y + (size_t)done * out_dim;
+        batch -= (uint32_t)done;
     }
     if (dtype != PDK_KQ_Q4K && !force_plain() && pdk_aligned(data, 16)) {
-        // Q4_0 below four tokens (and Q5_K / Q6_K outside the batch kernels' plan) have no batch kernel on the tensor path yet: one decode GEMV per token
-        // (17-25 us each at K=5120 N=25600, the later ones partly from L2) beats the plain f32
-        // kernel's 165 us per four tokens
+        // one token, and IQ4_XS, which has no batch kernel: one decode GEMV per token (17-29 us each at K=5120
+        // N=25600, the later ones partly from L2) beats the plain f32 kernel's 165 us per four tokens
         int rc = 0;
         for (uint32_t b = 0; b < batch && rc == 0; ++b)
             rc = more_gemv_i8(data, scales, (const float*)x + (size_t)b * in_dim, (float*)y + (size_t)b * out_dim, in_dim,

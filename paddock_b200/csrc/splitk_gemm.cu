@@ -27,8 +27,7 @@
 //   warps 2..5  nvfp4: warp 2 + c brings token rows 32 c .. 32 c + 31's activation scales into cell order,
 //               16 bytes per row and stage through registers (4-byte cp.async from the producer took four
 //               times the L1 requests and bound the kernel from 64 tokens on); then the epilogue
-#include <array>
-
+#include "cluster_caps.cuh"
 #include "nvf4_tc5.cuh"
 
 namespace {
@@ -37,7 +36,7 @@ enum Kind : int { kFp8 = 0, kNvf4 = 1 };
 
 constexpr uint32_t BM = 128, BKB = 128;
 constexpr uint32_t kABytes = BM * BKB, kSfBytes = 2048;
-constexpr uint32_t kMaxSplit = 8;      // portable cluster size
+constexpr uint32_t kMaxSplit = kPdkMaxCluster;
 constexpr uint32_t kThreads = 192;
 constexpr uint32_t kMaxStages = 5;
 constexpr uint32_t kSmemHalf = 115712;  // what lets two CTAs share an SM: 228 KB / 2 - 1 KB reserved
@@ -312,37 +311,17 @@ int launch_bn(const void* data, const void* xq, Args& a, uint32_t row_bytes, cud
     if (int rc = pdk_make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, data, row_bytes, a.out_dim, row_bytes, BKB, BM)) return rc;
     if (int rc = pdk_make_tmap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, row_bytes, a.batch, row_bytes, BKB, BN)) return rc;
     auto kern = splitk_gemm_kernel<KIND, BN, TO>;
-    static const cudaError_t attr_rc =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)C::kSmemBytes);
-    if (attr_rc != cudaSuccess) return (int)attr_rc;
     // How many clusters of s CTAs are resident at once (they stay within a GPC).  The driver counts one CTA per SM for
     // a kernel that allocates tensor memory; two run, so twice its answer (148, 74, 45, 33, 26, 22, 15, 15 on a B200).
-    static const std::array<uint32_t, kMaxSplit + 1> resident = [&] {
-        std::array<uint32_t, kMaxSplit + 1> r{};
-        for (uint32_t s = 1; s <= kMaxSplit; ++s) {
-            cudaLaunchConfig_t cfg = {};
-            cudaLaunchAttribute attr = {};
-            attr.id = cudaLaunchAttributeClusterDimension;
-            attr.val.clusterDim.x = s;
-            attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
-            cfg.gridDim = dim3(s);
-            cfg.blockDim = dim3(kThreads);
-            cfg.dynamicSmemBytes = C::kSmemBytes;
-            cfg.attrs = &attr;
-            cfg.numAttrs = 1;
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0) r[s] = 2u * (uint32_t)n;
-        }
-        (void)cudaGetLastError();
-        if (r[1] == 0u) r[1] = 2u * (uint32_t)pdk_sm_count();
-        return r;
-    }();
+    static PdkClusterCaps table;
+    const uint32_t* resident = nullptr;
+    if (int rc = pdk_cluster_caps(table, (const void*)kern, kThreads, C::kSmemBytes, &resident)) return rc;
     // The largest split whose clusters are all resident at once; more only add start-ups.  K = 5120, N = 5120, 7 tokens
     // (40 tiles): 11.4 us at S = 1, 7.6 at 4, 7.4 at 6, and 11.9 at 7, where a part of the clusters waits for a
     // second turn.  At least two stages per CTA, so that it streams more than it sets up.
     const uint32_t tiles_t = (a.batch + BN - 1u) / BN, tiles_w = (a.out_dim + BM - 1u) / BM;
     uint32_t split = a.num_kb / 2u < kMaxSplit ? a.num_kb / 2u : kMaxSplit;
-    while (split > 1u && (uint64_t)tiles_t * tiles_w > resident[split]) --split;
+    while (split > 1u && (uint64_t)tiles_t * tiles_w > 2u * resident[split]) --split;
     if (split == 0u) split = 1u;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(split, tiles_t, tiles_w);

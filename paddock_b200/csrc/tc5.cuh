@@ -355,6 +355,9 @@ __device__ __forceinline__ void mbar_arrive_leader(uint64_t* bar) {
 // Returns 0 or a cudaError_t.
 int pdk_make_tmap_2d(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t elem_bytes, const void* base,
                      uint64_t inner, uint64_t rows, uint64_t pitch, uint32_t box_inner, uint32_t box_rows);
+// The same with 64-byte swizzle (box rows up to 64 bytes).
+int pdk_make_tmap_2d_sw64(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t elem_bytes, const void* base,
+                          uint64_t inner, uint64_t rows, uint64_t pitch, uint32_t box_inner, uint32_t box_rows);
 // The same without swizzle (dense boxes, for stores): box_inner up to 256 elements.
 int pdk_make_tmap_2d_dense(CUtensorMap* map, CUtensorMapDataType dtype, uint32_t elem_bytes, const void* base,
                            uint64_t inner, uint64_t rows, uint64_t pitch, uint32_t box_inner, uint32_t box_rows);
