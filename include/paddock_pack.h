@@ -438,6 +438,11 @@ int pdk_moe_route_prep_f4(const void* logits, const void* router_bias, const voi
                           void* sorted_row, void* sorted_slot, void* block_expert, void* xq, void* xs, void* xstep,
                           uint32_t n_expert, uint32_t k, uint32_t rows, uint32_t dim, uint32_t bm, uint32_t max_blocks,
                           void* stream);
+/* The same for NVFP4 planes (natural element order, as pdk_moe_prep_act_f4n). */
+int pdk_moe_route_prep_f4n(const void* logits, const void* router_bias, const void* x, void* idx, void* w,
+                           void* sorted_row, void* sorted_slot, void* block_expert, void* xq, void* xs, void* xstep,
+                           uint32_t n_expert, uint32_t k, uint32_t rows, uint32_t dim, uint32_t bm, uint32_t max_blocks,
+                           void* stream);
 /* pdk_moe_prep_act_f4 with the natural element order of NVFP4 planes.  mode 0 gather; mode 1 gated
  * unit (min(g, limit) * sigmoid(alpha * that)) * (clamp(u, +-limit) + up_add); mode 2 relu(x)^2. */
 int pdk_moe_prep_act_f4n(const void* x, const void* up, const void* sorted_row, const void* block_expert, void* xq,

@@ -695,10 +695,9 @@ PDK_EXPORT int pdk_moe_prep_act_f4(const void* x, const void* up, const void* so
 // No counterpart in the reference.  moe_topk_batch + moe_align_bm + pdk_moe_prep_act_f4 (mode 0) in one
 // launch for decode widths: rows * k <= 32 pairs, rows <= 8, n_expert <= 512, max_blocks <= 32.  Writes
 // the same idx / w / sorted_row / sorted_slot / block_expert the three calls would, and the term rows.
-PDK_EXPORT int pdk_moe_route_prep_f4(const void* logits, const void* router_bias, const void* x, void* idx, void* w,
-                                     void* sorted_row, void* sorted_slot, void* block_expert, void* xq, void* xs, void* xstep,
-                                     uint32_t n_expert, uint32_t k, uint32_t rows, uint32_t dim, uint32_t bm,
-                                     uint32_t max_blocks, void* stream) {
+static int route_prep_impl(const void* logits, const void* router_bias, const void* x, void* idx, void* w, void* sorted_row,
+                           void* sorted_slot, void* block_expert, void* xq, void* xs, void* xstep, uint32_t n_expert, uint32_t k,
+                           uint32_t rows, uint32_t dim, uint32_t bm, uint32_t max_blocks, uint32_t natural, void* stream) {
     if (rows == 0 || max_blocks == 0) return 0;
     if (rows > 8u || k == 0 || k > 16u || rows * k > 32u || n_expert == 0 || n_expert > 512u || k > n_expert ||
         max_blocks > 32u || (bm != 8u && bm != 32u) || max_blocks * bm > kRouteMaxPos || dim == 0 || (dim & 31u) != 0u)
@@ -707,13 +706,30 @@ PDK_EXPORT int pdk_moe_route_prep_f4(const void* logits, const void* router_bias
     PrepArgs a{};
     a.x = (const float*)x;
     a.xq = (uint8_t*)xq; a.xs = (uint8_t*)xs; a.xstep = (float*)xstep;
-    a.dim = dim; a.bm = bm; a.mode = 0u; a.natural = 0u; a.alpha = 1.0f; a.limit = 0.0f; a.up_add = 0.0f;
+    a.dim = dim; a.bm = bm; a.mode = 0u; a.natural = natural; a.alpha = 1.0f; a.limit = 0.0f; a.up_add = 0.0f;
     RouteArgs r{};
     r.logits = (const float*)logits; r.bias = (const float*)router_bias;
     r.idx = (uint32_t*)idx; r.w = (float*)w;
     r.sorted_row = (uint32_t*)sorted_row; r.sorted_slot = (uint32_t*)sorted_slot; r.block_expert = (uint32_t*)block_expert;
     r.rows = rows; r.k = k; r.n_expert = n_expert; r.max_blocks = max_blocks;
     return pdk_launch_pdl(moe_route_prep_f4_kernel, dim3(max_blocks * bm), dim3(256), 0, (cudaStream_t)stream, a, r);
+}
+
+PDK_EXPORT int pdk_moe_route_prep_f4(const void* logits, const void* router_bias, const void* x, void* idx, void* w,
+                                     void* sorted_row, void* sorted_slot, void* block_expert, void* xq, void* xs, void* xstep,
+                                     uint32_t n_expert, uint32_t k, uint32_t rows, uint32_t dim, uint32_t bm,
+                                     uint32_t max_blocks, void* stream) {
+    return route_prep_impl(logits, router_bias, x, idx, w, sorted_row, sorted_slot, block_expert, xq, xs, xstep, n_expert, k, rows,
+                           dim, bm, max_blocks, 0u, stream);
+}
+
+// The same for NVFP4 expert planes (natural element order).
+PDK_EXPORT int pdk_moe_route_prep_f4n(const void* logits, const void* router_bias, const void* x, void* idx, void* w,
+                                      void* sorted_row, void* sorted_slot, void* block_expert, void* xq, void* xs, void* xstep,
+                                      uint32_t n_expert, uint32_t k, uint32_t rows, uint32_t dim, uint32_t bm,
+                                      uint32_t max_blocks, void* stream) {
+    return route_prep_impl(logits, router_bias, x, idx, w, sorted_row, sorted_slot, block_expert, xq, xs, xstep, n_expert, k, rows,
+                           dim, bm, max_blocks, 1u, stream);
 }
 
 // The same for NVFP4 expert planes: term rows packed in the natural element order (byte j = elements

@@ -267,11 +267,16 @@ def moe_nvf4_forward(ex, gate, up, down, ws, x, router_logits, out, gated=True, 
     c = ex.pack.call
     T, k, bm = ws.tokens, ws.n_active, ws.bm
     n_expert, embd, ff = up.n_expert, up.in_dim, up.rows
-    c("moe_topk_batch", router_logits, router_bias, n_expert, k, ws.idx, ws.w, T, stream=st)
     max_blocks = min(ws.max_blocks, min(T * k, T * k // bm + n_expert))
-    c("moe_align_bm", ws.idx, ws.sorted_row, ws.sorted_slot, ws.block_expert, T, k, n_expert, bm, max_blocks, stream=st)
-    c("pdk_moe_prep_act_f4n", x, None, ws.sorted_row, ws.block_expert, ws.x4q, ws.x4s, ws.x4step, embd, bm, max_blocks, 0,
-      alpha, limit, up_add, stream=st)
+    fused = T <= 8 and T * k <= 32 and n_expert <= 512 and max_blocks <= 32
+    if fused:      # decode widths: routing, alignment and the first activation preparation in one launch
+        c("pdk_moe_route_prep_f4n", router_logits, router_bias, x, ws.idx, ws.w, ws.sorted_row, ws.sorted_slot, ws.block_expert,
+          ws.x4q, ws.x4s, ws.x4step, n_expert, k, T, embd, bm, max_blocks, stream=st)
+    else:
+        c("moe_topk_batch", router_logits, router_bias, n_expert, k, ws.idx, ws.w, T, stream=st)
+        c("moe_align_bm", ws.idx, ws.sorted_row, ws.sorted_slot, ws.block_expert, T, k, n_expert, bm, max_blocks, stream=st)
+        c("pdk_moe_prep_act_f4n", x, None, ws.sorted_row, ws.block_expert, ws.x4q, ws.x4s, ws.x4step, embd, bm, max_blocks, 0,
+          alpha, limit, up_add, stream=st)
     if gated:
         c("pdk_nvf4_moe_gemm_tc5", gate.data, gate.tiled, gate.scale2, None, ws.g_raw, up.data, up.tiled, up.scale2, None,
           ws.u_raw, ws.x4q, ws.x4s, ws.x4step, ws.block_expert, ws.sorted_row, None, None, embd, ff, n_expert, bm,
@@ -288,4 +293,4 @@ def moe_nvf4_forward(ex, gate, up, down, ws, x, router_logits, out, gated=True, 
       ws.h4s, ws.h4step, ws.block_expert, ws.sorted_row, ws.sorted_slot, ws.w, ff, embd, n_expert, bm, max_blocks, k, 1,
       stream=st)
     c("moe_slot_combine", ws.part, out, embd, k, T, stream=st)
-    return 7
+    return 5 if fused else 7

@@ -139,9 +139,10 @@ def test_moe_block_tensor_core_path_matches_oracle(pack, tokens, n_expert, k, em
     (5, 8, 2, 512, 8),
     (2, 512, 8, 256, 32),
 ])
-def test_route_and_prepare_in_one_launch_equals_the_three_calls(pack, tokens, n_expert, k, embd, bm):
-    """pdk_moe_route_prep_f4 leaves the tables and the term rows of moe_topk_batch + moe_align_bm +
-    pdk_moe_prep_act_f4, byte for byte (routing weights bit for bit)."""
+@pytest.mark.parametrize("natural", [False, True])
+def test_route_and_prepare_in_one_launch_equals_the_three_calls(pack, tokens, n_expert, k, embd, bm, natural):
+    """pdk_moe_route_prep_f4 (..._f4n) leaves the tables and the term rows of moe_topk_batch + moe_align_bm +
+    pdk_moe_prep_act_f4 (..._f4n), byte for byte (routing weights bit for bit)."""
     ex = P.GpuExecutor(pack)
     c = ex.pack.call
     pairs = tokens * k
@@ -163,8 +164,11 @@ def test_route_and_prepare_in_one_launch_equals_the_three_calls(pack, tokens, n_
         a, b = buffers(), buffers()
         c("moe_topk_batch", logits, bias, n_expert, k, a["idx"], a["w"], tokens)
         c("moe_align_bm", a["idx"], a["row"], a["slot"], a["blk"], tokens, k, n_expert, bm, max_blocks)
-        c("pdk_moe_prep_act_f4", x, None, a["row"], a["blk"], a["q"], a["s"], a["step"], embd, bm, max_blocks, 0, 1.702, 7.0)
-        c("pdk_moe_route_prep_f4", logits, bias, x, b["idx"], b["w"], b["row"], b["slot"], b["blk"], b["q"], b["s"],
+        if natural:
+            c("pdk_moe_prep_act_f4n", x, None, a["row"], a["blk"], a["q"], a["s"], a["step"], embd, bm, max_blocks, 0, 1.702, 7.0, 1.0)
+        else:
+            c("pdk_moe_prep_act_f4", x, None, a["row"], a["blk"], a["q"], a["s"], a["step"], embd, bm, max_blocks, 0, 1.702, 7.0)
+        c("pdk_moe_route_prep_f4n" if natural else "pdk_moe_route_prep_f4", logits, bias, x, b["idx"], b["w"], b["row"], b["slot"], b["blk"], b["q"], b["s"],
           b["step"], n_expert, k, tokens, embd, bm, max_blocks)
         torch.cuda.synchronize()
         assert pack.device_error() == 0
