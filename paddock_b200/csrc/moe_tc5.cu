@@ -621,6 +621,201 @@ moe_tc5_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_co
     }
 }
 
+// Blocks of 32 tokens (prompts and large batches): the term rows of a block are 128 B rows, as many bytes per K step as the
+// weights, and one 128-row tile at a time fetched them again for every tile - 415 KB through L2 per 128 x 2880 tile, 3.8 GB a
+// call at 1024 tokens of 128 experts, which is what bound the kernel (14 TB/s from L2; HBM carried a third of that).
+// Here a tile is two weight tiles under one B: gate and up of the same rows, or two neighbouring row tiles of a
+// single plane.  The accumulators are 2 x 128 columns, so there is one pair of them and not two: the ring
+// (four stages of one slab) keeps filling while the epilogue empties it.
+constexpr uint32_t kDualBN = 128u, kDualStages = 4u;
+constexpr uint32_t kDualB = 2u * kABytes, kDualSfa = kDualB + kDualBN * BKB, kDualSfb = kDualSfa + 2u * kSfBytes;
+constexpr uint32_t kDualStage = kDualSfb + kSfBytes;
+constexpr uint32_t kDualSfCol0 = 2u * kDualBN, kDualSfCols = 48u;      // per stage: the cells of A0, A1 and B
+static_assert(kDualSfCol0 + kDualStages * kDualSfCols <= kTmemCols && kDualStages <= kMaxStages, "tensor memory, barriers");
+
+__global__ void __launch_bounds__(kThreads, 1)
+moe_tc5_dual_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
+                    const __grid_constant__ CUtensorMap tmap_x, const GemmArgs a) {
+    constexpr uint32_t BT = kDualBN / 4u, kIdesc = Cfg<kDualBN>::kIdesc;
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
+    Shared* sh = reinterpret_cast<Shared*>(tiles + kDualStages * kDualStage);
+    uint32_t* s_expert = reinterpret_cast<uint32_t*>(sh + 1);
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const bool two_planes = a.n_planes == 2u;
+    const uint32_t row_tiles = (a.out_dim + BM - 1u) / BM, per_block = two_planes ? row_tiles : (row_tiles + 1u) / 2u;
+    const uint32_t n_tiles = a.max_blocks * per_block;
+    const uint32_t n_mma = a.in_dim >> 6, num_kb = (n_mma + 3u) >> 2;
+
+    if (threadIdx.x == 0) {
+        for (uint32_t s = 0; s < kDualStages; ++s) {
+            tc5::mbar_init(&sh->full[s], 1);
+            tc5::mbar_init(&sh->empty[s], 1);
+        }
+        tc5::mbar_init(&sh->tmem_full[0], 1);
+        tc5::mbar_init(&sh->tmem_empty[0], 4);
+        sh->abort_flag = 0;
+        tc5::mbar_fence_init();
+        tc5::tma_prefetch_desc(&tmap_w0);
+        tc5::tma_prefetch_desc(&tmap_w1);
+        tc5::tma_prefetch_desc(&tmap_x);
+    }
+    if (warp == 1) {
+        tc5::tmem_alloc(&sh->tmem_base, kTmemCols);
+        tc5::tmem_relinquish();
+    }
+    pdk_pdl_launch_dependents();
+    pdk_pdl_wait();
+    for (uint32_t i = threadIdx.x; i < a.max_blocks; i += kThreads) s_expert[i] = a.block_expert[i];
+    tc5::fence_before_sync();
+    __syncthreads();
+    tc5::fence_after_sync();
+    const uint32_t tmem_base = sh->tmem_base;
+    const tc5::WaitCtx ctx{&sh->abort_flag, a.err_word};
+
+    // weight tile i (0, 1) of a tile: its row tile, and whether it is there (an odd last one of a single plane is alone)
+    struct Tile { uint32_t blk, expert, rt[2]; bool second; };
+    auto locate = [&](uint32_t tile) {
+        Tile t;
+        t.blk = tile / per_block;
+        const uint32_t rem = tile % per_block;
+        t.expert = s_expert[t.blk];
+        t.rt[0] = two_planes ? rem : 2u * rem;
+        t.rt[1] = two_planes ? rem : 2u * rem + 1u;
+        t.second = t.rt[1] < row_tiles;
+        return t;
+    };
+
+    if (warp == 0) {
+        // ------------------------------------------------------------ producer (whole warp, one lane issues)
+        uint32_t stage = 0, phase = 0;
+        bool ok = true;
+        for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+            const Tile t = locate(tile);
+            if (t.expert == PDK_MOE_PAD) continue;
+            const uint8_t* sf0 = a.w_sf[0] + ((size_t)t.expert * row_tiles + t.rt[0]) * num_kb * kSfBytes;
+            const uint8_t* sf1 = a.w_sf[two_planes ? 1 : 0] + ((size_t)t.expert * row_tiles + t.rt[1]) * num_kb * kSfBytes;
+            const uint8_t* xsf = a.x_sf + (size_t)t.blk * num_kb * kSfBytes;
+            for (uint32_t kb = 0; kb < num_kb; ++kb) {
+                ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, stage));
+                if (!ok) break;
+                uint8_t* st = tiles + stage * kDualStage;
+                uint64_t* full = &sh->full[stage];
+                tc5::mbar_arrive_expect_tx_elect(full, (t.second ? 2u : 1u) * (kABytes + kSfBytes) + kDualBN * BKB + kSfBytes);
+                const int32_t x = (int32_t)(kb * BKB), row = (int32_t)(t.expert * a.out_dim);
+                tc5::tma_load_2d_elect(st, &tmap_w0, full, x, row + (int32_t)(t.rt[0] * BM));
+                if (t.second) tc5::tma_load_2d_elect(st + kABytes, two_planes ? &tmap_w1 : &tmap_w0, full, x, row + (int32_t)(t.rt[1] * BM));
+                tc5::tma_load_2d_elect(st + kDualB, &tmap_x, full, x, (int32_t)(t.blk * kDualBN));
+                tc5::bulk_load_elect(st + kDualSfa, sf0 + (size_t)kb * kSfBytes, kSfBytes, full);
+                if (t.second) tc5::bulk_load_elect(st + kDualSfa + kSfBytes, sf1 + (size_t)kb * kSfBytes, kSfBytes, full);
+                tc5::bulk_load_elect(st + kDualSfb, xsf + (size_t)kb * kSfBytes, kSfBytes, full);
+                if (++stage == kDualStages) { stage = 0; phase ^= 1u; }
+            }
+        }
+        if (!ok && lane == 0)
+            for (int i = 0; i < 64; ++i) __nanosleep(1000);
+    } else if (warp == 1) {
+        // ------------------------------------------------------------ MMA issuer (whole warp, one lane issues)
+        uint32_t stage = 0, phase = 0, iter = 0;
+        bool ok = true;
+        for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+            const Tile t = locate(tile);
+            if (t.expert == PDK_MOE_PAD) continue;
+            ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->tmem_empty[0], (iter & 1u) ^ 1u, ctx, tc5::kErrTmemEmptyWait, 0u));
+            if (!ok) break;
+            ++iter;
+            tc5::fence_after_sync();
+            for (uint32_t kb = 0; kb < num_kb; ++kb) {
+                ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->full[stage], phase, ctx, tc5::kErrFullWait, stage));
+                if (!ok) break;
+                tc5::fence_after_sync();
+                const uint32_t s_addr = tc5::smem_u32(tiles + stage * kDualStage), steps = min(4u, n_mma - kb * 4u);
+                const uint32_t sf_t = tmem_base + kDualSfCol0 + stage * kDualSfCols, sfb_t = sf_t + 32u;
+                const uint64_t b_desc = tc5::smem_desc_sw128(s_addr + kDualB);
+                slab_nvf4<1u>(tmem_base, tc5::smem_desc_sw128(s_addr), b_desc, kIdesc, kb != 0u, sf_t, sfb_t, s_addr + kDualSfa,
+                              s_addr + kDualSfb, steps);
+                if (t.second)
+                    slab_nvf4<2u>(tmem_base + kDualBN, tc5::smem_desc_sw128(s_addr + kABytes), b_desc, kIdesc, kb != 0u, sf_t + 16u,
+                                  sfb_t, s_addr + kDualSfa + kSfBytes, s_addr + kDualSfb, steps);
+                tc5::mma_commit_elect(&sh->empty[stage]);
+                if (++stage == kDualStages) { stage = 0; phase ^= 1u; }
+            }
+            if (ok) tc5::mma_commit_elect(&sh->tmem_full[0]);
+        }
+    } else {
+        // ------------------------------------------------------------ epilogue
+        const uint32_t quarter = warp & 3u;
+        uint32_t iter = 0;
+        bool ok = true;
+        for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
+            const Tile t = locate(tile);
+            if (t.expert == PDK_MOE_PAD) continue;
+            ok = tc5::mbar_wait(&sh->tmem_full[0], iter & 1u, ctx, tc5::kErrTmemFullWait, 0u);
+            if (!ok) break;
+            ++iter;
+            __syncwarp();
+            tc5::fence_after_sync();
+            // lane = weight row; columns = term * BT + token
+            float v[2][BT];
+#pragma unroll
+            for (uint32_t s = 0; s < 2u; ++s) {
+                if (s == 1u && !t.second) break;
+                float c = 1.0f;
+#pragma unroll
+                for (uint32_t term = 0; term < 4u; ++term) {
+                    uint32_t r[32];
+                    tc5::tmem_ld_32x32(tmem_base + ((quarter * 32u) << 16) + s * kDualBN + term * 32u, r);
+                    tc5::tmem_ld_wait();
+#pragma unroll
+                    for (uint32_t i = 0; i < BT; ++i) v[s][i] = term == 0u ? __uint_as_float(r[i]) : fmaf(__uint_as_float(r[i]), c, v[s][i]);
+                    c *= 0.0625f;
+                }
+            }
+            tc5::fence_before_sync();
+            __syncwarp();
+            if (lane == 0) tc5::mbar_arrive(&sh->tmem_empty[0]);  // the accumulators are in registers now
+
+            // lane i fetches token i's routing data once; the loop below broadcasts it
+            const uint32_t my_pos = t.blk * BT + lane;
+            const uint32_t my_src = a.sorted_row[my_pos];
+            uint32_t my_row = my_pos;  // output row: block position, or the (token, slot) pair
+            float my_wgt = 1.0f;       // routing weight when scattering
+            if (a.scatter && my_src != PDK_MOE_PAD) {
+                my_row = my_src * a.n_active + a.sorted_slot[my_pos];
+                my_wgt = a.topk_w[my_row];
+            }
+            const float my_step = a.xstep[my_pos] * my_wgt;
+#pragma unroll
+            for (uint32_t s = 0; s < 2u; ++s) {
+                if (s == 1u && !t.second) break;
+                const uint32_t plane = two_planes ? s : 0u;
+                const float scale2 = a.scale2[plane][a.scale2_per_expert ? t.expert : 0u];
+                const uint32_t n = t.rt[s] * BM + quarter * 32u + lane;
+                float bias = 0.0f;
+                if (n < a.out_dim && a.bias[plane]) bias = a.bias[plane][(size_t)t.expert * a.out_dim + n];
+                float* out = a.out[plane];
+#pragma unroll
+                for (uint32_t i = 0; i < BT; ++i) {
+                    const uint32_t src = __shfl_sync(0xffffffffu, my_src, i);
+                    const uint32_t row = __shfl_sync(0xffffffffu, my_row, i);
+                    const float mul = __shfl_sync(0xffffffffu, my_step, i) * scale2;
+                    const float wgt = __shfl_sync(0xffffffffu, my_wgt, i);
+                    if (src == PDK_MOE_PAD || n >= a.out_dim) continue;
+                    // (acc * scale2 * step + bias) * routing weight
+                    out[(size_t)row * a.out_dim + n] = fmaf(v[s][i], mul, bias * wgt);
+                }
+            }
+        }
+    }
+
+    tc5::fence_before_sync();
+    __syncthreads();
+    if (warp == 1) {
+        tc5::fence_after_sync();
+        tc5::tmem_dealloc(tmem_base, kTmemCols);
+    }
+}
+
 constexpr uint32_t kMaxBlocks = 1024;  // block_expert[] is kept in shared memory
 
 template <uint32_t BN, bool WG = false>
@@ -635,6 +830,16 @@ int launch_gemm(const CUtensorMap& tw0, const CUtensorMap& tw1, const CUtensorMa
     uint32_t grid = (uint32_t)pdk_sm_count();
     if (grid > n_tiles) grid = n_tiles;
     return pdk_launch_pdl(kern, dim3(grid), dim3(kThreads), smem, st, tw0, tw1, tx, a);
+}
+
+int launch_dual(const CUtensorMap& tw0, const CUtensorMap& tw1, const CUtensorMap& tx, const GemmArgs& a, cudaStream_t st) {
+    const size_t smem = (size_t)kDualStages * kDualStage + sizeof(Shared) + kMaxBlocks * 4u + 1024u;
+    const cudaError_t e = cudaFuncSetAttribute(moe_tc5_dual_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return (int)e;
+    const uint32_t row_tiles = (a.out_dim + BM - 1u) / BM, per_block = a.n_planes == 2u ? row_tiles : (row_tiles + 1u) / 2u;
+    uint32_t grid = (uint32_t)pdk_sm_count();
+    if (grid > a.max_blocks * per_block) grid = a.max_blocks * per_block;
+    return pdk_launch_pdl(moe_tc5_dual_kernel, dim3(grid), dim3(kThreads), smem, st, tw0, tw1, tx, a);
 }
 
 }  // namespace
@@ -786,7 +991,7 @@ static int gemm_impl(const void* w0_data, const void* w0_sf, const float* w0_sca
     a.in_dim = in_dim; a.out_dim = out_dim; a.max_blocks = max_blocks; a.n_planes = w1_data ? 2u : 1u;
     a.n_active = n_active; a.scatter = scatter; a.err_word = pdk_error_word();
     auto st = (cudaStream_t)stream;
-    return bm == 8u ? launch_gemm<32>(tw0, tw1, tx, a, st) : launch_gemm<128>(tw0, tw1, tx, a, st);
+    return bm == 8u ? launch_gemm<32>(tw0, tw1, tx, a, st) : launch_dual(tw0, tw1, tx, a, st);
 }
 
 PDK_EXPORT int pdk_mxfp4_moe_gemm_tc5(const void* w0_data, const void* w0_sf, const void* w0_meta, const void* w0_bias,

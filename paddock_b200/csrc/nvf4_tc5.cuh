@@ -68,28 +68,30 @@ __device__ __forceinline__ void mma_nvf4(uint32_t d_tmem, uint64_t a_desc, uint6
 // (sfa_smem / sfb_smem: the slab's 2048-byte records) into tensor memory (sfa_t / sfb_t, four
 // columns per step).  One election, descriptors and addresses stepped inside the asm block:
 // issued this way the pair (two copies + MMA) takes the tensor core 92 cycles, the MMA alone 64;
-// one wrapper call per copy and per MMA took the issuing warp 200.
-template <bool kCopies>
+// one wrapper call per copy and per MMA took the issuing warp 200.  kCopies: 0 none, 1 both cells, 2 the A cell only
+// (another A tile under the same B: its cells are in tensor memory already).
+template <uint32_t kCopies>
 __device__ __forceinline__ void slab_nvf4(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                           uint32_t acc_first, uint32_t sfa_t, uint32_t sfb_t, uint32_t sfa_smem,
                                           uint32_t sfb_smem, uint32_t steps) {
     const uint64_t cell_a = (uint64_t)((sfa_smem >> 4) & 0x3FFFu) | ((uint64_t)1u << 16) | ((uint64_t)8u << 32);
     const uint64_t cell_b = (uint64_t)((sfb_smem >> 4) & 0x3FFFu) | ((uint64_t)1u << 16) | ((uint64_t)8u << 32);
 #define PDK_NV4_STEP(J, PRED)                                                                                        \
-    "setp.gt.and.u32 ej, %10, " #J ", e;\n\tsetp.gt.and.u32 cj, %10, " #J ", c;\n\t"                                  \
+    "setp.gt.and.u32 ej, %10, " #J ", e;\n\tsetp.gt.and.u32 cj, %10, " #J ", c;\n\tsetp.gt.and.u32 dj, %10, " #J ", d;\n\t" \
     "add.u64 a, %1, " #J "*2;\n\tadd.u64 b, %2, " #J "*2;\n\tadd.u32 sa, %5, " #J "*4;\n\tadd.u32 sb, %6, " #J "*4;\n\t" \
     "add.u64 ca, %7, " #J "*32;\n\tadd.u64 cb, %8, " #J "*32;\n\t"                                                    \
-    "@cj tcgen05.cp.cta_group::1.32x128b.warpx4 [sa], ca;\n\t@cj tcgen05.cp.cta_group::1.32x128b.warpx4 [sb], cb;\n\t" \
+    "@cj tcgen05.cp.cta_group::1.32x128b.warpx4 [sa], ca;\n\t@dj tcgen05.cp.cta_group::1.32x128b.warpx4 [sb], cb;\n\t" \
     "@ej tcgen05.mma.cta_group::1.kind::mxf4nvf4.block_scale.block16 [%0], a, b, %3, [sa], [sb], " PRED ";\n\t"
     asm volatile(
-        "{\n\t.reg .pred e, p, q, c, ej, cj;\n\t.reg .b64 a, b, ca, cb;\n\t.reg .b32 sa, sb;\n\t"
+        "{\n\t.reg .pred e, p, q, c, d, ej, cj, dj;\n\t.reg .b64 a, b, ca, cb;\n\t.reg .b32 sa, sb;\n\t"
         "elect.sync _|e, 0xffffffff;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
         "setp.eq.b32 q, 0, 0;\n\t"
         "setp.ne.and.b32 c, %9, 0, e;\n\t"
+        "setp.eq.and.b32 d, %9, 1, e;\n\t"
         PDK_NV4_STEP(0, "p") PDK_NV4_STEP(1, "q") PDK_NV4_STEP(2, "q") PDK_NV4_STEP(3, "q") "}" ::"r"(d_tmem),
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(acc_first), "r"(sfa_t), "r"(sfb_t), "l"(cell_a), "l"(cell_b),
-        "r"(kCopies ? 1u : 0u), "r"(steps)
+        "r"(kCopies), "r"(steps)
         : "memory");
 #undef PDK_NV4_STEP
 }
