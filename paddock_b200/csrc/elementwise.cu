@@ -46,7 +46,8 @@ PDK_EXPORT int pd_q8_0_dequant_f32(const void* in, void* out, uint64_t n_blocks,
 // whole number of 16-byte vectors), loads them as vectors, four or five in flight per thread, and reads each
 // block's payload back as the two 16-byte halves the plane stores: the payload sits at 34 b + 2, on a word for odd
 // b and half a word off for even b, where neighbouring words are funnelled together.  HBM bound; 4864 x 20246: 76 us with
-// the kernel below (two 2-byte loads per stored word), 34 us now (0.93 of the HBM copy rate).
+// the kernel below (two 2-byte loads per stored word), 34 us now (0.93 of the HBM copy rate).  Plain loads: with
+// ld.global.nc.L1::no_allocate the decode GEMV reads the plane slower ever after (see q4k_repack16_kernel).
 constexpr uint32_t kQ8RepackBlocks = 512;
 __global__ void __launch_bounds__(256)
 pdk_q8_0_repack16_kernel(const uint8_t* __restrict__ src, uint4* __restrict__ dst_data, uint16_t* __restrict__ dst_scale,
@@ -60,7 +61,7 @@ pdk_q8_0_repack16_kernel(const uint8_t* __restrict__ src, uint4* __restrict__ ds
     uint4 v[(kVecs + 255u) / 256u];
 #pragma unroll
     for (uint32_t i = 0; i < (kVecs + 255u) / 256u; ++i)
-        if (i * 256u + threadIdx.x < vecs) v[i] = pdk_ldg_stream16(s + i * 256u + threadIdx.x);
+        if (i * 256u + threadIdx.x < vecs) v[i] = s[i * 256u + threadIdx.x];
 #pragma unroll
     for (uint32_t i = 0; i < (kVecs + 255u) / 256u; ++i)
         if (i * 256u + threadIdx.x < vecs) reinterpret_cast<uint4*>(raw)[i * 256u + threadIdx.x] = v[i];

@@ -88,39 +88,42 @@ __global__ void q4k_dequant_kernel(const uint8_t* __restrict__ src, float* __res
     }
 }
 
-// Repack of 16-byte aligned planes.  A raw super-block is nine 16-byte vectors - header, then the
-// nibble payload as the plane stores it - so thread t of a 288-thread CTA (32 super-blocks x 9) always meets
-// the same vector of a super-block: the payload goes through as it is, the header threads unpack the
-// record.  Every load is a whole 16-byte vector of a contiguous run, kRepackDepth of them in flight per
-// thread.  HBM bound; 5120 x 25600: 60.5 us with the word-per-lane kernel below (a warp per super-block, one 4-byte
-// load in flight per thread), 22.8 us now (151.6 MB: the HBM copy rate).
-constexpr uint32_t kRepackDepth = 4, kRepackThreads = 288;
+// Repack of 16-byte aligned planes.  A raw super-block is nine 16-byte vectors - header, then the nibble payload as the plane
+// stores it.  The payload goes through as it is, eight lanes per super-block, so that a warp's store is four whole
+// 128-byte lines; one thread per super-block unpacks the header into the record.  Every load of a thread is in flight before
+// its first store.  HBM bound; 5120 x 25600: 60.5 us with the word-per-lane kernel below (a warp per super-block, one 4-byte load in
+// flight per thread), 24.8 us now (151.6 MB, 0.94 of the HBM copy rate; 26.6 with nine
+// consecutive lanes per super-block, whose stores begin and end inside lines).  Plain loads: with ld.global.nc.L1::no_allocate here the
+// repack takes as long, but the decode GEMV reads a plane of the same bytes slower ever after (18.10 against 17.92 us; Q8_0, the same
+// in elementwise.cu, 16.67 against 15.95), until something rewrites it - measured, the mechanism is not known.
+constexpr uint32_t kRepackDepth = 4, kRepackThreads = 256, kRepackSupers = kRepackThreads * kRepackDepth / 8u;
 __global__ void __launch_bounds__(kRepackThreads)
 q4k_repack16_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst_data, uint2* __restrict__ dst_scales, uint64_t n_super) {
-    const uint32_t j = threadIdx.x % 9u, s0 = threadIdx.x / 9u;
-    const uint64_t base = (uint64_t)blockIdx.x * (32u * kRepackDepth) + s0;
-    uint4 v[kRepackDepth];
-#pragma unroll
-    for (uint32_t i = 0; i < kRepackDepth; ++i)
-        if (base + i * 32u < n_super) v[i] = pdk_ldg_stream16(src + (base + i * 32u) * 9u + j);
+    const uint64_t s0 = (uint64_t)blockIdx.x * kRepackSupers;
+    uint4 v[kRepackDepth], head;
 #pragma unroll
     for (uint32_t i = 0; i < kRepackDepth; ++i) {
-        const uint64_t b = base + i * 32u;
-        if (b >= n_super) return;
-        if (j != 0u) {
-            dst_data[b * 8u + (j - 1u)] = v[i];
-            continue;
-        }
-        // scale bytes 0..3 | 4..7 | 8..11 = v.y | v.z | v.w: pairs 0..3 are the low six bits of the first two words,
-        // pairs 4..7 the nibbles of the third under the top two bits of those words
-        const uint32_t sc_lo = v[i].y & 0x3f3f3f3fu, m_lo = v[i].z & 0x3f3f3f3fu;
-        const uint32_t sc_hi = (v[i].w & 0x0f0f0f0fu) | ((v[i].y >> 2) & 0x30303030u);
-        const uint32_t m_hi = ((v[i].w >> 4) & 0x0f0f0f0fu) | ((v[i].z >> 2) & 0x30303030u);
-        uint2* rec = dst_scales + b * 3u;
-        rec[0] = make_uint2(v[i].x, sc_lo);
-        rec[1] = make_uint2(sc_hi, m_lo);
-        rec[2] = make_uint2(m_hi, 0u);
+        const uint32_t at = i * kRepackThreads + threadIdx.x;
+        if (s0 + (at >> 3) < n_super) v[i] = src[(s0 + (at >> 3)) * 9u + 1u + (at & 7u)];
     }
+    const uint64_t b = s0 + threadIdx.x;
+    const bool mine = threadIdx.x < kRepackSupers && b < n_super;
+    if (mine) head = pdk_ldg_stream16(src + b * 9u);
+#pragma unroll
+    for (uint32_t i = 0; i < kRepackDepth; ++i) {
+        const uint32_t at = i * kRepackThreads + threadIdx.x;
+        if (s0 + (at >> 3) < n_super) dst_data[s0 * 8u + at] = v[i];
+    }
+    if (!mine) return;
+    // scale bytes 0..3 | 4..7 | 8..11 = y | z | w: pairs 0..3 are the low six bits of the first two words,
+    // pairs 4..7 the nibbles of the third under the top two bits of those words
+    const uint32_t sc_lo = head.y & 0x3f3f3f3fu, m_lo = head.z & 0x3f3f3f3fu;
+    const uint32_t sc_hi = (head.w & 0x0f0f0f0fu) | ((head.y >> 2) & 0x30303030u);
+    const uint32_t m_hi = ((head.w >> 4) & 0x0f0f0f0fu) | ((head.z >> 2) & 0x30303030u);
+    uint2* rec = dst_scales + b * 3u;
+    rec[0] = make_uint2(head.x, sc_lo);
+    rec[1] = make_uint2(sc_hi, m_lo);
+    rec[2] = make_uint2(m_hi, 0u);
 }
 
 // Any alignment the slot takes: one warp per super-block, lane l moves one 4-byte word of the nibble payload
@@ -722,7 +725,7 @@ PDK_EXPORT int pd_kquant_repack(const void* src, void* dst_data, void* dst_scale
     const uint64_t blocks = (n_super + 7u) / 8u;
     if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
     if (pdk_aligned(src, 16) && pdk_aligned(dst_data, 16) && pdk_aligned(dst_scales, 8)) {
-        const uint64_t ctas = (n_super + 32u * kRepackDepth - 1u) / (32u * kRepackDepth);
+        const uint64_t ctas = (n_super + kRepackSupers - 1u) / kRepackSupers;
         q4k_repack16_kernel<<<(uint32_t)ctas, kRepackThreads, 0, (cudaStream_t)stream>>>((const uint4*)src, (uint4*)dst_data,
                                                                                       (uint2*)dst_scales, n_super);
         return pdk_launch_status();

@@ -622,11 +622,13 @@ moe_tc5_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_co
 }
 
 // Blocks of 32 tokens (prompts and large batches): the term rows of a block are 128 B rows, as many bytes per K step as the
-// weights, and one 128-row tile at a time fetched them again for every tile - 415 KB through L2 per 128 x 2880 tile, 3.8 GB a
-// call at 1024 tokens of 128 experts, which is what bound the kernel (14 TB/s from L2; HBM carried a third of that).
+// weights.  One 128-row tile at a time brought 36 KB per 256-element slab into shared memory for 32 KB that its four MMAs read
+// and 4 KB of scale cells: 72 KB or 562 cycles of the shared-memory port for 256 of the tensor core, and 415 KB through L2
+// per 128 x 2880 tile.
 // Here a tile is two weight tiles under one B: gate and up of the same rows, or two neighbouring row tiles of a
 // single plane.  The accumulators are 2 x 128 columns, so there is one pair of them and not two: the ring
-// (four stages of one slab) keeps filling while the epilogue empties it.
+// (four stages of one slab) keeps filling while the epilogue empties it.  Two tiles take 54 + 64 + 6 KB: 484 port cycles
+// each, and three quarters of the L2 bytes.  128 experts of 2880 x 2880, 4 active, 1024 tokens: the block's call 525 -> 502 us.
 constexpr uint32_t kDualBN = 128u, kDualStages = 4u;
 constexpr uint32_t kDualB = 2u * kABytes, kDualSfa = kDualB + kDualBN * BKB, kDualSfb = kDualSfa + 2u * kSfBytes;
 constexpr uint32_t kDualStage = kDualSfb + kSfBytes;
