@@ -435,13 +435,13 @@ def test_q4k_gemv_shard_stores_band_into_every_output(pack):
 
 
 def test_small_batch_scratch_is_per_stream(pack):
-    """The small-batch Q4_K GEMM keeps its activation image in library scratch, one slice per
-    (device, stream), two streams per device.  Three streams: the first two get slices, the third
-    takes the scratch-free route (same results within its own precision class); releasing a
-    stream hands its slice to the next newcomer."""
-    k, n, batch = 2048, 300, 4
+    """The integer batch kernel keeps its activation image in library scratch, one slice per (device,
+    stream), two streams per device.  Three streams: the first two get slices, the third takes
+    kq_batch.cu, which needs none (its 22-bit activations show: other bits, same results within their
+    precision); releasing a stream hands its slice to the next newcomer."""
+    k, n, batch = 1024, 14000, 4                    # wide enough that kquant.cu prefers the integer kernel
     w = oracle.fill_normal(n * k, seed_for(2, 900), 0.02)
-    x = bf16_activations(batch * k, seed_for(2, 901))
+    x = oracle.fill_normal(batch * k, seed_for(2, 901), 1.0)      # not bf16 values: the two kernels round them differently
     raw, d_data, d_sc = q4k_planes(pack, w, n, k)
     ref, ab = oracle.matmul_f64(oracle.dequant_q4_k(raw), x, k, n, batch, with_abs=True)
     d_x = dev_f32(x)
@@ -449,24 +449,28 @@ def test_small_batch_scratch_is_per_stream(pack):
     rel = pack._lib.pdk_stream_release
     rel.argtypes, rel.restype = [ctypes.c_void_p], None
     streams = [torch.cuda.Stream() for _ in range(3)]
-    outs = []
     torch.cuda.synchronize()
     rel(torch.cuda.current_stream().cuda_stream)    # earlier tests ran this route on the default stream
-    for st in streams:
-        y = torch.zeros(batch * n, dtype=torch.float32, device="cuda")
-        pack.call("pdk_kquant_gemm_f32", d_data, d_sc, d_x, y, k, n, batch, 12, stream=st.cuda_stream)
-        outs.append(y)
+
+    def run(st):
+        # the fill belongs to the stream of the launch: on the default stream nothing would order it before the GEMM
+        with torch.cuda.stream(st):
+            y = torch.full((batch * n,), float("nan"), dtype=torch.float32, device="cuda")
+            pack.call("pdk_kquant_gemm_f32", d_data, d_sc, d_x, y, k, n, batch, 12, stream=st.cuda_stream)
+        return y
+
+    outs = [run(st) for st in streams]
     torch.cuda.synchronize()
     assert pack.device_error() == 0
     for y in outs:
         got = y.cpu().numpy().reshape(batch, n)
         assert cond_err(got, ref, ab) < 1e-4 and rel_l2(got, ref) < 1e-3 < TOL
-    assert torch.equal(outs[0], outs[1])            # both on the integer tensor path
+    assert torch.equal(outs[0], outs[1])            # both on the integer kernel
+    assert not torch.equal(outs[0], outs[2])        # the third is not
     rel(streams[0].cuda_stream)
-    y3 = torch.zeros(batch * n, dtype=torch.float32, device="cuda")
-    pack.call("pdk_kquant_gemm_f32", d_data, d_sc, d_x, y3, k, n, batch, 12, stream=streams[2].cuda_stream)
+    y3 = run(streams[2])
     torch.cuda.synchronize()
-    assert torch.equal(y3, outs[0])                 # the third stream now runs the scratch route too
+    assert torch.equal(y3, outs[0])                 # the third stream now runs the integer kernel too
     for st in streams[1:]:
         rel(st.cuda_stream)
 
