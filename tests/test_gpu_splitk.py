@@ -42,3 +42,33 @@ def test_fp8(pack, m, n, k, out):
 @pytest.mark.parametrize("out", ["f32", "bf16"])
 def test_nvfp4(pack, m, n, k, out):
     check_nvf4_gemm_w4a4(pack, m, n, k, out)
+
+
+def test_nvfp4_first_call_behind_its_load(pack):
+    """Scale tiler, quantizer and GEMM on fresh buffers with nothing between them: the GEMM requests weights and scale
+    records ahead of its wait, and the quantizer in front of it must have held it back until the tiler's records are
+    complete.  Against the same calls with a synchronisation behind each; same bytes."""
+    k, n, m = 2048, 640, 5
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x = torch.randn(m * k, device="cuda", generator=g)
+
+    def run(w, s, sync):
+        tiled = torch.full((((n + 127) // 128) * (k // 256) * 2048,), 0x7F, dtype=torch.uint8, device="cuda")
+        xq = torch.zeros(m * k // 2, dtype=torch.uint8, device="cuda")
+        xs = torch.zeros(m * k // 16, dtype=torch.uint8, device="cuda")
+        y = torch.full((m * n,), float("nan"), dtype=torch.float32, device="cuda")
+        torch.cuda.synchronize()
+        for call in (("nvf4_tc5_tile_scales", s, tiled, k, n), ("quantize_nvf4", x, xq, xs, m * k),
+                     ("nvf4_gemm_tc5w", w, tiled, None, xq, xs, y, 1.0, k, n, m, None, 0)):
+            pack.call(*call)
+            if sync:
+                torch.cuda.synchronize()
+        torch.cuda.synchronize()
+        return y
+
+    for _ in range(20):
+        w = torch.randint(0, 256, (n * k // 2,), dtype=torch.uint8, device="cuda", generator=g)
+        s = torch.randint(0x28, 0x40, (n * k // 16,), dtype=torch.uint8, device="cuda", generator=g)
+        want, got = run(w, s, True), run(w, s, False)
+        assert torch.isfinite(want).all() and torch.equal(want, got)
+    assert pack.device_error() == 0
