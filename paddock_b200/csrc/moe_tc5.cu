@@ -621,14 +621,14 @@ moe_tc5_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_co
     }
 }
 
-// Blocks of 32 tokens (prompts and large batches): the term rows of a block are 128 B rows, as many bytes per K step as the
-// weights.  One 128-row tile at a time brought 36 KB per 256-element slab into shared memory for 32 KB that its four MMAs read
-// and 4 KB of scale cells: 72 KB or 562 cycles of the shared-memory port for 256 of the tensor core, and 415 KB through L2
-// per 128 x 2880 tile.
-// Here a tile is two weight tiles under one B: gate and up of the same rows, or two neighbouring row tiles of a
-// single plane.  The accumulators are 2 x 128 columns, so there is one pair of them and not two: the ring
-// (four stages of one slab) keeps filling while the epilogue empties it.  Two tiles take 54 + 64 + 6 KB: 484 port cycles
-// each, and three quarters of the L2 bytes.  128 experts of 2880 x 2880, 4 active, 1024 tokens: the block's call 525 -> 502 us.
+// Gate and up of blocks of 32 tokens where K is long: the term rows of a block are 128 B rows, as many bytes per K step as
+// the weights.  One 128-row tile at a time brings 36 KB per 256-element slab into shared memory for 32 KB that its four MMAs
+// read and 4 KB of scale cells: 72 KB or 562 cycles of the shared-memory port for 256 of the tensor core, and 415 KB
+// through L2 per 128 x 2880 tile.
+// Here a tile is the gate and the up tile of the same rows under one B.  The accumulators are 2 x 128 columns, so there is
+// one pair of them and not two: the ring (four stages of one slab) keeps filling while the epilogue empties it, but the
+// tensor core waits for the epilogue.  Two tiles take 54 + 64 + 6 KB: 484 port cycles each, and three quarters of the L2 bytes.
+// prefer_dual below has where that pays.
 constexpr uint32_t kDualBN = 128u, kDualStages = 4u;
 constexpr uint32_t kDualB = 2u * kABytes, kDualSfa = kDualB + kDualBN * BKB, kDualSfb = kDualSfa + 2u * kSfBytes;
 constexpr uint32_t kDualStage = kDualSfb + kSfBytes;
@@ -644,9 +644,7 @@ moe_tc5_dual_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_co
     Shared* sh = reinterpret_cast<Shared*>(tiles + kDualStages * kDualStage);
     uint32_t* s_expert = reinterpret_cast<uint32_t*>(sh + 1);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const bool two_planes = a.n_planes == 2u;
-    const uint32_t row_tiles = (a.out_dim + BM - 1u) / BM, per_block = two_planes ? row_tiles : (row_tiles + 1u) / 2u;
-    const uint32_t n_tiles = a.max_blocks * per_block;
+    const uint32_t row_tiles = (a.out_dim + BM - 1u) / BM, n_tiles = a.max_blocks * row_tiles;
     const uint32_t n_mma = a.in_dim >> 6, num_kb = (n_mma + 3u) >> 2;
 
     if (threadIdx.x == 0) {
@@ -675,42 +673,30 @@ moe_tc5_dual_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_co
     const uint32_t tmem_base = sh->tmem_base;
     const tc5::WaitCtx ctx{&sh->abort_flag, a.err_word};
 
-    // weight tile i (0, 1) of a tile: its row tile, and whether it is there (an odd last one of a single plane is alone)
-    struct Tile { uint32_t blk, expert, rt[2]; bool second; };
-    auto locate = [&](uint32_t tile) {
-        Tile t;
-        t.blk = tile / per_block;
-        const uint32_t rem = tile % per_block;
-        t.expert = s_expert[t.blk];
-        t.rt[0] = two_planes ? rem : 2u * rem;
-        t.rt[1] = two_planes ? rem : 2u * rem + 1u;
-        t.second = t.rt[1] < row_tiles;
-        return t;
-    };
-
     if (warp == 0) {
         // ------------------------------------------------------------ producer (whole warp, one lane issues)
         uint32_t stage = 0, phase = 0;
         bool ok = true;
         for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            const Tile t = locate(tile);
-            if (t.expert == PDK_MOE_PAD) continue;
-            const uint8_t* sf0 = a.w_sf[0] + ((size_t)t.expert * row_tiles + t.rt[0]) * num_kb * kSfBytes;
-            const uint8_t* sf1 = a.w_sf[two_planes ? 1 : 0] + ((size_t)t.expert * row_tiles + t.rt[1]) * num_kb * kSfBytes;
-            const uint8_t* xsf = a.x_sf + (size_t)t.blk * num_kb * kSfBytes;
+            const uint32_t blk = tile / row_tiles, rt = tile % row_tiles, expert = s_expert[blk];
+            if (expert == PDK_MOE_PAD) continue;
+            const size_t sf = ((size_t)expert * row_tiles + rt) * num_kb * kSfBytes;
+            const uint8_t* xsf = a.x_sf + (size_t)blk * num_kb * kSfBytes;
+            const int32_t row = (int32_t)(expert * a.out_dim + rt * BM);
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
                 ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, stage));
                 if (!ok) break;
                 uint8_t* st = tiles + stage * kDualStage;
                 uint64_t* full = &sh->full[stage];
-                tc5::mbar_arrive_expect_tx_elect(full, (t.second ? 2u : 1u) * (kABytes + kSfBytes) + kDualBN * BKB + kSfBytes);
-                const int32_t x = (int32_t)(kb * BKB), row = (int32_t)(t.expert * a.out_dim);
-                tc5::tma_load_2d_elect(st, &tmap_w0, full, x, row + (int32_t)(t.rt[0] * BM));
-                if (t.second) tc5::tma_load_2d_elect(st + kABytes, two_planes ? &tmap_w1 : &tmap_w0, full, x, row + (int32_t)(t.rt[1] * BM));
-                tc5::tma_load_2d_elect(st + kDualB, &tmap_x, full, x, (int32_t)(t.blk * kDualBN));
-                tc5::bulk_load_elect(st + kDualSfa, sf0 + (size_t)kb * kSfBytes, kSfBytes, full);
-                if (t.second) tc5::bulk_load_elect(st + kDualSfa + kSfBytes, sf1 + (size_t)kb * kSfBytes, kSfBytes, full);
-                tc5::bulk_load_elect(st + kDualSfb, xsf + (size_t)kb * kSfBytes, kSfBytes, full);
+                const size_t kb_sf = (size_t)kb * kSfBytes;
+                const int32_t x = (int32_t)(kb * BKB);
+                tc5::mbar_arrive_expect_tx_elect(full, kDualStage);
+                tc5::tma_load_2d_elect(st, &tmap_w0, full, x, row);
+                tc5::tma_load_2d_elect(st + kABytes, &tmap_w1, full, x, row);
+                tc5::tma_load_2d_elect(st + kDualB, &tmap_x, full, x, (int32_t)(blk * kDualBN));
+                tc5::bulk_load_elect(st + kDualSfa, a.w_sf[0] + sf + kb_sf, kSfBytes, full);
+                tc5::bulk_load_elect(st + kDualSfa + kSfBytes, a.w_sf[1] + sf + kb_sf, kSfBytes, full);
+                tc5::bulk_load_elect(st + kDualSfb, xsf + kb_sf, kSfBytes, full);
                 if (++stage == kDualStages) { stage = 0; phase ^= 1u; }
             }
         }
@@ -721,8 +707,7 @@ moe_tc5_dual_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_co
         uint32_t stage = 0, phase = 0, iter = 0;
         bool ok = true;
         for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            const Tile t = locate(tile);
-            if (t.expert == PDK_MOE_PAD) continue;
+            if (s_expert[tile / row_tiles] == PDK_MOE_PAD) continue;
             ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->tmem_empty[0], (iter & 1u) ^ 1u, ctx, tc5::kErrTmemEmptyWait, 0u));
             if (!ok) break;
             ++iter;
@@ -736,9 +721,8 @@ moe_tc5_dual_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_co
                 const uint64_t b_desc = tc5::smem_desc_sw128(s_addr + kDualB);
                 slab_nvf4<1u>(tmem_base, tc5::smem_desc_sw128(s_addr), b_desc, kIdesc, kb != 0u, sf_t, sfb_t, s_addr + kDualSfa,
                               s_addr + kDualSfb, steps);
-                if (t.second)
-                    slab_nvf4<2u>(tmem_base + kDualBN, tc5::smem_desc_sw128(s_addr + kABytes), b_desc, kIdesc, kb != 0u, sf_t + 16u,
-                                  sfb_t, s_addr + kDualSfa + kSfBytes, s_addr + kDualSfb, steps);
+                slab_nvf4<2u>(tmem_base + kDualBN, tc5::smem_desc_sw128(s_addr + kABytes), b_desc, kIdesc, kb != 0u, sf_t + 16u,
+                              sfb_t, s_addr + kDualSfa + kSfBytes, s_addr + kDualSfb, steps);
                 tc5::mma_commit_elect(&sh->empty[stage]);
                 if (++stage == kDualStages) { stage = 0; phase ^= 1u; }
             }
@@ -750,8 +734,8 @@ moe_tc5_dual_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_co
         uint32_t iter = 0;
         bool ok = true;
         for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            const Tile t = locate(tile);
-            if (t.expert == PDK_MOE_PAD) continue;
+            const uint32_t blk = tile / row_tiles, rt = tile % row_tiles, expert = s_expert[blk];
+            if (expert == PDK_MOE_PAD) continue;
             ok = tc5::mbar_wait(&sh->tmem_full[0], iter & 1u, ctx, tc5::kErrTmemFullWait, 0u);
             if (!ok) break;
             ++iter;
@@ -761,7 +745,6 @@ moe_tc5_dual_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_co
             float v[2][BT];
 #pragma unroll
             for (uint32_t s = 0; s < 2u; ++s) {
-                if (s == 1u && !t.second) break;
                 float c = 1.0f;
 #pragma unroll
                 for (uint32_t term = 0; term < 4u; ++term) {
@@ -777,34 +760,23 @@ moe_tc5_dual_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_co
             __syncwarp();
             if (lane == 0) tc5::mbar_arrive(&sh->tmem_empty[0]);  // the accumulators are in registers now
 
-            // lane i fetches token i's routing data once; the loop below broadcasts it
-            const uint32_t my_pos = t.blk * BT + lane;
+            // lane i fetches token i's step once; the loop below broadcasts it
+            const uint32_t my_pos = blk * BT + lane;
             const uint32_t my_src = a.sorted_row[my_pos];
-            uint32_t my_row = my_pos;  // output row: block position, or the (token, slot) pair
-            float my_wgt = 1.0f;       // routing weight when scattering
-            if (a.scatter && my_src != PDK_MOE_PAD) {
-                my_row = my_src * a.n_active + a.sorted_slot[my_pos];
-                my_wgt = a.topk_w[my_row];
-            }
-            const float my_step = a.xstep[my_pos] * my_wgt;
+            const float my_step = a.xstep[my_pos];
+            const uint32_t n = rt * BM + quarter * 32u + lane;
 #pragma unroll
             for (uint32_t s = 0; s < 2u; ++s) {
-                if (s == 1u && !t.second) break;
-                const uint32_t plane = two_planes ? s : 0u;
-                const float scale2 = a.scale2[plane][a.scale2_per_expert ? t.expert : 0u];
-                const uint32_t n = t.rt[s] * BM + quarter * 32u + lane;
+                const float scale2 = a.scale2[s][a.scale2_per_expert ? expert : 0u];
                 float bias = 0.0f;
-                if (n < a.out_dim && a.bias[plane]) bias = a.bias[plane][(size_t)t.expert * a.out_dim + n];
-                float* out = a.out[plane];
+                if (n < a.out_dim && a.bias[s]) bias = a.bias[s][(size_t)expert * a.out_dim + n];
+                float* out = a.out[s];
 #pragma unroll
                 for (uint32_t i = 0; i < BT; ++i) {
                     const uint32_t src = __shfl_sync(0xffffffffu, my_src, i);
-                    const uint32_t row = __shfl_sync(0xffffffffu, my_row, i);
                     const float mul = __shfl_sync(0xffffffffu, my_step, i) * scale2;
-                    const float wgt = __shfl_sync(0xffffffffu, my_wgt, i);
                     if (src == PDK_MOE_PAD || n >= a.out_dim) continue;
-                    // (acc * scale2 * step + bias) * routing weight
-                    out[(size_t)row * a.out_dim + n] = fmaf(v[s][i], mul, bias * wgt);
+                    out[(size_t)(blk * BT + i) * a.out_dim + n] = fmaf(v[s][i], mul, bias);
                 }
             }
         }
@@ -834,13 +806,24 @@ int launch_gemm(const CUtensorMap& tw0, const CUtensorMap& tw1, const CUtensorMa
     return pdk_launch_pdl(kern, dim3(grid), dim3(kThreads), smem, st, tw0, tw1, tx, a);
 }
 
+// Whether the two-tile kernel takes a gate | up call of 32-token blocks.  It saves port cycles and L2 bytes per slab and
+// pays an epilogue per tile that nothing overlaps, so it needs long K, and tiles enough that its half as many fill the last round.
+// Measured on a B200 (us, one tile at a time against two; 128 experts and 4 active unless stated): K = 2880, N = 2880: 272 / 251
+// at 1024 tokens, 200 / 199 at 256; K = 2048: 1.02 at 256 tokens (3680 tiles), 0.96 at 1024; K = 1024: 104 / 137 at 1024; K = 2880,
+// N = 768: 0.92 at 64 experts, 8 active, 2048 tokens (3456 tiles) but slower at 512 (1152 tiles).  A single plane (down), two
+// row tiles under one B, gained nothing at any of these sizes (147 / 141 at best, 16.4 / 24.4 at K = 1088, N = 1536).
+bool prefer_dual(const GemmArgs& a) {
+    const uint32_t num_kb = (a.in_dim + 255u) / 256u, row_tiles = (a.out_dim + BM - 1u) / BM;
+    return a.n_planes == 2u && num_kb >= 8u && (uint64_t)a.max_blocks * row_tiles >= 16ull * (uint32_t)pdk_sm_count();
+}
+
 int launch_dual(const CUtensorMap& tw0, const CUtensorMap& tw1, const CUtensorMap& tx, const GemmArgs& a, cudaStream_t st) {
     const size_t smem = (size_t)kDualStages * kDualStage + sizeof(Shared) + kMaxBlocks * 4u + 1024u;
     const cudaError_t e = cudaFuncSetAttribute(moe_tc5_dual_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
-    const uint32_t row_tiles = (a.out_dim + BM - 1u) / BM, per_block = a.n_planes == 2u ? row_tiles : (row_tiles + 1u) / 2u;
     uint32_t grid = (uint32_t)pdk_sm_count();
-    if (grid > a.max_blocks * per_block) grid = a.max_blocks * per_block;
+    const uint32_t n_tiles = a.max_blocks * ((a.out_dim + BM - 1u) / BM);
+    if (grid > n_tiles) grid = n_tiles;
     return pdk_launch_pdl(moe_tc5_dual_kernel, dim3(grid), dim3(kThreads), smem, st, tw0, tw1, tx, a);
 }
 
@@ -993,7 +976,8 @@ static int gemm_impl(const void* w0_data, const void* w0_sf, const float* w0_sca
     a.in_dim = in_dim; a.out_dim = out_dim; a.max_blocks = max_blocks; a.n_planes = w1_data ? 2u : 1u;
     a.n_active = n_active; a.scatter = scatter; a.err_word = pdk_error_word();
     auto st = (cudaStream_t)stream;
-    return bm == 8u ? launch_gemm<32>(tw0, tw1, tx, a, st) : launch_dual(tw0, tw1, tx, a, st);
+    if (bm == 8u) return launch_gemm<32>(tw0, tw1, tx, a, st);
+    return prefer_dual(a) ? launch_dual(tw0, tw1, tx, a, st) : launch_gemm<128>(tw0, tw1, tx, a, st);
 }
 
 PDK_EXPORT int pdk_mxfp4_moe_gemm_tc5(const void* w0_data, const void* w0_sf, const void* w0_meta, const void* w0_bias,

@@ -266,6 +266,35 @@ def test_nvf4_moe_block_matches_f64(pack, tokens, n_expert, k, embd, ff, bm, gat
     assert rel_l2(y, ref) < 2e-3 < TOL
 
 
+@pytest.mark.parametrize("in_dim,dual", [(1792, False), (2048, True), (2624, True)])
+def test_gate_and_up_in_one_tile_equal_one_plane_calls(pack, in_dim, dual):
+    """32-token blocks, both sides of prefer_dual's line (8 slabs of K; a whole and a ragged last slab, a ragged last row tile):
+    gate and up in one call give the bits of one call per plane, which always takes one tile at a time."""
+    n_expert, tokens, k, bm, out_dim = 8, 1024, 4, 32, 2400
+    gen = torch.Generator(device="cuda").manual_seed(in_dim)
+    rand = lambda lo, hi, n: torch.randint(lo, hi, (n,), dtype=torch.uint8, device="cuda", generator=gen)
+    max_blocks = tokens * k // bm + n_expert
+    slabs, row_tiles = (in_dim + 255) // 256, (out_dim + 127) // 128
+    assert (slabs >= 8 and max_blocks * row_tiles >= 16 * torch.cuda.get_device_properties(0).multi_processor_count) == dual
+    i32 = lambda n: torch.zeros(n, dtype=torch.int32, device="cuda")
+    idx, wgt, row, slot, blk = i32(tokens * k), torch.zeros(tokens * k, device="cuda"), i32(max_blocks * bm), i32(max_blocks * bm), i32(max_blocks)
+    pack.call("moe_topk_batch", torch.randn(tokens * n_expert, device="cuda", generator=gen), None, n_expert, k, idx, wgt, tokens)
+    pack.call("moe_align_bm", idx, row, slot, blk, tokens, k, n_expert, bm, max_blocks)
+    planes = [(rand(0, 256, n_expert * out_dim * in_dim // 2), rand(0x20, 0x40, n_expert * row_tiles * slabs * 2048),
+               torch.rand(n_expert, device="cuda", generator=gen) + 0.5) for _ in range(2)]
+    xq, xs = rand(0, 256, max_blocks * bm * 4 * in_dim // 2), rand(0x20, 0x40, max_blocks * slabs * 2048)
+    step = torch.rand(max_blocks * bm, device="cuda", generator=gen) + 0.5
+    outs = [torch.zeros(max_blocks * bm, out_dim, device="cuda") for _ in range(4)]
+    tail = (xq, xs, step, blk, row, None, None, in_dim, out_dim, n_expert, bm, max_blocks, k, 0)
+    pack.call("pdk_nvf4_moe_gemm_tc5", *planes[0], None, outs[0], *planes[1], None, outs[1], *tail)
+    for p in range(2):
+        pack.call("pdk_nvf4_moe_gemm_tc5", *planes[p], None, outs[2 + p], None, None, None, None, None, *tail)
+    torch.cuda.synchronize()
+    assert pack.device_error() == 0
+    for p in range(2):
+        assert torch.isfinite(outs[p]).all() and bool(outs[p].any()) and torch.equal(outs[p], outs[2 + p])
+
+
 # ---- the reference's own MoE slots (155 / 88 / 89 and the decode pair 92 / 93): int8 activations
 
 def _q8_roundtrip(v):
