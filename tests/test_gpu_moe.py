@@ -230,6 +230,11 @@ def nvf4_expert_plane(ex, n_expert, rows, cols, seed):
     (9, 8, 2, 128, 192, 8, True),
     (40, 8, 4, 256, 128, 32, True),
     (21, 4, 2, 1344, 320, 8, False),        # K = 5 slabs and a quarter, relu^2 experts
+    (1, 8, 4, 256, 192, 8, True),           # up to 8 tokens and 32 pairs: routing and first preparation in one launch
+    (8, 8, 4, 320, 128, 8, True),
+    (3, 16, 2, 256, 128, 32, True),
+    (50, 4, 2, 256, 320, 32, False),        # 32-token blocks, one plane, odd and even counts of 128-row tiles
+    (50, 4, 2, 320, 256, 32, False),
 ])
 def test_nvf4_moe_block_matches_f64(pack, tokens, n_expert, k, embd, ff, bm, gated):
     ex = P.GpuExecutor(pack)
