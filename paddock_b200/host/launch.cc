@@ -12,8 +12,9 @@
 //   Caller(resolve, slow, error)         callable (name, *args, stream=0): error is None -> returns the
 //                                        status, else raises error(name, status) when it is not 0
 //
-// Pointer arguments are None, integers or objects with data_ptr(); anything else (ctypes arrays)
-// sends the call to `slow`, the ctypes route, which takes what ctypes takes.
+// Pointer arguments are None, integers or objects with data_ptr(), numbers Python ints and floats, the
+// stream an int or None; anything else (ctypes objects, numpy scalars) sends the call to `slow`, the
+// ctypes route, which takes what ctypes takes.
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
@@ -132,6 +133,7 @@ int convert(char kind, PyObject* o, Slot* out) {
             return PyErr_Occurred() ? -1 : 0;
         }
         case 'f': {
+            if (!PyFloat_Check(o) && !PyLong_Check(o)) return 1;
             const double v = PyFloat_AsDouble(o);
             if (v == -1.0 && PyErr_Occurred()) return -1;
             out->f = (float)v;
@@ -174,16 +176,17 @@ PyObject* caller_call(PyObject* self, PyObject* const* args, size_t nargsf, PyOb
         return nullptr;
     }
     void* stream = nullptr;
+    bool plain = true;      // the stream is an int or None
     if (nk == 1) {
         PyObject* key = PyTuple_GET_ITEM(kwnames, 0);
         if (key != g_stream && PyUnicode_Compare(key, g_stream) != 0) {
             PyErr_Format(PyExc_TypeError, "unexpected keyword argument '%U'", key);
             return nullptr;
         }
-        if (args[n] != Py_None) {
-            const unsigned long long v = PyLong_AsUnsignedLongLongMask(args[n]);
-            if (v == (unsigned long long)-1 && PyErr_Occurred()) return nullptr;
-            stream = reinterpret_cast<void*>(static_cast<uintptr_t>(v));
+        if (PyLong_Check(args[n])) {
+            stream = reinterpret_cast<void*>(static_cast<uintptr_t>(PyLong_AsUnsignedLongLongMask(args[n])));
+        } else {
+            plain = args[n] == Py_None;
         }
     }
     PyObject* name = args[0];
@@ -205,8 +208,8 @@ PyObject* caller_call(PyObject* self, PyObject* const* args, size_t nargsf, PyOb
         return nullptr;
     }
     Slot slots[kMaxArgs];
-    for (Py_ssize_t i = 0; i < e->n; ++i) {
-        const int r = convert(e->sig[i], args[1 + i], &slots[i]);
+    for (Py_ssize_t i = 0; i < e->n || !plain; ++i) {
+        const int r = plain ? convert(e->sig[i], args[1 + i], &slots[i]) : 1;
         if (r < 0) return nullptr;
         if (r > 0) {
             PyObject* res = PyObject_Vectorcall(c->slow, args, (size_t)n, kwnames);

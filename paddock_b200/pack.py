@@ -10,7 +10,10 @@ import ctypes as C
 import os
 import re
 
-from . import _launch
+try:
+    from . import _launch        # host/launch.cc: the same calls in a third of the host time
+except ImportError:              # not built for this interpreter: calls go through ctypes
+    _launch = None
 
 PACK_MAGIC = 0x504B4450
 PACK_ABI_VERSION = 2
@@ -152,8 +155,11 @@ class KernelPack:
         # call(name, *args, stream=0): launch slot `name` (or a named extra) and raise LaunchError on a non-zero
         # status; status(...) returns the raw status instead.  Pointer arguments may be ints or torch tensors.
         # Native (host/launch.cc): the argument conversion of a ctypes call costs as much as a launch.
-        self.call = _launch.Caller(self._entry, self._slow_status, LaunchError)
-        self.status = _launch.Caller(self._entry, self._slow_status, None)
+        if _launch is not None:
+            self.call = _launch.Caller(self._entry, self._slow_status, LaunchError)
+            self.status = _launch.Caller(self._entry, self._slow_status, None)
+        else:
+            self.call, self.status = self._slow_call, self._slow_status
 
     @classmethod
     def load(cls, path=None):
@@ -240,16 +246,24 @@ class KernelPack:
         return _launch.Entry(C.cast(fn, C.c_void_p).value, _EXTRA_SIGS.get(name) or _SIGS[name], name)
 
     def _slow_status(self, name, *args, stream=0):
-        """status() through ctypes, for arguments the native path does not convert (ctypes arrays)."""
+        """status() through ctypes, for arguments the native path does not convert (ctypes objects, numpy scalars)."""
         f = self.extra(name) if name in _EXTRA_SIGS else self.fn(name)
-        return f(*[_arg(a) for a in args], stream)
+        sig = _EXTRA_SIGS.get(name) or _SIGS[name]
+        if len(args) != len(sig):
+            raise TypeError(f"{name} takes {len(sig)} arguments before the stream, got {len(args)}")
+        return f(*[_arg(a, c) for a, c in zip(args, sig)], stream)
+
+    def _slow_call(self, name, *args, stream=0):
+        rc = self._slow_status(name, *args, stream=stream)
+        if rc != 0:
+            raise LaunchError(name, rc)
 
     def bind(self, name, *args, stream=0):
         """A zero-argument callable that launches `name` with these arguments (converted once): for
         loops where the per-call argument marshalling would rival a short kernel's run time.  The
         tensors behind the pointers must outlive it; it raises LaunchError like call()."""
         f = self.extra(name) if name in _EXTRA_SIGS else self.fn(name)
-        conv = tuple(_arg(a) for a in args) + (stream,)
+        conv = tuple(_arg(a, c) for a, c in zip(args, _EXTRA_SIGS.get(name) or _SIGS[name], strict=True)) + (stream,)
 
         def launch():
             rc = f(*conv)
@@ -259,7 +273,11 @@ class KernelPack:
         return launch
 
 
-def _arg(a):
+def _arg(a, kind):
+    if kind != "p":
+        if hasattr(a, "data_ptr"):     # its address is no number, and its value would be a hidden synchronisation
+            raise TypeError("a tensor where the kernel takes a number")
+        return a
     if a is None:
         return None
     if hasattr(a, "data_ptr"):

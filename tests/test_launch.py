@@ -1,7 +1,9 @@
 """The native launch path of the binding: every argument of every entry point's signature reaches the C function."""
 import ctypes as C
 import subprocess
+import sys
 
+import numpy as np
 import pytest
 
 from paddock_b200 import _launch
@@ -66,3 +68,57 @@ def test_errors(echo):
         _launch.Entry(addr, "pfpfpf", "no such signature")
     with pytest.raises(TypeError):
         call("some_slot", *[0] * len(SIGS[1]), flow=1)
+
+
+def test_what_ctypes_takes_goes_through_ctypes(echo):
+    """The stream as a ctypes pointer, numbers as ctypes or numpy scalars: the slow route, nothing refused and nothing read."""
+    sig = "pppppufu"
+    i = SIGS.index(sig)
+    addr = C.cast(getattr(echo, f"echo{i}"), C.c_void_p).value
+    slow = []
+    caller = _launch.Caller(lambda name: _launch.Entry(addr, sig, name), lambda *a, **k: slow.append((a, k)) or 7, None)
+    args = [64, 128, 192, 256, 320, 3, 0.5, 9]
+    assert caller("x", *args, stream=None) == i % 3 and not slow
+    st = C.c_void_p(0x77)
+    assert caller("x", *args, stream=st) == 7 and slow.pop() == (("x", *args), {"stream": st})
+    for at, v in ((5, np.int64(3)), (5, C.c_uint32(3)), (6, np.float32(0.5)), (6, C.c_float(0.5)), (6, _Tensor(4096))):
+        odd = [*args[:at], v, *args[at + 1:]]
+        assert caller("x", *odd, stream=5) == 7 and slow.pop() == (("x", *odd), {"stream": 5})
+
+
+@pytest.mark.parametrize("native", [True, False])
+def test_pack_calls_with_and_without_the_extension(native):
+    """The package (file formats included) imports and calls the library without _launch as well; a tensor in a number's
+    place is refused either way.  In its own process: the extension is blocked before the first import."""
+    code = f"""
+import sys, ctypes as C
+if not {native}:
+    sys.modules['paddock_b200._launch'] = None
+import numpy as np
+from paddock_b200 import KernelPack, LaunchError, Open, formats, pack
+assert (pack._launch is not None) == {native}
+try:
+    KernelPack.load('/nonexistent/pack.so')
+    raise SystemExit('loaded')
+except Open:
+    pass
+p = KernelPack.load()
+args = lambda k, n, st=0: ('f8row_gemm', 0, 0, 0, 0, 0, k, n, 1)
+assert p.call(*args(16, 0)) is None and p.status(*args(16, 0), stream=C.c_void_p(0)) == 0     # no rows: nothing to do
+assert p.status(*args(3, 4)) == 1 and p.status(*args(np.uint32(3), 4)) == 1                  # K not a multiple of 16
+try:
+    p.call(*args(3, 4))
+    raise SystemExit('not refused')
+except LaunchError as e:
+    assert e.status == 1
+class Tensor:
+    def data_ptr(self): return 16
+for bad in (args(Tensor(), 4), args(16, 0)[:-1]):
+    for f in (p.call, p.status):
+        try:
+            f(*bad)
+            raise SystemExit('taken')
+        except TypeError:
+            pass
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, cwd=packmod.os.path.dirname(packmod._PKG))
