@@ -75,6 +75,7 @@ struct Args {
     float scale2;              // nvfp4
     void* y;
     uint32_t in_dim, out_dim, batch, num_kb;
+    uint32_t tile_t0, tile_w0; // the launch's first token and channel tile
     uint32_t vec_store;        // y rows take 4-channel vector stores
     uint32_t sf_vec;           // nvfp4: x_sf is 16-byte aligned
     unsigned int* err;
@@ -114,7 +115,7 @@ splitk_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     Shared* sh = reinterpret_cast<Shared*>(smem + C::kStages * C::kStageBytes);
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t split = gridDim.x, rank = blockIdx.x;   // the cluster spans x
-    const uint32_t t0 = blockIdx.y * BN, n0 = blockIdx.z * BM, n_tok = min(BN, a.batch - t0);
+    const uint32_t tw = a.tile_w0 + blockIdx.z, t0 = (a.tile_t0 + blockIdx.y) * BN, n0 = tw * BM, n_tok = min(BN, a.batch - t0);
     const uint32_t kb_lo = rank * a.num_kb / split, kb_hi = (rank + 1u) * a.num_kb / split;
 
     if (threadIdx.x == 0) {
@@ -157,7 +158,7 @@ splitk_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
             if (reused) tc5::tma_load_2d_elect(s, &tmap_w, &sh->full[stage], (int32_t)(kb * BKB), (int32_t)n0);
             else tc5::tma_load_2d_hint_elect(s, &tmap_w, &sh->full[stage], (int32_t)(kb * BKB), (int32_t)n0, stream_once);
             if constexpr (KIND == kNvf4)
-                tc5::bulk_load_elect(s + C::kOffSfa, a.w_sf + ((size_t)blockIdx.z * a.num_kb + kb) * kSfBytes, kSfBytes, &sh->full[stage]);
+                tc5::bulk_load_elect(s + C::kOffSfa, a.w_sf + ((size_t)tw * a.num_kb + kb) * kSfBytes, kSfBytes, &sh->full[stage]);
         };
         // weights depend on nothing the previous kernel in the stream writes: the first stages go out before the wait for it
         const uint32_t pre = min(kb_hi - kb_lo, C::kStages);
@@ -324,7 +325,6 @@ int launch_bn(const void* data, const void* xq, Args& a, uint32_t row_bytes, cud
     while (split > 1u && (uint64_t)tiles_t * tiles_w > 2u * resident[split]) --split;
     if (split == 0u) split = 1u;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(split, tiles_t, tiles_w);
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = C::kSmemBytes;
     cfg.stream = st;
@@ -337,8 +337,15 @@ int launch_bn(const void* data, const void* xq, Args& a, uint32_t row_bytes, cud
     attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, tx, a);
-    return e == cudaSuccess ? pdk_launch_status() : (int)e;
+    // one launch, unless a grid axis cannot hold the tiles (numbering them along x instead cost a division per CTA, 0.1 us)
+    constexpr uint32_t kAxis = 65535u;
+    for (a.tile_w0 = 0u; a.tile_w0 < tiles_w; a.tile_w0 += kAxis)
+        for (a.tile_t0 = 0u; a.tile_t0 < tiles_t; a.tile_t0 += kAxis) {
+            const uint32_t nt = tiles_t - a.tile_t0, nw = tiles_w - a.tile_w0;
+            cfg.gridDim = dim3(split, nt < kAxis ? nt : kAxis, nw < kAxis ? nw : kAxis);
+            if (cudaError_t e = cudaLaunchKernelEx(&cfg, kern, tw, tx, a); e != cudaSuccess) return (int)e;
+        }
+    return pdk_launch_status();
 }
 
 template <int KIND, typename TO>

@@ -72,3 +72,18 @@ def test_nvfp4_first_call_behind_its_load(pack):
         want, got = run(w, s, True), run(w, s, False)
         assert torch.isfinite(want).all() and torch.equal(want, got)
     assert pack.device_error() == 0
+
+
+def test_fp8_more_channels_than_a_grid_axis_has_tiles(pack):
+    """65,536 tiles of 128 channels and one more: tiles are numbered along the grid's first axis, which holds them."""
+    k, n = 16, 65536 * 128 + 5
+    g = torch.Generator(device="cuda").manual_seed(6)
+    w = torch.randint(0, 0x60, (n, k), dtype=torch.uint8, device="cuda", generator=g)
+    x = torch.randint(0, 0x60, (1, k), dtype=torch.uint8, device="cuda", generator=g)
+    one = torch.ones(n, device="cuda")
+    y = torch.full((1, n), float("nan"), device="cuda")
+    pack.call("f8row_gemm", w, one, x, one, y, k, n, 1)
+    torch.cuda.synchronize()
+    assert pack.device_error() == 0
+    ref = x.view(torch.float8_e4m3fn).double() @ w.view(torch.float8_e4m3fn).double().t()
+    assert float(((y.double() - ref).abs() / ref.clamp_min(1e-30)).max()) < 1e-6      # sixteen exact non-negative products
