@@ -92,6 +92,14 @@ __device__ __forceinline__ uint32_t cluster_addr(uint32_t saddr, uint32_t rank) 
 __device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
     asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
 }
+// A store that may be past the batch.  Predicated, not branched around: with `if (i < left)` in front of it the compiler
+// leaves a branch per store, about 50 cycles each, one microsecond for 32 tokens.
+__device__ __forceinline__ void store_if(float* p, float v, bool on) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.global.f32 [%0], %1;\n\t}" ::"l"(p), "f"(v), "r"((uint32_t)on) : "memory");
+}
+__device__ __forceinline__ void store_if(__nv_bfloat16* p, __nv_bfloat16 v, bool on) {
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\t@q st.global.b16 [%0], %1;\n\t}" ::"l"(p), "h"(__bfloat16_as_ushort(v)), "r"((uint32_t)on) : "memory");
+}
 
 template <typename TO>
 __device__ __forceinline__ void store4(TO* p, const float (&v)[4]);
@@ -253,6 +261,42 @@ splitk_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     // CTAs took 12.3 us instead of 9.7).
     const uint32_t cpr = ((BM + split - 1u) / split + 3u) & ~3u;
     float* red = reinterpret_cast<float*>(smem);
+    TO* y = reinterpret_cast<TO*>(a.y);
+    if (split == 1u) {
+        // The tile is whole: straight from tensor memory to y, 32 neighbouring channels per store.  By way of the partial
+        // sums' buffer below it took NVFP4, K = 1024, N = 5120 4.5 us instead of 3.2 at 32 tokens, 8.8 instead of 5.2 at 200.
+        if (warp >= 2u) {
+            const uint32_t quarter = warp & 3u, n = n0 + quarter * 32u + lane;
+            const bool live = n < a.out_dim;
+            const float ws = KIND == kFp8 && live ? __ldg(a.w_scale + n) : 0.0f;
+            const float bias = KIND == kNvf4 && live && a.bias != nullptr ? a.bias[n] : 0.0f;
+#pragma unroll 1
+            for (uint32_t c = 0; c < n_tok; c += 32u) {
+                uint32_t r[32];
+                tc5::tmem_ld_32x32(tmem_base + ((quarter * 32u) << 16) + c, r);
+                const float xs = KIND == kFp8 ? a.x_scale[t0 + min(c + lane, n_tok - 1u)] : 0.0f;
+                tc5::tmem_ld_wait();
+                TO* out = y + (size_t)(t0 + c) * a.out_dim + n;
+                const uint32_t left = live ? n_tok - c : 0u;
+#pragma unroll
+                for (uint32_t i = 0; i < 32u; ++i) {
+                    const float v = __uint_as_float(r[i]);
+                    float o;
+                    if constexpr (KIND == kFp8) o = v * (__shfl_sync(0xffffffffu, xs, i) * ws);
+                    else o = fmaf(v, a.scale2, bias);
+                    store_if(out, to_out(o, out), i < left);
+                    out += a.out_dim;
+                }
+            }
+            tc5::fence_before_sync();
+        }
+        __syncthreads();
+        if (warp == 1) {
+            tc5::fence_after_sync();
+            tc5::tmem_dealloc(tmem_base, C::kTmemCols);
+        }
+        return;
+    }
     if (warp >= 2u) {
         const uint32_t quarter = warp & 3u, ch = quarter * 32u + lane;      // a warp reads its own quarter of the tensor-memory lanes
         const uint32_t dst = cluster_addr(tc5::smem_u32(red), ch / cpr) + (rank * n_tok * cpr + ch % cpr) * 4u;
@@ -268,11 +312,9 @@ splitk_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
         }
         tc5::fence_before_sync();
     }
-    if (split > 1u) cluster_sync();
-    else __syncthreads();
+    cluster_sync();
 
     const uint32_t ch_lo = rank * cpr, groups = ch_lo < BM ? min(cpr, BM - ch_lo) / 4u : 0u;   // of four channels
-    TO* y = reinterpret_cast<TO*>(a.y);
     for (uint32_t i = threadIdx.x; i < groups * n_tok; i += kThreads) {
         const uint32_t tok = i / groups, g = (i - tok * groups) * 4u, n = n0 + ch_lo + g, t = t0 + tok;
         if (n >= a.out_dim) continue;
@@ -317,12 +359,18 @@ int launch_bn(const void* data, const void* xq, Args& a, uint32_t row_bytes, cud
     static PdkClusterCaps table;
     const uint32_t* resident = nullptr;
     if (int rc = pdk_cluster_caps(table, (const void*)kern, kThreads, C::kSmemBytes, &resident)) return rc;
-    // The largest split whose clusters are all resident at once; more only add start-ups.  K = 5120, N = 5120, 7 tokens
+    // The largest split whose clusters are all resident at once: more only add start-ups.  K = 5120, N = 5120, 7 tokens
     // (40 tiles): 11.4 us at S = 1, 7.6 at 4, 7.4 at 6, and 11.9 at 7, where a part of the clusters waits for a
     // second turn.  At least two stages per CTA, so that it streams more than it sets up.
     const uint32_t tiles_t = (a.batch + BN - 1u) / BN, tiles_w = (a.out_dim + BM - 1u) / BM;
     uint32_t split = a.num_kb / 2u < kMaxSplit ? a.num_kb / 2u : kMaxSplit;
     while (split > 1u && (uint64_t)tiles_t * tiles_w > 2u * resident[split]) --split;
+    // It has to save a CTA more slabs (0.3 us each) than the meeting of the partial sums costs, which grows with the tokens of a
+    // tile.  us whole / split: fp8 K = 1024, N = 1024: 3.6 / 3.4 at 1 token, 3.7 / 4.4 at 32, 5.3 / 7.1 at 128; nvfp4 K = 1024, N = 5120:
+    // 3.1 / 3.8 at 1, 4.7 / 8.4 at 128; K = 2048, N = 5120: 4.7 / 4.5 at 1, 4.8 / 5.3 at 32.  Over 1500 random shapes
+    // (K = 1024 ... 17408, N = 512 ... 27648, 1 ... 8192 tokens) this choice is within 1.2 % of the best of all eight splits on average.
+    const uint32_t tokens = tiles_t > 1u ? BN : a.batch, saved = split > 1u ? a.num_kb - (a.num_kb + split - 1u) / split : 0u;
+    if (KIND == kFp8 ? saved * 12u <= 6u * 12u + tokens : saved * 16u <= 4u * 16u + tokens) split = 1u;
     if (split == 0u) split = 1u;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(kThreads);

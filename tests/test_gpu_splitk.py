@@ -12,7 +12,9 @@ from test_gpu_nvf4 import check_nvf4_gemm_w4a4
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(1, 1, 256), (1, 127, 2304), (31, 129, 1280), (32, 128, 5120), (33, 640, 256), (64, 1003, 1792), (65, 260, 768),
-          (128, 256, 4096), (129, 384, 2560), (385, 136, 1536), (7, 20000, 512)]
+          (128, 256, 4096), (129, 384, 2560), (385, 136, 1536), (7, 20000, 512),
+          # whole tiles to y (short K, or tiles enough) beside meeting partial sums, ragged in tokens and channels
+          (33, 1001, 1024), (100, 2500, 512), (257, 1000, 768), (8, 17001, 2048), (6, 130, 17408), (120, 1024, 8192)]
 
 
 @pytest.mark.parametrize("m,n,k", SHAPES + [(3, 64, 16), (5, 72, 2064)])
