@@ -410,17 +410,17 @@ int launch(const void* data, const void* xq, Args& a, uint32_t row_bytes, cudaSt
 }  // namespace
 
 // Whether a pair kernel (256 x 256 tiles, two SMs each) beats this file's 128 x 128 tiles for a prompt.  Per SM the
-// pair tile moves fewer shared-memory bytes per flop, but it never splits K: its time hardly falls below that of one full tile,
-// while this kernel shares every tile among the CTAs that fit.  Where the two cross was measured (K = 1024, 4096, 16384,
-// N = 512 ... 17408, 130 ... 8192 tokens, on a B200): fp8 at about one small tile per SM (K = 4096, N = 5120: 300 tokens
-// 14.5 against 19.9 us, 400 tokens 20.6 against 20.2), earlier where K is short; nvfp4, whose pair kernel also
-// has a 128-token tile, at about two small tiles per K slab (K = 4096, N = 1280: 300 tokens 9.6 against 10.5, 400 tokens
-// 11.8 against 10.6; K = 16384, N = 2560: 400 tokens 21.3 against 23.7, 1000 tokens 42.4 against 41.7).
-// Up to 128 tokens, one token tile, the weight stream decides and this kernel keeps the call.
+// pair tile moves fewer shared-memory bytes per flop, but it starts later and its time hardly falls below that of one full
+// tile.  So the line falls with K, and lies at many small tiles where K is short.  Measured on a B200 (434 random shapes of 129 ...
+// 8192 tokens; the rule is within 1 % of the faster one on average, and 4 % behind it at worst where it used to choose
+// the other), us here / pair: fp8 K = 1024, N = 5120: 22.4 / 28.4 at 2500 tokens (800 small tiles); K = 2048, N = 5120: 31.0 / 32.4
+// there; K = 5120, N = 5120, 200 tokens: 15.3 / 21.6, N = 17408, 2500 tokens: 225 / 157.  nvfp4, whose pair kernel also has a 128-token tile and
+// re-tiles the activation scales first: K = 1024, N = 17408: 18.1 / 19.5 at 700 tokens, 34.5 / 32.5 at 1500; K = 8192, N = 9472: 108 / 83
+// at 2500.  Up to 128 tokens, one token tile, the weight stream decides and this kernel keeps the call.
 bool pdk_prefer_pair(uint32_t batch, uint32_t out_dim, uint32_t row_bytes, bool nvf4) {
     if (batch <= 128u) return false;
     const uint64_t small = (uint64_t)((batch + 127u) / 128u) * ((out_dim + 127u) / 128u), slabs = (row_bytes + BKB - 1u) / BKB;
-    return small > (uint64_t)pdk_sm_count() || small > slabs * (nvf4 ? 2u : 10u);
+    return small > 100u && (small - 100u) * slabs > (nvf4 ? 8000u : 6000u);
 }
 
 int pdk_f8row_gemm_splitk(const void* data, const void* w_scale, const void* xq, const void* x_scale, void* y, uint32_t in_dim,
