@@ -29,49 +29,13 @@
 // issue slots (450 instructions per unit).  Tiles of 32 rows halve the fragments but double the ring's stages, so that
 // fewer fit: 24.7 us at 1 token, but 45 at 8 and no plan at all for Q6_K, not kept.
 #include "cluster_caps.cuh"
+#include "kq_plan.cuh"
 #include "tc5.cuh"
 
 namespace {
 
-enum Fmt : int { kQ4K = 0, kQ40 = 1, kQ5K = 2, kQ6K = 3 };
-
-constexpr uint32_t kRows = 16;           // rows of a tile
-// One column tile (up to 8 tokens): 16 warps.  Two: 8 warps, whose fragments need the registers.
-template <uint32_t NT> constexpr uint32_t kWarpsOf = 16u;
-constexpr uint32_t kMaxSplit = kPdkMaxCluster;
-constexpr uint32_t kMaxStages = 6;
-constexpr uint32_t kSmemMax = 232448;    // 227 KB
-constexpr uint32_t kBox0 = kRows * 128u, kRecs = kRows * 24u;
-
-template <int F>
-struct Fmts {
-    static constexpr uint32_t kUnit = F == kQ6K ? 192u : F == kQ5K ? 160u : 128u;   // data bytes of 256 weights
-    static constexpr uint32_t kBox1 = kRows * (kUnit - 128u);                         // the high bits' box
-    static constexpr uint32_t kBlocks = F == kQ6K ? 16u : 8u;
-    static constexpr uint32_t kStage = kBox0 + kBox1 + kRecs;
-};
-
-// Shared memory: ring ([warp][stage] boxes, then high-bit boxes, then records), the activation image, the partial tiles,
-// the barriers.  When a round's weights are consumed its ring takes the partial sums that other CTAs send.
-struct Layout {
-    uint32_t off_box1, off_rec, off_b, pitch, off_step, off_xs, off_red, off_bar, total;
-};
-template <int F, uint32_t NT>
-__host__ __device__ __forceinline__ Layout layout(uint32_t stages, uint32_t batch, uint32_t ku, uint32_t tiles) {
-    using T = Fmts<F>;
-    Layout l;
-    const uint32_t n = kWarpsOf<NT> * stages;
-    l.off_box1 = n * kBox0;
-    l.off_rec = l.off_box1 + n * T::kBox1;
-    l.off_b = l.off_rec + n * kRecs;
-    l.pitch = ku * 1024u + 64u;            // the odd 64 bytes put two tokens' rows on distinct banks
-    l.off_step = l.off_b + batch * l.pitch;
-    l.off_xs = l.off_step + ((ku * batch * 4u + 15u) & ~15u);
-    l.off_red = l.off_xs + ku * batch * T::kBlocks * 4u;
-    l.off_bar = l.off_red + (tiles + kWarpsOf<NT>) * kRows * NT * 8u * 4u;
-    l.total = l.off_bar + n * 8u + 16u;
-    return l;
-}
+using namespace kq;
+static_assert(kMaxSplit == kPdkMaxCluster, "cluster_caps.cuh asks for these sizes");
 
 struct Args {
     const uint8_t* recs;
@@ -117,10 +81,10 @@ __device__ __forceinline__ float scale_f(uint32_t w, uint32_t i, bool up, float 
 }
 
 template <int F, uint32_t NT>
-__global__ void __launch_bounds__(kWarpsOf<NT> * 32u, 1)
+__global__ void __launch_bounds__(kWarps * 32u, 1)
 kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, const Args a) {
     using T = Fmts<F>;
-    constexpr uint32_t NCOLS = NT * 8u, kWarps = kWarpsOf<NT>, kThreads = kWarps * 32u, MT = kRows / 16u;
+    constexpr uint32_t NCOLS = NT * 8u, kThreads = kWarps * 32u, MT = kRows / 16u;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, t = lane & 3u;
     const uint32_t split = gridDim.x, rank = blockIdx.x;   // the cluster spans x
@@ -494,48 +458,10 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
     }
 }
 
-struct Plan {
-    uint32_t split, clusters, rounds, round_tiles, ku, stages;
-    size_t smem;
-};
-
-// S and the number of rounds by the longest warp's units.  A round costs about two units more (the ring fills and the partials
-// meet), a ring of two stages a fifth of the time.
-template <int F, uint32_t NT>
-bool make_plan(Plan& best, const uint32_t* cap, uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
-    constexpr uint32_t kWarps = kWarpsOf<NT>;
-    const uint32_t n_unit = in_dim >> 8, n_tiles = (out_dim + kRows - 1u) / kRows;
-    float best_cost = 0.0f;
-    best.split = 0u;
-    for (uint32_t s = 1; s <= kMaxSplit && s <= n_unit; ++s) {
-        if (cap[s] == 0u) continue;
-        const uint32_t ku = (n_unit + s - 1u) / s, clusters = cap[s] < n_tiles ? cap[s] : n_tiles;
-        const uint32_t per = (n_tiles + clusters - 1u) / clusters;
-        // one tile a round at two stages has to fit (the first test keeps the sizes below within 32 bits)
-        if (ku > 1024u || layout<F, NT>(2u, batch, ku, 1u).total > kSmemMax) continue;
-        for (uint32_t rounds = 1; rounds <= per; ++rounds) {
-            const uint32_t rt = (per + rounds - 1u) / rounds;
-            uint32_t d = kMaxStages;
-            while (d >= 2u && layout<F, NT>(d, batch, ku, rt).total > kSmemMax) --d;
-            // what the other CTAs send fits the ring
-            if (s * batch * ((rt * kRows + s - 1u) / s) * 4u > kWarps * d * Fmts<F>::kStage) d = 0u;
-            if (d < 2u) continue;
-            const uint32_t units = (rt * ku + kWarps - 1u) / kWarps;
-            const float cost = (float)rounds * ((float)units * (d == 2u ? 1.2f : 1.0f) + 2.0f) + (s > 1u ? 0.5f : 0.0f);
-            if (best.split == 0u || cost < best_cost) {
-                best_cost = cost;
-                best = Plan{s, clusters, rounds, rt, ku, d, layout<F, NT>(d, batch, ku, rt).total};
-            }
-            break;     // more rounds only cost more
-        }
-    }
-    return best.split != 0u;
-}
-
 template <int F, uint32_t NT>
 int launch(const void* data, const void* recs, const float* x, const int8_t* xq, const float* xq_scale, float* y, uint32_t in_dim,
            uint32_t out_dim, uint32_t batch, cudaStream_t st) {
-    constexpr uint32_t kThreads = kWarpsOf<NT> * 32u;
+    constexpr uint32_t kThreads = kWarps * 32u;
     auto kern = kq_batch_kernel<F, NT>;
     static PdkClusterCaps table;
     const uint32_t* cap = nullptr;       // one CTA per SM
