@@ -175,6 +175,9 @@ int pd_kquant_gemm_w4a8_sb(const void* data, const void* scales, const void* xq,
 int pdk_kquant_gemm_f32(const void* data, const void* scales, const void* x, void* y,
                         uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t dtype,
                         void* stream);
+/* Which kernel a small batch asks first, for tests and diagnostics (no device needed): 1 kq_batch.cu, 2 the integer
+ * kernel, 3 tcgen05; 0 = none of them (one token, IQ4_XS, more than 64 tokens). */
+int pdk_kquant_gemm_route(uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t dtype);
 
 /* ---- FP8 E4M3, one f32 scale per row ----------------------------------------- */
 

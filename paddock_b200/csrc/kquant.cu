@@ -17,6 +17,7 @@
 // bf16 hi + bf16 lo parts that ride in two columns of the same mma, and the
 // per-sub-block scale, the min term and the 128 offset are applied in f32 to
 // the 32-element partial sums.
+#include <cmath>
 #include <cstdlib>
 
 #include "pdk_common.cuh"
@@ -545,7 +546,9 @@ bool force_bf16_batch() {
     return v;
 }
 
-// From how many tokens on the tcgen05 kernel takes a call (PDK_Q4K_TC5_MIN, read once; 0 = never).
+enum Route : int { kRouteKq = 1, kRouteI8 = 2, kRouteTc5 = 3 };
+
+// From how many tokens on the tcgen05 kernel takes a Q4_K call (PDK_Q4K_TC5_MIN, read once; 0 = never).
 uint32_t tc5_min_tokens() {
     static const uint32_t v = [] {
         const char* e = getenv("PDK_Q4K_TC5_MIN");
@@ -554,21 +557,30 @@ uint32_t tc5_min_tokens() {
     return v;
 }
 
-// Where kq_batch.cu (clusters over K, any width) beats the kernels it shares a format with.
-//
-// Against the integer kernel of q4k_batch_i8.cu (Q4_K, Q5_K up to 8 tokens), whose time hardly falls below that of one round
-// of 64-row CTAs while this one splits K until the chip is full: kq_batch grows with tokens and plane, so the line falls
-// with both.  Measured (us, kq_batch against integer, Q4_K): K = 5120, N = 4096: 9.1 / 9.7 at 2 tokens, 10.7 / 9.8 at 4;
-// N = 2048: 8.7 / 9.6 at 4, 10.5 / 9.8 at 8; N = 1024: 7.9 / 9.5 at 8; N = 25600: 25.4 / 22.1 at 2; K = 1024, N = 9472:
-// 4.8 / 5.7 at 2, 4.9 / 5.5 at 4, 5.7 / 5.7 at 8; N = 13824: 6.3 / 5.6 at 2.
+// Where kq_batch.cu (clusters over K, any width) beats the integer kernel of q4k_batch_i8.cu (Q4_K, Q5_K up to 8 tokens), whose
+// time hardly falls below that of one round of 64-row CTAs while kq_batch splits K until the chip is full and grows with tokens
+// and plane.  Measured over 480 random shapes of both formats (K = 1024 ... 17408, N = 512 ... 27648; the rule is 1.1 % off the
+// faster one on average), us kq_batch / integer:
+//   K > 9216: the integer kernel's activation image leaves no L1: K = 11008, N = 2304, 2 tokens 10.2 / 41.5, N = 6208, 8 tokens 22.3 / 42.4;
+//   below, N (tokens + 8) against 680 sqrt(K): K = 8192, N = 3000, 8 tokens 11.8 / 14.3; K = 4096, N = 4096: 7.0 / 8.1 at 3, 9.6 / 8.1 at 8;
+//   K = 5120, N = 25600: 26.2 / 21.2 at 2, 32.1 / 22.2 at 8;
+//   narrow planes at short K, where both take a few us: kq_batch is one launch and keeps 22 activation bits where the
+//   integer kernel keeps 15.  K = 1024, N = 4096, 4 tokens: 4.6 / 5.5 launched one by one, 4.3 / 3.6 in a replayed graph.
 bool kq_beats_i8(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
+    if (in_dim > 9216u || (float)out_dim * (float)(batch + 8u) <= 680.0f * sqrtf((float)in_dim)) return true;
     const uint64_t limit = batch <= 2u ? 30000000u : batch <= 4u ? 20000000u : 10000000u;
     return (uint64_t)out_dim * (in_dim + 2048u) <= limit;
 }
-// Against the tcgen05 kernel of q4k_tc5.cu (Q4_0 from 4 tokens), which costs the same at 4 and at 16 tokens: K = 5120,
-// N = 25600: 26.4 / 29.2 at 4 tokens; N = 9472: 14.3 / 14.9 at 4, 16.2 / 15.2 at 8; N = 4096: 12.0 / 12.9 at 8.
-bool kq_beats_tc5(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
-    return batch <= 4u || (batch <= 8u && (uint64_t)out_dim * in_dim <= 25000000u);
+
+// The kernel that a pass over `batch` tokens asks first.  Q4_0 up to 8 tokens: kq_batch against the tcgen05 kernel (which costs the same
+// at 4 and at 16 tokens) is 0.4 % off the faster one over 180 random shapes, up to 5 times faster, at most 18 % slower (K = 5120,
+// N = 25600: 26.4 / 29.2 us at 4 tokens; N = 9472: 16.2 / 15.2 at 8).  Q5_K from 9 tokens on: two passes of the integer kernel would
+// be faster on wide planes (K = 5120, N = 25600, 16 tokens: 51.6 against 65.8 us), but kq_batch keeps 22 activation bits.
+Route batch_route(uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t dtype) {
+    const uint32_t from = dtype == PDK_KQ_Q4K ? tc5_min_tokens() : dtype == PDK_KQ_Q4_0 && tc5_min_tokens() != 0u ? 9u : 0u;
+    if (from != 0u && batch >= from) return kRouteTc5;
+    if ((dtype == PDK_KQ_Q4K || dtype == PDK_KQ_Q5K) && batch <= 8u && !kq_beats_i8(in_dim, out_dim, batch)) return kRouteI8;
+    return kRouteKq;
 }
 
 // Up to 16 tokens of `batch` through kq_batch.cu, in passes of one width (17 tokens are 9 + 8: the weights are read once per
@@ -584,12 +596,12 @@ int kq_pass(const void* data, const void* scales, const float* x, const int8_t* 
     return 0;
 }
 
-// 2 <= tokens of a Q4_K plane on the tensor paths: up to 32 tokens per launch on tcgen05 from tc5_min_tokens() on, up to 8 on
-// the integer kernel where kq_beats_i8 does not say otherwise, and whatever is outside their plans up to 16 on kq_batch.cu.
-// Activations f32 (x) or int8 with per-32 scales (xq, xs).  Returns the number of tokens done (all of them unless a
-// shape is outside every plan), or -(cudaError_t) - 1 on a launch error.
+// 2 <= tokens of a Q4_K, Q4_0, Q5_K or Q6_K plane on the tensor paths: up to 32 tokens per launch on tcgen05, up to 8 on the
+// integer kernel, and whatever is not theirs or outside their plans up to 16 on kq_batch.cu.  Activations f32 (x) or, for Q4_K, int8 with
+// per-32 scales (xq, xs).  Returns the number of tokens done (all of them unless a shape is outside every plan), or
+// -(cudaError_t) - 1 on a launch error.
 int small_batch(const void* data, const void* scales, const float* x, const int8_t* xq, const float* xs, float* y,
-                uint32_t in_dim, uint32_t out_dim, uint32_t batch, cudaStream_t st) {
+                uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t dtype, cudaStream_t st) {
     uint32_t b = 0;
     while (b < batch) {
         const uint32_t left = batch - b;
@@ -597,45 +609,21 @@ int small_batch(const void* data, const void* scales, const float* x, const int8
         const int8_t* qb = xq ? xq + (size_t)b * in_dim : nullptr;
         const float* sb = xs ? xs + (size_t)b * (in_dim >> 5) : nullptr;
         float* yb = y + (size_t)b * out_dim;
-        uint32_t take = 0;
-        int rc = -1;
-        if (tc5_min_tokens() != 0u && left >= tc5_min_tokens()) {
-            take = left < 32u ? left : 32u;
-            rc = pdk_q4k_tc5(data, scales, xb, qb, sb, yb, in_dim, out_dim, take, st);
-        }
-        if (rc == -1 && left <= 8u && !kq_beats_i8(in_dim, out_dim, left)) {
-            take = left;
-            rc = pdk_q4k_batch_i8(data, scales, xb, qb, sb, yb, in_dim, out_dim, take, st);
-        }
-        if (rc == -1) {
-            const int done = kq_pass(data, scales, xb, qb, sb, yb, in_dim, out_dim, left, PDK_KQ_Q4K, st);
-            if (done < 0) return done;
-            if (done == 0) break;
-            take = (uint32_t)done;
-            rc = 0;
-        }
-        if (rc != 0) return -rc - 1;
-        b += take;
-    }
-    return (int)b;
-}
-
-// The same for Q4_0 (tcgen05 where kq_beats_tc5 does not say otherwise), Q5_K (the integer kernel up to 8 tokens) and Q6_K.
-int small_batch_more(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim, uint32_t out_dim,
-                     uint32_t batch, uint32_t dtype, cudaStream_t st) {
-    uint32_t b = 0;
-    while (b < batch) {
-        const uint32_t left = batch - b;
-        const float* xb = x + (size_t)b * in_dim;
-        float* yb = y + (size_t)b * out_dim;
         uint32_t take = left < 32u ? left : 32u;
         int rc = -1;
-        if (dtype == PDK_KQ_Q4_0 && tc5_min_tokens() != 0u && !kq_beats_tc5(in_dim, out_dim, left))
-            rc = pdk_q4_0_tc5(data, scales, xb, yb, in_dim, out_dim, take, st);
-        if (dtype == PDK_KQ_Q5K && left <= 8u && !kq_beats_i8(in_dim, out_dim, left))
-            rc = pdk_q5k_batch_i8(data, scales, xb, yb, in_dim, out_dim, left, st);
+        switch (batch_route(in_dim, out_dim, left, dtype)) {
+            case kRouteTc5:
+                rc = dtype == PDK_KQ_Q4K ? pdk_q4k_tc5(data, scales, xb, qb, sb, yb, in_dim, out_dim, take, st)
+                                         : pdk_q4_0_tc5(data, scales, xb, yb, in_dim, out_dim, take, st);
+                break;
+            case kRouteI8:
+                rc = dtype == PDK_KQ_Q4K ? pdk_q4k_batch_i8(data, scales, xb, qb, sb, yb, in_dim, out_dim, take, st)
+                                         : pdk_q5k_batch_i8(data, scales, xb, yb, in_dim, out_dim, take, st);
+                break;
+            default: break;
+        }
         if (rc == -1) {
-            const int done = kq_pass(data, scales, xb, nullptr, nullptr, yb, in_dim, out_dim, left, dtype, st);
+            const int done = kq_pass(data, scales, xb, qb, sb, yb, in_dim, out_dim, left, dtype, st);
             if (done < 0) return done;
             if (done == 0) break;
             take = (uint32_t)done;
@@ -654,7 +642,7 @@ int gemm_any(const void* data, const void* scales, const float* x, float* y, uin
         if (rc != -1) return rc;
     }
     if (!force_plain() && !force_bf16_batch()) {
-        const int done = small_batch(data, scales, x, nullptr, nullptr, y, in_dim, out_dim, batch, st);
+        const int done = small_batch(data, scales, x, nullptr, nullptr, y, in_dim, out_dim, batch, PDK_KQ_Q4K, st);
         if (done < 0) return -done - 1;
         if ((uint32_t)done == batch) return 0;
         // outside both plans: the bf16 kernel or the plain route take what is left
@@ -748,13 +736,18 @@ PDK_EXPORT int pd_kquant_gemv(const void* data, const void* scales, const void* 
     return gemm_any(data, scales, (const float*)x, (float*)y, in_dim, out_dim, 1u, (cudaStream_t)stream);
 }
 
+PDK_EXPORT int pdk_kquant_gemm_route(uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t dtype) {
+    const bool known = dtype == PDK_KQ_Q4K || dtype == PDK_KQ_Q4_0 || dtype == PDK_KQ_Q5K || dtype == PDK_KQ_Q6K;
+    return known && batch >= 2u && batch <= 64u ? (int)batch_route(in_dim, out_dim, batch, dtype) : 0;
+}
+
 PDK_EXPORT int pdk_kquant_gemm_f32(const void* data, const void* scales, const void* x, void* y, uint32_t in_dim,
                                    uint32_t out_dim, uint32_t batch, uint32_t dtype, void* stream) {
     if (out_dim == 0 || batch == 0) return 0;
     if (batch > 64u) return cudaErrorInvalidValue;
     if (int rc = check_gemv(data, scales, x, y, in_dim, dtype)) return rc;
     if ((dtype == PDK_KQ_Q4_0 || dtype == PDK_KQ_Q5K || dtype == PDK_KQ_Q6K) && batch >= 2u && !force_plain()) {
-        const int done = small_batch_more(data, scales, (const float*)x, (float*)y, in_dim, out_dim, batch, dtype, (cudaStream_t)stream);
+        const int done = small_batch(data, scales, (const float*)x, nullptr, nullptr, (float*)y, in_dim, out_dim, batch, dtype, (cudaStream_t)stream);
         if (done < 0) return -done - 1;
         if ((uint32_t)done == batch) return 0;
         x = (const float*)x + (size_t)done * in_dim;   // outside every plan: the routes below take what is left
@@ -826,7 +819,7 @@ int w4a8_gemm(const void* data, const void* scales, const void* xq, const void* 
     }
     if (!force_plain() && !force_bf16_batch() && pdk_aligned(xq, 8)) {
         const int done = small_batch(data, scales, nullptr, (const int8_t*)xq, (const float*)xs, (float*)y, in_dim,
-                                     out_dim, batch, st);
+                                     out_dim, batch, PDK_KQ_Q4K, st);
         if (done < 0) return -done - 1;
         if ((uint32_t)done == batch) return 0;
         // outside both plans, or no scratch slice for this stream: the widening route takes what is left

@@ -1,5 +1,5 @@
 """The split plan of kq_batch.cu (csrc/kq_plan.cuh, compiled here for the host) over shapes of every size: what a plan puts into
-shared memory fits, the partial sums that a cluster sends fit the ring, the sizes do not wrap at the largest planes."""
+shared memory fits, the partial sums that a cluster sends fit the ring, the sizes do not wrap at the largest planes; and the rule that gives a call to that kernel or to another."""
 import os
 import subprocess
 
@@ -53,3 +53,27 @@ def test_plans_fit(tmp_path):
     csrc = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "paddock_b200", "csrc")
     subprocess.check_call(["g++", "-std=c++17", "-O2", "-I", csrc, "-o", str(tmp_path / "plan"), str(tmp_path / "plan.cc")])
     subprocess.check_call([str(tmp_path / "plan")], timeout=120)
+
+
+def test_routes_of_small_batches():
+    """Both sides of every line of the rule (kquant.cu), asked from the library: 1 kq_batch, 2 the integer kernel, 3 tcgen05, 0 other."""
+    import paddock_b200
+    lib = paddock_b200.KernelPack.load()._lib
+    route = lib.pdk_kquant_gemm_route
+    q4_0, q4_k, q5_k, q6_k, iq4_xs = 2, 12, 13, 14, 23
+    for dtype in (q4_k, q5_k):
+        assert route(9216, 27648, 2, dtype) == 2 and route(9472, 27648, 2, dtype) == 1         # K past the integer kernel's image
+        # N (tokens + 8) <= 680 sqrt(4096) = 43520
+        assert route(4096, 4352, 2, dtype) == 1 and route(4096, 4960, 2, dtype) == 2
+        assert route(4096, 2720, 8, dtype) == 1 and route(4096, 2721, 8, dtype) == 2
+        # N (K + 2048) <= 30, 20, 10 million up to 2, 4, 8 tokens
+        assert route(1024, 9765, 2, dtype) == 1 and route(1024, 9766, 2, dtype) == 2
+        assert route(1024, 6510, 4, dtype) == 1 and route(1024, 6511, 4, dtype) == 2
+        assert route(1024, 3255, 8, dtype) == 1 and route(1024, 3256, 8, dtype) == 2
+        assert route(5120, 25600, 1, dtype) == 0 and route(5120, 25600, 65, dtype) == 0
+        assert route(1 << 30, 1 << 30, 8, dtype) == 1 and route(256, (1 << 32) - 1, 2, dtype) == 2
+    assert [route(5120, 25600, m, q4_k) for m in (8, 9, 64)] == [2, 3, 3]
+    assert [route(5120, 25600, m, q5_k) for m in (8, 9, 64)] == [2, 1, 1]
+    assert [route(5120, 25600, m, q4_0) for m in (2, 8, 9, 64)] == [1, 1, 3, 3]
+    assert [route(5120, 25600, m, q6_k) for m in (2, 16, 64)] == [1, 1, 1]
+    assert route(5120, 25600, 4, iq4_xs) == 0
