@@ -199,12 +199,13 @@ def test_q4_k_small_batch_k5120_band(pack, batch):
     assert rel_l2(y, ref) < (1e-4 if batch <= 8 else 1e-3) < TOL
 
 
-@pytest.mark.parametrize("k,n,batch", [(5120, 1000, 2), (2048, 130, 8), (1024, 48, 5),      # int8 path, ragged rows
+@pytest.mark.parametrize("k,n,batch", [(5120, 1000, 2), (2048, 130, 8), (1024, 48, 5),      # kq_batch.cu, ragged rows
                                        (5120, 1000, 9), (2048, 300, 17), (4096, 257, 32),   # tcgen05, K halves
                                        (1536, 200, 16), (5120, 640, 40),                    # one K part; two launches
-                                       (1280, 64, 16)])                                     # odd super-block count: int8 path
+                                       (1280, 64, 16)])                                     # odd super-block count: kq_batch.cu
 def test_q4_k_batch_shapes(pack, k, n, batch):
-    """Every small-batch route of pdk_kquant_gemm_f32 on f32 activations that are not bf16 values."""
+    """pdk_kquant_gemm_f32 on f32 activations that are not bf16 values, narrow planes (the integer kernel's wide ones:
+    test_gpu_i8_batch.py)."""
     w = oracle.fill_normal(n * k, seed_for(2, 900 + k + n), 0.02)
     x = oracle.fill_normal(batch * k, seed_for(2, 901 + batch), 1.0)
     x[:k] *= 1.0e4                       # one token far outside the f16 range, one tiny, one zero
@@ -227,8 +228,8 @@ def test_q4_k_batch_shapes(pack, k, n, batch):
 @pytest.mark.parametrize("k,n", [(5120, 1000), (6144, 72), (2048, 33)])
 @pytest.mark.parametrize("batch", [2, 3, 8])
 def test_q4_k_two_to_eight_tokens(pack, k, n, batch):
-    """2 .. 8 tokens on the integer batch kernel: ragged rows, an all-zero token, a token of tiny
-    values; bit-identical from call to call."""
+    """2 .. 8 tokens of narrow planes (kq_batch.cu): ragged rows, an all-zero token, a token of tiny values; bit-identical
+    from call to call."""
     w = oracle.fill_normal(n * k, seed_for(2, 970 + k), 0.02)
     x = oracle.fill_normal(batch * k, seed_for(2, 971 + batch), 1.0)
     x[:k] = 0.0
@@ -328,7 +329,7 @@ def test_q4k_w4a8_slots(pack, k, n, batch):
             pack.call(name, d_data, d_sc, dev(q), dev_f32(s), dev_f32(sums), d_part, d_y, k, n, batch, 12)
         torch.cuda.synchronize()
         y = d_y.cpu().numpy().reshape(batch, n)
-        # up to 8 tokens run the integer path, more the f16-weight tcgen05 path
+        # up to 8 tokens of these narrow planes run kq_batch.cu, more the f16-weight tcgen05 path
         assert cond_err(y, ref, ab) < 1e-4 < TOL, name
 
 
@@ -379,7 +380,7 @@ def test_more_kquants_dequant_repack_gemv(pack, name, k, n):
             pack.call("pdk_kquant_gemm_f32", d_data, d_sc, dev_f32(x), d_out, k, n, batch, dtype)
         torch.cuda.synchronize()
         ref, ab = oracle.matmul_f64(want, x, k, n, batch, with_abs=True)
-        # Q4_0 from four tokens on (and K a multiple of 512) runs the f16-weight tcgen05 kernel
+        # Q4_0 from nine tokens on (and K a multiple of 512) runs the f16-weight tcgen05 kernel
         tol = 1e-4 if (name == "q4_0" and batch >= 4 and k % 512 == 0) else 1e-5
         assert cond_err(d_out.cpu().numpy().reshape(batch, n), ref, ab) < tol < TOL
 
@@ -387,8 +388,8 @@ def test_more_kquants_dequant_repack_gemv(pack, name, k, n):
 @pytest.mark.parametrize("name", ["q5_k", "q6_k"])
 @pytest.mark.parametrize("batch", [2, 8, 9, 16, 33])
 def test_q5_k_q6_k_tokens_as_columns(pack, name, batch):
-    """The integer batch kernels of Q5_K and Q6_K (eight or sixteen token columns per weight pass),
-    whole and ragged passes, rows that are not a multiple of the 16-row tile."""
+    """Q5_K and Q6_K through kq_batch.cu (eight or sixteen token columns per weight pass), whole and ragged passes, rows
+    that are not a multiple of the 16-row tile."""
     dtype, datab = KQ[name]
     k, n = 2048, 203
     ns = n * k // 256
@@ -403,7 +404,7 @@ def test_q5_k_q6_k_tokens_as_columns(pack, name, batch):
     torch.cuda.synchronize()
     assert pack.device_error() == 0
     ref, ab = oracle.matmul_f64(want, x, k, n, batch, with_abs=True)
-    # f32 activations: the batch kernels' 15-bit block floating point per 256 elements (the Q4_K batch tests' bound)
+    # the integer kernels' 15-bit block floating point per 256 elements (kq_batch.cu keeps 22 bits: test_gpu_kq_batch.py)
     err = cond_err(d_out.cpu().numpy().reshape(batch, n), ref, ab)
     assert err < 1e-4 < TOL, ("batch kernel", err)
     # each token alone through the decode GEMV: the same value up to the activations' block-floating step
