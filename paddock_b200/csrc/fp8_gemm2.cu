@@ -23,6 +23,7 @@
 namespace {
 
 using namespace tc5::pair;
+using tc5::cluster_sync;
 
 constexpr uint32_t BM = 128;            // tokens per CTA (256 per pair)
 constexpr uint32_t BN = 256;            // channels per pair

@@ -35,6 +35,9 @@
 namespace {
 
 using namespace kq;
+using tc5::cluster_addr;
+using tc5::cluster_sync;
+using tc5::st_cluster;
 static_assert(kMaxSplit == kPdkMaxCluster, "cluster_caps.cuh asks for these sizes");
 
 struct Args {
@@ -57,17 +60,6 @@ __device__ __forceinline__ void mma_f16_z(float (&d)[4], const uint32_t (&a)[4],
                  : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
                  : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.0f));
 }
-__device__ __forceinline__ uint32_t cluster_addr(uint32_t saddr, uint32_t rank) {
-    uint32_t a;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
-    return a;
-}
-__device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void cp_async8(uint32_t dst, const void* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(dst), "l"(src) : "memory");
 }
@@ -84,7 +76,7 @@ template <int F, uint32_t NT>
 __global__ void __launch_bounds__(kWarps * 32u, 1)
 kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, const Args a) {
     using T = Fmts<F>;
-    constexpr uint32_t NCOLS = NT * 8u, kThreads = kWarps * 32u, MT = kRows / 16u;
+    constexpr uint32_t NCOLS = NT * 8u, kThreads = kWarps * 32u;
     extern __shared__ __align__(1024) uint8_t smem[];
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, g = lane >> 2, t = lane & 3u;
     const uint32_t split = gridDim.x, rank = blockIdx.x;   // the cluster spans x
@@ -228,13 +220,11 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
             even[n] = min(2u * t + 8u * n, a.batch - 1u);
             odd[n] = min(2u * t + 1u + 8u * n, a.batch - 1u);
         }
-        float acc[MT][NT][4];
+        float acc[NT][4];
 #pragma unroll
-        for (uint32_t m = 0; m < MT; ++m)
+        for (uint32_t n = 0; n < NT; ++n)
 #pragma unroll
-            for (uint32_t n = 0; n < NT; ++n)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[m][n][i] = 0.0f;
+            for (int i = 0; i < 4; ++i) acc[n][i] = 0.0f;
         const float* ustep = reinterpret_cast<const float*>(smem + L.off_step);
         constexpr uint32_t kSteps = F == kQ6K ? 1u : 2u;
         constexpr float kBias = F == kQ6K ? 128.0f : 0.0f;
@@ -245,154 +235,136 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
             const uint8_t* b0 = box0 + stage * kBox0;
             const uint8_t* b1 = box1 + stage * T::kBox1;
             const uint8_t* rb = recs + stage * kRecs + row * 24u;
-            float U[MT][NT][4];
+            float U[NT][4];
 #pragma unroll
-            for (uint32_t m = 0; m < MT; ++m)
+            for (uint32_t n = 0; n < NT; ++n)
 #pragma unroll
-                for (uint32_t n = 0; n < NT; ++n)
-#pragma unroll
-                    for (int i = 0; i < 4; ++i) U[m][n][i] = 0.0f;
+                for (int i = 0; i < 4; ++i) U[n][i] = 0.0f;
             const uint8_t* bp[NT];
 #pragma unroll
             for (uint32_t n = 0; n < NT; ++n) bp[n] = smem + L.off_b + col[n] * L.pitch + c_u * 1024u + t * 16u;
 
-            uint32_t sw[MT][2][4];     // the scale bytes (Q6: raised by 128; Q4_0: eight f16 scales)
-            uint2 high[MT][2];         // Q5: the high-bit bytes 8t .. 8t+7
+            uint32_t sw[2][4];     // the scale bytes (Q6: raised by 128; Q4_0: eight f16 scales)
+            uint2 high[2];         // Q5: the high-bit bytes 8t .. 8t+7
 #pragma unroll
-            for (uint32_t m = 0; m < MT; ++m)
+            for (uint32_t h = 0; h < 2u; ++h) {
+                const uint32_t* rp = reinterpret_cast<const uint32_t*>(rb + h * 192u) + (F == kQ40 ? 0 : 1);
 #pragma unroll
-                for (uint32_t h = 0; h < 2u; ++h) {
-                    const uint32_t* rp = reinterpret_cast<const uint32_t*>(rb + (m * 16u + h * 8u) * 24u) + (F == kQ40 ? 0 : 1);
-#pragma unroll
-                    for (uint32_t i = 0; i < 4u; ++i)
-                        sw[m][h][i] = (F == kQ6K) ? rp[i] ^ 0x80808080u : (F == kQ40 || i < 2u) ? rp[i] : 0u;
-                    if constexpr (F == kQ5K) high[m][h] = *reinterpret_cast<const uint2*>(b1 + (row + m * 16u + h * 8u) * 32u + t * 8u);
-                }
+                for (uint32_t i = 0; i < 4u; ++i)
+                    sw[h][i] = (F == kQ6K) ? rp[i] ^ 0x80808080u : (F == kQ40 || i < 2u) ? rp[i] : 0u;
+                if constexpr (F == kQ5K) high[h] = *reinterpret_cast<const uint2*>(b1 + (row + h * 8u) * 32u + t * 8u);
+            }
             // A pair of blocks shares its bytes: the low nibbles' block and the high nibbles'
 #pragma unroll
             for (uint32_t p = 0; p < T::kBlocks / 2u; ++p) {
                 // Q6: p = half * 4 + h * 2 + (run & 1)
                 const uint32_t nh = p >> 2, hb = (p >> 1) & 1u, r01 = p & 1u;
-                uint32_t x[MT][2][kSteps], z[MT][2][kSteps];
+                uint32_t x[2][kSteps], z[2][kSteps];
 #pragma unroll
-                for (uint32_t m = 0; m < MT; ++m)
-#pragma unroll
-                    for (uint32_t h = 0; h < 2u; ++h) {
-                        const uint32_t r = row + m * 16u + h * 8u;
-                        if constexpr (F == kQ6K) {
-                            const uint32_t c = 4u * nh + 2u * r01 + hb;
-                            x[m][h][0] = *reinterpret_cast<const uint32_t*>(b0 + r * 128u + ((c ^ (row & 7u)) << 4) + t * 4u);
-                            z[m][h][0] = *reinterpret_cast<const uint32_t*>(b1 + r * 64u + (((2u * nh + hb) ^ ((row >> 1) & 3u)) << 4) + t * 4u);
-                        } else {
-                            const uint2 v = *reinterpret_cast<const uint2*>(b0 + r * 128u + (((2u * p + (t >> 1)) ^ (row & 7u)) << 4) + (t & 1u) * 8u);
-                            x[m][h][0] = v.x;
-                            x[m][h][kSteps - 1u] = v.y;
-                            z[m][h][0] = high[m][h].x;
-                            z[m][h][kSteps - 1u] = high[m][h].y;
-                        }
+                for (uint32_t h = 0; h < 2u; ++h) {
+                    const uint32_t r = row + h * 8u;
+                    if constexpr (F == kQ6K) {
+                        const uint32_t c = 4u * nh + 2u * r01 + hb;
+                        x[h][0] = *reinterpret_cast<const uint32_t*>(b0 + r * 128u + ((c ^ (row & 7u)) << 4) + t * 4u);
+                        z[h][0] = *reinterpret_cast<const uint32_t*>(b1 + r * 64u + (((2u * nh + hb) ^ ((row >> 1) & 3u)) << 4) + t * 4u);
+                    } else {
+                        const uint2 v = *reinterpret_cast<const uint2*>(b0 + r * 128u + (((2u * p + (t >> 1)) ^ (row & 7u)) << 4) + (t & 1u) * 8u);
+                        x[h][0] = v.x;
+                        x[h][kSteps - 1u] = v.y;
+                        z[h][0] = high[h].x;
+                        z[h][kSteps - 1u] = high[h].y;
                     }
+                }
 #pragma unroll
                 for (uint32_t up = 0; up < 2u; ++up) {
                     const uint32_t b = F == kQ6K ? 8u * nh + 2u * (r01 + 2u * up) + hb : 2u * p + up;
                     const uint32_t mq = up ? 0x00F000F0u : 0x000F000Fu;
-                    float d[MT][NT][4];
+                    float d[NT][4];
 #pragma unroll
                     for (uint32_t j = 0; j < kSteps; ++j) {
-                        uint32_t A[MT][4];       // {row g, row g + 8} x {bytes 0, 2 | bytes 1, 3}
+                        uint32_t A[4];       // {row g, row g + 8} x {bytes 0, 2 | bytes 1, 3}
 #pragma unroll
-                        for (uint32_t m = 0; m < MT; ++m)
-#pragma unroll
-                            for (uint32_t h = 0; h < 2u; ++h) {
-                                const uint32_t xv = x[m][h][j], zv = z[m][h][j];
-                                if constexpr (F == kQ6K) {
-                                    const uint32_t mh = up ? 0x03000300u : 0x00300030u, sh = r01 ? 2u : 4u;
-                                    A[m][h] = (xv & mq) | ((zv << sh) & mh);
-                                    A[m][2u + h] = ((xv >> 8) & mq) | ((zv >> (8u - sh)) & mh);
-                                } else {
-                                    A[m][h] = xv & mq;
-                                    A[m][2u + h] = (xv >> 8) & mq;
-                                    if constexpr (F == kQ5K) {
-                                        // bit b of a byte goes to bit 4 of its code (up: 8, the code being 4 bits up)
-                                        const uint32_t mh = up ? 0x01000100u : 0x00100010u, to = up ? 8u : 4u;
-                                        A[m][h] |= (to >= b ? zv << (to - b) : zv >> (b - to)) & mh;
-                                        A[m][2u + h] |= (zv >> (8u + b - to)) & mh;
-                                    }
+                        for (uint32_t h = 0; h < 2u; ++h) {
+                            const uint32_t xv = x[h][j], zv = z[h][j];
+                            if constexpr (F == kQ6K) {
+                                const uint32_t mh = up ? 0x03000300u : 0x00300030u, sh = r01 ? 2u : 4u;
+                                A[h] = (xv & mq) | ((zv << sh) & mh);
+                                A[2u + h] = ((xv >> 8) & mq) | ((zv >> (8u - sh)) & mh);
+                            } else {
+                                A[h] = xv & mq;
+                                A[2u + h] = (xv >> 8) & mq;
+                                if constexpr (F == kQ5K) {
+                                    // bit b of a byte goes to bit 4 of its code (up: 8, the code being 4 bits up)
+                                    const uint32_t mh = up ? 0x01000100u : 0x00100010u, to = up ? 8u : 4u;
+                                    A[h] |= (to >= b ? zv << (to - b) : zv >> (b - to)) & mh;
+                                    A[2u + h] |= (zv >> (8u + b - to)) & mh;
                                 }
                             }
+                        }
                         uint4 v[NT];
 #pragma unroll
                         for (uint32_t n = 0; n < NT; ++n) v[n] = *reinterpret_cast<const uint4*>(bp[n] + (b * kSteps + j) * 64u);
 #pragma unroll
-                        for (uint32_t m = 0; m < MT; ++m)
-#pragma unroll
-                            for (uint32_t n = 0; n < NT; ++n)
-                                if (j == 0u) mma_f16_z(d[m][n], A[m], v[n].x, v[n].y);
-                                else mma_f16(d[m][n], A[m], v[n].x, v[n].y);
-#pragma unroll
-                        for (uint32_t m = 0; m < MT; ++m)
-#pragma unroll
-                            for (uint32_t n = 0; n < NT; ++n) mma_f16(d[m][n], A[m], v[n].z, v[n].w);
-                    }
-#pragma unroll
-                    for (uint32_t m = 0; m < MT; ++m) {
-                        float s[2];
-#pragma unroll
-                        for (uint32_t h = 0; h < 2u; ++h) {
-                            if constexpr (F == kQ40) {
-                                const __half2 v = *reinterpret_cast<const __half2*>(&sw[m][h][p]);
-                                s[h] = up ? __high2float(v) * 0.0625f : __low2float(v);
-                            } else {
-                                s[h] = scale_f(sw[m][h][b >> 2], b & 3u, up != 0u, kBias);
-                            }
-                        }
-#pragma unroll
                         for (uint32_t n = 0; n < NT; ++n)
+                            if (j == 0u) mma_f16_z(d[n], A, v[n].x, v[n].y);
+                            else mma_f16(d[n], A, v[n].x, v[n].y);
 #pragma unroll
-                            for (int i = 0; i < 4; ++i) U[m][n][i] = fmaf(s[i >> 1], d[m][n][i], U[m][n][i]);
+                        for (uint32_t n = 0; n < NT; ++n) mma_f16(d[n], A, v[n].z, v[n].w);
                     }
+                    float s[2];
+#pragma unroll
+                    for (uint32_t h = 0; h < 2u; ++h) {
+                        if constexpr (F == kQ40) {
+                            const __half2 v = *reinterpret_cast<const __half2*>(&sw[h][p]);
+                            s[h] = up ? __high2float(v) * 0.0625f : __low2float(v);
+                        } else {
+                            s[h] = scale_f(sw[h][b >> 2], b & 3u, up != 0u, kBias);
+                        }
+                    }
+#pragma unroll
+                    for (uint32_t n = 0; n < NT; ++n)
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) U[n][i] = fmaf(s[i >> 1], d[n][i], U[n][i]);
                 }
             }
             // ---- scales x block sums
             const uint32_t sel = (t & 1u) ? 0x4342u : 0x4140u;     // bytes 2 (t & 1), + 1 into the halves
             const bool odd_w = (t & 2u) != 0u;
+            uint32_t A[4], dd[2];
 #pragma unroll
-            for (uint32_t m = 0; m < MT; ++m) {
-                uint32_t A[4], dd[2];
-#pragma unroll
-                for (uint32_t h = 0; h < 2u; ++h) {
-                    const uint32_t* rp = reinterpret_cast<const uint32_t*>(rb + (m * 16u + h * 8u) * 24u);
-                    dd[h] = rp[0];
-                    if constexpr (F == kQ6K) {
-                        // int8 scales as f16: 1024 + (sc + 128) by bit pattern, less 1152
-                        const __half2 off = __floats2half2_rn(1152.0f, 1152.0f);
-                        const uint32_t e = __byte_perm(odd_w ? sw[m][h][1] : sw[m][h][0], 0x64646464u, sel);
-                        const uint32_t f = __byte_perm(odd_w ? sw[m][h][3] : sw[m][h][2], 0x64646464u, sel);
-                        A[h] = h2_bits(__hsub2(*reinterpret_cast<const __half2*>(&e), off));
-                        A[2u + h] = h2_bits(__hsub2(*reinterpret_cast<const __half2*>(&f), off));
-                    } else if constexpr (F == kQ40) {
-                        A[h] = A[2u + h] = rp[t];
-                    } else {
-                        A[h] = A[2u + h] = __byte_perm(rp[3u + (t >> 1)], 0u, sel);
-                    }
+            for (uint32_t h = 0; h < 2u; ++h) {
+                const uint32_t* rp = reinterpret_cast<const uint32_t*>(rb + h * 192u);
+                dd[h] = rp[0];
+                if constexpr (F == kQ6K) {
+                    // int8 scales as f16: 1024 + (sc + 128) by bit pattern, less 1152
+                    const __half2 off = __floats2half2_rn(1152.0f, 1152.0f);
+                    const uint32_t e = __byte_perm(odd_w ? sw[h][1] : sw[h][0], 0x64646464u, sel);
+                    const uint32_t f = __byte_perm(odd_w ? sw[h][3] : sw[h][2], 0x64646464u, sel);
+                    A[h] = h2_bits(__hsub2(*reinterpret_cast<const __half2*>(&e), off));
+                    A[2u + h] = h2_bits(__hsub2(*reinterpret_cast<const __half2*>(&f), off));
+                } else if constexpr (F == kQ40) {
+                    A[h] = A[2u + h] = rp[t];
+                } else {
+                    A[h] = A[2u + h] = __byte_perm(rp[3u + (t >> 1)], 0u, sel);
                 }
-                const __half2 dh[2] = {*reinterpret_cast<const __half2*>(&dd[0]), *reinterpret_cast<const __half2*>(&dd[1])};
+            }
+            const __half2 dh[2] = {*reinterpret_cast<const __half2*>(&dd[0]), *reinterpret_cast<const __half2*>(&dd[1])};
 #pragma unroll
-                for (uint32_t n = 0; n < NT; ++n) {
-                    const uint32_t* xs = reinterpret_cast<const uint32_t*>(smem + L.off_xs + (c_u * a.batch + col[n]) * T::kBlocks * 4u);
-                    float M[4];
-                    mma_f16_z(M, A, xs[t], xs[4u + t]);      // Q4 / Q5: A twice along k, the high terms, then the low ones
-                    if constexpr (F == kQ6K) mma_f16(M, A, xs[8u + t], xs[12u + t]);
-                    const float* st = ustep + c_u * a.batch;
-                    const float se = st[even[n]], so = st[odd[n]];
+            for (uint32_t n = 0; n < NT; ++n) {
+                const uint32_t* xs = reinterpret_cast<const uint32_t*>(smem + L.off_xs + (c_u * a.batch + col[n]) * T::kBlocks * 4u);
+                float M[4];
+                mma_f16_z(M, A, xs[t], xs[4u + t]);      // Q4 / Q5: A twice along k, the high terms, then the low ones
+                if constexpr (F == kQ6K) mma_f16(M, A, xs[8u + t], xs[12u + t]);
+                const float* st = ustep + c_u * a.batch;
+                const float se = st[even[n]], so = st[odd[n]];
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const float dg = __low2float(dh[i >> 1]) * 16777216.0f;
-                        float v;
-                        if constexpr (F == kQ40) v = fmaf(U[m][n][i], 16777216.0f, -8.0f * M[i]);
-                        else if constexpr (F == kQ6K) v = dg * fmaf(-32.0f / 16777216.0f, M[i], U[m][n][i]);
-                        else v = dg * U[m][n][i] - __high2float(dh[i >> 1]) * (M[i] * 16777216.0f);
-                        acc[m][n][i] = fmaf((i & 1) ? so : se, v, acc[m][n][i]);
-                    }
+                for (int i = 0; i < 4; ++i) {
+                    const float dg = __low2float(dh[i >> 1]) * 16777216.0f;
+                    float v;
+                    if constexpr (F == kQ40) v = fmaf(U[n][i], 16777216.0f, -8.0f * M[i]);
+                    else if constexpr (F == kQ6K) v = dg * fmaf(-32.0f / 16777216.0f, M[i], U[n][i]);
+                    else v = dg * U[n][i] - __high2float(dh[i >> 1]) * (M[i] * 16777216.0f);
+                    acc[n][i] = fmaf((i & 1) ? so : se, v, acc[n][i]);
                 }
             }
             __syncwarp();
@@ -403,14 +375,12 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 // the (tile, warp) pairs that meet increase by one or two from each partial to the next: slot = tile + warp
                 float* dst = red + (size_t)(c_tile + warp) * kRows * NCOLS;
 #pragma unroll
-                for (uint32_t m = 0; m < MT; ++m)
-#pragma unroll
-                    for (uint32_t n = 0; n < NT; ++n) {
-                        float* to = dst + (row + m * 16u) * NCOLS + n * 8u + 2u * t;
-                        *reinterpret_cast<float2*>(to) = make_float2(acc[m][n][0], acc[m][n][1]);
-                        *reinterpret_cast<float2*>(to + 8u * NCOLS) = make_float2(acc[m][n][2], acc[m][n][3]);
-                        acc[m][n][0] = acc[m][n][1] = acc[m][n][2] = acc[m][n][3] = 0.0f;
-                    }
+                for (uint32_t n = 0; n < NT; ++n) {
+                    float* to = dst + row * NCOLS + n * 8u + 2u * t;
+                    *reinterpret_cast<float2*>(to) = make_float2(acc[n][0], acc[n][1]);
+                    *reinterpret_cast<float2*>(to + 8u * NCOLS) = make_float2(acc[n][2], acc[n][3]);
+                    acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
+                }
                 c_u = 0u;
                 ++c_tile;
             }

@@ -30,6 +30,7 @@ namespace {
 
 using namespace nvf4tc5;
 using namespace tc5::pair;
+using tc5::cluster_sync;
 
 template <uint32_t BN_>
 struct PairCfg {

@@ -1,7 +1,7 @@
 // nvf4_tc5.cuh - what the block-scaled e2m1 tcgen05 kernels share: the tile and
 // pipeline geometry, the shared-memory control block, the scale-cell copy and the
-// kind::mxf4nvf4 MMA issue.  (Used by the dense NVFP4 GEMM and by the grouped
-// MXFP4 expert GEMM.)
+// kind::mxf4nvf4 MMA issue.  (The geometry is the grouped expert GEMM's, moe_tc5.cu; the dense GEMMs, splitk_gemm.cu
+// and nvf4_gemm2.cu, use the scale-cell copy and the MMA issue.)
 #pragma once
 #include "tc5.cuh"
 
@@ -18,9 +18,8 @@ constexpr uint32_t kMaxStages = 4;
 // overlaps it; two slabs per hand-off halve that.
 constexpr uint32_t KS = 2;
 
-// Token tile BN: 128 for prefill widths (3 stages of two slabs); 32 or 64 for decode
-// widths, where the smaller activation box leaves room for 4 stages (8 slabs, 144 KB of
-// weights in flight per SM).
+// Operand columns BN, four term rows per token: 128 for blocks of 32 tokens (3 stages of two slabs); 32 for blocks of 8,
+// where the smaller activation box leaves room for 4 stages (8 slabs, 144 KB of weights in flight per SM).
 template <uint32_t BN>
 struct Cfg {
     static constexpr uint32_t kStages = BN == 128u ? 3u : 4u;

@@ -81,16 +81,15 @@ __device__ __forceinline__ void load_stage(Stage& s, const uint8_t* d0, const ui
 }
 
 // The activation image (built by q4k_act_limbs_kernel in global scratch, copied verbatim into
-// shared memory), NCOLS = 8 NT token columns:
+// shared memory), NCOLS = 8 token columns:
 //   planes : [NCOLS][pitch], pitch = 2K + 64 bytes; per 32-element block 64 bytes =
 //            4 x {8 hi limbs, 8 lo limbs} (lane t of a row reads its 16 bytes at once; the
 //            64 odd bytes per row put the 8 token rows of a quarter-warp read on distinct banks)
 //   ustep  : f32  [K/256][NCOLS]          step of (unit, token)
 //   isl    : int8 [K/256][3][NCOLS][8]    limbs of the eight block sums of (unit, token)
 // followed in shared memory by red : f32 [2][kSlots][kSlices][16][NCOLS] and the copy's mbarrier.
-template <uint32_t NT>
 struct Plan {
-    static constexpr uint32_t NCOLS = NT * 8u;
+    static constexpr uint32_t NCOLS = 8u;
     static __host__ __device__ uint32_t pitch(uint32_t in_dim) { return 2u * in_dim + 64u; }
     static __host__ __device__ size_t off_step(uint32_t in_dim) { return (size_t)NCOLS * pitch(in_dim); }
     static __host__ __device__ size_t off_isl(uint32_t in_dim) { return off_step(in_dim) + (size_t)(in_dim >> 8) * NCOLS * 4u; }
@@ -101,11 +100,10 @@ struct Plan {
 
 // Activations -> the image above, in global memory.  One warp per (token, unit), 8 elements
 // per lane; token columns at and past `batch` are written as zeros.
-template <uint32_t NT>
 __global__ void __launch_bounds__(256)
 q4k_act_limbs_kernel(const float* __restrict__ x, const int8_t* __restrict__ xq, const float* __restrict__ xq_scale,
                      uint8_t* __restrict__ img, uint32_t in_dim, uint32_t batch) {
-    using P = Plan<NT>;
+    using P = Plan;
     constexpr uint32_t NCOLS = P::NCOLS;
     const uint32_t n_unit = in_dim >> 8, pitch = P::pitch(in_dim);
     const uint32_t lane = threadIdx.x & 31u;
@@ -182,11 +180,12 @@ q4k_act_limbs_kernel(const float* __restrict__ x, const int8_t* __restrict__ xq,
 
 // K5: the plane is Q5_K repacked (kquant_more.cu) - per super-block 128 bytes of low nibbles in the Q4_K
 // convention, then 32 bytes of high bits; the codes become 5-bit and everything else is Q4_K's.
-template <uint32_t NT, uint32_t DEPTH, bool EARLY, bool K5>
+constexpr uint32_t DEPTH = 2;   // register stages of a warp
+template <bool K5>
 __global__ void __launch_bounds__(kThreads, 1)
 q4k_batch_i8_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict__ recs, const uint8_t* __restrict__ img,
                     float* __restrict__ y, uint32_t in_dim, uint32_t out_dim, uint32_t batch, unsigned int* err_word) {
-    using P = Plan<NT>;
+    using P = Plan;
     constexpr uint32_t NCOLS = P::NCOLS;
     extern __shared__ __align__(16) uint8_t smem[];
     const uint32_t n_unit = in_dim >> 8, pitch = P::pitch(in_dim);
@@ -260,25 +259,16 @@ q4k_batch_i8_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict_
     const bool landed = tc5::mbar_wait(bar, 0u, ctx, tc5::kErrFullWait, 0x40u);
     if (__syncthreads_or(!landed)) return;  // the copy never landed: error word set, the whole CTA leaves together
 
-    float acc[NT][4];
-#pragma unroll
-    for (uint32_t nt = 0; nt < NT; ++nt)
-#pragma unroll
-        for (int i = 0; i < 4; ++i) acc[nt][i] = 0.0f;
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
     uint32_t c_u = u_lo, c_tile = tile0, iter = 0;
-    // B operand rows of this lane: token column g of each n-tile, its 16 bytes {hi, lo} of a block
+    // B operand rows of this lane: token column g, its 16 bytes {hi, lo} of a block
     const uint8_t* bp = smem + (size_t)g * pitch + t * 16u;
 
     auto compute = [&](const Stage& s, auto&& prefetch) {
-        // EARLY: the loads for the stage consumed by the previous unit go out first (a whole unit
-        // of distance with two stages); otherwise after the main loop, when this unit's weight
-        // registers are dead
-        if (EARLY) prefetch();
-        int uh[NT][4], ul[NT][4];
-#pragma unroll
-        for (uint32_t nt = 0; nt < NT; ++nt)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) uh[nt][i] = ul[nt][i] = 0;
+        // the loads for the stage consumed by the previous unit go out first, a whole unit of distance with two stages
+        // (21.5 us at 4 tokens; three stages with the loads after the main loop, 22.9)
+        prefetch();
+        int uh[4] = {0, 0, 0, 0}, ul[4] = {0, 0, 0, 0};
         const uint8_t* bu = bp + c_u * 512u;
 #pragma unroll
         for (uint32_t b = 0; b < 8u; ++b) {
@@ -293,21 +283,18 @@ q4k_batch_i8_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict_
             }
             const int sc_g = (int)((s.sc[0][b >> 2] >> (8u * (b & 3u))) & 0xffu);
             const int sc_g8 = (int)((s.sc[1][b >> 2] >> (8u * (b & 3u))) & 0xffu);
-#pragma unroll
-            for (uint32_t nt = 0; nt < NT; ++nt) {
-                const uint4 v = *reinterpret_cast<const uint4*>(bu + (size_t)nt * 8u * pitch + b * 64u);
-                int th[4], tl[4];
-                mma_s8_z(th, a0, a1, a2, a3, v.x, v.y);
-                mma_s8_z(tl, a0, a1, a2, a3, v.z, v.w);
-                uh[nt][0] += sc_g * th[0];
-                uh[nt][1] += sc_g * th[1];
-                uh[nt][2] += sc_g8 * th[2];
-                uh[nt][3] += sc_g8 * th[3];
-                ul[nt][0] += sc_g * tl[0];
-                ul[nt][1] += sc_g * tl[1];
-                ul[nt][2] += sc_g8 * tl[2];
-                ul[nt][3] += sc_g8 * tl[3];
-            }
+            const uint4 v = *reinterpret_cast<const uint4*>(bu + b * 64u);
+            int th[4], tl[4];
+            mma_s8_z(th, a0, a1, a2, a3, v.x, v.y);
+            mma_s8_z(tl, a0, a1, a2, a3, v.z, v.w);
+            uh[0] += sc_g * th[0];
+            uh[1] += sc_g * th[1];
+            uh[2] += sc_g8 * th[2];
+            uh[3] += sc_g8 * th[3];
+            ul[0] += sc_g * tl[0];
+            ul[1] += sc_g * tl[1];
+            ul[2] += sc_g8 * tl[2];
+            ul[3] += sc_g8 * tl[3];
         }
         // min term: A = m[row][block] in k-slots 0..7 (lanes t = 0, 1), B = one limb of the block sums
         const uint32_t am0 = t < 2u ? s.mw[0] : 0u, am1 = t < 2u ? s.mw[1] : 0u;
@@ -315,22 +302,18 @@ q4k_batch_i8_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict_
         const __half2 dh1 = *reinterpret_cast<const __half2*>(&s.dd[1]);
         const float d_g = __low2float(dh0), dmin_g = __high2float(dh0);
         const float d_g8 = __low2float(dh1), dmin_g8 = __high2float(dh1);
-        if (!EARLY) prefetch();
+        const uint8_t* ip = isl + ((size_t)(c_u * 3u) * NCOLS + g) * 8u + (t & 1u) * 4u;
+        int m0[4], m1[4], m2[4];
+        mma_s8_z(m0, am0, am1, 0u, 0u, *reinterpret_cast<const uint32_t*>(ip), 0u);
+        mma_s8_z(m1, am0, am1, 0u, 0u, *reinterpret_cast<const uint32_t*>(ip + NCOLS * 8u), 0u);
+        mma_s8_z(m2, am0, am1, 0u, 0u, *reinterpret_cast<const uint32_t*>(ip + 2u * NCOLS * 8u), 0u);
+        const float2 stp = *reinterpret_cast<const float2*>(ustep + c_u * NCOLS + 2u * t);
 #pragma unroll
-        for (uint32_t nt = 0; nt < NT; ++nt) {
-            const uint8_t* ip = isl + ((size_t)(c_u * 3u) * NCOLS + nt * 8u + g) * 8u + (t & 1u) * 4u;
-            int m0[4], m1[4], m2[4];
-            mma_s8_z(m0, am0, am1, 0u, 0u, *reinterpret_cast<const uint32_t*>(ip), 0u);
-            mma_s8_z(m1, am0, am1, 0u, 0u, *reinterpret_cast<const uint32_t*>(ip + NCOLS * 8u), 0u);
-            mma_s8_z(m2, am0, am1, 0u, 0u, *reinterpret_cast<const uint32_t*>(ip + 2u * NCOLS * 8u), 0u);
-            const float2 stp = *reinterpret_cast<const float2*>(ustep + c_u * NCOLS + nt * 8u + 2u * t);
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const float mainv = fmaf((float)uh[nt][i], 256.0f, (float)ul[nt][i]);
-                const float minv = (float)(m0[i] + 256 * m1[i] + 65536 * m2[i]);
-                const float d = i < 2 ? d_g : d_g8, dm = i < 2 ? dmin_g : dmin_g8;
-                acc[nt][i] = fmaf((i & 1) ? stp.y : stp.x, d * mainv - dm * minv, acc[nt][i]);
-            }
+        for (int i = 0; i < 4; ++i) {
+            const float mainv = fmaf((float)uh[i], 256.0f, (float)ul[i]);
+            const float minv = (float)(m0[i] + 256 * m1[i] + 65536 * m2[i]);
+            const float d = i < 2 ? d_g : d_g8, dm = i < 2 ? dmin_g : dmin_g8;
+            acc[i] = fmaf((i & 1) ? stp.y : stp.x, d * mainv - dm * minv, acc[i]);
         }
 
         // ---- end of this warp's K slice for the tile: the four slices meet in shared memory
@@ -338,23 +321,16 @@ q4k_batch_i8_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict_
             c_u = u_lo;
             float* rbuf = red + ((size_t)(iter & 1u) * kSlots + slot) * (kSlices * 16u * NCOLS);
             float* mine = rbuf + (size_t)slice * 16u * NCOLS;
-#pragma unroll
-            for (uint32_t nt = 0; nt < NT; ++nt) {
-                *reinterpret_cast<float2*>(mine + g * NCOLS + nt * 8u + 2u * t) = make_float2(acc[nt][0], acc[nt][1]);
-                *reinterpret_cast<float2*>(mine + (g + 8u) * NCOLS + nt * 8u + 2u * t) = make_float2(acc[nt][2], acc[nt][3]);
-                acc[nt][0] = acc[nt][1] = acc[nt][2] = acc[nt][3] = 0.0f;
-            }
+            *reinterpret_cast<float2*>(mine + g * NCOLS + 2u * t) = make_float2(acc[0], acc[1]);
+            *reinterpret_cast<float2*>(mine + (g + 8u) * NCOLS + 2u * t) = make_float2(acc[2], acc[3]);
+            acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
             bar_sync(1u + slot, kSlices * 32u);
-            // 128 threads, 16 rows x NCOLS tokens: thread -> (row = idx % 16, token = idx / 16 [+ 8])
+            // 128 threads, 16 rows x NCOLS tokens: thread -> (row = idx % 16, token = idx / 16)
             const uint32_t idx = slice * 32u + lane;
-            const uint32_t row = c_tile * 16u + (idx & 15u);
-#pragma unroll
-            for (uint32_t nt = 0; nt < NT; ++nt) {
-                const uint32_t tok = nt * 8u + (idx >> 4);
-                const uint32_t o = (idx & 15u) * NCOLS + tok;
-                const float v = (rbuf[o] + rbuf[16u * NCOLS + o]) + (rbuf[32u * NCOLS + o] + rbuf[48u * NCOLS + o]);
-                if (row < out_dim && tok < batch) y[(size_t)tok * out_dim + row] = v;
-            }
+            const uint32_t row = c_tile * 16u + (idx & 15u), tok = idx >> 4;
+            const uint32_t o = (idx & 15u) * NCOLS + tok;
+            const float v = (rbuf[o] + rbuf[16u * NCOLS + o]) + (rbuf[32u * NCOLS + o] + rbuf[48u * NCOLS + o]);
+            if (row < out_dim && tok < batch) y[(size_t)tok * out_dim + row] = v;
             c_tile += tile_stride;
             ++iter;
         }
@@ -381,21 +357,21 @@ __device__ __align__(1024) uint8_t g_q4k_img[kImgLanes][kImgSliceBytes];
 PDK_SLICE_TABLE(img_slice_table, g_q4k_img, kImgSliceBytes, kImgLanes);
 uint8_t* img_slice(cudaStream_t st) { return img_slice_table.slice(st); }
 
-template <uint32_t NT, uint32_t DEPTH, bool EARLY, bool K5>
+template <bool K5>
 int launch(const void* data, const void* recs, const float* x, const int8_t* xq, const float* xq_scale, float* y,
            uint32_t in_dim, uint32_t out_dim, uint32_t batch, cudaStream_t st) {
-    using P = Plan<NT>;
+    using P = Plan;
     const uint32_t n_unit = in_dim >> 8;
     if ((in_dim & 255u) != 0u || n_unit < kSlices) return -1;
     const size_t smem = P::total(in_dim);
     if (smem > 227u * 1024u) return -1;
     uint8_t* img = img_slice(st);
     if (img == nullptr) return -1;
-    auto kern = q4k_batch_i8_kernel<NT, DEPTH, EARLY, K5>;
+    auto kern = q4k_batch_i8_kernel<K5>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const uint32_t tasks = P::NCOLS * n_unit;
-    if (int rc = pdk_launch_pdl(q4k_act_limbs_kernel<NT>, dim3((tasks + 7u) / 8u), dim3(256), 0, st, x, xq, xq_scale, img,
+    if (int rc = pdk_launch_pdl(q4k_act_limbs_kernel, dim3((tasks + 7u) / 8u), dim3(256), 0, st, x, xq, xq_scale, img,
                                 in_dim, batch))
         return rc;
     const uint32_t n_tiles = (out_dim + 15u) / 16u;
@@ -417,14 +393,12 @@ int launch(const void* data, const void* recs, const float* x, const int8_t* xq,
 int pdk_q4k_batch_i8(const void* data, const void* scales, const float* x, const int8_t* xq, const float* xq_scale,
                      float* y, uint32_t in_dim, uint32_t out_dim, uint32_t batch, cudaStream_t st) {
     if (batch == 0u || batch > 8u) return -1;
-    // Two stages with the loads issued first measured the same as three stages with the loads
-    // issued after the main loop (21.5 against 22.9 us at 4 tokens).
-    return launch<1, 2, true, false>(data, scales, x, xq, xq_scale, y, in_dim, out_dim, batch, st);
+    return launch<false>(data, scales, x, xq, xq_scale, y, in_dim, out_dim, batch, st);
 }
 
 // The same for a Q5_K plane (f32 activations).
 int pdk_q5k_batch_i8(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim, uint32_t out_dim,
                      uint32_t batch, cudaStream_t st) {
     if (batch == 0u || batch > 8u) return -1;
-    return launch<1, 2, true, true>(data, scales, x, nullptr, nullptr, y, in_dim, out_dim, batch, st);
+    return launch<true>(data, scales, x, nullptr, nullptr, y, in_dim, out_dim, batch, st);
 }

@@ -32,6 +32,10 @@
 
 namespace {
 
+using tc5::cluster_addr;
+using tc5::cluster_sync;
+using tc5::st_cluster;
+
 enum Kind : int { kFp8 = 0, kNvf4 = 1 };
 
 constexpr uint32_t BM = 128, BKB = 128;
@@ -81,17 +85,6 @@ struct Args {
     unsigned int* err;
 };
 
-__device__ __forceinline__ void cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t cluster_addr(uint32_t saddr, uint32_t rank) {
-    uint32_t a;
-    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(saddr), "r"(rank));
-    return a;
-}
-__device__ __forceinline__ void st_cluster(uint32_t addr, float v) {
-    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
 // A store that may be past the batch.  Predicated, not branched around: with `if (i < left)` in front of it the compiler
 // leaves a branch per store, about 50 cycles each, one microsecond for 32 tokens.
 __device__ __forceinline__ void store_if(float* p, float v, bool on) {

@@ -136,6 +136,7 @@ template <int kKind>
 __global__ void __launch_bounds__(kProbeThreads)
 tc5_issue_probe_pair_kernel(uint32_t n_mma, unsigned int* err, unsigned long long* cycles) {
     using namespace tc5::pair;
+    using tc5::cluster_sync;
     extern __shared__ uint8_t probe_raw[];
     __shared__ uint64_t done_bar;
     __shared__ uint32_t tmem_slot;
