@@ -62,10 +62,8 @@ __device__ __forceinline__ uint32_t nvf4_codes4(const float4& v, float recip) {
 // One thread per 8 elements (half a block); the lane pair closes the 16-element amax.
 __global__ void quantize_nvf4_kernel(const float* __restrict__ x, uint8_t* __restrict__ q,
                                      uint8_t* __restrict__ scale, uint32_t n) {
-    // The wait comes first: the GEMM behind this kernel reads its weight plane ahead of its own wait, so it may start
-    // only when all that was launched before the quantizer (a load's repack or scale tiler, say) is complete and visible
-    pdk_pdl_wait();
     pdk_pdl_launch_dependents();
+    pdk_pdl_wait();
     const uint32_t i = (blockIdx.x * 256u + threadIdx.x) * 8u;
     if (i >= n) return;  // n % 32 == 0: lane pairs leave together
     const float4 a = *reinterpret_cast<const float4*>(x + i);
@@ -208,6 +206,7 @@ __global__ void nvf4_tile_scales_kernel(const uint8_t* __restrict__ scale, uint3
     uint32_t v = 0u;
     if (row < out_dim) v = *reinterpret_cast<const uint32_t*>(scale + (size_t)row * kb16 + kb * 16u + j * 4u);
     tiled[w] = v;
+    pdk_plane_written();
 }
 
 // W4A16 decode GEMV, f32 activations: a warp per output row, 8 rows per CTA.

@@ -48,8 +48,8 @@ def test_nvfp4(pack, m, n, k, out):
 
 def test_nvfp4_first_call_behind_its_load(pack):
     """Scale tiler, quantizer and GEMM on fresh buffers with nothing between them: the GEMM requests weights and scale
-    records ahead of its wait, and the quantizer in front of it must have held it back until the tiler's records are
-    complete.  Against the same calls with a synchronisation behind each; same bytes."""
+    records ahead of its wait, behind a quantizer that releases it early, so the tiler makes its stores visible before its
+    blocks leave.  Against the same calls with a synchronisation behind each; same bytes."""
     k, n, m = 2048, 640, 5
     g = torch.Generator(device="cuda").manual_seed(5)
     x = torch.randn(m * k, device="cuda", generator=g)
