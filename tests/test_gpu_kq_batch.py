@@ -57,6 +57,27 @@ def test_edges(pack, name, k, n, batch):
         assert not y[2].any()
 
 
+@pytest.mark.parametrize("name", sorted(FORMATS))
+@pytest.mark.parametrize("batch", [5, 12])
+def test_one_token_that_is_not_finite(pack, name, batch):
+    """An infinite and a NaN activation reach their own token alone: the other tokens keep their bits."""
+    k, n = 1280, 40                       # an odd super-block count: no other kernel takes 12 tokens
+    _, d_data, d_sc, dtype = planes(pack, name, k, n, 350)
+    x = oracle.fill_normal(batch * k, 351 + batch, 1.0).reshape(batch, k)
+    outs = []
+    for bad in (False, True):
+        if bad:
+            x[1, 3], x[3, 700] = np.inf, np.nan
+        y = torch.full((batch, n), 7.0, dtype=torch.float32, device="cuda")
+        pack.call("pdk_kquant_gemm_f32", d_data, d_sc, dev_f32(x.reshape(-1)), y, k, n, batch, dtype)
+        torch.cuda.synchronize()
+        outs.append(y)
+    assert pack.device_error() == 0
+    keep = [t for t in range(batch) if t not in (1, 3)]
+    assert torch.equal(outs[0][keep], outs[1][keep]) and torch.isfinite(outs[0]).all()
+    assert not torch.isfinite(outs[1][[1, 3]]).any()
+
+
 @pytest.mark.parametrize("name,batch", [("q6_k", 8), ("q6_k", 12), ("q5_k", 16)])
 def test_several_rounds_of_a_cluster(pack, name, batch):
     """5120 x 25600: more partial tiles than shared memory holds at 12 and 16 tokens, so that a ring refills where the
