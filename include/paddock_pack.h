@@ -17,10 +17,10 @@
  *   - the pack never allocates, synchronizes or creates streams.
  *   - weight planes (data, scales, tiled scale records) are load-time operands: decode and GEMM kernels
  *     are launched as programmatic dependents and may read a plane ahead of their wait for the launch
- *     before them.  Planes that this pack's repack, bf16_to_f8row and scale-tiling launchers write may be
- *     read by the next call on the stream; a host that writes a plane with kernels of its own, or
- *     copies into one between calls, puts an event wait or a synchronisation between that and
- *     the next call that reads it.
+ *     before them.  The pack's repack, bf16_to_f8row and scale-tiling launchers are ordinary launches,
+ *     whose blocks have left before a later call of the stream starts.  A host that writes a plane with
+ *     kernels of its own, or copies into one between calls, puts an event wait or a synchronisation
+ *     between that and the next call that reads it.
  *
  * The launchers are also exported by name (pd_*), with the signatures the
  * reference gives the same names in packs/cuda/src/abi.cuh, so a host that

@@ -83,8 +83,6 @@ pdk_q8_0_repack16_kernel(const uint8_t* __restrict__ src, uint4* __restrict__ ds
         dst_data[b0 * 2u + i] = o;
     }
     for (uint32_t b = threadIdx.x; b < n; b += 256u) dst_scale[b0 + b] = reinterpret_cast<const uint16_t*>(raw)[b * 17u];
-    __syncthreads();
-    if (threadIdx.x == 0u) pdk_plane_written();
 }
 
 // Any alignment the slot takes: eight threads per block, one 4-byte word of the int8 payload each (read as
@@ -100,7 +98,6 @@ __global__ void pdk_q8_0_repack_kernel(const uint8_t* __restrict__ src, uint32_t
     uint32_t lo = s[1u + 2u * w], hi = s[2u + 2u * w];
     dst_data[b * 8u + w] = lo | (hi << 16);
     if (w == 0) dst_scale[b] = s[0];
-    pdk_plane_written();
 }
 
 PDK_EXPORT int pd_q8_0_repack(const void* src, void* dst_data, void* dst_scale, uint64_t n_blocks, void* stream) {

@@ -110,19 +110,16 @@ q4k_repack16_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst_data,
         const uint32_t at = i * kRepackThreads + threadIdx.x;
         if (s0 + (at >> 3) < n_super) dst_data[s0 * 8u + at] = v[i];
     }
-    if (mine) {
-        // scale bytes 0..3 | 4..7 | 8..11 = y | z | w: pairs 0..3 are the low six bits of the first two words,
-        // pairs 4..7 the nibbles of the third under the top two bits of those words
-        const uint32_t sc_lo = head.y & 0x3f3f3f3fu, m_lo = head.z & 0x3f3f3f3fu;
-        const uint32_t sc_hi = (head.w & 0x0f0f0f0fu) | ((head.y >> 2) & 0x30303030u);
-        const uint32_t m_hi = ((head.w >> 4) & 0x0f0f0f0fu) | ((head.z >> 2) & 0x30303030u);
-        uint2* rec = dst_scales + b * 3u;
-        rec[0] = make_uint2(head.x, sc_lo);
-        rec[1] = make_uint2(sc_hi, m_lo);
-        rec[2] = make_uint2(m_hi, 0u);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0u) pdk_plane_written();
+    if (!mine) return;
+    // scale bytes 0..3 | 4..7 | 8..11 = y | z | w: pairs 0..3 are the low six bits of the first two words,
+    // pairs 4..7 the nibbles of the third under the top two bits of those words
+    const uint32_t sc_lo = head.y & 0x3f3f3f3fu, m_lo = head.z & 0x3f3f3f3fu;
+    const uint32_t sc_hi = (head.w & 0x0f0f0f0fu) | ((head.y >> 2) & 0x30303030u);
+    const uint32_t m_hi = ((head.w >> 4) & 0x0f0f0f0fu) | ((head.z >> 2) & 0x30303030u);
+    uint2* rec = dst_scales + b * 3u;
+    rec[0] = make_uint2(head.x, sc_lo);
+    rec[1] = make_uint2(sc_hi, m_lo);
+    rec[2] = make_uint2(m_hi, 0u);
 }
 
 // Any alignment the slot takes: one warp per super-block, lane l moves one 4-byte word of the nibble payload
@@ -146,7 +143,6 @@ __global__ void q4k_repack_kernel(const uint8_t* __restrict__ src, uint8_t* __re
     } else if (lane < 16u) {
         rec[8u + lane] = 0;             // pad bytes 20..23
     }
-    pdk_plane_written();
 }
 
 // ===========================================================================

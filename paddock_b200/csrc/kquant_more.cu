@@ -150,7 +150,6 @@ __global__ void kq_repack_kernel(const uint8_t* __restrict__ src, uint8_t* __res
         if (l < 8u) { rec[2u * l] = s[l * 18u]; rec[2u * l + 1u] = s[l * 18u + 1u]; }
         if (l >= 16u && l < 24u) rec[l] = 0;
     }
-    pdk_plane_written();
 }
 
 // ---------------------------------------------------------------- GEMV / small-batch GEMM, f32

@@ -195,7 +195,7 @@ __global__ void nvf4_dequant_kernel(const uint8_t* __restrict__ data, const uint
 //   byte l*16 + c*4 + b  of cell j  =  scale[rt*128 + c*32 + l][kb*16 + j*4 + b]
 // (rows past out_dim read as 0).  One thread per 4-byte word of the output.
 __global__ void nvf4_tile_scales_kernel(const uint8_t* __restrict__ scale, uint32_t* __restrict__ tiled,
-                                        uint32_t in_dim, uint32_t out_dim, uint64_t n_words) {
+                                        uint32_t in_dim, uint32_t out_dim, uint64_t n_words, bool plane) {
     const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= n_words) return;
     const uint32_t n_slab = in_dim >> 8, kb16 = in_dim >> 4;
@@ -206,7 +206,9 @@ __global__ void nvf4_tile_scales_kernel(const uint8_t* __restrict__ scale, uint3
     uint32_t v = 0u;
     if (row < out_dim) v = *reinterpret_cast<const uint32_t*>(scale + (size_t)row * kb16 + kb * 16u + j * 4u);
     tiled[w] = v;
-    pdk_plane_written();
+    // Records of a weight plane: the GEMM requests its first ones ahead of its wait and starts behind a quantizer that releases
+    // it early, when these blocks have left but nothing has waited for this grid's flush.  So they leave with their stores visible.
+    if (plane) asm volatile("fence.acq_rel.gpu;\n\tfence.proxy.async.global;" ::: "memory");
 }
 
 // W4A16 decode GEMV, f32 activations: a warp per output row, 8 rows per CTA.
@@ -333,17 +335,17 @@ PDK_EXPORT int pd_nvf4_dequant(const void* data, const void* scale, float scale2
 }
 
 // slot 853, packs/cuda/src/gemm/dense_nvf4_tc5.cuh:845-861,981-994
-PDK_EXPORT int pd_nvf4_tc5_tile_scales(const void* scale, void* tiled, uint32_t in_dim, uint32_t out_dim,
-                                       void* stream) {
+int pdk_nvf4_tile_scales(const void* scale, void* tiled, uint32_t in_dim, uint32_t out_dim, bool plane, cudaStream_t st) {
     if (out_dim == 0 || in_dim == 0) return 0;
     if ((in_dim & 255u) != 0u || !pdk_aligned(scale, 4) || !pdk_aligned(tiled, 16)) return cudaErrorInvalidValue;
     const uint64_t n_words = (uint64_t)((out_dim + 127u) / 128u) * (in_dim >> 8) * 512u;
     const uint64_t blocks = (n_words + 255u) / 256u;
     if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
-    nvf4_tile_scales_kernel<<<(uint32_t)blocks, 256, 0, (cudaStream_t)stream>>>((const uint8_t*)scale,
-                                                                                (uint32_t*)tiled, in_dim, out_dim,
-                                                                                n_words);
+    nvf4_tile_scales_kernel<<<(uint32_t)blocks, 256, 0, st>>>((const uint8_t*)scale, (uint32_t*)tiled, in_dim, out_dim, n_words, plane);
     return pdk_launch_status();
+}
+PDK_EXPORT int pd_nvf4_tc5_tile_scales(const void* scale, void* tiled, uint32_t in_dim, uint32_t out_dim, void* stream) {
+    return pdk_nvf4_tile_scales(scale, tiled, in_dim, out_dim, true, (cudaStream_t)stream);
 }
 
 // slot 394, packs/cuda/src/quant/nvf4.cuh:4436-4779

@@ -18,6 +18,8 @@ int pdk_nvf4_gemm_pair_f32(const void*, const void*, const void*, const void*, c
 int pdk_nvf4_gemm_pair_bf16(const void*, const void*, const void*, const void*, const void*, void*, float, uint32_t, uint32_t,
                             uint32_t, cudaStream_t);
 
+// nvf4_elem.cu; plane: the records are a weight plane's
+int pdk_nvf4_tile_scales(const void* scale, void* tiled, uint32_t in_dim, uint32_t out_dim, bool plane, cudaStream_t st);
 // splitk_gemm.cu
 bool pdk_prefer_pair(uint32_t batch, uint32_t out_dim, uint32_t row_bytes, bool nvf4);
 int pdk_nvf4_gemm_splitk(const void* data, const void* scale_tiled, const void* bias, const void* xq, const void* xs, void* y,
@@ -40,7 +42,8 @@ bool pair_enabled() {
 // K-elements costs the L2 as many requests again as the operand boxes, one 2 KB bulk copy per slab does
 // not.  The buffer lives in the library (the pack allocates nothing at run time); one slice per stream,
 // for the first kXsfLanes streams that make such calls - further streams, and calls too large for a
-// slice, take the K-split kernel, which gathers.
+// slice, take the K-split kernel's whole tiles, which bring the scales through registers: 8192 tokens, K = 17408, N = 4096
+// (9.4 MB of records) 300 us, 4096 tokens, K = N = 5120 66 us where the pair kernel takes 59.
 constexpr size_t kXsfSliceBytes = 8u << 20;  // batch * in_dim / 16 bytes, padded to 128 tokens
 constexpr int kXsfLanes = 2;
 __device__ __align__(1024) uint8_t g_xsf_scratch[kXsfLanes][kXsfSliceBytes];
@@ -62,7 +65,7 @@ int launch(const void* data, const void* scale_tiled, const void* bias, const vo
     if (pair_enabled() && pdk_prefer_pair(batch, out_dim, in_dim >> 1, true)) {
         const size_t need = (size_t)((batch + 127u) / 128u) * (in_dim >> 8) * kSfBytes;
         if (uint8_t* xt = xsf_slice(st, need)) {
-            if (int rc = pd_nvf4_tc5_tile_scales(xs, xt, in_dim, batch, st)) return rc;
+            if (int rc = pdk_nvf4_tile_scales(xs, xt, in_dim, batch, false, st)) return rc;
             if constexpr (sizeof(TO) == 4) return pdk_nvf4_gemm_pair_f32(data, scale_tiled, bias, xq, xt, y, scale2, in_dim, out_dim, batch, st);
             else return pdk_nvf4_gemm_pair_bf16(data, scale_tiled, bias, xq, xt, y, scale2, in_dim, out_dim, batch, st);
         }

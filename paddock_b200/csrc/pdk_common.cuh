@@ -52,12 +52,6 @@ __device__ __forceinline__ void pdk_pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 __device__ __forceinline__ void pdk_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// The end of a kernel that writes weight planes.  Readers request their first weights, through TMA too, ahead of that wait.  They start
-// when this grid's blocks have left, but behind a kernel that releases its dependents early nothing waits for this grid's
-// flush: its stores are made visible here, before the blocks leave.  One thread behind a barrier does it for its block.
-__device__ __forceinline__ void pdk_plane_written() {
-    asm volatile("fence.acq_rel.gpu;\n\tfence.proxy.async.global;" ::: "memory");
-}
 
 __device__ __forceinline__ float pdk_warp_sum(float v) {
 #pragma unroll

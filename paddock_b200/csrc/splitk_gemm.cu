@@ -11,7 +11,8 @@
 // plane that HBM delivers in 4), so K is split as well: a tile is 128 channels x BN tokens, and a
 // cluster of S CTAs shares it, each summing every S-th part of K.  The partial accumulators meet
 // through distributed shared memory and are added in rank order: same sum whatever the timing, no
-// scratch, no zeroing, no second launch.
+// scratch, no zeroing, no second launch.  Where K is short or the tokens are many the meeting costs more
+// than the split saves: one CTA takes the tile and stores it from tensor memory (launch_bn has the line).
 //
 // Two CTAs share an SM (about 100 KB of stages and at most half the tensor memory each): while one meets
 // its cluster and stores, the other streams, and a CTA's start-up (barriers, tensor memory, first boxes)
