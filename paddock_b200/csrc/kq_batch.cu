@@ -22,9 +22,9 @@
 // tile that it touched, and the partials meet once per round (as many tiles as shared memory holds partials of; one, mostly), in a fixed order, across the cluster in distributed
 // shared memory: the same sum whatever the timing, no scratch, no zeroing of y, one launch.
 //
-// Measured on a B200 (us, before -> here).  Q6_K, K = 17408, N = 5003: 57.6 -> 28.4 at 2 tokens, 115 -> 31.7 at 4, 229 -> 32.6 at 8 (the
-// activations did not fit one CTA: a GEMV per token); K = 5120, N = 25600: 41.0 -> 33 at 2, 41.4 -> 38 at 8, 82.7 -> 76 at 16;
-// N = 1024: 15.7 -> 7.0 at 2, 31 -> 11.5 at 16.  Q4_K, K = 17408, N = 5120: 80.9 -> 24.4 at 2.  What bounds it now: the shared
+// Measured on a B200 (us, before -> here).  Q6_K, K = 17408, N = 5003: 56.4 -> 28.4 at 2 tokens, 114 -> 28.8 at 4, 226 -> 34.1 at 8 (the
+// activations did not fit one CTA: a GEMV per token); K = 5120, N = 25600: 40.9 -> 33 at 2, 41.3 -> 38 at 8, 82.5 -> 76 at 16;
+// N = 1024: 15.2 -> 6.5 at 2, 30 -> 10.1 at 16.  Q4_K, K = 17408, N = 5120: 81.1 -> 23.7 at 2.  What bounds it now: the shared
 // memory pipe (118 wavefronts per unit, 64 of them the activation fragments: 13 of the 25 us of Q4_K, K = 5120, N = 25600) and
 // issue slots (450 instructions per unit).  Tiles of 32 rows halve the fragments but double the ring's stages, so that
 // fewer fit: 24.7 us at 1 token, but 45 at 8 and no plan at all for Q6_K, not kept.

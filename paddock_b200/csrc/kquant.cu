@@ -274,7 +274,7 @@ bool kq_beats_i8(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
 // The kernel that a pass over `batch` tokens asks first.  Q4_0 up to 8 tokens: kq_batch against the tcgen05 kernel (which costs the same
 // at 4 and at 16 tokens) is 0.4 % off the faster one over 180 random shapes, up to 5 times faster, at most 18 % slower (K = 5120,
 // N = 25600: 26.4 / 29.2 us at 4 tokens; N = 9472: 16.2 / 15.2 at 8).  Q5_K from 9 tokens on: two passes of the integer kernel would
-// be faster on wide planes (K = 5120, N = 25600, 16 tokens: 51.6 against 65.8 us), but kq_batch keeps 22 activation bits.
+// be faster on wide planes (K = 5120, N = 25600, 16 tokens: 51.6 against 64.5 us), but kq_batch keeps 22 activation bits.
 Route batch_route(uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t dtype) {
     const uint32_t from = dtype == PDK_KQ_Q4K ? tc5_min_tokens() : dtype == PDK_KQ_Q4_0 && tc5_min_tokens() != 0u ? 9u : 0u;
     if (from != 0u && batch >= from) return kRouteTc5;
