@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(256) moe_route_prep_f4_kernel(const PrepArgs a
     __syncthreads();
     if (warp == 0u) {
         const bool valid = lane < npairs;
-        const uint32_t e = valid ? s_idx[lane] : 0xfffffff0u + lane;     // idle lanes: distinct keys that match nobody
+        const uint32_t e = valid ? s_idx[lane] : 0x80000000u + lane;     // idle lanes: distinct keys that match nobody
         const uint32_t grp = __match_any_sync(0xffffffffu, e);
         const uint32_t rank = __popc(grp & ((1u << lane) - 1u)), cnt = __popc(grp);
         const uint32_t nblk = (valid && rank == 0u) ? (cnt + a.bm - 1u) / a.bm : 0u;   // counted once, by the group's first lane

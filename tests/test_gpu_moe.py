@@ -138,6 +138,7 @@ def test_moe_block_tensor_core_path_matches_oracle(pack, tokens, n_expert, k, em
     (3, 16, 4, 2880, 8),
     (5, 8, 2, 512, 8),
     (2, 512, 8, 256, 32),
+    (8, 2, 2, 256, 8),       # whole blocks of two experts, half the lanes without a pair
 ])
 @pytest.mark.parametrize("natural", [False, True])
 def test_route_and_prepare_in_one_launch_equals_the_three_calls(pack, tokens, n_expert, k, embd, bm, natural):
