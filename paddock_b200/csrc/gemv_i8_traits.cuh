@@ -496,6 +496,7 @@ __device__ __forceinline__ void limb_load8(const float* __restrict__ x, const in
         for (int i = 0; i < 8; ++i) v[i] = (float)(int8_t)((i < 4 ? q.x >> (8 * i) : q.y >> (8 * (i - 4))) & 0xff) * s;
     }
 }
+template <uint32_t kBlock = 32u>
 __device__ __forceinline__ void limb_store8(const float (&v)[8], uint32_t grp, uint8_t* xs_hi, uint8_t* xs_lo,
                                             float2* xmeta) {
     float amax = 0.0f;
@@ -529,6 +530,10 @@ __device__ __forceinline__ void limb_store8(const float (&v)[8], uint32_t grp, u
     *reinterpret_cast<uint2*>(xs_hi + (size_t)grp * 8u) = hi;
     *reinterpret_cast<uint2*>(xs_lo + (size_t)grp * 8u) = lo;
     isum += __shfl_xor_sync(0xffffffffu, isum, 1);
+    if constexpr (kBlock == 16u) {      // the sums of 16 elements, the step of their 32
+        if ((grp & 1u) == 0u) xmeta[grp >> 1] = make_float2(step, step * (float)isum);
+        return;
+    }
     isum += __shfl_xor_sync(0xffffffffu, isum, 2);
     if ((grp & 3u) == 0u) xmeta[grp >> 2] = make_float2(step, step * (float)isum);
 }

@@ -235,7 +235,7 @@ gemv_q6k_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict__ re
 
 // Returns 0 / a cudaError_t, or -1 when the shape is outside the kernel's plan (K not a multiple
 // of 256, fewer than four super-blocks per row, activations too long for shared memory).
-int pdk_q6k_gemv_i8(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim, uint32_t out_dim,
+int pdk_q6k_gemv_i8_regs(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim, uint32_t out_dim,
                     cudaStream_t st) {
     const uint32_t n_unit = in_dim >> 8;
     if ((in_dim & 255u) != 0u || n_unit < kSlices) return -1;

@@ -34,6 +34,7 @@
 // leaves waits (bounded again) for the copies it still has in flight.
 #include <cstdlib>
 
+#include "cluster_caps.cuh"
 #include "gemv_i8_traits.cuh"
 #include "tc5.cuh"
 
@@ -41,17 +42,22 @@ namespace {
 
 using namespace gemv_i8;
 
-constexpr uint32_t kMaxWarps = 12;
+constexpr uint32_t kMaxWarps = 12;                      // with 168 registers a thread
+constexpr uint32_t kManyWarps = 20, kMaxTeams = 10;     // with 96
 constexpr uint32_t kMaxDepth = 4;
-constexpr uint32_t kRedBufs = 8;
+constexpr uint32_t kRedBufs = 8;                        // of a team
 constexpr uint32_t kSmemMax = 232448;  // 227 KB per CTA on sm_100
 constexpr uint32_t kBoxBytes = 2048;   // 16 rows x 128 bytes
 
 struct RingPlan {
-    uint32_t W;          // warps
+    uint32_t W;          // warps of a team
+    uint32_t teams;      // teams of a CTA: tile i of the CTA is team i % teams'
     uint32_t D;          // stages per warp
-    uint32_t invariant;  // W == pairs per row: a warp's pair never changes
-    uint32_t off_xmeta, off_red, off_bar, off_rec, off_data, smem_bytes;
+    uint32_t split;      // CTAs of a cluster, which share tiles and split the pairs of a row
+    uint32_t clusters;
+    uint32_t invariant;  // W >= pairs of a row's part: a warp's pair never changes
+    uint32_t k_part;     // elements of a row that a CTA's activations cover, at most
+    uint32_t off_xmeta, off_red, off_recv, off_bar, off_rec, off_data, smem_bytes;
 };
 
 enum : unsigned int { kErrRingFull = 0x11, kErrRingFold = 0x13, kErrRingDrain = 0x14, kErrRingFree = 0x15 };
@@ -73,7 +79,9 @@ __device__ __forceinline__ uint32_t word4(const uint4& v, uint32_t i) { return i
 // load_ring arguments: `box` = the unit's first data box, o0 / o1 = swz(g, 2t) / swz(g, 2t + 1)
 // (rows g + 8 lie 1024 bytes further), `rec` = row g's record of the unit (row g + 8: 8 box rows on).
 struct RQ4K : Q4K {
-    static constexpr uint32_t kDataBoxes = 1;
+    static constexpr uint32_t kDataBoxes = 1, kHighBytes = 0, kPasses = 2, kSub = 4, kBlock = 32;
+    static constexpr bool kMany = true;
+    static constexpr float kStepCost = 0.055f, kManyCost = 0.05f, kRegsCost = 1.05f;   // make_plan
     // pass p of lane t feeds block 2t + p: the low (p = 0) or high nibbles of ggml group t, whose
     // first 16 bytes (chunk 2t) sit in k-slots 4t.. and whose second 16 (chunk 2t+1) in slots 16+4t..
     __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return 2u * t + p; }
@@ -85,8 +93,8 @@ struct RQ4K : Q4K {
         a2 = word4(s.q[1], j) & mask;
         a3 = word4(s.q[3], j) & mask;
     }
-    __device__ static __forceinline__ void load_ring(Stage& s, const uint8_t* box, const uint8_t* rec, uint32_t rec8,
-                                                     uint32_t o0, uint32_t o1, uint32_t t) {
+    __device__ static __forceinline__ void load_ring(Stage& s, const uint8_t* box, const uint8_t*, const uint8_t* rec, uint32_t rec8,
+                                                     uint32_t o0, uint32_t o1, uint32_t, uint32_t t) {
         s.q[0] = *reinterpret_cast<const uint4*>(box + o0);
         s.q[1] = *reinterpret_cast<const uint4*>(box + o1);
         s.q[2] = *reinterpret_cast<const uint4*>(box + o0 + 1024u);
@@ -102,7 +110,9 @@ struct RQ4K : Q4K {
 };
 
 struct RQ40 : Q40 {
-    static constexpr uint32_t kDataBoxes = 1;
+    static constexpr uint32_t kDataBoxes = 1, kHighBytes = 0, kPasses = 2, kSub = 4, kBlock = 32;
+    static constexpr bool kMany = true;
+    static constexpr float kStepCost = 0.052f, kManyCost = 0.047f, kRegsCost = 0.95f;   // make_plan
     __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return 2u * t + p; }
     __device__ static __forceinline__ void a_pass(const Stage& s, uint32_t p, uint32_t j, uint32_t& a0, uint32_t& a1,
                                                   uint32_t& a2, uint32_t& a3) {
@@ -112,8 +122,8 @@ struct RQ40 : Q40 {
         a2 = word4(s.q[1], j) & mask;
         a3 = word4(s.q[3], j) & mask;
     }
-    __device__ static __forceinline__ void load_ring(Stage& s, const uint8_t* box, const uint8_t* rec, uint32_t rec8,
-                                                     uint32_t o0, uint32_t o1, uint32_t t) {
+    __device__ static __forceinline__ void load_ring(Stage& s, const uint8_t* box, const uint8_t*, const uint8_t* rec, uint32_t rec8,
+                                                     uint32_t o0, uint32_t o1, uint32_t, uint32_t t) {
         s.q[0] = *reinterpret_cast<const uint4*>(box + o0);
         s.q[1] = *reinterpret_cast<const uint4*>(box + o1);
         s.q[2] = *reinterpret_cast<const uint4*>(box + o0 + 1024u);
@@ -125,6 +135,9 @@ struct RQ40 : Q40 {
 
 struct RQ80 : Q80 {
     static constexpr uint32_t kDataBoxes = 2;  // blocks 0..3 | blocks 4..7 of the unit
+    static constexpr uint32_t kHighBytes = 0, kPasses = 2, kSub = 4, kBlock = 32;
+    static constexpr bool kMany = false;       // two boxes a unit leave no room for the stages, and the loads spill
+    static constexpr float kStepCost = 0.096f, kManyCost = 0.0f, kRegsCost = 1.6f;   // make_plan
     // pass p of lane t feeds block t + 4p: box p holds blocks 4p..4p+3, chunk 2t its block t's first
     // 16 bytes (k-slots 4t..), chunk 2t+1 the second 16 (slots 16+4t..)
     __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return t + 4u * p; }
@@ -135,8 +148,8 @@ struct RQ80 : Q80 {
         a2 = word4(s.q[2u * p + 1u], j);
         a3 = word4(s.q[5u + 2u * p], j);
     }
-    __device__ static __forceinline__ void load_ring(Stage& s, const uint8_t* box, const uint8_t* rec, uint32_t rec8,
-                                                     uint32_t o0, uint32_t o1, uint32_t t) {
+    __device__ static __forceinline__ void load_ring(Stage& s, const uint8_t* box, const uint8_t*, const uint8_t* rec, uint32_t rec8,
+                                                     uint32_t o0, uint32_t o1, uint32_t, uint32_t t) {
         s.q[0] = *reinterpret_cast<const uint4*>(box + o0);
         s.q[1] = *reinterpret_cast<const uint4*>(box + o1);
         s.q[2] = *reinterpret_cast<const uint4*>(box + kBoxBytes + o0);
@@ -152,86 +165,221 @@ struct RQ80 : Q80 {
     }
 };
 
-template <class F>
-__global__ void __launch_bounds__(kMaxWarps * 32u, 1)
-gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant__ CUtensorMap rmap,
-                 const float* __restrict__ bias, const float* __restrict__ x, float* __restrict__ y, uint32_t in_dim,
-                 uint32_t out_dim, const int8_t* __restrict__ xq, const float* __restrict__ xq_scale, const PeerOut peers,
+// Q5_K: the Q4_K nibbles and record, and 32 bytes whose bit b is bit 4 of block b's codes.  Lane t's blocks 2t and 2t + 1 take
+// two bits of every byte.
+struct RQ5K : Q4K {
+    static constexpr uint32_t kDataBytes = 160;
+    static constexpr uint32_t kDataBoxes = 1, kHighBytes = 32, kPasses = 2, kSub = 4, kBlock = 32;
+    static constexpr bool kMany = true;
+    static constexpr float kStepCost = 0.13f, kManyCost = 0.065f, kRegsCost = 1.45f;
+    static constexpr int kHiShift = 0;
+    struct Stage : Q4K::Stage {
+        uint4 h[4];   // rows g, g + 8: the high-bit bytes, shifted so that block 2t's bit is bit 0
+    };
+    __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return 2u * t + p; }
+    __device__ static __forceinline__ void a_pass(const Stage& s, uint32_t p, uint32_t j, uint32_t& a0, uint32_t& a1,
+                                                  uint32_t& a2, uint32_t& a3) {
+        auto code = [p](uint32_t w, uint32_t h) {
+            return p ? ((w >> 4) & 0x0F0F0F0Fu) | ((h << 3) & 0x10101010u) : (w & 0x0F0F0F0Fu) | ((h << 4) & 0x10101010u);
+        };
+        a0 = code(word4(s.q[0], j), word4(s.h[0], j));
+        a1 = code(word4(s.q[2], j), word4(s.h[2], j));
+        a2 = code(word4(s.q[1], j), word4(s.h[1], j));
+        a3 = code(word4(s.q[3], j), word4(s.h[3], j));
+    }
+    __device__ static __forceinline__ void load_ring(Stage& s, const uint8_t* box, const uint8_t* high, const uint8_t* rec, uint32_t rec8,
+                                                     uint32_t o0, uint32_t o1, uint32_t g, uint32_t t) {
+        RQ4K::load_ring(s, box, nullptr, rec, rec8, o0, o1, g, t);
+#pragma unroll
+        for (uint32_t i = 0; i < 4u; ++i) {
+            const uint4 v = *reinterpret_cast<const uint4*>(high + (g + (i >> 1) * 8u) * 32u + (i & 1u) * 16u);
+            s.h[i] = make_uint4(v.x >> (2u * t), v.y >> (2u * t), v.z >> (2u * t), v.w >> (2u * t));
+        }
+    }
+};
+
+// Q6_K: sixteen blocks of 16 weights, so four passes of two mmas.  Lane t holds, of the 128-weight half t / 2, the blocks at
+// elements 16 (t & 1) + 32 p (p = pass): low nibbles of two 16-byte chunks of ql for p = 0, 1, high nibbles for p = 2, 3,
+// and bits 2p, 2p + 1 of one chunk of qh.  Codes stay unsigned; the -32 goes through the 16-element sums of the activations.
+struct RQ6K {
+    static constexpr uint32_t kDataBytes = 192, kRecBytes = 24;
+    static constexpr uint32_t kDataBoxes = 1, kHighBytes = 64, kPasses = 4, kSub = 2, kBlock = 16;
+    static constexpr bool kMany = true;
+    static constexpr float kStepCost = 0.13f, kManyCost = 0.065f, kRegsCost = 1.4f;
+    static constexpr bool kUnsignedA = true;
+    static constexpr int kHiShift = 0;
+    struct Stage {
+        uint4 q[4];      // row g: ql chunks of p = 0, 2 and of p = 1, 3; row g + 8 likewise
+        uint4 h[2];      // qh chunk of rows g, g + 8
+        uint32_t d[2];   // f16 d of the two rows (low half)
+        uint2 sc[2];     // the half's eight int8 scales, for this lane's blocks: bytes 2 p of the eight, shifted by t & 1
+    };
+    __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return 8u * (t >> 1) + 2u * p + (t & 1u); }
+    __device__ static __forceinline__ void a_pass(const Stage& s, uint32_t p, uint32_t j, uint32_t& a0, uint32_t& a1,
+                                                  uint32_t& a2, uint32_t& a3) {
+        auto code = [p](uint32_t w, uint32_t h) {
+            const uint32_t lo = (p >> 1) ? (w >> 4) & 0x0F0F0F0Fu : w & 0x0F0F0F0Fu;
+            return lo | ((p == 0u ? h << 4 : p == 1u ? h << 2 : p == 2u ? h : h >> 2) & 0x30303030u);
+        };
+        const uint32_t c = p & 1u;
+        a0 = code(word4(s.q[c], j), word4(s.h[0], j));
+        a1 = code(word4(s.q[2u + c], j), word4(s.h[1], j));
+        a2 = code(word4(s.q[c], 2u + j), word4(s.h[0], 2u + j));
+        a3 = code(word4(s.q[2u + c], 2u + j), word4(s.h[1], 2u + j));
+    }
+    __device__ static __forceinline__ void load_ring(Stage& s, const uint8_t* box, const uint8_t* high, const uint8_t* rec, uint32_t rec8,
+                                                     uint32_t, uint32_t, uint32_t g, uint32_t t) {
+        const uint32_t c0 = 4u * (t >> 1) + (t & 1u);
+#pragma unroll
+        for (uint32_t h = 0; h < 2u; ++h) {
+            s.q[2u * h] = *reinterpret_cast<const uint4*>(box + h * 1024u + swz(g, c0));
+            s.q[2u * h + 1u] = *reinterpret_cast<const uint4*>(box + h * 1024u + swz(g, c0 + 2u));
+            // 64-byte rows under the 64-byte swizzle: chunk index xor bits 1..2 of the row
+            s.h[h] = *reinterpret_cast<const uint4*>(high + (g + h * 8u) * 64u + ((t ^ ((g >> 1) & 3u)) << 4));
+            const uint8_t* r = rec + h * rec8;
+            s.d[h] = *reinterpret_cast<const uint32_t*>(r);
+            const uint32_t w0 = *reinterpret_cast<const uint32_t*>(r + 4u + 8u * (t >> 1)), w1 = *reinterpret_cast<const uint32_t*>(r + 8u + 8u * (t >> 1));
+            s.sc[h] = make_uint2(w0 >> (8u * (t & 1u)), w1 >> (8u * (t & 1u)));
+        }
+    }
+    __device__ static __forceinline__ void fold(const Stage& s, const int (&c)[4][4], const float2 (&xm)[4], float& acc_g, float& acc_g8) {
+        float v[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (uint32_t h = 0; h < 2u; ++h)
+#pragma unroll
+            for (uint32_t p = 0; p < 4u; ++p) {
+                const uint32_t w = (p >> 1) ? s.sc[h].y : s.sc[h].x;
+                const float f = fmaf((float)(c[p][2u * h] * 256 + c[p][2u * h + 1u]), xm[p].x, -32.0f * xm[p].y);
+                v[h] = fmaf((float)(int8_t)((w >> (16u * (p & 1u))) & 0xffu), f, v[h]);
+            }
+        acc_g = fmaf(__half2float(__ushort_as_half((unsigned short)s.d[0])), v[0], acc_g);
+        acc_g8 = fmaf(__half2float(__ushort_as_half((unsigned short)s.d[1])), v[1], acc_g8);
+    }
+};
+
+__device__ __forceinline__ void cp_async8_fill(uint32_t dst, const void* src, bool valid) {     // zeros where not valid
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(valid ? 8u : 0u) : "memory");
+}
+
+// MANY: up to kManyWarps warps in one or more teams, the units of a pair one after the other; else one team of up to kMaxWarps.
+// RECS_ASYNC: a row's records are not a multiple of 16 bytes (an odd number of 24-byte records): the lanes copy them.
+// SPLIT: a cluster of pl.split CTAs shares its tiles and splits the pairs of a row.  (As template arguments: an instance that can
+// do it all takes 0.2 us longer to start and 5 % longer at N = 6016.)
+template <class F, bool MANY, bool RECS_ASYNC, bool SPLIT>
+__global__ void __launch_bounds__((MANY ? kManyWarps : kMaxWarps) * 32u, 1)
+gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant__ CUtensorMap hmap, const __grid_constant__ CUtensorMap rmap,
+                 const uint8_t* __restrict__ recs, const float* __restrict__ bias, const float* __restrict__ x, float* __restrict__ y,
+                 uint32_t in_dim, uint32_t out_dim, const int8_t* __restrict__ xq, const float* __restrict__ xq_scale, const PeerOut peers,
                  const RingPlan pl, unsigned int* __restrict__ err) {
     using Stage = typename F::Stage;
-    constexpr uint32_t kUnitData = F::kDataBoxes * kBoxBytes;       // one unit's boxes
+    constexpr uint32_t kUnitData = F::kDataBoxes * kBoxBytes, kUnitHigh = 16u * F::kHighBytes;   // one unit's boxes
     constexpr uint32_t kRecRow = 2u * F::kRecBytes;                 // a pair's records of one row
-    constexpr uint32_t kStageData = 2u * kUnitData, kStageRec = 16u * kRecRow;
+    constexpr uint32_t kStageHigh = 2u * kUnitData, kStageData = kStageHigh + 2u * kUnitHigh, kStageRec = 16u * kRecRow;
+    constexpr uint32_t kPasses = F::kPasses, kSub = F::kSub;
     extern __shared__ __align__(1024) uint8_t smem[];
-    const uint32_t n_pair = in_dim >> 9;
     uint8_t* xs_hi = smem;
-    uint8_t* xs_lo = smem + in_dim;
-    uint8_t* zeros = smem + 2u * (size_t)in_dim;
+    uint8_t* xs_lo = smem + pl.k_part;
+    uint8_t* zeros = smem + 2u * (size_t)pl.k_part;
     float2* xmeta = reinterpret_cast<float2*>(smem + pl.off_xmeta);
-    float* red = reinterpret_cast<float*>(smem + pl.off_red);
-    uint64_t* full = reinterpret_cast<uint64_t*>(smem + pl.off_bar);  // [W][kMaxDepth]
-    uint64_t* red_full = full + kMaxWarps * kMaxDepth;
-    uint64_t* red_free = red_full + kRedBufs;
-    volatile int* abort_flag = reinterpret_cast<volatile int*>(red_free + kRedBufs);
-
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    const uint32_t tid = threadIdx.x, lane = tid & 31u;
     const uint32_t W = pl.W, D = pl.D;
-    const uint32_t n_tiles = (out_dim + 15u) >> 4;
-    const uint32_t tile_lo = (uint32_t)((uint64_t)blockIdx.x * n_tiles / gridDim.x);
-    const uint32_t tile_hi = (uint32_t)((uint64_t)(blockIdx.x + 1u) * n_tiles / gridDim.x);
-    const uint32_t my_tiles = tile_hi - tile_lo;
-    // this warp's pairs of a tile: warp, warp + W, ... below n_pair
+    uint32_t warp = tid >> 5, team = 0u;
+    const uint32_t cta_warp = warp, teams = MANY ? pl.teams : 1u;
+    if (MANY)
+        for (; warp >= W; warp -= W) ++team;
+    float* red = reinterpret_cast<float*>(smem + pl.off_red) + team * kRedBufs * (W * 16u);
+    float* recv = reinterpret_cast<float*>(smem + pl.off_recv);
+    uint64_t* full = reinterpret_cast<uint64_t*>(smem + pl.off_bar);  // [warp][kMaxDepth], then per team the fold barriers
+    uint64_t* red_full = full + W * teams * kMaxDepth + 2u * team * kRedBufs;
+    uint64_t* red_free = red_full + kRedBufs;
+    volatile int* abort_flag = reinterpret_cast<volatile int*>(full + W * teams * kMaxDepth + 2u * teams * kRedBufs);
+
+    const uint32_t split = SPLIT ? pl.split : 1u, rank = SPLIT ? blockIdx.x % split : 0u, cl = SPLIT ? blockIdx.x / split : blockIdx.x;
+    const uint32_t all_pairs = (in_dim + 511u) >> 9;
+    const uint32_t p_lo = SPLIT ? rank * all_pairs / split : 0u, n_pair = (SPLIT ? (rank + 1u) * all_pairs / split : all_pairs) - p_lo;
+    const uint32_t n_tiles = (out_dim + 15u) >> 4, n_cl = SPLIT ? pl.clusters : gridDim.x;
+    const uint32_t tile_lo = (uint32_t)((uint64_t)cl * n_tiles / n_cl);
+    const uint32_t tile_hi = (uint32_t)((uint64_t)(cl + 1u) * n_tiles / n_cl);
+    const uint32_t cta_tiles = tile_hi - tile_lo;
+    // the team's tiles team, team + teams, ..., and this warp's pairs of a tile: warp, warp + W, ... below n_pair
+    const uint32_t my_tiles = MANY ? (team < cta_tiles ? (cta_tiles - team + teams - 1u) / teams : 0u) : cta_tiles;
     const uint32_t my_pairs = warp < n_pair ? (n_pair - warp + W - 1u) / W : 0u;
     const uint32_t total = my_tiles * my_pairs;
 
-    uint64_t* my_full = full + warp * kMaxDepth;
-    uint8_t* my_data = smem + pl.off_data + (size_t)warp * D * kStageData;
-    uint8_t* my_rec = smem + pl.off_rec + (size_t)warp * D * kStageRec;
+    uint64_t* my_full = full + cta_warp * kMaxDepth;
+    uint8_t* my_data = smem + pl.off_data + (size_t)cta_warp * D * kStageData;
+    uint8_t* my_rec = smem + pl.off_rec + (size_t)cta_warp * D * kStageRec;
+    const size_t rec_pitch = (size_t)(in_dim >> 8) * F::kRecBytes;
 
     // (tile, pair) number i of this warp -> stage i % D; issue = arm the barrier, then the copies.
     // Called by the whole (converged) warp: one elected lane issues, so addresses and the
-    // tensor-map pointers stay in uniform registers.
+    // tensor-map pointers stay in uniform registers.  What lies beyond a row's end is filled with zeros.
     const uint64_t stream_once = tc5::l2_policy_evict_first();   // a plane is read once per launch
     auto issue = [&](uint32_t stage, uint32_t tl, uint32_t pr) {
         uint64_t* bar = my_full + stage;
-        tc5::mbar_arrive_expect_tx_elect(bar, kStageData + kStageRec);
+        const uint32_t gp = p_lo + pr;
+        tc5::mbar_arrive_expect_tx_elect(bar, kStageData + (RECS_ASYNC ? 0u : kStageRec));
         const int32_t row = (int32_t)((tile_lo + tl) * 16u);
+        uint8_t* st = my_data + stage * kStageData;
 #pragma unroll
-        for (uint32_t b = 0; b < 2u * F::kDataBoxes; ++b)
-            tc5::tma_load_2d_hint_elect(my_data + stage * kStageData + b * kBoxBytes, &dmap, bar,
-                                        (int32_t)(pr * 2u * F::kDataBytes + b * 128u), row, stream_once);
-        tc5::tma_load_2d_hint_elect(my_rec + stage * kStageRec, &rmap, bar, (int32_t)(pr * kRecRow), row, stream_once);
+        for (uint32_t u = 0; u < 2u; ++u) {
+#pragma unroll
+            for (uint32_t b = 0; b < F::kDataBoxes; ++b)
+                tc5::tma_load_2d_hint_elect(st + u * kUnitData + b * kBoxBytes, &dmap, bar, (int32_t)((gp * 2u + u) * F::kDataBytes + b * 128u), row,
+                                            stream_once);
+            if constexpr (F::kHighBytes != 0u)
+                tc5::tma_load_2d_hint_elect(st + kStageHigh + u * kUnitHigh, &hmap, bar, (int32_t)((gp * 2u + u) * F::kDataBytes + 128u), row, stream_once);
+        }
+        if constexpr (!RECS_ASYNC) {
+            tc5::tma_load_2d_hint_elect(my_rec + stage * kStageRec, &rmap, bar, (int32_t)(gp * kRecRow), row, stream_once);
+        } else {
+            constexpr uint32_t kPieces = kRecRow / 8u;      // of a row
+            const uint32_t dst = tc5::smem_u32(my_rec + stage * kStageRec), last = out_dim - 1u;
+#pragma unroll
+            for (uint32_t i = 0; i < kPieces / 2u; ++i) {
+                const uint32_t c = i * 32u + lane, r = c / kPieces, off = gp * kRecRow + (c - r * kPieces) * 8u;
+                const bool valid = off < rec_pitch;
+                cp_async8_fill(dst + c * 8u, recs + (size_t)min((uint32_t)row + r, last) * rec_pitch + (valid ? off : 0u), valid);
+            }
+            asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc5::smem_u32(bar)) : "memory");
+        }
     };
 
     // ---- prologue: every warp arms its own barriers and requests its first D stages; only then
     // does the CTA meet (shared barriers of the tile fold) and wait for the previous kernel
     if (lane == 0u) {
-        for (uint32_t s = 0; s < D; ++s) tc5::mbar_init(my_full + s, 1u);
+        for (uint32_t s = 0; s < D; ++s) tc5::mbar_init(my_full + s, RECS_ASYNC ? 33u : 1u);
         tc5::mbar_fence_init();
     }
     __syncwarp();
-    uint32_t i_tl = 0, i_pr = warp, issued = 0;  // issue cursor
+    uint32_t i_tl = team, i_pr = warp, issued = 0;  // issue cursor
     auto issue_next = [&]() {
         issue(issued % D, i_tl, i_pr);
         ++issued;
         i_pr += W;
-        if (i_pr >= n_pair) { i_pr = warp; ++i_tl; }
+        if (i_pr >= n_pair) { i_pr = warp; i_tl += teams; }
     };
     // the first stage of every warp goes out alone: it is what the first iteration waits for, and
     // it arrives sooner when the chip's first burst is a quarter of the ring
     if (total > 0u) issue_next();
-    if (tid == 0u) {
+    if (warp == 0u && lane == 0u) {
         for (uint32_t b = 0; b < kRedBufs; ++b) {
             tc5::mbar_init(&red_full[b], W);
             tc5::mbar_init(&red_free[b], 1u);
         }
-        *abort_flag = 0;
+        if (team == 0u) *abort_flag = 0;
         tc5::mbar_fence_init();
     }
     if (tid < 8u) reinterpret_cast<uint32_t*>(zeros)[tid] = 0u;
     // The CTA meets once, here, where it would wait for the previous kernel anyway: the fold
-    // barriers and the zero line are shared, everything after is per warp (invariant plans).
-    __syncthreads();
+    // barriers and the zero line are shared, everything after is per warp (invariant plans of one team).
+    // A cluster meets too: its CTAs store into one another's shared memory later.
+    if constexpr (SPLIT) {
+        __syncwarp();
+        tc5::cluster_sync();
+    } else {
+        __syncthreads();
+    }
     // Programmatic dependent launch: the next kernel of the stream may start its prologue (its own
     // first requests: weights never depend on this kernel) as soon as this one's CTAs have all started.
     pdk_pdl_launch_dependents();
@@ -240,23 +388,36 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
     const bool peer_deferred = peers.n != 0u && peers.signal == 2u && blockIdx.x == 0u && tid == 0u;
     if (peer_deferred) peer_step = peer_post_previous(peers);
     const bool invariant = pl.invariant != 0u;
+    const uint32_t x0 = p_lo * 64u, x_groups = in_dim >> 3;     // groups of 8 elements before this part, of a row
+    // what lies beyond the row's end counts as zero; the load itself is unconditional, so that two of them are in flight at once
+    auto load8 = [&](uint32_t grp, float (&v)[8]) { limb_load8(x, xq, xq_scale, min(x0 + grp, x_groups - 1u), v); };
+    auto store8 = [&](float (&v)[8], uint32_t grp) {
+        if (x0 + grp >= x_groups) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] = 0.0f;
+        }
+        limb_store8<F::kBlock>(v, grp, xs_hi, xs_lo, xmeta);
+    };
     if (invariant) {
-        // A warp only ever meets its own pair's 512 activations: it builds their limbs itself.  The
+        // A warp only ever meets its own pair's 512 activations: it builds their limbs itself (the first team for all).  The
         // loads of x go out before the rest of the ring is requested, so they do not queue behind it.
         const uint32_t g0 = warp * 64u + lane;   // groups of 8 elements: this lane's two
         float v0[8], v1[8];
-        limb_load8(x, xq, xq_scale, g0, v0);
-        limb_load8(x, xq, xq_scale, g0 + 32u, v1);
+        load8(g0, v0);
+        load8(g0 + 32u, v1);
         while (issued < D && issued < total) issue_next();
-        limb_store8(v0, g0, xs_hi, xs_lo, xmeta);
-        limb_store8(v1, g0 + 32u, xs_hi, xs_lo, xmeta);
-        __syncwarp();
+        if (team == 0u && warp < n_pair) {
+            store8(v0, g0);
+            store8(v1, g0 + 32u);
+        }
+        if (MANY) __syncthreads();
+        else __syncwarp();
     } else {
-        const uint32_t groups = in_dim >> 3;
-        for (uint32_t grp = tid; grp < groups; grp += W * 32u) {
+        const uint32_t groups = n_pair * 64u;
+        for (uint32_t grp = tid; grp < groups; grp += W * teams * 32u) {
             float v[8];
-            limb_load8(x, xq, xq_scale, grp, v);
-            limb_store8(v, grp, xs_hi, xs_lo, xmeta);
+            load8(grp, v);
+            store8(v, grp);
         }
         while (issued < D && issued < total) issue_next();
         __syncthreads();
@@ -268,48 +429,59 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
     // lane (g, t) feeds limb g & 1 of block blk(p, t) when g >> 1 == t, and zeros otherwise.
     const bool role = (g >> 1) == t;
     const uint8_t* my_limb = (g & 1u) ? xs_lo : xs_hi;
-    uint32_t vb[2][2][8];  // [unit of the pair][pass]: words 0..3 -> b0 of mma j, words 4..7 -> b1
-    float4 xm[2];          // per unit: {step, sum} of blocks blk(0, t) and blk(1, t), the two this lane folds
-    auto load_b = [&](uint32_t pr) {
+    // Where a thread has registers for it, both units of a pair side by side (independent accumulator chains), and
+    // with an invariant pair B stays in registers; else one unit after the other.
+    constexpr uint32_t kSide = MANY ? 1u : 2u;
+    uint32_t vb[kSide][kPasses][2u * kSub];  // [unit][pass]: words 0.. -> b0 of mma j, words kSub.. -> b1
+    float2 xm[kSide][kPasses];               // {step, sum} of the blocks this lane folds
+    auto load_b = [&](uint32_t first) {
 #pragma unroll
-        for (uint32_t i = 0; i < 2u; ++i) {
-            const uint32_t u = 2u * pr + i;
+        for (uint32_t i = 0; i < kSide; ++i) {
+            const uint32_t u = first + i;
 #pragma unroll
-            for (uint32_t p = 0; p < 2u; ++p) {
-                const uint8_t* src = role ? my_limb + u * 256u + F::blk(p, t) * 32u : zeros;
-                const uint4 a = *reinterpret_cast<const uint4*>(src);
-                const uint4 b = *reinterpret_cast<const uint4*>(src + 16u);
-                vb[i][p][0] = a.x; vb[i][p][1] = a.y; vb[i][p][2] = a.z; vb[i][p][3] = a.w;
-                vb[i][p][4] = b.x; vb[i][p][5] = b.y; vb[i][p][6] = b.z; vb[i][p][7] = b.w;
+            for (uint32_t p = 0; p < kPasses; ++p) {
+                const uint8_t* src = role ? my_limb + u * 256u + F::blk(p, t) * F::kBlock : zeros;
+#pragma unroll
+                for (uint32_t c = 0; c < kSub / 2u; ++c) {
+                    const uint4 a = *reinterpret_cast<const uint4*>(src + 16u * c);
+                    vb[i][p][4u * c] = a.x; vb[i][p][4u * c + 1u] = a.y; vb[i][p][4u * c + 2u] = a.z; vb[i][p][4u * c + 3u] = a.w;
+                }
+                xm[i][p] = xmeta[u * (256u / F::kBlock) + F::blk(p, t)];
             }
-            const float2 m0 = xmeta[u * 8u + F::blk(0u, t)], m1 = xmeta[u * 8u + F::blk(1u, t)];
-            xm[i] = make_float4(m0.x, m0.y, m1.x, m1.y);
         }
     };
-    if (invariant && warp < n_pair) load_b(warp);
+    if (!MANY && invariant && warp < n_pair) load_b(2u * warp);
 
     // per-lane offsets inside a stage
     const uint32_t o0 = swz(g, 2u * t), o1 = swz(g, 2u * t + 1u);
     const uint32_t rec_g = g * kRecRow, rec8 = 8u * kRecRow;
 
-    // ---- tile fold.  Per tile each warp leaves 16 partial row sums in buffer tl % kRedBufs and
-    // arrives on the buffer's barrier (fire and forget).  The tile belongs to warp tl % W, which
+    // ---- tile fold.  Per tile each warp of the team leaves 16 partial row sums in buffer tl % kRedBufs (tl counts the team's
+    // tiles) and arrives on the buffer's barrier (fire and forget).  The tile belongs to the team's warp tl % W, which
     // looks at the barrier once per later iteration and, when all W warps have arrived, adds the
     // partials in warp order, stores y and hands the buffer back; it blocks only before taking on
-    // another tile, and at the end.  A buffer is written again (tile tl + kRedBufs) only after
-    // its fold.
+    // another tile, before it would wait for that very buffer, and at the end.  A buffer is written again (tile tl + kRedBufs)
+    // only after its fold.  With K split, the sum goes to the CTA of the cluster that adds up the row.
     constexpr uint32_t kNone = 0xffffffffu;
-    uint32_t pend = kNone;  // local index of the tile this warp still has to fold
+    uint32_t pend = kNone;  // the team's tile this warp still has to fold
     bool alive = true;
+    const uint32_t rows = cta_tiles * 16u, rpo = SPLIT ? (rows + split - 1u) / split : 0u;   // rows per owner
     auto fold_tile = [&](uint32_t tl_f) {
         const uint32_t rbf = tl_f % kRedBufs;
         const float* rbuf = red + (size_t)rbf * (W * 16u);
-        const uint32_t row = (tile_lo + tl_f) * 16u + lane;
+        const uint32_t r = (team + tl_f * teams) * 16u + lane, row = tile_lo * 16u + r;
         float v = 0.0f;
         if (lane < 16u)
             for (uint32_t w = 0; w < W; ++w) v += rbuf[w * 16u + lane];
         __syncwarp();
         if (lane == 0u) tc5::mbar_arrive(&red_free[rbf]);
+        if constexpr (SPLIT) {
+            if (lane < 16u) {
+                const uint32_t owner = r / rpo;
+                tc5::st_cluster(tc5::cluster_addr(tc5::smem_u32(recv), owner) + (rank * rpo + r - owner * rpo) * 4u, v);
+            }
+            return;
+        }
         if (lane < 16u && row < out_dim) {
             if (bias) v += bias[row];
             if (peers.n == 0u) {
@@ -344,35 +516,44 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
         for (uint32_t pr = warp; pr < n_pair; pr += W) {
             if (alive) alive = __all_sync(0xffffffffu, tc5::mbar_wait(my_full + stage, phase, ctx, kErrRingFull, stage));
             if (alive) {
-                Stage st[2];
                 const uint8_t* sd = my_data + stage * kStageData;
                 const uint8_t* sr = my_rec + stage * kStageRec + rec_g;
-                F::load_ring(st[0], sd, sr, rec8, o0, o1, t);
-                F::load_ring(st[1], sd + kUnitData, sr + F::kRecBytes, rec8, o0, o1, t);
-                if (!invariant) load_b(pr);
-                // four independent accumulator chains: [unit][pass], {hi, lo} of row g, {hi, lo} of row g + 8
-                int c[2][2][4] = {};
+                // [unit][pass], {hi, lo} of row g, {hi, lo} of row g + 8
 #pragma unroll
-                for (uint32_t j = 0; j < 4u; ++j) {
+                for (uint32_t i0 = 0; i0 < 2u; i0 += kSide) {
+                    Stage st[kSide];
 #pragma unroll
-                    for (uint32_t i = 0; i < 2u; ++i) {
+                    for (uint32_t i = 0; i < kSide; ++i)
+                        F::load_ring(st[i], sd + (i0 + i) * kUnitData, sd + kStageHigh + (i0 + i) * kUnitHigh, sr + (i0 + i) * F::kRecBytes, rec8, o0, o1, g, t);
+                    if (MANY || !invariant) load_b(2u * pr + i0);
+                    int c[kSide][kPasses][4] = {};
 #pragma unroll
-                        for (uint32_t p = 0; p < 2u; ++p) {
-                            uint32_t a0, a1, a2, a3;
-                            F::a_pass(st[i], p, j, a0, a1, a2, a3);
-                            if constexpr (F::kUnsignedA) mma_u8s8_nv(c[i][p], a0, a1, a2, a3, vb[i][p][j], vb[i][p][4u + j]);
-                            else mma_s8_nv(c[i][p], a0, a1, a2, a3, vb[i][p][j], vb[i][p][4u + j]);
+                    for (uint32_t j = 0; j < kSub; ++j) {
+#pragma unroll
+                        for (uint32_t i = 0; i < kSide; ++i) {
+#pragma unroll
+                            for (uint32_t p = 0; p < kPasses; ++p) {
+                                uint32_t a0, a1, a2, a3;
+                                F::a_pass(st[i], p, j, a0, a1, a2, a3);
+                                if constexpr (F::kUnsignedA) mma_u8s8_nv(c[i][p], a0, a1, a2, a3, vb[i][p][j], vb[i][p][kSub + j]);
+                                else mma_s8_nv(c[i][p], a0, a1, a2, a3, vb[i][p][j], vb[i][p][kSub + j]);
+                            }
                         }
                     }
-                }
 #pragma unroll
-                for (uint32_t i = 0; i < 2u; ++i) {
-                    float f[4];
-                    f[0] = (float)(c[i][0][0] * 256 + c[i][0][1]) * xm[i].x;
-                    f[1] = (float)((c[i][1][0] * 256 + c[i][1][1]) >> F::kHiShift) * xm[i].z;
-                    f[2] = (float)(c[i][0][2] * 256 + c[i][0][3]) * xm[i].x;
-                    f[3] = (float)((c[i][1][2] * 256 + c[i][1][3]) >> F::kHiShift) * xm[i].z;
-                    F::fold(st[i], f, xm[i].y, xm[i].w, acc_g, acc_g8);
+                    for (uint32_t i = 0; i < kSide; ++i) {
+                        const float2 (&m)[kPasses] = xm[i];
+                        if constexpr (kPasses == 4u) {
+                            F::fold(st[i], c[i], m, acc_g, acc_g8);
+                        } else {
+                            float f[4];
+                            f[0] = (float)(c[i][0][0] * 256 + c[i][0][1]) * m[0].x;
+                            f[1] = (float)((c[i][1][0] * 256 + c[i][1][1]) >> F::kHiShift) * m[1].x;
+                            f[2] = (float)(c[i][0][2] * 256 + c[i][0][3]) * m[0].x;
+                            f[3] = (float)((c[i][1][2] * 256 + c[i][1][3]) >> F::kHiShift) * m[1].x;
+                            F::fold(st[i], f, m[0].y, m[1].y, acc_g, acc_g8);
+                        }
+                    }
                 }
                 // Every register the stage's loads filled has been consumed by now, so those loads
                 // are complete: the stage can take its next copy.
@@ -387,6 +568,7 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
         a += __shfl_xor_sync(0xffffffffu, a, 2);
         b += __shfl_xor_sync(0xffffffffu, b, 2);
         float* rbuf = red + (size_t)rb * (W * 16u);
+        if (pend != kNone && pend + kRedBufs == tl) poll_fold(true);   // the wait below is for this warp's own fold
         if (alive && tl >= kRedBufs)
             alive = __all_sync(0xffffffffu, tc5::mbar_wait(&red_free[rb], rb_phase ^ 1u, ctx, kErrRingFree, rb));
         if (alive) {
@@ -406,6 +588,17 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
         if (++rb == kRedBufs) { rb = 0; rb_phase ^= 1u; }
     }
     poll_fold(true);
+    if constexpr (SPLIT) {
+        __syncwarp();
+        tc5::cluster_sync();     // every CTA's sums are here
+        for (uint32_t r = tid; r < rpo; r += W * teams * 32u) {
+            const uint32_t at = rank * rpo + r, row = tile_lo * 16u + at;
+            if (at >= rows || row >= out_dim) break;
+            float v = 0.0f;
+            for (uint32_t s = 0; s < split; ++s) v += recv[s * rpo + r];
+            y[row] = bias ? v + bias[row] : v;
+        }
+    }
     if (peers.n != 0u && peers.signal == 1u) {   // uniform over the grid
         __syncthreads();
         if (tid == 0u) peer_signal(peers, err);
@@ -428,41 +621,71 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
     }
 }
 
+// What a CTA keeps in shared memory; false when fewer than two stages per warp fit.
 template <class F>
-bool make_plan(uint32_t in_dim, RingPlan& best) {
-    if (in_dim == 0u || (in_dim & 511u) != 0u) return false;  // whole pairs of units
-    const uint32_t n_pair = in_dim >> 9;
-    if (n_pair < 4u) return false;
-    constexpr uint32_t kStage = 2u * F::kDataBoxes * kBoxBytes + 32u * F::kRecBytes;
-    double best_cost = 1e30;
+bool ring_layout(RingPlan& p, uint32_t in_dim, uint32_t out_dim) {
+    constexpr uint32_t kData = 2u * (F::kDataBoxes * kBoxBytes + 16u * F::kHighBytes), kRec = 32u * F::kRecBytes;
+    const uint32_t n = p.W * p.teams, pairs = ((in_dim + 511u) / 512u + p.split - 1u) / p.split;
+    const uint64_t tiles = ((out_dim + 15u) / 16u + p.clusters - 1u) / p.clusters;
+    const uint64_t recv = p.split > 1u ? (uint64_t)p.split * ((tiles * 16u + p.split - 1u) / p.split) * 4u : 0u;
+    if (pairs > 512u || recv > kSmemMax) return false;
+    p.invariant = p.W >= pairs ? 1u : 0u;
+    p.k_part = pairs * 512u;
+    p.off_xmeta = 2u * p.k_part + 32u;
+    p.off_red = p.off_xmeta + (p.k_part / F::kBlock) * 8u;
+    p.off_recv = p.off_red + kRedBufs * n * 64u;
+    p.off_bar = (p.off_recv + (uint32_t)recv + 7u) & ~7u;
+    p.off_rec = (p.off_bar + (n * kMaxDepth + 2u * kRedBufs * p.teams + 1u) * 8u + 127u) & ~127u;
+    for (p.D = kMaxDepth; p.D >= 2u; --p.D) {
+        p.off_data = (p.off_rec + n * p.D * kRec + 1023u) & ~1023u;  // swizzled boxes start on 1 KB
+        p.smem_bytes = p.off_data + n * p.D * kData;
+        if (p.smem_bytes <= kSmemMax) return true;
+    }
+    return false;
+}
+
+// The split with the shortest estimate, in us; false where the register-staged kernel (gemv_i8.cu, gemv_q6k.cu) has a shorter one.
+//   one team     1.7 + steps (0.9 + kStepCost W): a step is a pair of a tile, and the longer the more warps share the SM
+//   many warps   2.0 + steps (0.75 + kManyCost warps) + 0.8 per tile of a team (its fold)
+//   split        0.5 more for two CTAs, 0.9 for more; 0.03 per pair of the part for the activations that every CTA converts
+//   registers    1.2 + rounds of 64 rows per SM x K / 1024 x kRegsCost, up to 1.35 times that when its four slots are full
+// Measured (us; register kernel -> here): Q6_K 17152 x 1024 25.2 -> 8.1 (four CTAs), 9472 x 2560 15.6 -> 9.8, 5120 x 25600 23.5 -> 20.1; Q8_0
+// 5376 x 6016 11.7 -> 7.6, 17152 x 520 29.3 -> 5.3; Q4_K 9472 x 1024 12.0 -> 5.1; and the other way round Q4_K 1792 x 9792 6.1 -> 4.6.  Q4_K 5120 x
+// 25600: one team of ten 17.2, two of ten 17.5, four of five 15.6; 4096 x 25600: eight 14.5, six teams of three 13.0.
+template <class F>
+bool make_plan(uint32_t in_dim, uint32_t out_dim, bool whole, const uint32_t* cap, RingPlan& best) {
+    const uint32_t all = (in_dim + 511u) / 512u, n_tiles = (out_dim + 15u) / 16u, slots = 4u * cap[1];
+    float best_cost = 0.0f;
     bool found = false;
-    for (uint32_t W = kMaxWarps; W >= 4u; --W) {
-        RingPlan p{};
-        p.W = W;
-        const uint32_t rounds = (n_pair + W - 1u) / W;
-        p.invariant = (W == n_pair) ? 1u : 0u;
-        p.off_xmeta = (2u * in_dim + 32u + 15u) & ~15u;
-        p.off_red = p.off_xmeta + (in_dim >> 5) * 8u;
-        p.off_bar = p.off_red + kRedBufs * W * 64u;
-        p.off_rec = (p.off_bar + (kMaxWarps * kMaxDepth + 2u * kRedBufs) * 8u + 16u + 127u) & ~127u;
-        const uint32_t fixed = p.off_rec;
-        if (fixed + 1024u + 2u * W * kStage > kSmemMax) continue;
-        p.D = (kSmemMax - fixed - 1024u) / (W * kStage);
-        if (p.D > kMaxDepth) p.D = kMaxDepth;
-        p.off_data = (p.off_rec + W * p.D * 32u * F::kRecBytes + 1023u) & ~1023u;  // swizzled boxes start on 1 KB
-        p.smem_bytes = p.off_data + W * p.D * 2u * F::kDataBoxes * kBoxBytes;
-        if (p.smem_bytes > kSmemMax) continue;
-        double cost = (double)(rounds * W) / (double)n_pair;   // idle warps in a tile's last round
-        if (p.D < 3u) cost += 0.04 * (3u - p.D);
-        if (W < 8u) cost += 0.03 * (8u - W);
-        cost -= 1e-9 * (double)(W * p.D * kStage);            // ties: more bytes in flight
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = p;
-            found = true;
+    for (uint32_t s = 1; s <= (whole ? 1u : kPdkMaxCluster) && s <= all; ++s) {
+        if (cap[s] == 0u || s == 5u || s == 7u) continue;
+        const uint32_t np = (all + s - 1u) / s, clusters = cap[s] < n_tiles ? cap[s] : n_tiles, per = (n_tiles + clusters - 1u) / clusters;
+        const float fixed = (s == 1u ? 0.0f : s == 2u ? 0.5f : 0.9f) + 0.03f * (float)np;
+        for (uint32_t rounds = 1; rounds <= 5u && rounds <= np; ++rounds) {
+            const uint32_t W = (np + rounds - 1u) / rounds;
+            if (W > kManyWarps) continue;
+            const uint32_t most = kManyWarps / W, teams[5] = {1u, 2u, kMaxWarps / W, most / 2u, most};
+            for (uint32_t i = 0; i < 5u; ++i) {
+                const uint32_t T = teams[i] < kMaxTeams ? teams[i] : kMaxTeams, n = W * T, folds = T != 0u ? (per + T - 1u) / T : 0u;
+                if (T == 0u || n > kManyWarps || (i > 0u && T <= teams[i - 1u])) continue;
+                const bool many = T > 1u || n > kMaxWarps;
+                if (many && !F::kMany) continue;
+                const float steps = (float)(folds * rounds);
+                const float cost = fixed + (many ? 2.0f + steps * (0.75f + F::kManyCost * (float)n) + 0.8f * (float)folds
+                                                 : 1.7f + steps * (0.9f + F::kStepCost * (float)n));
+                if (found && cost >= best_cost) continue;
+                RingPlan p{};
+                p.W = W; p.teams = T; p.split = s; p.clusters = clusters;
+                if (!ring_layout<F>(p, in_dim, out_dim)) continue;
+                best_cost = cost;
+                best = p;
+                found = true;
+            }
         }
     }
-    return found;
+    const float fill = n_tiles < slots ? (float)n_tiles / (float)slots : 1.0f;
+    const float regs = 1.2f + (float)((n_tiles + slots - 1u) / slots) * (float)in_dim / 1024.0f * F::kRegsCost * (1.0f + 0.35f * fill);
+    return found && best_cost <= regs;
 }
 
 // PDK_GEMV_REGS=1 sends every call to the register-staged kernel (A/B switch, read once).
@@ -479,50 +702,52 @@ bool force_regs() {
 // boxes of a unit pair's records x 16 dense.
 struct MapEntry {
     const void *data, *recs;
-    uint32_t in_dim, out_dim, rec_box;
-    CUtensorMap dmap, rmap;
+    uint32_t in_dim, out_dim, format;     // format: data bytes and record bytes of a unit
+    CUtensorMap dmap, hmap, rmap;
 };
+// whether a row's records can be described by a tensor map
+template <class F>
+bool recs_by_tma(uint32_t in_dim) { return ((in_dim >> 8) * F::kRecBytes) % 16u == 0u; }
+
 template <class F>
 int plane_maps(const void* data, const void* recs, uint32_t in_dim, uint32_t out_dim, const MapEntry** out) {
     constexpr int kEntries = 16;
+    constexpr uint32_t kFormat = F::kDataBytes << 8 | F::kRecBytes;
     thread_local MapEntry cache[kEntries];
     thread_local int next = 0, used = 0;
     for (int i = 0; i < used; ++i) {
         const MapEntry& e = cache[i];
-        if (e.data == data && e.recs == recs && e.in_dim == in_dim && e.out_dim == out_dim && e.rec_box == 2u * F::kRecBytes) {
+        if (e.data == data && e.recs == recs && e.in_dim == in_dim && e.out_dim == out_dim && e.format == kFormat) {
             *out = &e;
             return 0;
         }
     }
     MapEntry& e = cache[next];
     const uint32_t n_unit = in_dim >> 8;
-    int rc = pdk_make_tmap_2d(&e.dmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1u, data, (uint64_t)n_unit * F::kDataBytes, out_dim,
-                              (uint64_t)n_unit * F::kDataBytes, 128u, 16u);
-    if (rc == 0)
+    const uint64_t pitch = (uint64_t)n_unit * F::kDataBytes;
+    int rc = pdk_make_tmap_2d(&e.dmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1u, data, pitch, out_dim, pitch, 128u, 16u);
+    e.hmap = e.rmap = e.dmap;
+    if (rc == 0 && F::kHighBytes == 32u) rc = pdk_make_tmap_2d_dense(&e.hmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1u, data, pitch, out_dim, pitch, 32u, 16u);
+    if (rc == 0 && F::kHighBytes == 64u) rc = pdk_make_tmap_2d_sw64(&e.hmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1u, data, pitch, out_dim, pitch, 64u, 16u);
+    if (rc == 0 && recs_by_tma<F>(in_dim))
         rc = pdk_make_tmap_2d_dense(&e.rmap, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1u, recs, (uint64_t)n_unit * F::kRecBytes,
                                     out_dim, (uint64_t)n_unit * F::kRecBytes, 2u * F::kRecBytes, 16u);
     if (rc != 0) {
         e.data = nullptr;
         return rc;
     }
-    e.data = data; e.recs = recs; e.in_dim = in_dim; e.out_dim = out_dim; e.rec_box = 2u * F::kRecBytes;
+    e.data = data; e.recs = recs; e.in_dim = in_dim; e.out_dim = out_dim; e.format = kFormat;
     *out = &e;
     next = (next + 1) % kEntries;
     if (used < kEntries) ++used;
     return 0;
 }
 
-template <class F>
-int launch_ring(const void* data, const void* recs, const float* bias, const float* x, float* y, uint32_t in_dim,
-                uint32_t out_dim, cudaStream_t st, const int8_t* xq = nullptr, const float* xq_scale = nullptr,
-                const PeerOut* peers = nullptr) {
-    if (force_regs() || !pdk_aligned(recs, 16)) return -1;  // tensor maps start on 16 bytes
-    RingPlan pl;
-    if (!make_plan<F>(in_dim, pl)) return -1;
-    const MapEntry* maps = nullptr;
-    if (plane_maps<F>(data, recs, in_dim, out_dim, &maps) != 0) return -1;
-    auto kern = gemv_ring_kernel<F>;
-    static bool attr_set[64] = {false};  // per device, per format (one instance of this function per F)
+template <class F, bool MANY, bool RECS_ASYNC, bool SPLIT>
+int launch_plan(const MapEntry& m, const void* recs, const float* bias, const float* x, float* y, uint32_t in_dim, uint32_t out_dim,
+                cudaStream_t st, const int8_t* xq, const float* xq_scale, const PeerOut& po, const RingPlan& pl) {
+    auto kern = gemv_ring_kernel<F, MANY, RECS_ASYNC, SPLIT>;
+    static bool attr_set[64] = {false};  // per device, per instance
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
@@ -533,13 +758,65 @@ int launch_ring(const void* data, const void* recs, const float* bias, const flo
     }
     unsigned int* err = pdk_error_word();
     if (err == nullptr) return (int)cudaErrorUnknown;
-    const uint32_t n_tiles = (out_dim + 15u) / 16u;
-    uint32_t grid = (uint32_t)pdk_sm_count();
-    if (grid > n_tiles) grid = n_tiles;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(pl.split * pl.clusters);
+    cfg.blockDim = dim3(pl.W * pl.teams * 32u);
+    cfg.dynamicSmemBytes = pl.smem_bytes;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = pdk_pdl_enabled() ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = pl.split;
+    attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = SPLIT ? 2 : 1;
+    e = cudaLaunchKernelEx(&cfg, kern, m.dmap, m.hmap, m.rmap, (const uint8_t*)recs, bias, x, y, in_dim, out_dim, xq, xq_scale, po, pl, err);
+    return e == cudaSuccess ? pdk_launch_status() : (int)e;
+}
+
+// -1: outside the plan (rows of less than four units, planes that do not start on 16 bytes, activations too long), or the
+// register-staged kernel is faster.
+template <class F>
+int launch_ring(const void* data, const void* recs, const float* bias, const float* x, float* y, uint32_t in_dim,
+                uint32_t out_dim, cudaStream_t st, const int8_t* xq = nullptr, const float* xq_scale = nullptr,
+                const PeerOut* peers = nullptr) {
+    if (force_regs() || in_dim < 1024u || (in_dim & 255u) != 0u || out_dim > 0x40000000u) return -1;
+    const bool tma = recs_by_tma<F>(in_dim);
+    if (!pdk_aligned(recs, tma ? 16 : 8)) return -1;
+    // clusters of s CTAs that are resident at once: one CTA per SM, whatever the instance
+    static PdkClusterCaps table;
+    const uint32_t* cap = nullptr;
+    if (int rc = pdk_cluster_caps(table, (const void*)gemv_ring_kernel<F, false, false, true>, kMaxWarps * 32u, kSmemMax, &cap)) return rc;
+    // the plans of the shapes a thread met last
+    struct Known { const uint32_t* cap; uint32_t in_dim, out_dim, whole, ok; RingPlan plan; };
+    constexpr uint32_t kKnown = 32;
+    thread_local Known known[kKnown] = {};
+    const uint32_t whole = peers != nullptr ? 1u : 0u;
+    Known& k = known[(in_dim / 256u * 7u + out_dim / 8u + whole * 3u) % kKnown];
+    if (k.cap != cap || k.in_dim != in_dim || k.out_dim != out_dim || k.whole != whole) {
+        k = Known{cap, in_dim, out_dim, whole, 0u, RingPlan{}};
+        k.ok = make_plan<F>(in_dim, out_dim, whole != 0u, cap, k.plan) ? 1u : 0u;
+    }
+    if (k.ok == 0u) return -1;
+    const RingPlan& pl = k.plan;
+    const MapEntry* maps = nullptr;
+    if (plane_maps<F>(data, recs, in_dim, out_dim, &maps) != 0) return -1;
     PeerOut po{};
     if (peers) po = *peers;
-    return pdk_launch_pdl(kern, dim3(grid), dim3(pl.W * 32u), (size_t)pl.smem_bytes, st, maps->dmap, maps->rmap, bias, x, y,
-                          in_dim, out_dim, xq, xq_scale, po, pl, err);
+#define PDK_RING(M, A, S) return launch_plan<F, M, A, S>(*maps, recs, bias, x, y, in_dim, out_dim, st, xq, xq_scale, po, pl)
+    if constexpr (F::kMany) {
+        if (pl.teams > 1u || pl.W > kMaxWarps) {
+            if (pl.split > 1u) { if (tma) PDK_RING(true, false, true); else PDK_RING(true, true, true); }
+            if (tma) PDK_RING(true, false, false); else PDK_RING(true, true, false);
+        }
+    }
+    if constexpr (F::kRecBytes % 16u != 0u) {
+        if (!tma) { if (pl.split > 1u) PDK_RING(false, true, true); else PDK_RING(false, true, false); }
+    }
+    if (pl.split > 1u) PDK_RING(false, false, true);
+    PDK_RING(false, false, false);
+#undef PDK_RING
 }
 
 
@@ -816,6 +1093,7 @@ bool make_batch_plan(uint32_t in_dim, BatchPlan& p) {
 int pdk_q4k_gemv_i8_regs(const void*, const void*, const float*, float*, uint32_t, uint32_t, cudaStream_t);
 int pdk_q4_0_gemv_i8_regs(const void*, const void*, const float*, float*, uint32_t, uint32_t, cudaStream_t);
 int pdk_q5k_gemv_i8_regs(const void*, const void*, const float*, float*, uint32_t, uint32_t, cudaStream_t);
+int pdk_q6k_gemv_i8_regs(const void*, const void*, const float*, float*, uint32_t, uint32_t, cudaStream_t);
 int pdk_q8_0_gemv_i8_regs(const void*, const void*, const float*, const float*, float*, uint32_t, uint32_t, cudaStream_t);
 int pdk_q4k_gemv_i8_q8act_regs(const void*, const void*, const int8_t*, const float*, float*, uint32_t, uint32_t,
                                cudaStream_t);
@@ -841,7 +1119,13 @@ int pdk_q4_0_gemv_i8(const void* data, const void* scales, const float* x, float
 
 int pdk_q5k_gemv_i8(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim,
                     uint32_t out_dim, cudaStream_t st) {
-    return pdk_q5k_gemv_i8_regs(data, scales, x, y, in_dim, out_dim, st);
+    const int rc = launch_ring<RQ5K>(data, scales, nullptr, x, y, in_dim, out_dim, st);
+    return rc != -1 ? rc : pdk_q5k_gemv_i8_regs(data, scales, x, y, in_dim, out_dim, st);
+}
+
+int pdk_q6k_gemv_i8(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim, uint32_t out_dim, cudaStream_t st) {
+    const int rc = launch_ring<RQ6K>(data, scales, nullptr, x, y, in_dim, out_dim, st);
+    return rc != -1 ? rc : pdk_q6k_gemv_i8_regs(data, scales, x, y, in_dim, out_dim, st);
 }
 
 int pdk_q8_0_gemv_i8(const void* data, const void* scale, const float* bias, const float* x, float* y,
