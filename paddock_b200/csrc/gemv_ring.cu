@@ -81,7 +81,7 @@ __device__ __forceinline__ uint32_t word4(const uint4& v, uint32_t i) { return i
 struct RQ4K : Q4K {
     static constexpr uint32_t kDataBoxes = 1, kHighBytes = 0, kPasses = 2, kSub = 4, kBlock = 32;
     static constexpr bool kMany = true;
-    static constexpr float kStepCost = 0.055f, kManyCost = 0.05f, kRegsCost = 1.05f;   // make_plan
+    static constexpr float kStepCost = 0.048f, kManyCost = 0.057f, kRegsCost = 1.10f;   // make_plan
     // pass p of lane t feeds block 2t + p: the low (p = 0) or high nibbles of ggml group t, whose
     // first 16 bytes (chunk 2t) sit in k-slots 4t.. and whose second 16 (chunk 2t+1) in slots 16+4t..
     __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return 2u * t + p; }
@@ -112,7 +112,7 @@ struct RQ4K : Q4K {
 struct RQ40 : Q40 {
     static constexpr uint32_t kDataBoxes = 1, kHighBytes = 0, kPasses = 2, kSub = 4, kBlock = 32;
     static constexpr bool kMany = true;
-    static constexpr float kStepCost = 0.052f, kManyCost = 0.047f, kRegsCost = 0.95f;   // make_plan
+    static constexpr float kStepCost = 0.048f, kManyCost = 0.057f, kRegsCost = 0.83f;   // make_plan
     __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return 2u * t + p; }
     __device__ static __forceinline__ void a_pass(const Stage& s, uint32_t p, uint32_t j, uint32_t& a0, uint32_t& a1,
                                                   uint32_t& a2, uint32_t& a3) {
@@ -137,7 +137,7 @@ struct RQ80 : Q80 {
     static constexpr uint32_t kDataBoxes = 2;  // blocks 0..3 | blocks 4..7 of the unit
     static constexpr uint32_t kHighBytes = 0, kPasses = 2, kSub = 4, kBlock = 32;
     static constexpr bool kMany = false;       // two boxes a unit leave no room for the stages, and the loads spill
-    static constexpr float kStepCost = 0.096f, kManyCost = 0.0f, kRegsCost = 1.6f;   // make_plan
+    static constexpr float kStepCost = 0.093f, kManyCost = 0.0f, kRegsCost = 1.62f;   // make_plan
     // pass p of lane t feeds block t + 4p: box p holds blocks 4p..4p+3, chunk 2t its block t's first
     // 16 bytes (k-slots 4t..), chunk 2t+1 the second 16 (slots 16+4t..)
     __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return t + 4u * p; }
@@ -171,7 +171,7 @@ struct RQ5K : Q4K {
     static constexpr uint32_t kDataBytes = 160;
     static constexpr uint32_t kDataBoxes = 1, kHighBytes = 32, kPasses = 2, kSub = 4, kBlock = 32;
     static constexpr bool kMany = true;
-    static constexpr float kStepCost = 0.13f, kManyCost = 0.065f, kRegsCost = 1.45f;
+    static constexpr float kStepCost = 0.143f, kManyCost = 0.090f, kRegsCost = 1.32f;
     static constexpr int kHiShift = 0;
     struct Stage : Q4K::Stage {
         uint4 h[4];   // rows g, g + 8: the high-bit bytes, shifted so that block 2t's bit is bit 0
@@ -205,7 +205,7 @@ struct RQ6K {
     static constexpr uint32_t kDataBytes = 192, kRecBytes = 24;
     static constexpr uint32_t kDataBoxes = 1, kHighBytes = 64, kPasses = 4, kSub = 2, kBlock = 16;
     static constexpr bool kMany = true;
-    static constexpr float kStepCost = 0.13f, kManyCost = 0.065f, kRegsCost = 1.4f;
+    static constexpr float kStepCost = 0.143f, kManyCost = 0.090f, kRegsCost = 1.75f;
     static constexpr bool kUnsignedA = true;
     static constexpr int kHiShift = 0;
     struct Stage {
@@ -262,12 +262,12 @@ __device__ __forceinline__ void cp_async8_fill(uint32_t dst, const void* src, bo
 }
 
 // MANY: up to kManyWarps warps in one or more teams, the units of a pair one after the other; else one team of up to kMaxWarps.
-// RECS_ASYNC: a row's records are not a multiple of 16 bytes (an odd number of 24-byte records): the lanes copy them.
-// SPLIT: a cluster of pl.split CTAs shares its tiles and splits the pairs of a row.  (As template arguments: an instance that can
-// do it all takes 0.2 us longer to start and 5 % longer at N = 6016.)
-template <class F, bool MANY, bool RECS_ASYNC, bool SPLIT>
+// ODD: the last pair of a row is one unit and zeros; 24-byte records of such a row are not a multiple of 16 bytes, and the lanes copy them.
+// SPLIT: a cluster of pl.split CTAs shares its tiles and splits the pairs of a row.  (As template arguments: what an instance
+// does not need costs it 0.1 to 0.25 of its 3 to 5 us where there are few tiles.)
+template <class F, bool MANY, bool ODD, bool SPLIT>
 __global__ void __launch_bounds__((MANY ? kManyWarps : kMaxWarps) * 32u, 1)
-gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant__ CUtensorMap hmap, const __grid_constant__ CUtensorMap rmap,
+gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant__ CUtensorMap rmap, const __grid_constant__ CUtensorMap hmap,
                  const uint8_t* __restrict__ recs, const float* __restrict__ bias, const float* __restrict__ x, float* __restrict__ y,
                  uint32_t in_dim, uint32_t out_dim, const int8_t* __restrict__ xq, const float* __restrict__ xq_scale, const PeerOut peers,
                  const RingPlan pl, unsigned int* __restrict__ err) {
@@ -276,10 +276,12 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
     constexpr uint32_t kRecRow = 2u * F::kRecBytes;                 // a pair's records of one row
     constexpr uint32_t kStageHigh = 2u * kUnitData, kStageData = kStageHigh + 2u * kUnitHigh, kStageRec = 16u * kRecRow;
     constexpr uint32_t kPasses = F::kPasses, kSub = F::kSub;
+    constexpr bool RECS_ASYNC = ODD && F::kRecBytes % 16u != 0u;
     extern __shared__ __align__(1024) uint8_t smem[];
+    const uint32_t k_part = ODD || SPLIT ? pl.k_part : in_dim;
     uint8_t* xs_hi = smem;
-    uint8_t* xs_lo = smem + pl.k_part;
-    uint8_t* zeros = smem + 2u * (size_t)pl.k_part;
+    uint8_t* xs_lo = smem + k_part;
+    uint8_t* zeros = smem + 2u * (size_t)k_part;
     float2* xmeta = reinterpret_cast<float2*>(smem + pl.off_xmeta);
     const uint32_t tid = threadIdx.x, lane = tid & 31u;
     const uint32_t W = pl.W, D = pl.D;
@@ -295,7 +297,7 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
     volatile int* abort_flag = reinterpret_cast<volatile int*>(full + W * teams * kMaxDepth + 2u * teams * kRedBufs);
 
     const uint32_t split = SPLIT ? pl.split : 1u, rank = SPLIT ? blockIdx.x % split : 0u, cl = SPLIT ? blockIdx.x / split : blockIdx.x;
-    const uint32_t all_pairs = (in_dim + 511u) >> 9;
+    const uint32_t all_pairs = (ODD ? in_dim + 511u : in_dim) >> 9;
     const uint32_t p_lo = SPLIT ? rank * all_pairs / split : 0u, n_pair = (SPLIT ? (rank + 1u) * all_pairs / split : all_pairs) - p_lo;
     const uint32_t n_tiles = (out_dim + 15u) >> 4, n_cl = SPLIT ? pl.clusters : gridDim.x;
     const uint32_t tile_lo = (uint32_t)((uint64_t)cl * n_tiles / n_cl);
@@ -390,9 +392,9 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
     const bool invariant = pl.invariant != 0u;
     const uint32_t x0 = p_lo * 64u, x_groups = in_dim >> 3;     // groups of 8 elements before this part, of a row
     // what lies beyond the row's end counts as zero; the load itself is unconditional, so that two of them are in flight at once
-    auto load8 = [&](uint32_t grp, float (&v)[8]) { limb_load8(x, xq, xq_scale, min(x0 + grp, x_groups - 1u), v); };
+    auto load8 = [&](uint32_t grp, float (&v)[8]) { limb_load8(x, xq, xq_scale, ODD ? min(x0 + grp, x_groups - 1u) : x0 + grp, v); };
     auto store8 = [&](float (&v)[8], uint32_t grp) {
-        if (x0 + grp >= x_groups) {
+        if (ODD && x0 + grp >= x_groups) {
 #pragma unroll
             for (int i = 0; i < 8; ++i) v[i] = 0.0f;
         }
@@ -406,7 +408,7 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
         load8(g0, v0);
         load8(g0 + 32u, v1);
         while (issued < D && issued < total) issue_next();
-        if (team == 0u && warp < n_pair) {
+        if ((!MANY || team == 0u) && (!(MANY || SPLIT) || warp < n_pair)) {      // one team, no split: every warp has its pair
             store8(v0, g0);
             store8(v1, g0 + 32u);
         }
@@ -568,9 +570,11 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
         a += __shfl_xor_sync(0xffffffffu, a, 2);
         b += __shfl_xor_sync(0xffffffffu, b, 2);
         float* rbuf = red + (size_t)rb * (W * 16u);
-        if (pend != kNone && pend + kRedBufs == tl) poll_fold(true);   // the wait below is for this warp's own fold
-        if (alive && tl >= kRedBufs)
-            alive = __all_sync(0xffffffffu, tc5::mbar_wait(&red_free[rb], rb_phase ^ 1u, ctx, kErrRingFree, rb));
+        if (alive && tl >= kRedBufs) {
+            if (pend + kRedBufs == tl) poll_fold(true);   // the buffer waits for this warp's own fold
+            if (alive)
+                alive = __all_sync(0xffffffffu, tc5::mbar_wait(&red_free[rb], rb_phase ^ 1u, ctx, kErrRingFree, rb));
+        }
         if (alive) {
             if (t == 0u) {
                 rbuf[warp * 16u + g] = a;
@@ -645,10 +649,11 @@ bool ring_layout(RingPlan& p, uint32_t in_dim, uint32_t out_dim) {
 }
 
 // The split with the shortest estimate, in us; false where the register-staged kernel (gemv_i8.cu, gemv_q6k.cu) has a shorter one.
-//   one team     1.7 + steps (0.9 + kStepCost W): a step is a pair of a tile, and the longer the more warps share the SM
-//   many warps   2.0 + steps (0.75 + kManyCost warps) + 0.8 per tile of a team (its fold)
-//   split        0.5 more for two CTAs, 0.9 for more; 0.03 per pair of the part for the activations that every CTA converts
-//   registers    1.2 + rounds of 64 rows per SM x K / 1024 x kRegsCost, up to 1.35 times that when its four slots are full
+//   one team     1.3 + steps (1.03 + kStepCost W): a step is a pair of a tile, and the longer the more warps share the SM
+//   many warps   2.0 + steps (0.69 + kManyCost warps) + 1.7 per tile of a team (its fold)
+//   split        1.4 more for two CTAs, 2.2 for more
+//   registers    1.34 + rounds of 64 rows per SM x K / 1024 x kRegsCost, up to 1.33 times that when its four slots are full
+// Fitted to every split of 528 shapes (K = 1280 ... 17408, N = 520 ... 25600, all formats): 1.5 % over the best of them on average, 25 % at worst.
 // Measured (us; register kernel -> here): Q6_K 17152 x 1024 25.2 -> 8.1 (four CTAs), 9472 x 2560 15.6 -> 9.8, 5120 x 25600 23.5 -> 20.1; Q8_0
 // 5376 x 6016 11.7 -> 7.6, 17152 x 520 29.3 -> 5.3; Q4_K 9472 x 1024 12.0 -> 5.1; and the other way round Q4_K 1792 x 9792 6.1 -> 4.6.  Q4_K 5120 x
 // 25600: one team of ten 17.2, two of ten 17.5, four of five 15.6; 4096 x 25600: eight 14.5, six teams of three 13.0.
@@ -660,7 +665,7 @@ bool make_plan(uint32_t in_dim, uint32_t out_dim, bool whole, const uint32_t* ca
     for (uint32_t s = 1; s <= (whole ? 1u : kPdkMaxCluster) && s <= all; ++s) {
         if (cap[s] == 0u || s == 5u || s == 7u) continue;
         const uint32_t np = (all + s - 1u) / s, clusters = cap[s] < n_tiles ? cap[s] : n_tiles, per = (n_tiles + clusters - 1u) / clusters;
-        const float fixed = (s == 1u ? 0.0f : s == 2u ? 0.5f : 0.9f) + 0.03f * (float)np;
+        const float fixed = s == 1u ? 0.0f : s == 2u ? 1.4f : 2.2f;
         for (uint32_t rounds = 1; rounds <= 5u && rounds <= np; ++rounds) {
             const uint32_t W = (np + rounds - 1u) / rounds;
             if (W > kManyWarps) continue;
@@ -671,8 +676,8 @@ bool make_plan(uint32_t in_dim, uint32_t out_dim, bool whole, const uint32_t* ca
                 const bool many = T > 1u || n > kMaxWarps;
                 if (many && !F::kMany) continue;
                 const float steps = (float)(folds * rounds);
-                const float cost = fixed + (many ? 2.0f + steps * (0.75f + F::kManyCost * (float)n) + 0.8f * (float)folds
-                                                 : 1.7f + steps * (0.9f + F::kStepCost * (float)n));
+                const float cost = fixed + (many ? 2.0f + steps * (0.69f + F::kManyCost * (float)n) + 1.7f * (float)folds
+                                                 : 1.3f + steps * (1.03f + F::kStepCost * (float)n));
                 if (found && cost >= best_cost) continue;
                 RingPlan p{};
                 p.W = W; p.teams = T; p.split = s; p.clusters = clusters;
@@ -684,7 +689,7 @@ bool make_plan(uint32_t in_dim, uint32_t out_dim, bool whole, const uint32_t* ca
         }
     }
     const float fill = n_tiles < slots ? (float)n_tiles / (float)slots : 1.0f;
-    const float regs = 1.2f + (float)((n_tiles + slots - 1u) / slots) * (float)in_dim / 1024.0f * F::kRegsCost * (1.0f + 0.35f * fill);
+    const float regs = 1.34f + (float)((n_tiles + slots - 1u) / slots) * (float)in_dim / 1024.0f * F::kRegsCost * (1.0f + 0.33f * fill);
     return found && best_cost <= regs;
 }
 
@@ -743,10 +748,10 @@ int plane_maps(const void* data, const void* recs, uint32_t in_dim, uint32_t out
     return 0;
 }
 
-template <class F, bool MANY, bool RECS_ASYNC, bool SPLIT>
+template <class F, bool MANY, bool ODD, bool SPLIT>
 int launch_plan(const MapEntry& m, const void* recs, const float* bias, const float* x, float* y, uint32_t in_dim, uint32_t out_dim,
                 cudaStream_t st, const int8_t* xq, const float* xq_scale, const PeerOut& po, const RingPlan& pl) {
-    auto kern = gemv_ring_kernel<F, MANY, RECS_ASYNC, SPLIT>;
+    auto kern = gemv_ring_kernel<F, MANY, ODD, SPLIT>;
     static bool attr_set[64] = {false};  // per device, per instance
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -771,7 +776,7 @@ int launch_plan(const MapEntry& m, const void* recs, const float* bias, const fl
     attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = SPLIT ? 2 : 1;
-    e = cudaLaunchKernelEx(&cfg, kern, m.dmap, m.hmap, m.rmap, (const uint8_t*)recs, bias, x, y, in_dim, out_dim, xq, xq_scale, po, pl, err);
+    e = cudaLaunchKernelEx(&cfg, kern, m.dmap, m.rmap, m.hmap, (const uint8_t*)recs, bias, x, y, in_dim, out_dim, xq, xq_scale, po, pl, err);
     return e == cudaSuccess ? pdk_launch_status() : (int)e;
 }
 
@@ -804,17 +809,16 @@ int launch_ring(const void* data, const void* recs, const float* bias, const flo
     if (plane_maps<F>(data, recs, in_dim, out_dim, &maps) != 0) return -1;
     PeerOut po{};
     if (peers) po = *peers;
-#define PDK_RING(M, A, S) return launch_plan<F, M, A, S>(*maps, recs, bias, x, y, in_dim, out_dim, st, xq, xq_scale, po, pl)
+#define PDK_RING(M, O, S) return launch_plan<F, M, O, S>(*maps, recs, bias, x, y, in_dim, out_dim, st, xq, xq_scale, po, pl)
+    const bool odd = (in_dim & 511u) != 0u;
     if constexpr (F::kMany) {
         if (pl.teams > 1u || pl.W > kMaxWarps) {
-            if (pl.split > 1u) { if (tma) PDK_RING(true, false, true); else PDK_RING(true, true, true); }
-            if (tma) PDK_RING(true, false, false); else PDK_RING(true, true, false);
+            if (pl.split > 1u) { if (odd) PDK_RING(true, true, true); else PDK_RING(true, false, true); }
+            if (odd) PDK_RING(true, true, false); else PDK_RING(true, false, false);
         }
     }
-    if constexpr (F::kRecBytes % 16u != 0u) {
-        if (!tma) { if (pl.split > 1u) PDK_RING(false, true, true); else PDK_RING(false, true, false); }
-    }
-    if (pl.split > 1u) PDK_RING(false, false, true);
+    if (pl.split > 1u) { if (odd) PDK_RING(false, true, true); else PDK_RING(false, false, true); }
+    if (odd) PDK_RING(false, true, false);
     PDK_RING(false, false, false);
 #undef PDK_RING
 }
