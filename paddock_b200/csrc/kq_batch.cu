@@ -45,6 +45,7 @@ struct Args {
     const float* x;            // f32 activations, or null:
     const int8_t* xq;          // int8 activations ...
     const float* xq_scale;     // ... with one scale per 32 elements
+    const float* bias;         // [out_dim] or null
     float* y;
     uint32_t in_dim, out_dim, batch, stages, ku_max, round_tiles;
     unsigned int* err;
@@ -90,7 +91,7 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
     const tc5::WaitCtx ctx{abort_flag, a.err};
     uint8_t* box0 = smem + warp * a.stages * kBox0;
     uint8_t* box1 = smem + L.off_box1 + warp * a.stages * T::kBox1;
-    uint8_t* recs = smem + L.off_rec + warp * a.stages * kRecs;
+    uint8_t* recs = smem + L.off_rec + warp * a.stages * T::kRecs;
     float* red = reinterpret_cast<float*>(smem + L.off_red);
 
     pdk_pdl_launch_dependents();
@@ -105,15 +106,16 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
     const uint64_t stream_once = tc5::l2_policy_evict_first();
     uint32_t l_tile = 0u, l_u = 0u, rec_off[2];
     const uint8_t* rec_src = a.recs;
-    auto seek = [&](uint32_t tile, uint32_t u) {       // the 48 eight-byte pieces of a tile's records: one or two per lane
+    constexpr uint32_t kPieces = T::kRec / 8u, kCopies = (kRows * kPieces + 31u) / 32u;   // eight-byte pieces of a row's record, copies of a lane
+    auto seek = [&](uint32_t tile, uint32_t u) {
         l_tile = tile;
         l_u = u;
         const uint32_t row0 = min(tile * kRows, a.out_dim - 1u), last = a.out_dim - 1u - row0;
-        rec_src = a.recs + ((size_t)row0 * n_unit + u_lo + u) * 24u;
+        rec_src = a.recs + ((size_t)row0 * n_unit + u_lo + u) * T::kRec;
 #pragma unroll
-        for (uint32_t i = 0; i < 2u; ++i) {
-            const uint32_t c = i * 32u + lane, r = c / 3u;
-            rec_off[i] = min(r, last) * n_unit * 24u + (c - 3u * r) * 8u;
+        for (uint32_t i = 0; i < kCopies; ++i) {
+            const uint32_t c = i * 32u + lane, r = c / kPieces;
+            rec_off[i] = min(r, last) * n_unit * T::kRec + (c - kPieces * r) * 8u;
         }
     };
     auto issue = [&](uint32_t s) {
@@ -122,12 +124,12 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         tc5::tma_load_2d_hint_elect(box0 + s * kBox0, &tm0, &bars[s], (int32_t)(u * T::kUnit), (int32_t)(l_tile * kRows), stream_once);
         if constexpr (T::kBox1 != 0u)
             tc5::tma_load_2d_hint_elect(box1 + s * T::kBox1, &tm1, &bars[s], (int32_t)(u * T::kUnit + 128u), (int32_t)(l_tile * kRows), stream_once);
-        const uint32_t dst = tc5::smem_u32(recs + s * kRecs) + lane * 8u;
+        const uint32_t dst = tc5::smem_u32(recs + s * T::kRecs) + lane * 8u;
 #pragma unroll
-        for (uint32_t i = 0; i < 2u; ++i)
+        for (uint32_t i = 0; i < kCopies; ++i)
             if (i == 0u || lane < 16u) cp_async8(dst + i * 256u, rec_src + rec_off[i]);
         asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(tc5::smem_u32(&bars[s])) : "memory");
-        rec_src += 24;
+        rec_src += T::kRec;
         if (++l_u == ku) seek(l_tile + 1u, 0u);
     };
     uint32_t stage = 0u, phase = 0u;
@@ -228,13 +230,14 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         const float* ustep = reinterpret_cast<const float*>(smem + L.off_step);
         constexpr uint32_t kSteps = F == kQ6K ? 1u : 2u;
         constexpr float kBias = F == kQ6K ? 128.0f : 0.0f;
+        constexpr bool kF16Scales = F == kQ40 || F == kQ80;
 
         for (uint32_t q = 0; q < mine; ++q) {
             ok = __all_sync(0xffffffffu, ok && tc5::mbar_wait(&bars[stage], phase, ctx, tc5::kErrFullWait, 0x50u + warp));
             if (!ok) break;
             const uint8_t* b0 = box0 + stage * kBox0;
             const uint8_t* b1 = box1 + stage * T::kBox1;
-            const uint8_t* rb = recs + stage * kRecs + row * 24u;
+            const uint8_t* rb = recs + stage * T::kRecs + row * T::kRec;
             float U[NT][4];
 #pragma unroll
             for (uint32_t n = 0; n < NT; ++n)
@@ -244,17 +247,17 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 #pragma unroll
             for (uint32_t n = 0; n < NT; ++n) bp[n] = smem + L.off_b + col[n] * L.pitch + c_u * 1024u + t * 16u;
 
-            uint32_t sw[2][4];     // the scale bytes (Q6: raised by 128; Q4_0: eight f16 scales)
+            uint32_t sw[2][4];     // the scale bytes (Q6: raised by 128; Q4_0, Q8_0: eight f16 scales)
             uint2 high[2];         // Q5: the high-bit bytes 8t .. 8t+7
 #pragma unroll
             for (uint32_t h = 0; h < 2u; ++h) {
-                const uint32_t* rp = reinterpret_cast<const uint32_t*>(rb + h * 192u) + (F == kQ40 ? 0 : 1);
+                const uint32_t* rp = reinterpret_cast<const uint32_t*>(rb + h * 8u * T::kRec) + (kF16Scales ? 0 : 1);
 #pragma unroll
                 for (uint32_t i = 0; i < 4u; ++i)
-                    sw[h][i] = (F == kQ6K) ? rp[i] ^ 0x80808080u : (F == kQ40 || i < 2u) ? rp[i] : 0u;
+                    sw[h][i] = (F == kQ6K) ? rp[i] ^ 0x80808080u : (kF16Scales || i < 2u) ? rp[i] : 0u;
                 if constexpr (F == kQ5K) high[h] = *reinterpret_cast<const uint2*>(b1 + (row + h * 8u) * 32u + t * 8u);
             }
-            // A pair of blocks shares its bytes: the low nibbles' block and the high nibbles'
+            // A pair of blocks shares its bytes: the low nibbles' block and the high nibbles' (Q8_0: blocks p and 4 + p, of the two boxes)
 #pragma unroll
             for (uint32_t p = 0; p < T::kBlocks / 2u; ++p) {
                 // Q6: p = half * 4 + h * 2 + (run & 1)
@@ -268,16 +271,18 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                         x[h][0] = *reinterpret_cast<const uint32_t*>(b0 + r * 128u + ((c ^ (row & 7u)) << 4) + t * 4u);
                         z[h][0] = *reinterpret_cast<const uint32_t*>(b1 + r * 64u + (((2u * nh + hb) ^ ((row >> 1) & 3u)) << 4) + t * 4u);
                     } else {
-                        const uint2 v = *reinterpret_cast<const uint2*>(b0 + r * 128u + (((2u * p + (t >> 1)) ^ (row & 7u)) << 4) + (t & 1u) * 8u);
+                        const uint32_t at = r * 128u + (((2u * p + (t >> 1)) ^ (row & 7u)) << 4) + (t & 1u) * 8u;
+                        const uint2 v = *reinterpret_cast<const uint2*>(b0 + at);
                         x[h][0] = v.x;
                         x[h][kSteps - 1u] = v.y;
-                        z[h][0] = high[h].x;
-                        z[h][kSteps - 1u] = high[h].y;
+                        const uint2 w = F == kQ80 ? *reinterpret_cast<const uint2*>(b1 + at) : high[h];
+                        z[h][0] = w.x;
+                        z[h][kSteps - 1u] = w.y;
                     }
                 }
 #pragma unroll
                 for (uint32_t up = 0; up < 2u; ++up) {
-                    const uint32_t b = F == kQ6K ? 8u * nh + 2u * (r01 + 2u * up) + hb : 2u * p + up;
+                    const uint32_t b = F == kQ6K ? 8u * nh + 2u * (r01 + 2u * up) + hb : F == kQ80 ? 4u * up + p : 2u * p + up;
                     const uint32_t mq = up ? 0x00F000F0u : 0x000F000Fu;
                     float d[NT][4];
 #pragma unroll
@@ -290,6 +295,11 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                                 const uint32_t mh = up ? 0x03000300u : 0x00300030u, sh = r01 ? 2u : 4u;
                                 A[h] = (xv & mq) | ((zv << sh) & mh);
                                 A[2u + h] = ((xv >> 8) & mq) | ((zv >> (8u - sh)) & mh);
+                            } else if constexpr (F == kQ80) {
+                                // int8 raised by 128: 0..255, subnormal too
+                                const uint32_t wv = (up ? zv : xv) ^ 0x80808080u;
+                                A[h] = wv & 0x00FF00FFu;
+                                A[2u + h] = (wv >> 8) & 0x00FF00FFu;
                             } else {
                                 A[h] = xv & mq;
                                 A[2u + h] = (xv >> 8) & mq;
@@ -314,7 +324,10 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                     float s[2];
 #pragma unroll
                     for (uint32_t h = 0; h < 2u; ++h) {
-                        if constexpr (F == kQ40) {
+                        if constexpr (F == kQ80) {
+                            const __half2 v = *reinterpret_cast<const __half2*>(&sw[h][b >> 1]);
+                            s[h] = (b & 1u) ? __high2float(v) : __low2float(v);
+                        } else if constexpr (F == kQ40) {
                             const __half2 v = *reinterpret_cast<const __half2*>(&sw[h][p]);
                             s[h] = up ? __high2float(v) * 0.0625f : __low2float(v);
                         } else {
@@ -333,7 +346,7 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
             uint32_t A[4], dd[2];
 #pragma unroll
             for (uint32_t h = 0; h < 2u; ++h) {
-                const uint32_t* rp = reinterpret_cast<const uint32_t*>(rb + h * 192u);
+                const uint32_t* rp = reinterpret_cast<const uint32_t*>(rb + h * 8u * T::kRec);
                 dd[h] = rp[0];
                 if constexpr (F == kQ6K) {
                     // int8 scales as f16: 1024 + (sc + 128) by bit pattern, less 1152
@@ -342,7 +355,7 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                     const uint32_t f = __byte_perm(odd_w ? sw[h][3] : sw[h][2], 0x64646464u, sel);
                     A[h] = h2_bits(__hsub2(*reinterpret_cast<const __half2*>(&e), off));
                     A[2u + h] = h2_bits(__hsub2(*reinterpret_cast<const __half2*>(&f), off));
-                } else if constexpr (F == kQ40) {
+                } else if constexpr (kF16Scales) {
                     A[h] = A[2u + h] = rp[t];
                 } else {
                     A[h] = A[2u + h] = __byte_perm(rp[3u + (t >> 1)], 0u, sel);
@@ -361,7 +374,7 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 for (int i = 0; i < 4; ++i) {
                     const float dg = __low2float(dh[i >> 1]) * 16777216.0f;
                     float v;
-                    if constexpr (F == kQ40) v = fmaf(U[n][i], 16777216.0f, -8.0f * M[i]);
+                    if constexpr (kF16Scales) v = fmaf(U[n][i], 16777216.0f, (F == kQ80 ? -128.0f : -8.0f) * M[i]);
                     else if constexpr (F == kQ6K) v = dg * fmaf(-32.0f / 16777216.0f, M[i], U[n][i]);
                     else v = dg * U[n][i] - __high2float(dh[i >> 1]) * (M[i] * 16777216.0f);
                     acc[n][i] = fmaf((i & 1) ? so : se, v, acc[n][i]);
@@ -404,7 +417,7 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 const uint32_t owner = r / rpo;
                 st_cluster(cluster_addr(part, owner) + ((rank * a.batch + tok) * rpo + (r - owner * rpo)) * 4u, v);
             } else if (r0 * kRows + r < a.out_dim) {
-                a.y[(size_t)tok * a.out_dim + r0 * kRows + r] = v;
+                a.y[(size_t)tok * a.out_dim + r0 * kRows + r] = a.bias ? v + a.bias[r0 * kRows + r] : v;
             }
         }
         if (split > 1u) {
@@ -418,7 +431,7 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 const uint32_t tok = i / own, r = i - tok * own, n = r0 * kRows + rank * rpo + r;
                 float v = 0.0f;
                 for (uint32_t s = 0; s < split; ++s) v += got[(s * a.batch + tok) * rpo + r];
-                if (n < a.out_dim) a.y[(size_t)tok * a.out_dim + n] = v;
+                if (n < a.out_dim) a.y[(size_t)tok * a.out_dim + n] = a.bias ? v + a.bias[n] : v;
             }
         }
         if (r0 + a.round_tiles < t_hi) {
@@ -429,8 +442,8 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
 }
 
 template <int F, uint32_t NT>
-int launch(const void* data, const void* recs, const float* x, const int8_t* xq, const float* xq_scale, float* y, uint32_t in_dim,
-           uint32_t out_dim, uint32_t batch, cudaStream_t st) {
+int launch(const void* data, const void* recs, const float* bias, const float* x, const int8_t* xq, const float* xq_scale, float* y,
+           uint32_t in_dim, uint32_t out_dim, uint32_t batch, cudaStream_t st) {
     constexpr uint32_t kThreads = kWarps * 32u;
     auto kern = kq_batch_kernel<F, NT>;
     static PdkClusterCaps table;
@@ -448,7 +461,7 @@ int launch(const void* data, const void* recs, const float* x, const int8_t* xq,
     } else if constexpr (F == kQ6K) {
         if (int rc = pdk_make_tmap_2d_sw64(&t1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, data, pitch, out_dim, pitch, 64u, kRows)) return rc;
     }
-    const Args a{(const uint8_t*)recs, x, xq, xq_scale, y, in_dim, out_dim, batch, p.stages, p.ku, p.round_tiles, pdk_error_word()};
+    const Args a{(const uint8_t*)recs, x, xq, xq_scale, bias, y, in_dim, out_dim, batch, p.stages, p.ku, p.round_tiles, pdk_error_word()};
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(p.split, p.clusters);
     cfg.blockDim = dim3(kThreads);
@@ -469,9 +482,9 @@ int launch(const void* data, const void* recs, const float* x, const int8_t* xq,
 
 template <int F>
 int launch_f(const void* data, const void* recs, const float* x, const int8_t* xq, const float* xs, float* y, uint32_t in_dim,
-             uint32_t out_dim, uint32_t batch, cudaStream_t st) {
-    return batch <= 8u ? launch<F, 1>(data, recs, x, xq, xs, y, in_dim, out_dim, batch, st)
-                       : launch<F, 2>(data, recs, x, xq, xs, y, in_dim, out_dim, batch, st);
+             uint32_t out_dim, uint32_t batch, cudaStream_t st, const float* bias = nullptr) {
+    return batch <= 8u ? launch<F, 1>(data, recs, bias, x, xq, xs, y, in_dim, out_dim, batch, st)
+                       : launch<F, 2>(data, recs, bias, x, xq, xs, y, in_dim, out_dim, batch, st);
 }
 
 }  // namespace
@@ -489,4 +502,11 @@ int pdk_kq_batch(const void* data, const void* scales, const float* x, const int
         case 14u: return launch_f<kQ6K>(data, scales, x, xq, xq_scale, y, in_dim, out_dim, batch, st);
         default: return -1;
     }
+}
+
+// The same for repacked Q8_0 planes (data int8 [out_dim][in_dim], scale f16 [out_dim][in_dim / 32], bias [out_dim] or null).
+int pdk_kq_batch_q8(const void* data, const void* scale, const float* bias, const float* x, float* y, uint32_t in_dim, uint32_t out_dim,
+                    uint32_t batch, cudaStream_t st) {
+    if (batch == 0u || batch > 16u || in_dim == 0u || (in_dim & 255u) != 0u || out_dim > 0x40000000u || !pdk_aligned(scale, 8)) return -1;
+    return launch_f<kQ80>(data, scale, x, nullptr, nullptr, y, in_dim, out_dim, batch, st, bias);
 }

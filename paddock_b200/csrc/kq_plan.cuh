@@ -10,24 +10,25 @@
 
 namespace kq {
 
-enum Fmt : int { kQ4K = 0, kQ40 = 1, kQ5K = 2, kQ6K = 3 };
+enum Fmt : int { kQ4K = 0, kQ40 = 1, kQ5K = 2, kQ6K = 3, kQ80 = 4 };
 
 constexpr uint32_t kRows = 16;           // rows of a tile
 constexpr uint32_t kWarps = 16;          // of a CTA, whatever its column tiles (NT: tiles of 8 tokens, one or two)
 constexpr uint32_t kMaxSplit = 8;        // portable cluster size
 constexpr uint32_t kMaxStages = 6;
 constexpr uint32_t kSmemMax = 232448;    // 227 KB
-constexpr uint32_t kBox0 = kRows * 128u, kRecs = kRows * 24u;
+constexpr uint32_t kBox0 = kRows * 128u;
 
 template <int F>
 struct Fmts {
-    static constexpr uint32_t kUnit = F == kQ6K ? 192u : F == kQ5K ? 160u : 128u;   // data bytes of 256 weights
-    static constexpr uint32_t kBox1 = kRows * (kUnit - 128u);                         // the high bits' box
+    static constexpr uint32_t kUnit = F == kQ80 ? 256u : F == kQ6K ? 192u : F == kQ5K ? 160u : 128u;   // data bytes of 256 weights
+    static constexpr uint32_t kBox1 = kRows * (kUnit - 128u);                         // the high bits' box, or the second half's
     static constexpr uint32_t kBlocks = F == kQ6K ? 16u : 8u;
+    static constexpr uint32_t kRec = F == kQ80 ? 16u : 24u, kRecs = kRows * kRec;     // scale records, of a row and of a tile
     static constexpr uint32_t kStage = kBox0 + kBox1 + kRecs;
 };
 
-// Shared memory: ring ([warp][stage] boxes, then high-bit boxes, then records), the activation image, the partial tiles,
+// Shared memory: ring ([warp][stage] boxes, then second boxes, then records), the activation image, the partial tiles,
 // the barriers.  When a round's weights are consumed its ring takes the partial sums that other CTAs send.
 struct Layout {
     uint32_t off_box1, off_rec, off_b, pitch, off_step, off_xs, off_red, off_bar, total;
@@ -39,7 +40,7 @@ __host__ __device__ __forceinline__ Layout layout(uint32_t stages, uint32_t batc
     const uint32_t n = kWarps * stages;
     l.off_box1 = n * kBox0;
     l.off_rec = l.off_box1 + n * T::kBox1;
-    l.off_b = l.off_rec + n * kRecs;
+    l.off_b = l.off_rec + n * T::kRecs;
     l.pitch = ku * 1024u + 64u;            // the odd 64 bytes put two tokens' rows on distinct banks
     l.off_step = l.off_b + batch * l.pitch;
     l.off_xs = l.off_step + ((ku * batch * 4u + 15u) & ~15u);

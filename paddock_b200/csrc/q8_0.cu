@@ -11,6 +11,8 @@
 
 #include "pdk_common.cuh"
 
+int pdk_kq_batch_q8(const void* data, const void* scale, const float* bias, const float* x, float* y, uint32_t in_dim,
+                    uint32_t out_dim, uint32_t batch, cudaStream_t st);   // kq_batch.cu
 int pdk_q8_0_gemm_i8(const void* data, const void* scale, const float* bias, const float* x, float* y, uint32_t in_dim,
                      uint32_t out_dim, uint32_t batch, cudaStream_t st);
 int pdk_q8_0_gemv_i8(const void* data, const void* scale, const float* bias, const float* x, float* y,
@@ -158,6 +160,14 @@ PDK_EXPORT int pd_q8_0_gemv_repacked(const void* data, const void* scale, const 
     return dispatch<1>(data, scale, bias, (const float*)x, (float*)y, in_dim, out_dim, 0u, (cudaStream_t)stream);
 }
 
+// Where kq_batch.cu takes two and more tokens although the ring's plan holds.  From 9 tokens the ring reads the weights twice, and on narrow
+// planes that is all there is (us, ring / kq_batch: 5120 x 520, 9 tokens 10.4 / 7.0, 16 tokens 10.7 / 8.6; 5120 x 1800 12.1 / 10.8, 12.4 / 12.8);
+// up to four tokens on wide planes of short rows the ring is short of issue slots (2048 x 25600, 2 tokens 14.5 / 11.6; 4096 x 25600 22.0 / 18.8;
+// 5120 x 25600, 4 tokens 25.3 / 27.7).  Elsewhere the ring: 4096 x 6016, 8 tokens 8.0 / 11.4.
+static bool kq_beats_ring(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
+    return (batch >= 9u && batch <= 16u && out_dim <= 1024u) || (batch <= 4u && out_dim >= 16384u && in_dim <= 4096u);
+}
+
 PDK_EXPORT int pd_q8_0_gemm_repacked(const void* data, const void* scale, const void* bias, const void* x, void* y,
                                      uint32_t in_dim, uint32_t out_dim, uint32_t batch, void* stream) {
     if (out_dim == 0 || batch == 0) return 0;
@@ -166,11 +176,27 @@ PDK_EXPORT int pd_q8_0_gemm_repacked(const void* data, const void* scale, const 
     float* yf = (float*)y;
     auto st = (cudaStream_t)stream;
     if (!force_plain()) {
-        // two or more tokens: the tokens-as-columns kernel on the TMA ring (one weight pass per eight
-        // tokens); shapes outside its plan take one decode GEMV per token, which still beats the plain
+        // two or more tokens: the tokens-as-columns kernel on the TMA ring (K = 2048, 2560 ... 5632; one weight pass per eight
+        // tokens) or kq_batch.cu; shapes outside both plans take one decode GEMV per token, which still beats the plain
         // f32 kernel below (169 us per four tokens against 18 us per token at K=5120 N=17408)
-        int rc = batch >= 2u ? pdk_q8_0_gemm_i8(data, scale, (const float*)bias, xf, yf, in_dim, out_dim, batch, st) : -1;
+        int rc = batch >= 2u && !kq_beats_ring(in_dim, out_dim, batch)
+                     ? pdk_q8_0_gemm_i8(data, scale, (const float*)bias, xf, yf, in_dim, out_dim, batch, st) : -1;
         if (rc != -1) return rc;
+        uint32_t done = 0u;
+        while (batch >= 2u && in_dim >= 1024u && done < batch) {      // shorter rows belong to the f32 kernels
+            // passes of one width, or narrower ones where K is so long that the activations of 16 tokens do not fit
+            const uint32_t left = batch - done, passes = (left + 15u) / 16u;
+            uint32_t take = (left + passes - 1u) / passes;
+            for (rc = -1; rc == -1 && take != 0u;) {
+                rc = pdk_kq_batch_q8(data, scale, (const float*)bias, xf + (size_t)done * in_dim, yf + (size_t)done * out_dim, in_dim,
+                                     out_dim, take, st);
+                if (rc == -1) take = take > 8u ? 8u : take / 2u;
+            }
+            if (rc == -1) break;     // outside the plan at one token too, so nothing is done yet
+            if (rc != 0) return rc;
+            done += take;
+        }
+        if (done == batch) return 0;
         rc = 0;
         for (uint32_t t = 0; t < batch && rc == 0; ++t)
             rc = pdk_q8_0_gemv_i8(data, scale, (const float*)bias, xf + (size_t)t * in_dim, yf + (size_t)t * out_dim, in_dim,
