@@ -73,7 +73,9 @@ __device__ __forceinline__ float scale_f(uint32_t w, uint32_t i, bool up, float 
     return up ? fmaf(f, 0.0625f, -(8388608.0f + bias) * 0.0625f) : f - (8388608.0f + bias);
 }
 
-template <int F, uint32_t NT>
+// HL: up to four tokens.  The mma's columns are (token, term) pairs: one mma and an 8-byte fragment per step where a column per
+// token takes two mmas and 16 bytes, and the two terms' sums are added when a tile is done.
+template <int F, uint32_t NT, bool HL>
 __global__ void __launch_bounds__(kWarps * 32u, 1)
 kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__ CUtensorMap tm1, const Args a) {
     using T = Fmts<F>;
@@ -218,9 +220,9 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         uint32_t col[NT], even[NT], odd[NT];       // columns past the batch repeat its last token
 #pragma unroll
         for (uint32_t n = 0; n < NT; ++n) {
-            col[n] = min(g + 8u * n, a.batch - 1u);
-            even[n] = min(2u * t + 8u * n, a.batch - 1u);
-            odd[n] = min(2u * t + 1u + 8u * n, a.batch - 1u);
+            col[n] = min(HL ? g >> 1 : g + 8u * n, a.batch - 1u);
+            even[n] = min(HL ? t : 2u * t + 8u * n, a.batch - 1u);
+            odd[n] = HL ? even[n] : min(2u * t + 1u + 8u * n, a.batch - 1u);
         }
         float acc[NT][4];
 #pragma unroll
@@ -245,7 +247,7 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 for (int i = 0; i < 4; ++i) U[n][i] = 0.0f;
             const uint8_t* bp[NT];
 #pragma unroll
-            for (uint32_t n = 0; n < NT; ++n) bp[n] = smem + L.off_b + col[n] * L.pitch + c_u * 1024u + t * 16u;
+            for (uint32_t n = 0; n < NT; ++n) bp[n] = smem + L.off_b + col[n] * L.pitch + c_u * 1024u + t * 16u + (HL ? (g & 1u) * 8u : 0u);
 
             uint32_t sw[2][4];     // the scale bytes (Q6: raised by 128; Q4_0, Q8_0: eight f16 scales)
             uint2 high[2];         // Q5: the high-bit bytes 8t .. 8t+7
@@ -311,6 +313,12 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                                 }
                             }
                         }
+                        if constexpr (HL) {
+                            const uint2 v = *reinterpret_cast<const uint2*>(bp[0] + (b * kSteps + j) * 64u);
+                            if (j == 0u) mma_f16_z(d[0], A, v.x, v.y);
+                            else mma_f16(d[0], A, v.x, v.y);
+                            continue;
+                        }
                         uint4 v[NT];
 #pragma unroll
                         for (uint32_t n = 0; n < NT; ++n) v[n] = *reinterpret_cast<const uint4*>(bp[n] + (b * kSteps + j) * 64u);
@@ -366,8 +374,10 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
             for (uint32_t n = 0; n < NT; ++n) {
                 const uint32_t* xs = reinterpret_cast<const uint32_t*>(smem + L.off_xs + (c_u * a.batch + col[n]) * T::kBlocks * 4u);
                 float M[4];
-                mma_f16_z(M, A, xs[t], xs[4u + t]);      // Q4 / Q5: A twice along k, the high terms, then the low ones
-                if constexpr (F == kQ6K) mma_f16(M, A, xs[8u + t], xs[12u + t]);
+                const bool takes = !HL || (g & 1u) == 0u;     // the first term's column has both terms' sums
+                auto xsum = [&](uint32_t i) { return takes ? xs[i] : 0u; };
+                mma_f16_z(M, A, xsum(t), xsum(4u + t));      // Q4 / Q5: A twice along k, the high terms, then the low ones
+                if constexpr (F == kQ6K) mma_f16(M, A, xsum(8u + t), xsum(12u + t));
                 const float* st = ustep + c_u * a.batch;
                 const float se = st[even[n]], so = st[odd[n]];
 #pragma unroll
@@ -389,9 +399,14 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 float* dst = red + (size_t)(c_tile + warp) * kRows * NCOLS;
 #pragma unroll
                 for (uint32_t n = 0; n < NT; ++n) {
-                    float* to = dst + row * NCOLS + n * 8u + 2u * t;
-                    *reinterpret_cast<float2*>(to) = make_float2(acc[n][0], acc[n][1]);
-                    *reinterpret_cast<float2*>(to + 8u * NCOLS) = make_float2(acc[n][2], acc[n][3]);
+                    if constexpr (HL) {
+                        dst[row * NCOLS + t] = acc[n][0] + acc[n][1];
+                        dst[(row + 8u) * NCOLS + t] = acc[n][2] + acc[n][3];
+                    } else {
+                        float* to = dst + row * NCOLS + n * 8u + 2u * t;
+                        *reinterpret_cast<float2*>(to) = make_float2(acc[n][0], acc[n][1]);
+                        *reinterpret_cast<float2*>(to + 8u * NCOLS) = make_float2(acc[n][2], acc[n][3]);
+                    }
                     acc[n][0] = acc[n][1] = acc[n][2] = acc[n][3] = 0.0f;
                 }
                 c_u = 0u;
@@ -441,11 +456,11 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
     }
 }
 
-template <int F, uint32_t NT>
+template <int F, uint32_t NT, bool HL>
 int launch(const void* data, const void* recs, const float* bias, const float* x, const int8_t* xq, const float* xq_scale, float* y,
            uint32_t in_dim, uint32_t out_dim, uint32_t batch, cudaStream_t st) {
     constexpr uint32_t kThreads = kWarps * 32u;
-    auto kern = kq_batch_kernel<F, NT>;
+    auto kern = kq_batch_kernel<F, NT, HL>;
     static PdkClusterCaps table;
     const uint32_t* cap = nullptr;       // one CTA per SM
     if (int rc = pdk_cluster_caps(table, (const void*)kern, kThreads, kSmemMax, &cap)) return rc;
@@ -483,8 +498,9 @@ int launch(const void* data, const void* recs, const float* bias, const float* x
 template <int F>
 int launch_f(const void* data, const void* recs, const float* x, const int8_t* xq, const float* xs, float* y, uint32_t in_dim,
              uint32_t out_dim, uint32_t batch, cudaStream_t st, const float* bias = nullptr) {
-    return batch <= 8u ? launch<F, 1>(data, recs, bias, x, xq, xs, y, in_dim, out_dim, batch, st)
-                       : launch<F, 2>(data, recs, bias, x, xq, xs, y, in_dim, out_dim, batch, st);
+    if (batch <= 4u) return launch<F, 1, true>(data, recs, bias, x, xq, xs, y, in_dim, out_dim, batch, st);
+    return batch <= 8u ? launch<F, 1, false>(data, recs, bias, x, xq, xs, y, in_dim, out_dim, batch, st)
+                       : launch<F, 2, false>(data, recs, bias, x, xq, xs, y, in_dim, out_dim, batch, st);
 }
 
 }  // namespace
