@@ -271,13 +271,27 @@ bool kq_beats_i8(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
     return (uint64_t)out_dim * (in_dim + 2048u) <= limit;
 }
 
+// 9 and more tokens of Q4_K or Q4_0: both kernels' times in us, fitted to 560 timings (K = 1024 ... 12800, N = 520 ... 25600, 9 ... 32 tokens).
+// tcgen05 takes up to 32 tokens for one price: 4.3 us and 0.75 per super-block of a work item, 128 rows x all of K, or half of it where
+// that is whole box pairs (K % 1024 == 0); a narrow plane has fewer items than SMs.  kq_batch pays for weights x tokens, 16 tokens a
+// pass, but fills the chip whatever N is and has exact weights.  Measured (us, kq_batch / tcgen05): Q4_K 9728 x 1100, 9 tokens 11.0 / 31.6,
+// 16 tokens 12.6 / 31.8; 12800 x 5000, 12 tokens 31.8 / 40.7; 5120 x 2560, 16 tokens 12.6 / 12.4; 5120 x 25600, 16 tokens 53.7 / 30.3; 9728 x 520, 32 tokens 20.3 / 30.3.
+bool kq_beats_tc5(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
+    const uint32_t units = in_dim >> 8, split = (units & 3u) == 0u ? 2u : 1u, passes = (batch + 15u) / 16u, take = (batch + passes - 1u) / passes;
+    const float items = (float)((out_dim + 127u) / 128u * split), sms = 148.0f;
+    const float tc5 = (float)((batch + 31u) / 32u) * (4.3f + 0.75f * (float)(units / split) * ceilf(items / sms));
+    const float kq = (float)passes * (5.0f + (float)in_dim / 3000.0f + 0.1f * ((float)take - 9.0f) +
+                                      (float)out_dim * (float)in_dim * (2.25e-7f + 1.0e-8f * (float)take));
+    return kq < tc5;
+}
+
 // The kernel that a pass over `batch` tokens asks first.  Q4_0 up to 8 tokens: kq_batch against the tcgen05 kernel (which costs the same
 // at 4 and at 16 tokens) is 0.4 % off the faster one over 180 random shapes, up to 5 times faster, at most 18 % slower (K = 5120,
 // N = 25600: 26.4 / 29.2 us at 4 tokens; N = 9472: 16.2 / 15.2 at 8).  Q5_K from 9 tokens on: two passes of the integer kernel would
 // be faster on wide planes (K = 5120, N = 25600, 16 tokens: 51.6 against 64.5 us), but kq_batch keeps 22 activation bits.
 Route batch_route(uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t dtype) {
     const uint32_t from = dtype == PDK_KQ_Q4K ? tc5_min_tokens() : dtype == PDK_KQ_Q4_0 && tc5_min_tokens() != 0u ? 9u : 0u;
-    if (from != 0u && batch >= from) return kRouteTc5;
+    if (from != 0u && batch >= from) return kq_beats_tc5(in_dim, out_dim, batch) ? kRouteKq : kRouteTc5;
     if ((dtype == PDK_KQ_Q4K || dtype == PDK_KQ_Q5K) && batch <= 8u && !kq_beats_i8(in_dim, out_dim, batch)) return kRouteI8;
     return kRouteKq;
 }

@@ -40,7 +40,7 @@ int main() {
         for (unsigned n : {1u, 5u, 16u, 17u, 512u, 5003u, 27648u, 262144u, 1u << 24, (1u << 29) + 7u, 0x3fffffffu, 0x40000000u})
             for (unsigned b = 1; b <= 16; ++b)
                 for (const uint32_t* cap : {b200, part}) {
-                    all<kQ4K>(k, n, b, cap); all<kQ40>(k, n, b, cap); all<kQ5K>(k, n, b, cap); all<kQ6K>(k, n, b, cap);
+                    all<kQ4K>(k, n, b, cap); all<kQ40>(k, n, b, cap); all<kQ5K>(k, n, b, cap); all<kQ6K>(k, n, b, cap); all<kQ80>(k, n, b, cap);
                 }
     std::printf("%llu plans, %llu without\n", checked, refused);
     return checked > 5000 ? 0 : 2;
@@ -73,6 +73,10 @@ def test_routes_of_small_batches():
         assert route(5120, 25600, 1, dtype) == 0 and route(5120, 25600, 65, dtype) == 0
         assert route(1 << 30, 1 << 30, 8, dtype) == 1 and route(256, (1 << 32) - 1, 2, dtype) == 2
     assert [route(5120, 25600, m, q4_k) for m in (8, 9, 64)] == [2, 3, 3]
+    for dtype in (q4_k, q4_0):      # narrow planes, few of tcgen05's work items: kq_batch; 32 tokens are two of its passes
+        assert [route(9728, n, 9, dtype) for n in (1100, 7000, 9000)] == [1, 1, 3]
+        assert [route(9728, n, 32, dtype) for n in (520, 2560)] == [1, 3]
+        assert [route(5120, n, 16, dtype) for n in (1100, 5000)] == [1, 3]
     assert [route(5120, 25600, m, q5_k) for m in (8, 9, 64)] == [2, 1, 1]
     assert [route(5120, 25600, m, q4_0) for m in (2, 8, 9, 64)] == [1, 1, 3, 3]
     assert [route(5120, 25600, m, q6_k) for m in (2, 16, 64)] == [1, 1, 1]
