@@ -81,7 +81,7 @@ __device__ __forceinline__ uint32_t word4(const uint4& v, uint32_t i) { return i
 struct RQ4K : Q4K {
     static constexpr uint32_t kDataBoxes = 1, kHighBytes = 0, kPasses = 2, kSub = 4, kBlock = 32;
     static constexpr bool kMany = true;
-    static constexpr float kStepCost = 0.048f, kManyCost = 0.057f, kRegsCost = 1.10f;   // make_plan
+    static constexpr float kStepCost = 0.048f, kManyCost = 0.052f, kRegsCost = 0.90f;   // make_plan
     // pass p of lane t feeds block 2t + p: the low (p = 0) or high nibbles of ggml group t, whose
     // first 16 bytes (chunk 2t) sit in k-slots 4t.. and whose second 16 (chunk 2t+1) in slots 16+4t..
     __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return 2u * t + p; }
@@ -112,7 +112,7 @@ struct RQ4K : Q4K {
 struct RQ40 : Q40 {
     static constexpr uint32_t kDataBoxes = 1, kHighBytes = 0, kPasses = 2, kSub = 4, kBlock = 32;
     static constexpr bool kMany = true;
-    static constexpr float kStepCost = 0.048f, kManyCost = 0.057f, kRegsCost = 0.83f;   // make_plan
+    static constexpr float kStepCost = 0.048f, kManyCost = 0.052f, kRegsCost = 0.83f;   // make_plan
     __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return 2u * t + p; }
     __device__ static __forceinline__ void a_pass(const Stage& s, uint32_t p, uint32_t j, uint32_t& a0, uint32_t& a1,
                                                   uint32_t& a2, uint32_t& a3) {
@@ -137,7 +137,7 @@ struct RQ80 : Q80 {
     static constexpr uint32_t kDataBoxes = 2;  // blocks 0..3 | blocks 4..7 of the unit
     static constexpr uint32_t kHighBytes = 0, kPasses = 2, kSub = 4, kBlock = 32;
     static constexpr bool kMany = false;       // two boxes a unit leave no room for the stages, and the loads spill
-    static constexpr float kStepCost = 0.093f, kManyCost = 0.0f, kRegsCost = 1.62f;   // make_plan
+    static constexpr float kStepCost = 0.120f, kManyCost = 0.0f, kRegsCost = 1.91f;   // make_plan
     // pass p of lane t feeds block t + 4p: box p holds blocks 4p..4p+3, chunk 2t its block t's first
     // 16 bytes (k-slots 4t..), chunk 2t+1 the second 16 (slots 16+4t..)
     __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return t + 4u * p; }
@@ -171,7 +171,7 @@ struct RQ5K : Q4K {
     static constexpr uint32_t kDataBytes = 160;
     static constexpr uint32_t kDataBoxes = 1, kHighBytes = 32, kPasses = 2, kSub = 4, kBlock = 32;
     static constexpr bool kMany = true;
-    static constexpr float kStepCost = 0.143f, kManyCost = 0.090f, kRegsCost = 1.32f;
+    static constexpr float kStepCost = 0.127f, kManyCost = 0.087f, kRegsCost = 1.55f;
     static constexpr int kHiShift = 0;
     struct Stage : Q4K::Stage {
         uint4 h[4];   // rows g, g + 8: the high-bit bytes, shifted so that block 2t's bit is bit 0
@@ -205,7 +205,7 @@ struct RQ6K {
     static constexpr uint32_t kDataBytes = 192, kRecBytes = 24;
     static constexpr uint32_t kDataBoxes = 1, kHighBytes = 64, kPasses = 4, kSub = 2, kBlock = 16;
     static constexpr bool kMany = true;
-    static constexpr float kStepCost = 0.143f, kManyCost = 0.090f, kRegsCost = 1.75f;
+    static constexpr float kStepCost = 0.127f, kManyCost = 0.087f, kRegsCost = 1.49f;
     static constexpr bool kUnsignedA = true;
     static constexpr int kHiShift = 0;
     struct Stage {
@@ -649,23 +649,27 @@ bool ring_layout(RingPlan& p, uint32_t in_dim, uint32_t out_dim) {
 }
 
 // The split with the shortest estimate, in us; false where the register-staged kernel (gemv_i8.cu, gemv_q6k.cu) has a shorter one.
-//   one team     1.3 + steps (1.03 + kStepCost W): a step is a pair of a tile, and the longer the more warps share the SM
-//   many warps   2.0 + steps (0.69 + kManyCost warps) + 1.7 per tile of a team (its fold)
-//   split        1.4 more for two CTAs, 2.2 for more
-//   registers    1.34 + rounds of 64 rows per SM x K / 1024 x kRegsCost, up to 1.33 times that when its four slots are full
-// Fitted to every split of 528 shapes (K = 1280 ... 17408, N = 520 ... 25600, all formats): 1.5 % over the best of them on average, 25 % at worst.
+//   one team     1.19 + steps (1.035 + kStepCost W): a step is a pair of a tile, and the longer the more warps share the SM
+//   many warps   2.36 + steps (0.65 + kManyCost warps) + 1.61 per tile of a team (its fold)
+//   the stream   1.26 + 22 ns per KB of the CTA; the shorter of it and the above counts 4.4 % on top of the longer
+//   split        1.45 more for two CTAs, 2.18 for more
+//   registers    1.43 + rounds of 64 rows per SM x K / 1024 x kRegsCost, up to 1.32 times that when its four slots are full
+// Fitted to every split of 973 shapes (K = 1280 ... 17408, N = 520 ... 25600, all formats): 1.7 % over the best of them on average, 45 % at worst
+// (Q4_K 6912 x 520: 4.9 us, four CTAs 3.4).
 // Measured (us; register kernel -> here): Q6_K 17152 x 1024 25.2 -> 8.1 (four CTAs), 9472 x 2560 15.6 -> 9.8, 5120 x 25600 23.5 -> 20.1; Q8_0
 // 5376 x 6016 11.7 -> 7.6, 17152 x 520 29.3 -> 5.3; Q4_K 9472 x 1024 12.0 -> 5.1; and the other way round Q4_K 1792 x 9792 6.1 -> 4.6.  Q4_K 5120 x
 // 25600: one team of ten 17.2, two of ten 17.5, four of five 15.6; 4096 x 25600: eight 14.5, six teams of three 13.0.
 template <class F>
 bool make_plan(uint32_t in_dim, uint32_t out_dim, bool whole, const uint32_t* cap, RingPlan& best) {
     const uint32_t all = (in_dim + 511u) / 512u, n_tiles = (out_dim + 15u) / 16u, slots = 4u * cap[1];
+    constexpr float kPairKb = (float)(2u * (F::kDataBoxes * kBoxBytes + 16u * F::kHighBytes) + 32u * F::kRecBytes) / 1000.0f;
     float best_cost = 0.0f;
     bool found = false;
     for (uint32_t s = 1; s <= (whole ? 1u : kPdkMaxCluster) && s <= all; ++s) {
-        if (cap[s] == 0u || s == 5u || s == 7u) continue;
+        if (cap[s] == 0u || s == 5u || s == 7u || (s > 1u && n_tiles > 3u * cap[1])) continue;    // wide planes fill the chip unsplit
         const uint32_t np = (all + s - 1u) / s, clusters = cap[s] < n_tiles ? cap[s] : n_tiles, per = (n_tiles + clusters - 1u) / clusters;
-        const float fixed = s == 1u ? 0.0f : s == 2u ? 1.4f : 2.2f;
+        const float fixed = s == 1u ? 0.0f : s == 2u ? 1.45f : 2.18f;
+        const float stream = 1.26f + (float)((uint64_t)per * np) * kPairKb * 0.022f;
         for (uint32_t rounds = 1; rounds <= 5u && rounds <= np; ++rounds) {
             const uint32_t W = (np + rounds - 1u) / rounds;
             if (W > kManyWarps) continue;
@@ -676,8 +680,9 @@ bool make_plan(uint32_t in_dim, uint32_t out_dim, bool whole, const uint32_t* ca
                 const bool many = T > 1u || n > kMaxWarps;
                 if (many && !F::kMany) continue;
                 const float steps = (float)(folds * rounds);
-                const float cost = fixed + (many ? 2.0f + steps * (0.69f + F::kManyCost * (float)n) + 1.7f * (float)folds
-                                                 : 1.3f + steps * (1.03f + F::kStepCost * (float)n));
+                const float work = many ? 2.36f + steps * (0.65f + F::kManyCost * (float)n) + 1.61f * (float)folds
+                                        : 1.19f + steps * (1.035f + F::kStepCost * (float)n);
+                const float cost = fixed + (work > stream ? work + 0.044f * stream : stream + 0.044f * work);
                 if (found && cost >= best_cost) continue;
                 RingPlan p{};
                 p.W = W; p.teams = T; p.split = s; p.clusters = clusters;
@@ -689,7 +694,7 @@ bool make_plan(uint32_t in_dim, uint32_t out_dim, bool whole, const uint32_t* ca
         }
     }
     const float fill = n_tiles < slots ? (float)n_tiles / (float)slots : 1.0f;
-    const float regs = 1.34f + (float)((n_tiles + slots - 1u) / slots) * (float)in_dim / 1024.0f * F::kRegsCost * (1.0f + 0.33f * fill);
+    const float regs = 1.43f + (float)((n_tiles + slots - 1u) / slots) * (float)in_dim / 1024.0f * F::kRegsCost * (1.0f + 0.32f * fill);
     return found && best_cost <= regs;
 }
 
@@ -780,13 +785,13 @@ int launch_plan(const MapEntry& m, const void* recs, const float* bias, const fl
     return e == cudaSuccess ? pdk_launch_status() : (int)e;
 }
 
-// -1: outside the plan (rows of less than four units, planes that do not start on 16 bytes, activations too long), or the
+// -1: outside the plan (rows of up to four units: Q6_K 1024 x 618 2.2 us on registers, 2.5 here; planes that do not start on 16 bytes, activations too long), or the
 // register-staged kernel is faster.
 template <class F>
 int launch_ring(const void* data, const void* recs, const float* bias, const float* x, float* y, uint32_t in_dim,
                 uint32_t out_dim, cudaStream_t st, const int8_t* xq = nullptr, const float* xq_scale = nullptr,
                 const PeerOut* peers = nullptr) {
-    if (force_regs() || in_dim < 1024u || (in_dim & 255u) != 0u || out_dim > 0x40000000u) return -1;
+    if (force_regs() || in_dim <= 1024u || (in_dim & 255u) != 0u || out_dim > 0x40000000u) return -1;
     const bool tma = recs_by_tma<F>(in_dim);
     if (!pdk_aligned(recs, tma ? 16 : 8)) return -1;
     // clusters of s CTAs that are resident at once: one CTA per SM, whatever the instance
