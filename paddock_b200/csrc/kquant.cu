@@ -35,7 +35,7 @@ int pdk_q5k_gemv_i8(const void* data, const void* scales, const float* x, float*
 int pdk_iq4xs_gemv_i8(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim, uint32_t out_dim,
                       cudaStream_t st);  // gemv_i8.cu
 int pdk_q6k_gemv_i8(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim,
-                    uint32_t out_dim, cudaStream_t st);  // gemv_q6k.cu
+                    uint32_t out_dim, cudaStream_t st);  // gemv_ring.cu
 // kq_batch.cu: 1..16 tokens of every format here, f32 or int8 activations; -1 = shape outside its plan
 int pdk_kq_batch(const void* data, const void* scales, const float* x, const int8_t* xq, const float* xq_scale, float* y,
                  uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t dtype, cudaStream_t st);
@@ -272,14 +272,14 @@ bool kq_beats_i8(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
 }
 
 // 9 and more tokens of Q4_K or Q4_0: both kernels' times in us, fitted to 560 timings (K = 1024 ... 12800, N = 520 ... 25600, 9 ... 32 tokens).
-// tcgen05 takes up to 32 tokens for one price: 4.3 us and 0.75 per super-block of a work item, 128 rows x all of K, or half of it where
-// that is whole box pairs (K % 1024 == 0); a narrow plane has fewer items than SMs.  kq_batch pays for weights x tokens, 16 tokens a
+// tcgen05 takes up to 32 tokens for one price: 4.3 us and 0.75 per super-block of a CTA's run (q4k_tc5.cu: equal runs, or half tiles of 128 rows where
+// the plane has fewer of them than the chip has SMs).  kq_batch pays for weights x tokens, 16 tokens a
 // pass, but fills the chip whatever N is and has exact weights.  Measured (us, kq_batch / tcgen05): Q4_K 9728 x 1100, 9 tokens 11.0 / 31.6,
 // 16 tokens 12.6 / 31.8; 12800 x 5000, 12 tokens 31.8 / 40.7; 5120 x 2560, 16 tokens 12.6 / 12.4; 5120 x 25600, 16 tokens 53.7 / 30.3; 9728 x 520, 32 tokens 20.3 / 30.3.
 bool kq_beats_tc5(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
-    const uint32_t units = in_dim >> 8, split = (units & 3u) == 0u ? 2u : 1u, passes = (batch + 15u) / 16u, take = (batch + passes - 1u) / passes;
-    const float items = (float)((out_dim + 127u) / 128u * split), sms = 148.0f;
-    const float tc5 = (float)((batch + 31u) / 32u) * (4.3f + 0.75f * (float)(units / split) * ceilf(items / sms));
+    const uint32_t pairs = in_dim >> 9, tiles = (out_dim + 127u) / 128u, sms = 148u, passes = (batch + 15u) / 16u, take = (batch + passes - 1u) / passes;
+    const float run = tiles >= sms ? ceilf((float)tiles * (float)pairs / (float)sms) : 2u * tiles > sms ? (float)pairs : (float)((pairs + 1u) / 2u);   // of the busiest CTA
+    const float tc5 = (float)((batch + 31u) / 32u) * (4.3f + 1.5f * run);
     const float kq = (float)passes * (5.0f + (float)in_dim / 3000.0f + 0.1f * ((float)take - 9.0f) +
                                       (float)out_dim * (float)in_dim * (2.25e-7f + 1.0e-8f * (float)take));
     return kq < tc5;

@@ -12,12 +12,11 @@
 // splits it into two f16 terms x = hi + lo (exact for bf16-valued activations, 22 bits
 // otherwise), stored as 2 * tokens rows of a library-resident f16 matrix that TMA boxes are
 // cut from.  The accumulator [128 rows][hi columns | lo columns] stays in tensor memory over
-// the whole K range of a work item; the epilogue adds the two column groups, undoes the token
+// the whole of a run's part of a tile; the epilogue adds the two column groups, undoes the token
 // scale and adds into y.
 //
-// A work item is (128-row tile, half of K): twice as many items as tiles keeps 148 SMs evenly
-// loaded at 200 tiles.  The two halves of a tile add into y with red.global.add.f32; y is
-// zeroed by the kernel in front, and with exactly two addends per element the sum does not
+// A CTA takes a contiguous run of (tile, unit pair)s, cut at pairs, half tiles or tiles (range_start; launch picks).  A tile that two CTAs share is added into y by both with red.global.add.f32; y is
+// zeroed by the kernel in front, and with at most two addends per element the sum does not
 // depend on their order.
 //
 // What paces it (cycle counters in every role at 16 tokens): the tensor core.  A kind::f16 MMA with the
@@ -322,11 +321,23 @@ __device__ __forceinline__ void dequant_regs(const uint4& q, const SlabScale& sc
     }
 }
 
+// Where CTA c's run of unit pairs starts; the pairs of tile t are t ppt .. (t + 1) ppt.  Cut: equal runs of pairs (no run shorter than a tile),
+// half tiles, or whole tiles.  Either way a tile has at most two CTAs, and the sum of two addends on a zeroed y does not
+// depend on their order.
+enum Cut : uint32_t { kCutPairs = 0u, kCutHalves = 1u, kCutTiles = 2u };
+__device__ __forceinline__ uint32_t range_start(uint32_t c, uint32_t grid, uint32_t out_dim, uint32_t ppt, uint32_t cut) {
+    const uint32_t tiles = (out_dim + BM - 1u) / BM;
+    if (cut == kCutPairs) return (uint32_t)((uint64_t)c * tiles * ppt / grid);
+    if (cut == kCutTiles) return (uint32_t)((uint64_t)c * tiles / grid) * ppt;
+    const uint32_t h = (uint32_t)((uint64_t)c * 2u * tiles / grid);
+    return (h >> 1) * ppt + (h & 1u) * (ppt >> 1);
+}
+
 template <uint32_t NC, bool Q40>
 __global__ void __launch_bounds__(kThreads, 1)
 q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                const __grid_constant__ CUtensorMap tmap_r, const float* __restrict__ tokscale, float* __restrict__ y,
-               uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t ksplit, unsigned int* err_word) {
+               uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t cut, unsigned int* err_word) {
     using C = Cfg<NC>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
@@ -335,8 +346,8 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
     Shared* sh = reinterpret_cast<Shared*>(tiles + kStages * C::kStageBytes);
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t n_unit = in_dim >> 8, upi = n_unit / ksplit;  // units per item (even)
-    const uint32_t n_items = ((out_dim + BM - 1u) / BM) * ksplit;
+    const uint32_t ppt = in_dim >> 9;                            // unit pairs (weight boxes) of a tile
+    const uint32_t p_lo = range_start(blockIdx.x, gridDim.x, out_dim, ppt, cut), p_hi = range_start(blockIdx.x + 1u, gridDim.x, out_dim, ppt, cut);
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < kRawStages; ++s) {
@@ -382,10 +393,10 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         const uint32_t qd = pw & 3u, hf = pw >> 2;
         const uint32_t r_in = qd * 32u + lane, swz = r_in & 7u;
         const uint32_t line_off = (r_in >> 3) * 1024u + swz * 128u;  // the row's 128-byte line in a weight box
-        const uint32_t my_items = blockIdx.x < n_items ? (n_items - blockIdx.x + gridDim.x - 1u) / gridDim.x : 0u;
-        const uint32_t total = my_items * upi;
+        const uint32_t total = 2u * (p_hi - p_lo);
+        uint32_t tile = p_lo / ppt, seg_end = min(p_hi, (tile + 1u) * ppt) - p_lo, iter = 0u;   // the part of this tile ends here
         bool ok = true;
-        // unit n of this CTA's sequence: box n / 2 (unit n % 2 of it: upi is even, so that is the set), operand
+        // unit n of this CTA's sequence: box n / 2 (unit n % 2 of it, so that is the set), operand
         // stage n % kStages
         for (uint32_t n = set; n < total && ok; n += kProdSets) {
             const uint32_t j = n & 1u, box = n >> 1;
@@ -429,18 +440,17 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                 tc5::mbar_arrive(&sh->full[stage]);
                 tc5::mbar_arrive(&sh->raw_empty[rs]);  // every lane has consumed its bytes of the box
             }
-            if (n % upi + kProdSets >= upi && warp < 4u) {
-                // ---- set 0 has written its last unit of the item: warps 0..3 drain the item's accumulator
+            if (box + 1u == seg_end) {
+                // ---- set 0 has written its last unit of the tile's part: warps 0..3 drain the accumulator
                 // (full once set 1's last unit has gone through the tensor core too)
-                {
-                    const uint32_t iter = n / upi, c_item = blockIdx.x + iter * gridDim.x;
+                if (warp < 4u) {
                     const uint32_t buf = iter & 1u, aphase = (iter >> 1) & 1u;
                     if (iter == 0u) pdk_pdl_wait();  // tokscale and the zeroed y are the previous kernel's output
                     ok = mbar_wait_park(&sh->tmem_full[buf], aphase, ctx, tc5::kErrTmemFullWait, buf);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     tc5::fence_after_sync();
-                    const uint32_t row = (c_item / ksplit) * BM + warp * 32u + lane;
+                    const uint32_t row = tile * BM + warp * 32u + lane;
                     constexpr uint32_t HC = NC / 2u;  // token columns
 #pragma unroll 1
                     for (uint32_t t0 = 0; t0 < HC; t0 += 16u) {
@@ -462,6 +472,9 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
                     __syncwarp();
                     if (lane == 0) tc5::mbar_arrive(&sh->tmem_empty[buf]);
                 }
+                ++tile;
+                ++iter;
+                seg_end = min(p_hi, (tile + 1u) * ppt) - p_lo;
             }
         }
     } else if (warp == kRawWarp) {
@@ -469,8 +482,9 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         // Weights depend on nothing the previous kernel in the stream writes: no wait for it.
         uint32_t rs = 0, rphase = 0;
         bool ok = true, waited = false;
-        for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const uint32_t row0 = (item / ksplit) * BM, u0 = (item % ksplit) * upi;
+        for (uint32_t at = p_lo; at < p_hi && ok;) {
+            const uint32_t tile = at / ppt, row0 = tile * BM, u0 = 2u * (at - tile * ppt), upi = 2u * (min(p_hi, (tile + 1u) * ppt) - at);
+            at += upi >> 1;
             for (uint32_t u = 0; u < upi; u += 2u) {
                 ok = mbar_wait_park(&sh->raw_empty[rs], rphase ^ 1u, ctx, tc5::kErrEmptyWait, 0x20u + rs);
                 ok = __all_sync(0xffffffffu, ok);
@@ -501,8 +515,9 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         uint32_t stage = 0, phase = 0;
         bool ok = true;
         pdk_pdl_wait();  // the f16 rows are the previous kernel's output
-        for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-            const uint32_t u0 = (item % ksplit) * upi;
+        for (uint32_t at = p_lo; at < p_hi && ok;) {
+            const uint32_t tile = at / ppt, u0 = 2u * (at - tile * ppt), upi = 2u * (min(p_hi, (tile + 1u) * ppt) - at);
+            at += upi >> 1;
             for (uint32_t u = 0; u < upi; ++u) {
                 ok = mbar_wait_park(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, 0x10u + stage);
                 ok = __all_sync(0xffffffffu, ok);
@@ -522,7 +537,9 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         // ------------------------------------------------------------ MMA issuer (whole warp, one lane issues)
         uint32_t stage = 0, phase = 0, iter = 0, rs = 0, rphase = 0;
         bool ok = true;
-        for (uint32_t item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++iter) {
+        for (uint32_t at = p_lo; at < p_hi && ok; ++iter) {
+            const uint32_t upi = 2u * (min(p_hi, (at / ppt + 1u) * ppt) - at);
+            at += upi >> 1;
             const uint32_t buf = iter & 1u, aphase = (iter >> 1) & 1u;
             ok = mbar_wait_park(&sh->tmem_empty[buf], aphase ^ 1u, ctx, tc5::kErrTmemEmptyWait, buf);
             ok = __all_sync(0xffffffffu, ok);
@@ -600,13 +617,24 @@ int launch(const void* data, const void* recs, const float* x, const int8_t* xq,
     if (int rc = pdk_launch_pdl(q4k_act_f16_kernel, dim3(NC / 2u + kZeroCtas), dim3(kActThreads), 0, st, x, xq, xq_scale, xh,
                                 tokscale, y, in_dim, out_dim, batch, NC / 2u))
         return rc;
-    // two K halves per tile when each half is a whole number of record boxes
-    const uint32_t ksplit = (n_unit & 3u) == 0u ? 2u : 1u;
-    const uint32_t n_items = ((out_dim + BM - 1u) / BM) * ksplit;
-    uint32_t grid = (uint32_t)pdk_sm_count();
-    if (grid > n_items) grid = n_items;
+    // Half tiles where the plane has at most half a tile per SM (also of an odd number of pairs: 9728 x 6528, 9 tokens 31.6 us whole, 19.5 in halves), whole
+    // tiles up to one per SM.  From there runs or whole tiles by the busiest CTA's estimate: 1.5 us per pair, 1.3 per tile that it touches
+    // (its accumulator is drained while nothing is produced), 0.5 for runs.  4608 x 19968, 10 tokens: whole tiles 32.2 us, runs 22.7;
+    // 1536 x 25856, 20 tokens: 15.9, 17.3; 5120 x 25600, 16 tokens: half tiles in turn 30.1, runs 29.8.
+    const uint32_t tiles = (out_dim + BM - 1u) / BM, sms = (uint32_t)pdk_sm_count(), ppt = n_unit >> 1;
+    uint32_t cut = kCutTiles, grid = tiles;
+    if (2u * tiles <= sms && ppt >= 2u) {
+        cut = kCutHalves;
+        grid = 2u * tiles;
+    } else if (tiles > sms) {
+        const uint32_t whole = (tiles + sms - 1u) / sms;
+        const uint64_t run = ((uint64_t)tiles * ppt + sms - 1u) / sms;
+        const float by_tiles = (1.5f * (float)ppt + 1.3f) * (float)whole, by_pairs = 1.5f * (float)run + 1.3f * (float)(whole + 1u) + 0.5f;
+        cut = by_tiles <= by_pairs ? kCutTiles : kCutPairs;
+        grid = sms;
+    }
     return pdk_launch_pdl(kern, dim3(grid), dim3(kThreads), smem, st, tx, tw, tr, (const float*)tokscale, y, in_dim,
-                          out_dim, batch, ksplit, pdk_error_word());
+                          out_dim, batch, cut, pdk_error_word());
 }
 
 }  // namespace
