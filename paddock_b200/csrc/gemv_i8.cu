@@ -279,7 +279,8 @@ int launch(const void* data, const void* recs, const float* bias, const float* x
 
 }  // namespace
 
-// The register-staged kernel: the route for the shapes the ring kernel (gemv_ring.cu) declines.
+// The register-staged kernel: the route for short rows, where it starts faster than the ring kernel (gemv_ring.cu, make_plan), and for
+// what that one declines.
 // All return 0 / a cudaError_t, or -1 when the shape is outside this kernel's plan too (K not a
 // multiple of 256, fewer than four units per row, or activations too long for shared memory).
 int pdk_q4k_gemv_i8_regs(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim,

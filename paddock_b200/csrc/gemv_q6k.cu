@@ -1,4 +1,5 @@
-// gemv_q6k.cu - single-token decode GEMV for repacked Q6_K planes on the int8 tensor path.
+// gemv_q6k.cu - single-token decode GEMV for repacked Q6_K planes on the int8 tensor path, operands in registers: the route for
+// short rows and for what the ring kernel (gemv_ring.cu) declines.
 //
 // Q6_K: 256 weights per super-block as 16 blocks of 16, w = d * sc[block] * (q - 32) with 6-bit
 // codes q (low nibbles in ql[128], two high bits in qh[64]), int8 block scales and one f16 d.

@@ -1,4 +1,4 @@
-// gemv_ring.cu - single-token decode GEMV for Q4_K, Q4_0 and Q8_0 planes with the weights staged
+// gemv_ring.cu - single-token decode GEMV for Q4_K, Q5_K, Q6_K, Q4_0 and Q8_0 planes with the weights staged
 // in shared memory by TMA, every warp running its own ring.
 //
 // The arithmetic is that of gemv_i8.cu (integer dot products on mma m16n8k32, activations as two
@@ -10,10 +10,12 @@
 // the warps hold in registers, and requests them at kernel start, before the wait on the previous
 // kernel in the stream (programmatic dependent launch).
 //
-//   * A CTA (one per SM) owns a contiguous range of 16-row tiles; warp w takes units w, w + W, ...
-//     of every tile (unit = 256 weights of a row).  Per (tile, unit) the warp's elected lane issues
-//     one 2-D TMA copy of the 16 rows x 128 bytes of packed weights (two for Q8_0's 256 bytes) and
-//     one of the rows' scale records.  The planes stay in the byte layout the repack slots write
+//   * A CTA (one per SM) owns a contiguous range of 16-row tiles, its teams of W warps take them in turn, and warp w of a team
+//     takes pairs w, w + W, ... of a tile (pair = two units, unit = 256 weights of a row; the last pair of an odd row is
+//     half zeros).  On narrow planes of long rows a cluster of CTAs shares the tiles and splits the pairs, and the sums meet in
+//     distributed shared memory.  Per (tile, pair) the warp's elected lane issues
+//     2-D TMA copies of the 16 rows x 128 bytes of packed weights of each unit (two for Q8_0's 256 bytes; a second box for the high bits of
+//     Q5_K and Q6_K) and one of the rows' scale records.  The planes stay in the byte layout the repack slots write
 //     (super-block local: the engine concatenates planes at super-block offsets); the tensor maps
 //     describe them as [rows][row bytes].
 //   * The weight boxes are written with the 128-byte swizzle, which puts the 16-byte chunks that
@@ -22,10 +24,10 @@
 //   * A warp is the only reader of its stages: it waits on its own mbarrier, moves the fragments
 //     to registers, and re-arms the stage itself after the mma sequence has consumed them.  No
 //     producer warp, no cross-warp hand-shake in the weight path, so a warp that falls behind
-//     delays nobody's loads.  When W equals the units of a row (K = 5120: 20 warps) a warp meets
+//     delays nobody's loads.  When W equals the pairs of a row (one team) a warp meets
 //     the same slice of the activations in every tile and keeps its B operand in registers.
-//   * Per tile each warp leaves 16 partial row sums in one of kRedBufs shared buffers and arrives
-//     on the buffer's mbarrier without waiting; warp (tile mod W) adds the W partials in warp order
+//   * Per tile each warp leaves 16 partial row sums in one of the team's kRedBufs shared buffers and arrives
+//     on the buffer's mbarrier without waiting; warp (tile mod W) of the team adds the W partials in warp order
 //     once they are all there - it looks once per iteration - and stores y (or, row sharded, the
 //     band into every rank's y).
 //

@@ -1,4 +1,4 @@
-// kq_batch.cu - Q4_K, Q5_K, Q6_K and Q4_0 planes times 1..16 tokens per launch on mma.sync f16, weights exact.
+// kq_batch.cu - Q4_K, Q5_K, Q6_K, Q4_0 and Q8_0 planes times 1..16 tokens per launch on mma.sync f16, weights exact.
 //
 // The work is a stream of weights; what the kernel is built around is what it costs to get a weight byte in front of
 // the tensor core and a scale behind it:
@@ -8,12 +8,13 @@
 //     34 requests that touch eight rows each, and the L1 request rate (about 270 cycles a unit) set the time;
 //   * a code is its own f16 operand: the bit pattern of q in 0..63 is the subnormal number q 2^-24, which the tensor core
 //     multiplies exactly.  A high nibble stays where it is (16 q 2^-24; its block's scale is divided by 16), so two weights
-//     cost one AND (an AND-OR with the high bits of Q5_K / Q6_K) and no conversion;
+//     cost one AND (an AND-OR with the high bits of Q5_K / Q6_K) and no conversion.  Q8_0's int8 codes are raised by 128 on the way (XOR);
 //   * activations: per token and unit a power of two brings the largest element below 2^10, and x = hi + lo in two f16
 //     terms (22 bits, exact for bf16 values).  Both terms accumulate into one f32 tile, so a block is folded into the unit's
 //     sum with four FFMAs per 16 x 8 tile (an int8 fold takes eight IMADs at half their rate, and an s8 m16n8k16 for
-//     Q6_K's 16-weight blocks takes the tensor pipe as long, 8 cycles, as an f16 one);
-//   * the min term (Q4_K, Q5_K), the -32 (Q6_K) and the -8 (Q4_0) are products of the block scales with the block
+//     Q6_K's 16-weight blocks takes the tensor pipe as long, 8 cycles, as an f16 one).  Up to four tokens the terms are columns of
+//     their own: one mma and half the fragment bytes per step;
+//   * the min term (Q4_K, Q5_K), the -32 (Q6_K), the -8 (Q4_0) and the -128 (Q8_0) are products of the block scales with the block
 //     sums of x: one or two more MMAs per unit.
 //
 // Split: a cluster of S CTAs shares a run of 16-row tiles, each CTA one part of K - its part of the activations (4 bytes
@@ -22,10 +23,10 @@
 // tile that it touched, and the partials meet once per round (as many tiles as shared memory holds partials of; one, mostly), in a fixed order, across the cluster in distributed
 // shared memory: the same sum whatever the timing, no scratch, no zeroing of y, one launch.
 //
-// Measured on a B200 (us, before -> here).  Q6_K, K = 17408, N = 5003: 56.4 -> 28.4 at 2 tokens, 114 -> 28.8 at 4, 226 -> 34.1 at 8 (the
-// activations did not fit one CTA: a GEMV per token); K = 5120, N = 25600: 40.9 -> 33 at 2, 41.3 -> 38 at 8, 82.5 -> 76 at 16;
-// N = 1024: 15.2 -> 6.5 at 2, 30 -> 10.1 at 16.  Q4_K, K = 17408, N = 5120: 81.1 -> 23.7 at 2.  What bounds it now: the shared
-// memory pipe (118 wavefronts per unit, 64 of them the activation fragments: 13 of the 25 us of Q4_K, K = 5120, N = 25600) and
+// Measured on a B200 (us; up to 4 tokens: terms as two mmas -> as columns).  Q6_K, K = 17408, N = 5003: 28.2 -> 26.0 at 2 tokens, 27.8 -> 25.6 at 3,
+// 28.7 -> 26.5 at 4, 34.1 at 8; K = 5120, N = 25600: 33.2 -> 30.4 at 2, 38 at 8, 76 at 16.  Q4_K, K = 17408, N = 5120: 23.6 -> 20.6 at 2; Q4_0, K = 5120,
+// N = 25600: 25.4 -> 21.5.  Q8_0 (a GEMV per token before): 7424 x 520, 8 tokens 108 -> 6.7; 2816 x 6016, 16 tokens 96 -> 16.  What bounds it from 5 tokens: the shared
+// memory pipe (118 wavefronts per unit, 64 of them the activation fragments: 13 of the 25 us of Q4_K, K = 5120, N = 25600 at 2 tokens with two mmas) and
 // issue slots (450 instructions per unit).  Tiles of 32 rows halve the fragments but double the ring's stages, so that
 // fewer fit: 24.7 us at 1 token, but 45 at 8 and no plan at all for Q6_K, not kept.
 #include "cluster_caps.cuh"

@@ -127,8 +127,8 @@ def test_q4_k_gemv_shapes(pack, k, n):
 
 
 # Shapes chosen for the ring-staged decode GEMV's plans: 8 units per row (the smallest it takes),
-# stages that do not divide the row (18, 22, 68, 108 units), an odd unit count (43: the ring
-# kernel declines Q4_K's 24-byte records there and the register-staged kernel runs), fewer than 16
+# stages that do not divide the row (18, 22, 68, 108 units), an odd unit count (43: the lanes
+# copy Q4_K's 24-byte records there), fewer than 16
 # rows, a last tile of one row, and more tiles than SMs so that the ring wraps many times.
 RING_SHAPES = [(2048, 7), (2048, 4099), (4608, 33), (5632, 100), (11008, 49), (17408, 161), (27648, 40), (4096, 16 * 148 * 3 + 1)]
 
