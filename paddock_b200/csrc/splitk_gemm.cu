@@ -12,7 +12,7 @@
 // cluster of S CTAs shares it, each summing every S-th part of K.  The partial accumulators meet
 // through distributed shared memory and are added in rank order: same sum whatever the timing, no
 // scratch, no zeroing, no second launch.  Where K is short or the tokens are many the meeting costs more
-// than the split saves: one CTA takes the tile and stores it from tensor memory (launch_bn has the line).
+// than the split saves: one CTA takes the tile and stores it from tensor memory (plan_split has the line).
 //
 // Two CTAs share an SM (about 100 KB of stages and at most half the tensor memory each): while one meets
 // its cluster and stores, the other streams, and a CTA's start-up (barriers, tensor memory, first boxes)
@@ -341,31 +341,40 @@ splitk_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     }
 }
 
+// The CTAs that share a tile of BN tokens (the split of K) in a call: 0 or a cudaError_t.
 template <int KIND, uint32_t BN, typename TO>
-int launch_bn(const void* data, const void* xq, Args& a, uint32_t row_bytes, cudaStream_t st) {
-    using C = Cfg<KIND, BN>;
-    CUtensorMap tw, tx;
-    if (int rc = pdk_make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, data, row_bytes, a.out_dim, row_bytes, BKB, BM)) return rc;
-    if (int rc = pdk_make_tmap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, row_bytes, a.batch, row_bytes, BKB, BN)) return rc;
-    auto kern = splitk_gemm_kernel<KIND, BN, TO>;
+int plan_split(const Args& a, uint32_t& split, uint32_t& sms) {
     // How many clusters of s CTAs are resident at once (they stay within a GPC).  The driver counts one CTA per SM for
     // a kernel that allocates tensor memory; two run, so twice its answer (148, 74, 45, 33, 26, 22, 15, 15 on a B200).
     static PdkClusterCaps table;
     const uint32_t* resident = nullptr;
-    if (int rc = pdk_cluster_caps(table, (const void*)kern, kThreads, C::kSmemBytes, &resident)) return rc;
+    if (int rc = pdk_cluster_caps(table, (const void*)splitk_gemm_kernel<KIND, BN, TO>, kThreads, Cfg<KIND, BN>::kSmemBytes, &resident)) return rc;
     // The largest split whose clusters are all resident at once: more only add start-ups.  K = 5120, N = 5120, 7 tokens
     // (40 tiles): 11.4 us at S = 1, 7.6 at 4, 7.4 at 6, and 11.9 at 7, where a part of the clusters waits for a
     // second turn.  At least two stages per CTA, so that it streams more than it sets up.
     const uint32_t tiles_t = (a.batch + BN - 1u) / BN, tiles_w = (a.out_dim + BM - 1u) / BM;
-    uint32_t split = a.num_kb / 2u < kMaxSplit ? a.num_kb / 2u : kMaxSplit;
+    split = a.num_kb / 2u < kMaxSplit ? a.num_kb / 2u : kMaxSplit;
     while (split > 1u && (uint64_t)tiles_t * tiles_w > 2u * resident[split]) --split;
     // It has to save a CTA more slabs (0.3 us each) than the meeting of the partial sums costs, which grows with the tokens of a
     // tile.  us whole / split: fp8 K = 1024, N = 1024: 3.6 / 3.4 at 1 token, 3.7 / 4.4 at 32, 5.3 / 7.1 at 128; nvfp4 K = 1024, N = 5120:
     // 3.1 / 3.8 at 1, 4.7 / 8.4 at 128; K = 2048, N = 5120: 4.7 / 4.5 at 1, 4.8 / 5.3 at 32.  Over 1500 random shapes
     // (K = 1024 ... 17408, N = 512 ... 27648, 1 ... 8192 tokens) this choice is within 1.2 % of the best of all eight splits on average.
-    const uint32_t tokens = tiles_t > 1u ? BN : a.batch, saved = split > 1u ? a.num_kb - (a.num_kb + split - 1u) / split : 0u;
+    // Several tiles of 64 tokens count as tiles of 128, there are as many more of them (nvfp4 K = 3584, N = 1088, 265 tokens: 7.3 whole, 7.9 split).
+    const uint32_t tokens = tiles_t > 1u ? (BN < 128u ? 128u : BN) : a.batch, saved = split > 1u ? a.num_kb - (a.num_kb + split - 1u) / split : 0u;
     if (KIND == kFp8 ? saved * 12u <= 6u * 12u + tokens : saved * 16u <= 4u * 16u + tokens) split = 1u;
     if (split == 0u) split = 1u;
+    sms = resident[1];
+    return 0;
+}
+
+template <int KIND, uint32_t BN, typename TO>
+int launch_bn(const void* data, const void* xq, Args& a, uint32_t row_bytes, uint32_t split, cudaStream_t st) {
+    using C = Cfg<KIND, BN>;
+    CUtensorMap tw, tx;
+    if (int rc = pdk_make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, data, row_bytes, a.out_dim, row_bytes, BKB, BM)) return rc;
+    if (int rc = pdk_make_tmap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, row_bytes, a.batch, row_bytes, BKB, BN)) return rc;
+    auto kern = splitk_gemm_kernel<KIND, BN, TO>;
+    const uint32_t tiles_t = (a.batch + BN - 1u) / BN, tiles_w = (a.out_dim + BM - 1u) / BM;
     cudaLaunchConfig_t cfg = {};
     cfg.blockDim = dim3(kThreads);
     cfg.dynamicSmemBytes = C::kSmemBytes;
@@ -396,9 +405,32 @@ int launch(const void* data, const void* xq, Args& a, uint32_t row_bytes, cudaSt
     a.vec_store = (a.out_dim & 3u) == 0u && pdk_aligned(a.y, 4u * sizeof(TO)) ? 1u : 0u;
     a.sf_vec = pdk_aligned(a.x_sf, 16) ? 1u : 0u;
     a.err = pdk_error_word();
-    if (a.batch <= 32u) return launch_bn<KIND, 32, TO>(data, xq, a, row_bytes, st);
-    if (a.batch <= 64u) return launch_bn<KIND, 64, TO>(data, xq, a, row_bytes, st);
-    return launch_bn<KIND, 128, TO>(data, xq, a, row_bytes, st);
+    uint32_t split = 1u, sms = 0u;
+    if (a.batch <= 32u) {
+        if (int rc = plan_split<KIND, 32, TO>(a, split, sms)) return rc;
+        return launch_bn<KIND, 32, TO>(data, xq, a, row_bytes, split, st);
+    }
+    if (int rc = plan_split<KIND, 64, TO>(a, split, sms)) return rc;
+    if (a.batch > 64u) {
+        // Tiles of 64 or of 128 tokens (figures: us with 128 / with 64).  64 while they are all resident, two CTAs per SM: a tile starts and ends sooner,
+        // and there are twice as many to fill the chip (fp8 1024 x 5120, 100 tokens 6.3 / 5.0, 160 tokens 6.9 / 5.1; 5120 x 17408, 128 tokens
+        // 23.6 / 20.7; nvfp4 5120 x 5120, 200 tokens 13.1 / 9.6; beyond it fp8 1024 x 25600, 96 tokens 8.5 / 10.8).  128
+        //  - where 64 leaves a CTA more slabs of K and the tokens are few (fp8 8192 x 9728: 65 tokens 18.5 / 22.9, 17408 x 5120, 80 tokens 20.8 / 23.0);
+        //  - for up to 80 tokens on a split row: 128 moves no more partial sums than there are tokens, and a second tile is
+        //    mostly padding (fp8 2048 x 2560, 65 tokens 6.5 / 7.1; nvfp4 10240 x 632, 68 tokens 6.4 / 6.8; even at 80);
+        //  - for long rows of many tiles: 64 reads each weight twice as often, and L2 paces that (fp8 14592 x 3528, 323 tokens, 19152 slabs in all:
+        //    25.2 / 35.2; 15104 x 2424, 283 tokens, 11210: 20.5 / 23.5; 9728 x 2264, 332 tokens, 8208: even);
+        //  - above 512 tokens, where 64 was not measured.
+        // Over 67 FP8 and 81 NVFP4 shapes of 65 ... 700 tokens: 0.88 - 0.90 of the time with 128 alone, 3 % longer at worst.
+        uint32_t split128 = 1u;
+        if (int rc = plan_split<KIND, 128, TO>(a, split128, sms)) return rc;
+        const uint64_t tiles = (uint64_t)((a.batch + 63u) / 64u) * ((a.out_dim + BM - 1u) / BM);
+        const uint32_t slabs = (a.num_kb + split - 1u) / split, slabs128 = (a.num_kb + split128 - 1u) / split128;
+        if (tiles > 2u * sms || a.batch > 512u || (a.batch <= 80u && split128 > 1u) || (slabs > slabs128 && 3u * (slabs - slabs128) + 40u > a.batch) ||
+            (a.num_kb > 64u && a.num_kb * tiles > 8000u && a.batch > 128u))
+            return launch_bn<KIND, 128, TO>(data, xq, a, row_bytes, split128, st);
+    }
+    return launch_bn<KIND, 64, TO>(data, xq, a, row_bytes, split, st);
 }
 
 }  // namespace

@@ -89,3 +89,19 @@ def test_fp8_more_channels_than_a_grid_axis_has_tiles(pack):
     assert pack.device_error() == 0
     ref = x.view(torch.float8_e4m3fn).double() @ w.view(torch.float8_e4m3fn).double().t()
     assert float(((y.double() - ref).abs() / ref.clamp_min(1e-30)).max()) < 1e-6      # sixteen exact non-negative products
+
+
+# The line between tiles of 64 and of 128 tokens, one shape on each side of each of its conditions (296 tiles, 80 tokens on a split
+# row, slabs against tokens, 512 tokens, long rows of many tiles), and second tiles of one and of all but one token.
+TILES_64_128 = [(65, 260, 768), (127, 260, 768), (80, 130, 8192), (81, 130, 8192), (129, 300, 5120), (193, 136, 2560), (100, 18944, 256),
+                (100, 18945, 256), (512, 136, 768), (513, 136, 768), (90, 5000, 4096), (120, 5000, 4096)]
+
+
+@pytest.mark.parametrize("m,n,k", TILES_64_128 + [(129, 2700, 16640)])
+def test_fp8_token_tiles(pack, m, n, k):
+    test_fp8(pack, m, n, k, "f32")
+
+
+@pytest.mark.parametrize("m,n,k", TILES_64_128)
+def test_nvfp4_token_tiles(pack, m, n, k):
+    check_nvf4_gemm_w4a4(pack, m, n, k, "bf16")
