@@ -328,7 +328,11 @@ enum Cut : uint32_t { kCutPairs = 0u, kCutHalves = 1u, kCutTiles = 2u };
 __device__ __forceinline__ uint32_t range_start(uint32_t c, uint32_t grid, uint32_t out_dim, uint32_t ppt, uint32_t cut) {
     const uint32_t tiles = (out_dim + BM - 1u) / BM;
     if (cut == kCutPairs) return (uint32_t)((uint64_t)c * tiles * ppt / grid);
-    if (cut == kCutTiles) return (uint32_t)((uint64_t)c * tiles / grid) * ppt;
+    if (cut == kCutTiles) {
+        // the CTAs with one tile more are the first ones (spread evenly over the grid: 1536 x 25856, 20 tokens 17.5 us, this way 15.9)
+        const uint32_t rem = tiles % grid;
+        return (c * (tiles / grid) + (c < rem ? c : rem)) * ppt;
+    }
     const uint32_t h = (uint32_t)((uint64_t)c * 2u * tiles / grid);
     return (h >> 1) * ppt + (h & 1u) * (ppt >> 1);
 }
