@@ -32,6 +32,8 @@
 
 #include "gemv_i8_traits.cuh"
 
+unsigned int* pdk_error_word();   // fp8_quant.cu
+
 namespace {
 
 constexpr uint32_t kSlots = 4;    // 16-row tiles in flight per CTA
@@ -53,7 +55,8 @@ template <class F>
 __global__ void __launch_bounds__(kThreads, kCtasPerSm)
 gemv_i8_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict__ recs, const float* __restrict__ bias,
                const float* __restrict__ x, float* __restrict__ y, uint32_t in_dim, uint32_t out_dim,
-               const int8_t* __restrict__ xq, const float* __restrict__ xq_scale, const PeerOut peers) {
+               const int8_t* __restrict__ xq, const float* __restrict__ xq_scale, const PeerOut peers,
+               unsigned int* __restrict__ err) {
     using Stage = typename F::Stage;
     constexpr uint32_t DEPTH = F::kDepth;
     extern __shared__ __align__(16) uint8_t smem[];
@@ -233,7 +236,7 @@ gemv_i8_kernel(const uint8_t* __restrict__ data, const uint8_t* __restrict__ rec
         __syncthreads();
         if (tid == 0u) peer_signal(peers);
     }
-    if (peer_deferred) peer_check_previous(peers, peer_step, nullptr);
+    if (peer_deferred) peer_check_previous(peers, peer_step, err);
 }
 
 // PDK_NO_PDL=1 launches without programmatic stream serialization (A/B switch, read once).
@@ -272,8 +275,10 @@ int launch(const void* data, const void* recs, const float* bias, const float* x
     cfg.numAttrs = 1;
     PeerOut po{};
     if (peers) po = *peers;
+    unsigned int* err = peers ? pdk_error_word() : nullptr;   // only a wait for peers can run out here
+    if (peers && err == nullptr) return (int)cudaErrorUnknown;
     e = cudaLaunchKernelEx(&cfg, kern, (const uint8_t*)data, (const uint8_t*)recs, bias, x, y, in_dim, out_dim, xq,
-                           xq_scale, po);
+                           xq_scale, po, err);
     return e == cudaSuccess ? pdk_launch_status() : (int)e;
 }
 

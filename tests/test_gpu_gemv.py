@@ -527,7 +527,8 @@ def test_q4k_gemv_shard_sync_raises_flags_and_wait_is_bounded(pack):
     assert int(flags1[0]) == 3 and int(flags1[8]) == 3 and ctr1.tolist() == [0, 3]
 
 
-def test_q4k_gemv_shard_lagged_checks_the_previous_step_on_the_device(pack):
+@pytest.mark.parametrize("k,n", [(5120, 160), (1024, 160), (4096, 8192)])      # the ring kernel; the register kernel for short rows and by its price
+def test_q4k_gemv_shard_lagged_checks_the_previous_step_on_the_device(pack, k, n):
     """The form for loops that rotate y buffers: a launch signals the PREVIOUS launch of its stream (when
     it starts) and checks that every rank's previous step has arrived (before it ends); the last launch
     is signalled by pdk_peer_flags_post.  One rank alone: every check passes, and a closing wait on "my
@@ -535,7 +536,6 @@ def test_q4k_gemv_shard_lagged_checks_the_previous_step_on_the_device(pack):
     up on rank 1 after its bounded wait and says so."""
     import ctypes
     import time
-    k, n = 5120, 160
     w = oracle.fill_normal(n * k, seed_for(2, 960), 0.02)
     raw, d_data, d_sc = q4k_planes(pack, w, n, k)
     d_x = dev_f32(bf16_activations(k, seed_for(2, 961)))
