@@ -470,6 +470,16 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
     uint32_t pend = kNone;  // the team's tile this warp still has to fold
     bool alive = true;
     const uint32_t rows = cta_tiles * 16u, rpo = SPLIT ? (rows + split - 1u) / split : 0u;   // rows per owner
+    auto put = [&](uint32_t row, float v) {
+        if (bias) v += bias[row];
+        if (peers.n == 0u) {
+            y[row] = v;
+            return;
+        }
+#pragma unroll
+        for (uint32_t p = 0; p < 8u; ++p)  // constant indices: the pointers stay in the parameter bank
+            if (p < peers.n) peers.ptr[p][peers.row0 + row] = v;
+    };
     auto fold_tile = [&](uint32_t tl_f) {
         const uint32_t rbf = tl_f % kRedBufs;
         const float* rbuf = red + (size_t)rbf * (W * 16u);
@@ -486,16 +496,7 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
             }
             return;
         }
-        if (lane < 16u && row < out_dim) {
-            if (bias) v += bias[row];
-            if (peers.n == 0u) {
-                y[row] = v;
-            } else {
-#pragma unroll
-                for (uint32_t p = 0; p < 8u; ++p)  // constant indices: the pointers stay in the parameter bank
-                    if (p < peers.n) peers.ptr[p][peers.row0 + row] = v;
-            }
-        }
+        if (lane < 16u && row < out_dim) put(row, v);
     };
     auto poll_fold = [&](bool block) {
         if (pend == kNone || !alive) return;
@@ -602,7 +603,7 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
             if (at >= rows || row >= out_dim) break;
             float v = 0.0f;
             for (uint32_t s = 0; s < split; ++s) v += recv[s * rpo + r];
-            y[row] = bias ? v + bias[row] : v;
+            put(row, v);
         }
     }
     if (peers.n != 0u && peers.signal == 1u) {   // uniform over the grid
@@ -662,12 +663,12 @@ bool ring_layout(RingPlan& p, uint32_t in_dim, uint32_t out_dim) {
 // 5376 x 6016 11.7 -> 7.6, 17152 x 520 29.3 -> 5.3; Q4_K 9472 x 1024 12.0 -> 5.1; and the other way round Q4_K 1792 x 9792 6.1 -> 4.6.  Q4_K 5120 x
 // 25600: one team of ten 17.2, two of ten 17.5, four of five 15.6; 4096 x 25600: eight 14.5, six teams of three 13.0.
 template <class F>
-bool make_plan(uint32_t in_dim, uint32_t out_dim, bool whole, const uint32_t* cap, RingPlan& best) {
+bool make_plan(uint32_t in_dim, uint32_t out_dim, const uint32_t* cap, RingPlan& best) {
     const uint32_t all = (in_dim + 511u) / 512u, n_tiles = (out_dim + 15u) / 16u, slots = 4u * cap[1];
     constexpr float kPairKb = (float)(2u * (F::kDataBoxes * kBoxBytes + 16u * F::kHighBytes) + 32u * F::kRecBytes) / 1000.0f;
     float best_cost = 0.0f;
     bool found = false;
-    for (uint32_t s = 1; s <= (whole ? 1u : kPdkMaxCluster) && s <= all; ++s) {
+    for (uint32_t s = 1; s <= kPdkMaxCluster && s <= all; ++s) {
         if (cap[s] == 0u || s == 5u || s == 7u || (s > 1u && n_tiles > 3u * cap[1])) continue;    // wide planes fill the chip unsplit
         const uint32_t np = (all + s - 1u) / s, clusters = cap[s] < n_tiles ? cap[s] : n_tiles, per = (n_tiles + clusters - 1u) / clusters;
         const float fixed = s == 1u ? 0.0f : s == 2u ? 1.45f : 2.18f;
@@ -801,14 +802,13 @@ int launch_ring(const void* data, const void* recs, const float* bias, const flo
     const uint32_t* cap = nullptr;
     if (int rc = pdk_cluster_caps(table, (const void*)gemv_ring_kernel<F, false, false, true>, kMaxWarps * 32u, kSmemMax, &cap)) return rc;
     // the plans of the shapes a thread met last
-    struct Known { const uint32_t* cap; uint32_t in_dim, out_dim, whole, ok; RingPlan plan; };
+    struct Known { const uint32_t* cap; uint32_t in_dim, out_dim, ok; RingPlan plan; };
     constexpr uint32_t kKnown = 32;
     thread_local Known known[kKnown] = {};
-    const uint32_t whole = peers != nullptr ? 1u : 0u;
-    Known& k = known[(in_dim / 256u * 7u + out_dim / 8u + whole * 3u) % kKnown];
-    if (k.cap != cap || k.in_dim != in_dim || k.out_dim != out_dim || k.whole != whole) {
-        k = Known{cap, in_dim, out_dim, whole, 0u, RingPlan{}};
-        k.ok = make_plan<F>(in_dim, out_dim, whole != 0u, cap, k.plan) ? 1u : 0u;
+    Known& k = known[(in_dim / 256u * 7u + out_dim / 8u) % kKnown];
+    if (k.cap != cap || k.in_dim != in_dim || k.out_dim != out_dim) {
+        k = Known{cap, in_dim, out_dim, 0u, RingPlan{}};
+        k.ok = make_plan<F>(in_dim, out_dim, cap, k.plan) ? 1u : 0u;
     }
     if (k.ok == 0u) return -1;
     const RingPlan& pl = k.plan;

@@ -415,11 +415,13 @@ def test_q5_k_q6_k_tokens_as_columns(pack, name, batch):
     assert one < 1e-4, ("decode GEMV", one)
 
 
-def test_q4k_gemv_shard_stores_band_into_every_output(pack):
-    """pdk_q4k_gemv_shard with two destination vectors on one GPU (the multi-GPU case points the
+# (8192, 3200) and (17408, 3200): the ring kernel splits the pairs of a row over a cluster; (1024, 160): the register kernel
+@pytest.mark.parametrize("k,n", [(5120, 512), (8192, 3200), (17408, 3200), (17408, 2560), (1024, 160)])
+def test_q4k_gemv_shard_stores_band_into_every_output(pack, k, n):
+    """pdk_q4k_gemv_shard and _sync with two destination vectors on one GPU (the multi-GPU case points the
     second at a peer's buffer): both receive the band at row0, bit-identical to kquant_gemv."""
     import ctypes
-    k, n, full, row0 = 5120, 512, 2048, 1024
+    row0, full = 1024, 1024 + n + 512
     w = oracle.fill_normal(n * k, 730, 0.02)
     raw, d_data, d_sc = q4k_planes(pack, w, n, k)
     x = dev_f32(bf16_activations(k, seed_for(2, 9)))
@@ -427,11 +429,20 @@ def test_q4k_gemv_shard_stores_band_into_every_output(pack):
     pack.call("kquant_gemv", d_data, d_sc, x, d_ref, k, n, 12)
     outs = [torch.full((full,), -1.0, dtype=torch.float32, device="cuda") for _ in range(2)]
     ptrs = (ctypes.c_void_p * 2)(*[o.data_ptr() for o in outs])
-    pack.call("pdk_q4k_gemv_shard", d_data, d_sc, x, ctypes.addressof(ptrs), 2, row0, k, n)
-    torch.cuda.synchronize()
-    for o in outs:
-        assert torch.equal(o[row0:row0 + n], d_ref)
-        assert bool((o[:row0] == -1.0).all()) and bool((o[row0 + n:] == -1.0).all())
+    flags, ctr = torch.zeros(32, dtype=torch.int32, device="cuda"), torch.zeros(2, dtype=torch.int32, device="cuda")
+    fptrs = (ctypes.c_void_p * 2)(flags.data_ptr(), flags.data_ptr() + 64)
+    for sync in (False, True):
+        for o in outs:
+            o.fill_(-1.0)
+        if sync:
+            pack.call("pdk_q4k_gemv_shard_sync", d_data, d_sc, x, ctypes.addressof(ptrs), ctypes.addressof(fptrs), ctr, 2, 1, row0, 5, k, n)
+        else:
+            pack.call("pdk_q4k_gemv_shard", d_data, d_sc, x, ctypes.addressof(ptrs), 2, row0, k, n)
+        torch.cuda.synchronize()
+        for o in outs:
+            assert torch.equal(o[row0:row0 + n], d_ref)
+            assert bool((o[:row0] == -1.0).all()) and bool((o[row0 + n:] == -1.0).all())
+    assert int(flags[1]) == 5 and int(flags[17]) == 5 and ctr.tolist() == [0, 0] and pack.device_error() == 0
     assert pack.status("pdk_q4k_gemv_shard", d_data, d_sc, x, ctypes.addressof(ptrs), 9, row0, k, n) == 1
 
 
