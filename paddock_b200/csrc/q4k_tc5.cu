@@ -15,9 +15,9 @@
 // the whole of a run's part of a tile; the epilogue adds the two column groups, undoes the token
 // scale and adds into y.
 //
-// A CTA takes a contiguous run of (tile, unit pair)s, cut at pairs, half tiles or tiles (range_start; launch picks).  A tile that two CTAs share is added into y by both with red.global.add.f32; y is
-// zeroed by the kernel in front, and with at most two addends per element the sum does not
-// depend on their order.
+// A CTA takes a contiguous run of (tile, unit pair)s, cut at pairs, half tiles or tiles (q4k_runs.cuh).  A tile that two
+// CTAs share is added into y by both with red.global.add.f32; y is zeroed by the kernel in front, and with at most two
+// addends per element the sum does not depend on their order.
 //
 // What paces it (cycle counters in every role at 16 tokens): the tensor core.  A kind::f16 MMA with the
 // A operand in tensor memory takes 64 cycles at M128 K16 however few columns (32) it has, 16 of them per
@@ -29,11 +29,12 @@
 // operands is 3e-4, the condition-relative error 3e-5.
 #include <cuda_fp16.h>
 
+#include "q4k_runs.cuh"
 #include "tc5.cuh"
 
 namespace {
 
-constexpr uint32_t BM = 128;          // weight rows per work item (MMA M)
+constexpr uint32_t BM = q4k_runs::kTileRows;   // weight rows of a tile (MMA M)
 constexpr uint32_t kProdWarps = 8;    // dequantizing warps per unit (super-block column of the tile)
 // Two sets of producer warps take the units in turn (set 0 the even ones, set 1 the odd ones): a
 // producer's chain for a unit - box read, nibble arithmetic, tensor-memory stores, barrier - is
@@ -321,27 +322,11 @@ __device__ __forceinline__ void dequant_regs(const uint4& q, const SlabScale& sc
     }
 }
 
-// Where CTA c's run of unit pairs starts; the pairs of tile t are t ppt .. (t + 1) ppt.  Cut: equal runs of pairs (no run shorter than a tile),
-// half tiles, or whole tiles.  Either way a tile has at most two CTAs, and the sum of two addends on a zeroed y does not
-// depend on their order.
-enum Cut : uint32_t { kCutPairs = 0u, kCutHalves = 1u, kCutTiles = 2u };
-__device__ __forceinline__ uint32_t range_start(uint32_t c, uint32_t grid, uint32_t out_dim, uint32_t ppt, uint32_t cut) {
-    const uint32_t tiles = (out_dim + BM - 1u) / BM;
-    if (cut == kCutPairs) return (uint32_t)((uint64_t)c * tiles * ppt / grid);
-    if (cut == kCutTiles) {
-        // the CTAs with one tile more are the first ones (spread evenly over the grid: 1536 x 25856, 20 tokens 17.5 us, this way 15.9)
-        const uint32_t rem = tiles % grid;
-        return (c * (tiles / grid) + (c < rem ? c : rem)) * ppt;
-    }
-    const uint32_t h = (uint32_t)((uint64_t)c * 2u * tiles / grid);
-    return (h >> 1) * ppt + (h & 1u) * (ppt >> 1);
-}
-
 template <uint32_t NC, bool Q40>
 __global__ void __launch_bounds__(kThreads, 1)
 q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_w,
                const __grid_constant__ CUtensorMap tmap_r, const float* __restrict__ tokscale, float* __restrict__ y,
-               uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t cut, unsigned int* err_word) {
+               uint32_t in_dim, uint32_t out_dim, uint32_t batch, const q4k_runs::Runs runs, unsigned int* err_word) {
     using C = Cfg<NC>;
     extern __shared__ uint8_t smem_raw[];
     uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
@@ -351,7 +336,8 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
 
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint32_t ppt = in_dim >> 9;                            // unit pairs (weight boxes) of a tile
-    const uint32_t p_lo = range_start(blockIdx.x, gridDim.x, out_dim, ppt, cut), p_hi = range_start(blockIdx.x + 1u, gridDim.x, out_dim, ppt, cut);
+    const uint32_t p_lo = q4k_runs::start(runs, blockIdx.x, ppt), p_hi = q4k_runs::start(runs, blockIdx.x + 1u, ppt);
+    const uint32_t tile_lo = p_lo / ppt;
 
     if (threadIdx.x == 0) {
         for (uint32_t s = 0; s < kRawStages; ++s) {
@@ -398,7 +384,7 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         const uint32_t r_in = qd * 32u + lane, swz = r_in & 7u;
         const uint32_t line_off = (r_in >> 3) * 1024u + swz * 128u;  // the row's 128-byte line in a weight box
         const uint32_t total = 2u * (p_hi - p_lo);
-        uint32_t tile = p_lo / ppt, seg_end = min(p_hi, (tile + 1u) * ppt) - p_lo, iter = 0u;   // the part of this tile ends here
+        uint32_t tile = tile_lo, seg_end = min(p_hi, (tile + 1u) * ppt) - p_lo, iter = 0u;   // the part of this tile ends here
         bool ok = true;
         // unit n of this CTA's sequence: box n / 2 (unit n % 2 of it, so that is the set), operand
         // stage n % kStages
@@ -486,8 +472,8 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         // Weights depend on nothing the previous kernel in the stream writes: no wait for it.
         uint32_t rs = 0, rphase = 0;
         bool ok = true, waited = false;
-        for (uint32_t at = p_lo; at < p_hi && ok;) {
-            const uint32_t tile = at / ppt, row0 = tile * BM, u0 = 2u * (at - tile * ppt), upi = 2u * (min(p_hi, (tile + 1u) * ppt) - at);
+        for (uint32_t at = p_lo, tile = tile_lo; at < p_hi && ok; ++tile) {
+            const uint32_t row0 = tile * BM, u0 = 2u * (at - tile * ppt), upi = 2u * (min(p_hi, (tile + 1u) * ppt) - at);
             at += upi >> 1;
             for (uint32_t u = 0; u < upi; u += 2u) {
                 ok = mbar_wait_park(&sh->raw_empty[rs], rphase ^ 1u, ctx, tc5::kErrEmptyWait, 0x20u + rs);
@@ -519,8 +505,8 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         uint32_t stage = 0, phase = 0;
         bool ok = true;
         pdk_pdl_wait();  // the f16 rows are the previous kernel's output
-        for (uint32_t at = p_lo; at < p_hi && ok;) {
-            const uint32_t tile = at / ppt, u0 = 2u * (at - tile * ppt), upi = 2u * (min(p_hi, (tile + 1u) * ppt) - at);
+        for (uint32_t at = p_lo, tile = tile_lo; at < p_hi && ok; ++tile) {
+            const uint32_t u0 = 2u * (at - tile * ppt), upi = 2u * (min(p_hi, (tile + 1u) * ppt) - at);
             at += upi >> 1;
             for (uint32_t u = 0; u < upi; ++u) {
                 ok = mbar_wait_park(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, 0x10u + stage);
@@ -542,7 +528,7 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         uint32_t stage = 0, phase = 0, iter = 0, rs = 0, rphase = 0;
         bool ok = true;
         for (uint32_t at = p_lo; at < p_hi && ok; ++iter) {
-            const uint32_t upi = 2u * (min(p_hi, (at / ppt + 1u) * ppt) - at);
+            const uint32_t upi = 2u * (min(p_hi, (tile_lo + iter + 1u) * ppt) - at);
             at += upi >> 1;
             const uint32_t buf = iter & 1u, aphase = (iter >> 1) & 1u;
             ok = mbar_wait_park(&sh->tmem_empty[buf], aphase ^ 1u, ctx, tc5::kErrTmemEmptyWait, buf);
@@ -621,24 +607,9 @@ int launch(const void* data, const void* recs, const float* x, const int8_t* xq,
     if (int rc = pdk_launch_pdl(q4k_act_f16_kernel, dim3(NC / 2u + kZeroCtas), dim3(kActThreads), 0, st, x, xq, xq_scale, xh,
                                 tokscale, y, in_dim, out_dim, batch, NC / 2u))
         return rc;
-    // Half tiles where the plane has at most half a tile per SM (also of an odd number of pairs: 9728 x 6528, 9 tokens 31.6 us whole, 19.5 in halves), whole
-    // tiles up to one per SM.  From there runs or whole tiles by the busiest CTA's estimate: 1.5 us per pair, 1.3 per tile that it touches
-    // (its accumulator is drained while nothing is produced), 0.5 for runs.  4608 x 19968, 10 tokens: whole tiles 32.2 us, runs 22.7;
-    // 1536 x 25856, 20 tokens: 15.9, 17.3; 5120 x 25600, 16 tokens: half tiles in turn 30.1, runs 29.8.
-    const uint32_t tiles = (out_dim + BM - 1u) / BM, sms = (uint32_t)pdk_sm_count(), ppt = n_unit >> 1;
-    uint32_t cut = kCutTiles, grid = tiles;
-    if (2u * tiles <= sms && ppt >= 2u) {
-        cut = kCutHalves;
-        grid = 2u * tiles;
-    } else if (tiles > sms) {
-        const uint32_t whole = (tiles + sms - 1u) / sms;
-        const uint64_t run = ((uint64_t)tiles * ppt + sms - 1u) / sms;
-        const float by_tiles = (1.5f * (float)ppt + 1.3f) * (float)whole, by_pairs = 1.5f * (float)run + 1.3f * (float)(whole + 1u) + 0.5f;
-        cut = by_tiles <= by_pairs ? kCutTiles : kCutPairs;
-        grid = sms;
-    }
-    return pdk_launch_pdl(kern, dim3(grid), dim3(kThreads), smem, st, tx, tw, tr, (const float*)tokscale, y, in_dim,
-                          out_dim, batch, cut, pdk_error_word());
+    const q4k_runs::Runs runs = q4k_runs::pick((out_dim + BM - 1u) / BM, n_unit >> 1, (uint32_t)pdk_sm_count());
+    return pdk_launch_pdl(kern, dim3(runs.grid), dim3(kThreads), smem, st, tx, tw, tr, (const float*)tokscale, y, in_dim,
+                          out_dim, batch, runs, pdk_error_word());
 }
 
 }  // namespace
