@@ -178,6 +178,10 @@ int pdk_kquant_gemm_f32(const void* data, const void* scales, const void* x, voi
 /* Which kernel a small batch asks first, for tests and diagnostics (no device needed): 1 kq_batch.cu, 2 the integer
  * kernel, 3 tcgen05; 0 = none of them (one token, IQ4_XS, more than 64 tokens). */
 int pdk_kquant_gemm_route(uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t dtype);
+/* How a one-token call (pd_kquant_gemv, or pd_q8_0_gemv_repacked with dtype 8) of such a plane runs on the current device, for tests and
+ * diagnostics: plan[4] = warps of a team, teams, CTAs of a cluster and stages of the ring kernel; all 0 where the register-staged
+ * kernel is faster or the shape is outside the ring's plans.  0 or a cudaError_t. */
+int pdk_gemv_plan(uint32_t in_dim, uint32_t out_dim, uint32_t dtype, uint32_t* plan);
 
 /* ---- FP8 E4M3, one f32 scale per row ----------------------------------------- */
 

@@ -38,29 +38,15 @@
 
 #include "cluster_caps.cuh"
 #include "gemv_i8_traits.cuh"
+#include "ring_plan.cuh"
 #include "tc5.cuh"
 
 namespace {
 
 using namespace gemv_i8;
 
-constexpr uint32_t kMaxWarps = 12;                      // with 168 registers a thread
-constexpr uint32_t kManyWarps = 20, kMaxTeams = 10;     // with 96
-constexpr uint32_t kMaxDepth = 4;
-constexpr uint32_t kRedBufs = 8;                        // of a team
-constexpr uint32_t kSmemMax = 232448;  // 227 KB per CTA on sm_100
-constexpr uint32_t kBoxBytes = 2048;   // 16 rows x 128 bytes
-
-struct RingPlan {
-    uint32_t W;          // warps of a team
-    uint32_t teams;      // teams of a CTA: tile i of the CTA is team i % teams'
-    uint32_t D;          // stages per warp
-    uint32_t split;      // CTAs of a cluster, which share tiles and split the pairs of a row
-    uint32_t clusters;
-    uint32_t invariant;  // W >= pairs of a row's part: a warp's pair never changes
-    uint32_t k_part;     // elements of a row that a CTA's activations cover, at most
-    uint32_t off_xmeta, off_red, off_recv, off_bar, off_rec, off_data, smem_bytes;
-};
+using namespace ring;
+static_assert(kMaxSplit == kPdkMaxCluster, "cluster_caps.cuh asks for these sizes");
 
 enum : unsigned int { kErrRingFull = 0x11, kErrRingFold = 0x13, kErrRingDrain = 0x14, kErrRingFree = 0x15 };
 
@@ -80,10 +66,9 @@ __device__ __forceinline__ uint32_t word4(const uint4& v, uint32_t i) { return i
 
 // load_ring arguments: `box` = the unit's first data box, o0 / o1 = swz(g, 2t) / swz(g, 2t + 1)
 // (rows g + 8 lie 1024 bytes further), `rec` = row g's record of the unit (row g + 8: 8 box rows on).
-struct RQ4K : Q4K {
-    static constexpr uint32_t kDataBoxes = 1, kHighBytes = 0, kPasses = 2, kSub = 4, kBlock = 32;
-    static constexpr bool kMany = true;
-    static constexpr float kStepCost = 0.048f, kManyCost = 0.052f, kRegsCost = 0.90f;   // make_plan
+struct RQ4K : Q4K, Q4KPlane {
+    using Q4KPlane::kDataBytes, Q4KPlane::kRecBytes;
+    static constexpr uint32_t kPasses = 2, kSub = 4;
     // pass p of lane t feeds block 2t + p: the low (p = 0) or high nibbles of ggml group t, whose
     // first 16 bytes (chunk 2t) sit in k-slots 4t.. and whose second 16 (chunk 2t+1) in slots 16+4t..
     __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return 2u * t + p; }
@@ -111,10 +96,9 @@ struct RQ4K : Q4K {
     }
 };
 
-struct RQ40 : Q40 {
-    static constexpr uint32_t kDataBoxes = 1, kHighBytes = 0, kPasses = 2, kSub = 4, kBlock = 32;
-    static constexpr bool kMany = true;
-    static constexpr float kStepCost = 0.048f, kManyCost = 0.052f, kRegsCost = 0.83f;   // make_plan
+struct RQ40 : Q40, Q40Plane {
+    using Q40Plane::kDataBytes, Q40Plane::kRecBytes;
+    static constexpr uint32_t kPasses = 2, kSub = 4;
     __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return 2u * t + p; }
     __device__ static __forceinline__ void a_pass(const Stage& s, uint32_t p, uint32_t j, uint32_t& a0, uint32_t& a1,
                                                   uint32_t& a2, uint32_t& a3) {
@@ -135,11 +119,9 @@ struct RQ40 : Q40 {
     }
 };
 
-struct RQ80 : Q80 {
-    static constexpr uint32_t kDataBoxes = 2;  // blocks 0..3 | blocks 4..7 of the unit
-    static constexpr uint32_t kHighBytes = 0, kPasses = 2, kSub = 4, kBlock = 32;
-    static constexpr bool kMany = false;       // two boxes a unit leave no room for the stages, and the loads spill
-    static constexpr float kStepCost = 0.120f, kManyCost = 0.0f, kRegsCost = 1.91f;   // make_plan
+struct RQ80 : Q80, Q80Plane {     // boxes: blocks 0..3 | blocks 4..7 of the unit
+    using Q80Plane::kDataBytes, Q80Plane::kRecBytes;
+    static constexpr uint32_t kPasses = 2, kSub = 4;
     // pass p of lane t feeds block t + 4p: box p holds blocks 4p..4p+3, chunk 2t its block t's first
     // 16 bytes (k-slots 4t..), chunk 2t+1 the second 16 (slots 16+4t..)
     __device__ static __forceinline__ uint32_t blk(uint32_t p, uint32_t t) { return t + 4u * p; }
@@ -169,11 +151,9 @@ struct RQ80 : Q80 {
 
 // Q5_K: the Q4_K nibbles and record, and 32 bytes whose bit b is bit 4 of block b's codes.  Lane t's blocks 2t and 2t + 1 take
 // two bits of every byte.
-struct RQ5K : Q4K {
-    static constexpr uint32_t kDataBytes = 160;
-    static constexpr uint32_t kDataBoxes = 1, kHighBytes = 32, kPasses = 2, kSub = 4, kBlock = 32;
-    static constexpr bool kMany = true;
-    static constexpr float kStepCost = 0.127f, kManyCost = 0.087f, kRegsCost = 1.55f;
+struct RQ5K : Q4K, Q5KPlane {
+    using Q5KPlane::kDataBytes, Q5KPlane::kRecBytes;
+    static constexpr uint32_t kPasses = 2, kSub = 4;
     static constexpr int kHiShift = 0;
     struct Stage : Q4K::Stage {
         uint4 h[4];   // rows g, g + 8: the high-bit bytes, shifted so that block 2t's bit is bit 0
@@ -203,11 +183,8 @@ struct RQ5K : Q4K {
 // Q6_K: sixteen blocks of 16 weights, so four passes of two mmas.  Lane t holds, of the 128-weight half t / 2, the blocks at
 // elements 16 (t & 1) + 32 p (p = pass): low nibbles of two 16-byte chunks of ql for p = 0, 1, high nibbles for p = 2, 3,
 // and bits 2p, 2p + 1 of one chunk of qh.  Codes stay unsigned; the -32 goes through the 16-element sums of the activations.
-struct RQ6K {
-    static constexpr uint32_t kDataBytes = 192, kRecBytes = 24;
-    static constexpr uint32_t kDataBoxes = 1, kHighBytes = 64, kPasses = 4, kSub = 2, kBlock = 16;
-    static constexpr bool kMany = true;
-    static constexpr float kStepCost = 0.127f, kManyCost = 0.087f, kRegsCost = 1.49f;
+struct RQ6K : Q6KPlane {
+    static constexpr uint32_t kPasses = 4, kSub = 2;
     static constexpr bool kUnsignedA = true;
     static constexpr int kHiShift = 0;
     struct Stage {
@@ -628,79 +605,6 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
     }
 }
 
-// What a CTA keeps in shared memory; false when fewer than two stages per warp fit.
-template <class F>
-bool ring_layout(RingPlan& p, uint32_t in_dim, uint32_t out_dim) {
-    constexpr uint32_t kData = 2u * (F::kDataBoxes * kBoxBytes + 16u * F::kHighBytes), kRec = 32u * F::kRecBytes;
-    const uint32_t n = p.W * p.teams, pairs = ((in_dim + 511u) / 512u + p.split - 1u) / p.split;
-    const uint64_t tiles = ((out_dim + 15u) / 16u + p.clusters - 1u) / p.clusters;
-    const uint64_t recv = p.split > 1u ? (uint64_t)p.split * ((tiles * 16u + p.split - 1u) / p.split) * 4u : 0u;
-    if (pairs > 512u || recv > kSmemMax) return false;
-    p.invariant = p.W >= pairs ? 1u : 0u;
-    p.k_part = pairs * 512u;
-    p.off_xmeta = 2u * p.k_part + 32u;
-    p.off_red = p.off_xmeta + (p.k_part / F::kBlock) * 8u;
-    p.off_recv = p.off_red + kRedBufs * n * 64u;
-    p.off_bar = (p.off_recv + (uint32_t)recv + 7u) & ~7u;
-    p.off_rec = (p.off_bar + (n * kMaxDepth + 2u * kRedBufs * p.teams + 1u) * 8u + 127u) & ~127u;
-    for (p.D = kMaxDepth; p.D >= 2u; --p.D) {
-        p.off_data = (p.off_rec + n * p.D * kRec + 1023u) & ~1023u;  // swizzled boxes start on 1 KB
-        p.smem_bytes = p.off_data + n * p.D * kData;
-        if (p.smem_bytes <= kSmemMax) return true;
-    }
-    return false;
-}
-
-// The split with the shortest estimate, in us; false where the register-staged kernel (gemv_i8.cu, gemv_q6k.cu) has a shorter one.
-//   one team     1.19 + steps (1.035 + kStepCost W): a step is a pair of a tile, and the longer the more warps share the SM
-//   many warps   2.36 + steps (0.65 + kManyCost warps) + 1.61 per tile of a team (its fold)
-//   the stream   1.26 + 22 ns per KB of the CTA; the shorter of it and the above counts 4.4 % on top of the longer
-//   split        1.45 more for two CTAs, 2.18 for more
-//   registers    1.43 + rounds of 64 rows per SM x K / 1024 x kRegsCost, up to 1.32 times that when its four slots are full
-// Fitted to every split of 973 shapes (K = 1280 ... 17408, N = 520 ... 25600, all formats): 1.7 % over the best of them on average, 45 % at worst
-// (Q4_K 6912 x 520: 4.9 us, four CTAs 3.4).
-// Measured (us; register kernel -> here): Q6_K 17152 x 1024 25.2 -> 8.1 (four CTAs), 9472 x 2560 15.6 -> 9.8, 5120 x 25600 23.5 -> 20.1; Q8_0
-// 5376 x 6016 11.7 -> 7.6, 17152 x 520 29.3 -> 5.3; Q4_K 9472 x 1024 12.0 -> 5.1; and the other way round Q4_K 1792 x 9792 6.1 -> 4.6.  Q4_K 5120 x
-// 25600: one team of ten 17.2, two of ten 17.5, four of five 15.6; 4096 x 25600: eight 14.5, six teams of three 13.0.
-template <class F>
-bool make_plan(uint32_t in_dim, uint32_t out_dim, const uint32_t* cap, RingPlan& best) {
-    const uint32_t all = (in_dim + 511u) / 512u, n_tiles = (out_dim + 15u) / 16u, slots = 4u * cap[1];
-    constexpr float kPairKb = (float)(2u * (F::kDataBoxes * kBoxBytes + 16u * F::kHighBytes) + 32u * F::kRecBytes) / 1000.0f;
-    float best_cost = 0.0f;
-    bool found = false;
-    for (uint32_t s = 1; s <= kPdkMaxCluster && s <= all; ++s) {
-        if (cap[s] == 0u || s == 5u || s == 7u || (s > 1u && n_tiles > 3u * cap[1])) continue;    // wide planes fill the chip unsplit
-        const uint32_t np = (all + s - 1u) / s, clusters = cap[s] < n_tiles ? cap[s] : n_tiles, per = (n_tiles + clusters - 1u) / clusters;
-        const float fixed = s == 1u ? 0.0f : s == 2u ? 1.45f : 2.18f;
-        const float stream = 1.26f + (float)((uint64_t)per * np) * kPairKb * 0.022f;
-        for (uint32_t rounds = 1; rounds <= 5u && rounds <= np; ++rounds) {
-            const uint32_t W = (np + rounds - 1u) / rounds;
-            if (W > kManyWarps) continue;
-            const uint32_t most = kManyWarps / W, teams[5] = {1u, 2u, kMaxWarps / W, most / 2u, most};
-            for (uint32_t i = 0; i < 5u; ++i) {
-                const uint32_t T = teams[i] < kMaxTeams ? teams[i] : kMaxTeams, n = W * T, folds = T != 0u ? (per + T - 1u) / T : 0u;
-                if (T == 0u || n > kManyWarps || (i > 0u && T <= teams[i - 1u])) continue;
-                const bool many = T > 1u || n > kMaxWarps;
-                if (many && !F::kMany) continue;
-                const float steps = (float)(folds * rounds);
-                const float work = many ? 2.36f + steps * (0.65f + F::kManyCost * (float)n) + 1.61f * (float)folds
-                                        : 1.19f + steps * (1.035f + F::kStepCost * (float)n);
-                const float cost = fixed + (work > stream ? work + 0.044f * stream : stream + 0.044f * work);
-                if (found && cost >= best_cost) continue;
-                RingPlan p{};
-                p.W = W; p.teams = T; p.split = s; p.clusters = clusters;
-                if (!ring_layout<F>(p, in_dim, out_dim)) continue;
-                best_cost = cost;
-                best = p;
-                found = true;
-            }
-        }
-    }
-    const float fill = n_tiles < slots ? (float)n_tiles / (float)slots : 1.0f;
-    const float regs = 1.43f + (float)((n_tiles + slots - 1u) / slots) * (float)in_dim / 1024.0f * F::kRegsCost * (1.0f + 0.32f * fill);
-    return found && best_cost <= regs;
-}
-
 // PDK_GEMV_REGS=1 sends every call to the register-staged kernel (A/B switch, read once).
 bool force_regs() {
     static const bool v = [] {
@@ -788,15 +692,10 @@ int launch_plan(const MapEntry& m, const void* recs, const float* bias, const fl
     return e == cudaSuccess ? pdk_launch_status() : (int)e;
 }
 
-// -1: outside the plan (rows of up to four units: Q6_K 1024 x 618 2.2 us on registers, 2.5 here; planes that do not start on 16 bytes, activations too long), or the
-// register-staged kernel is faster.
+// The plan of a shape on the current device: 0, a cudaError_t, or -1 where there is none or the register-staged kernel is faster.
 template <class F>
-int launch_ring(const void* data, const void* recs, const float* bias, const float* x, float* y, uint32_t in_dim,
-                uint32_t out_dim, cudaStream_t st, const int8_t* xq = nullptr, const float* xq_scale = nullptr,
-                const PeerOut* peers = nullptr) {
-    if (force_regs() || in_dim <= 1024u || (in_dim & 255u) != 0u || out_dim > 0x40000000u) return -1;
-    const bool tma = recs_by_tma<F>(in_dim);
-    if (!pdk_aligned(recs, tma ? 16 : 8)) return -1;
+int shape_plan(uint32_t in_dim, uint32_t out_dim, const RingPlan** plan) {
+    if (in_dim <= 1024u || (in_dim & 255u) != 0u || out_dim > 0x40000000u) return -1;
     // clusters of s CTAs that are resident at once: one CTA per SM, whatever the instance
     static PdkClusterCaps table;
     const uint32_t* cap = nullptr;
@@ -810,8 +709,22 @@ int launch_ring(const void* data, const void* recs, const float* bias, const flo
         k = Known{cap, in_dim, out_dim, 0u, RingPlan{}};
         k.ok = make_plan<F>(in_dim, out_dim, cap, k.plan) ? 1u : 0u;
     }
-    if (k.ok == 0u) return -1;
-    const RingPlan& pl = k.plan;
+    *plan = &k.plan;
+    return k.ok != 0u ? 0 : -1;
+}
+
+// -1: outside the plan (rows of up to four units: Q6_K 1024 x 618 2.2 us on registers, 2.5 here; planes that do not start on 16 bytes, activations too long), or the
+// register-staged kernel is faster.
+template <class F>
+int launch_ring(const void* data, const void* recs, const float* bias, const float* x, float* y, uint32_t in_dim,
+                uint32_t out_dim, cudaStream_t st, const int8_t* xq = nullptr, const float* xq_scale = nullptr,
+                const PeerOut* peers = nullptr) {
+    if (force_regs()) return -1;
+    const bool tma = recs_by_tma<F>(in_dim);
+    if (!pdk_aligned(recs, tma ? 16 : 8)) return -1;
+    const RingPlan* plan = nullptr;
+    if (int rc = shape_plan<F>(in_dim, out_dim, &plan)) return rc;
+    const RingPlan& pl = *plan;
     const MapEntry* maps = nullptr;
     if (plane_maps<F>(data, recs, in_dim, out_dim, &maps) != 0) return -1;
     PeerOut po{};
@@ -1175,6 +1088,28 @@ int pdk_q8_0_gemm_i8(const void* data, const void* scale, const float* bias, con
                                       nb, pl, err, t0 + 8u >= batch ? 1u : 0u);
         if (rc != 0) return rc;
     }
+    return 0;
+}
+
+// warps of a team, teams, CTAs of a cluster, stages of the ring kernel's plan for a one-token call on this device; all 0 = not its call
+PDK_EXPORT int pdk_gemv_plan(uint32_t in_dim, uint32_t out_dim, uint32_t dtype, uint32_t* plan) {
+    if (plan == nullptr || out_dim == 0u) return cudaErrorInvalidValue;
+    const RingPlan* p = nullptr;
+    int rc;
+    switch (dtype) {
+        case PDK_KQ_Q4K: rc = shape_plan<RQ4K>(in_dim, out_dim, &p); break;
+        case PDK_KQ_Q4_0: rc = shape_plan<RQ40>(in_dim, out_dim, &p); break;
+        case PDK_KQ_Q5K: rc = shape_plan<RQ5K>(in_dim, out_dim, &p); break;
+        case PDK_KQ_Q6K: rc = shape_plan<RQ6K>(in_dim, out_dim, &p); break;
+        case 8u: rc = shape_plan<RQ80>(in_dim, out_dim, &p); break;      // ggml's Q8_0
+        default: return cudaErrorInvalidValue;
+    }
+    if (rc > 0) return rc;
+    const bool on = rc == 0 && !force_regs();
+    plan[0] = on ? p->W : 0u;
+    plan[1] = on ? p->teams : 0u;
+    plan[2] = on ? p->split : 0u;
+    plan[3] = on ? p->D : 0u;
     return 0;
 }
 
