@@ -1,6 +1,7 @@
 // q4k_runs.cuh - which super-blocks of a plane a CTA of q4k_tc5.cu takes (plain C++: tests/test_q4k_runs.py compiles it for the host).
 #pragma once
 #include <cstdint>
+#include <initializer_list>
 #ifndef __CUDACC__
 #define __host__
 #define __device__
@@ -28,25 +29,34 @@ __host__ __device__ __forceinline__ uint32_t start(const Runs& r, uint32_t c, ui
     return (i >> 1) * ppt + (i & 1u) * (ppt >> 1);
 }
 
-// Half tiles where the plane has at most half a tile per SM (also of an odd number of pairs: 9728 x 6528, 9 tokens 31.6 us whole, 19.5 in halves), whole
-// tiles up to one per SM.  From there runs or whole tiles by the busiest CTA's estimate: 1.5 us per pair, 1.3 per tile that it touches
-// (its accumulator is drained while nothing is produced), 0.5 for runs.  4608 x 19968, 10 tokens: whole tiles 32.2 us, runs 22.7;
-// 1536 x 25856, 20 tokens: 15.9, 17.3; 5120 x 25600, 16 tokens: half tiles in turn 30.1, runs 29.8.
-inline Runs pick(uint32_t tiles, uint32_t ppt, uint32_t sms) {
-    Cut cut = kTiles;
-    uint32_t grid = tiles;
-    if (2u * tiles <= sms && ppt >= 2u) {
-        cut = kHalves;
-        grid = 2u * tiles;
-    } else if (tiles > sms) {
-        const uint32_t whole = (tiles + sms - 1u) / sms;
-        const uint64_t run = ((uint64_t)tiles * ppt + sms - 1u) / sms;
-        const float by_tiles = (1.5f * (float)ppt + 1.3f) * (float)whole, by_pairs = 1.5f * (float)run + 1.3f * (float)(whole + 1u) + 0.5f;
-        cut = by_tiles <= by_pairs ? kTiles : kPairs;
-        grid = sms;
+// The cut with the shortest estimate, in us, of the busiest CTA: 1.3 per pair and 0.2 per tile that it touches (its accumulator is drained while nothing
+// is produced); and where the grid leaves the kernel in front (`ahead` CTAs, an SM each) no room, its CTAs start that much
+// later: 0.02 per CTA too many, 0.04 with two token tiles.  Fitted to 434 shapes of 9 ... 32 tokens (K = 1024 ... 16384, N = 512 ... 27648): 0.2 % over
+// the best cut on average, 11 % at worst.  us, tiles / halves / pairs:
+//   4608 x 19968, 10 tokens    32.2 / 28.0 / 21.5     runs of pairs balance whatever the tiles are
+//   2048 x 25856, 20 tokens    18.3 / 15.7 / 16.2     halves touch two tiles at most, runs three
+//   1024 x 23040, 10 tokens    11.6 / 10.3 / 10.3
+//   9728 x 6528, 9 tokens      31.6 / 19.5            at most half a tile per SM: halves fill the chip
+//   1536 x 9216, 25 tokens      9.2 /  9.8            but not where a pair saved is less than the later start
+// Between half a tile and a tile per SM a cut saves the busiest CTA nothing.
+inline Runs pick(uint32_t tiles, uint32_t ppt, uint32_t sms, uint32_t ahead, bool wide) {
+    Runs best{};
+    float best_cost = 0.0f;
+    for (uint32_t cut : {kTiles, kHalves, kPairs}) {
+        if (cut == kHalves && (ppt < 2u || (2u * tiles > sms && tiles < sms))) continue;
+        if (cut == kPairs && tiles < sms) continue;      // a run would be shorter than a tile
+        const uint64_t pieces = (uint64_t)tiles * (cut == kPairs ? ppt : cut == kHalves ? 2u : 1u);
+        const uint32_t grid = pieces < sms ? (uint32_t)pieces : sms;
+        const uint32_t most = (uint32_t)((pieces + grid - 1u) / grid);
+        const uint32_t pairs = cut == kPairs ? most : cut == kTiles ? most * ppt : most / 2u * ppt + (most & 1u) * ((ppt + 1u) / 2u);
+        const uint32_t touched = cut == kPairs ? (most + ppt - 2u) / ppt + 1u : cut == kTiles ? most : most / 2u + 1u;
+        const float cost = 1.3f * (float)pairs + 0.2f * (float)touched +
+                           (grid + ahead > sms ? (float)(grid + ahead - sms) * (wide ? 0.04f : 0.02f) : 0.0f);
+        if (best.grid != 0u && cost >= best_cost) continue;
+        best_cost = cost;
+        best = Runs{cut, grid, (uint32_t)(pieces / grid), (uint32_t)(pieces % grid)};
     }
-    const uint64_t pieces = (uint64_t)tiles * (cut == kPairs ? ppt : cut == kHalves ? 2u : 1u);
-    return Runs{cut, grid, (uint32_t)(pieces / grid), (uint32_t)(pieces % grid)};
+    return best;
 }
 
 }  // namespace q4k_runs

@@ -607,7 +607,7 @@ int launch(const void* data, const void* recs, const float* x, const int8_t* xq,
     if (int rc = pdk_launch_pdl(q4k_act_f16_kernel, dim3(NC / 2u + kZeroCtas), dim3(kActThreads), 0, st, x, xq, xq_scale, xh,
                                 tokscale, y, in_dim, out_dim, batch, NC / 2u))
         return rc;
-    const q4k_runs::Runs runs = q4k_runs::pick((out_dim + BM - 1u) / BM, n_unit >> 1, (uint32_t)pdk_sm_count());
+    const q4k_runs::Runs runs = q4k_runs::pick((out_dim + BM - 1u) / BM, n_unit >> 1, (uint32_t)pdk_sm_count(), NC / 2u + kZeroCtas, NC > 32u);
     return pdk_launch_pdl(kern, dim3(runs.grid), dim3(kThreads), smem, st, tx, tw, tr, (const float*)tokscale, y, in_dim,
                           out_dim, batch, runs, pdk_error_word());
 }
