@@ -457,14 +457,20 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
     }
 }
 
+// Clusters of s CTAs that are resident at once: one CTA per SM.
+template <int F, uint32_t NT, bool HL>
+int cluster_caps(const uint32_t** cap) {
+    static PdkClusterCaps table;
+    return pdk_cluster_caps(table, (const void*)kq_batch_kernel<F, NT, HL>, kWarps * 32u, kSmemMax, cap);
+}
+
 template <int F, uint32_t NT, bool HL>
 int launch(const void* data, const void* recs, const float* bias, const float* x, const int8_t* xq, const float* xq_scale, float* y,
            uint32_t in_dim, uint32_t out_dim, uint32_t batch, cudaStream_t st) {
     constexpr uint32_t kThreads = kWarps * 32u;
     auto kern = kq_batch_kernel<F, NT, HL>;
-    static PdkClusterCaps table;
-    const uint32_t* cap = nullptr;       // one CTA per SM
-    if (int rc = pdk_cluster_caps(table, (const void*)kern, kThreads, kSmemMax, &cap)) return rc;
+    const uint32_t* cap = nullptr;
+    if (int rc = cluster_caps<F, NT, HL>(&cap)) return rc;
     Plan p;
     if (!make_plan<F, NT>(p, cap, in_dim, out_dim, batch)) return -1;
     using T = Fmts<F>;
@@ -519,6 +525,19 @@ int pdk_kq_batch(const void* data, const void* scales, const float* x, const int
         case 14u: return launch_f<kQ6K>(data, scales, x, xq, xq_scale, y, in_dim, out_dim, batch, st);
         default: return -1;
     }
+}
+
+// The estimate of the plan for 9 .. 16 tokens of a Q4_K or Q4_0 plane (kq_plan.cuh: super-blocks of a warp); 0 = none.  Without a device, a B200's.
+float pdk_kq_batch_cost(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
+    static const uint32_t b200[kMaxSplit + 1u] = {0, 148, 74, 45, 33, 26, 22, 15, 15};
+    const uint32_t* cap = nullptr;
+    if (cluster_caps<kQ4K, 2, false>(&cap) != 0) {
+        (void)cudaGetLastError();
+        cap = b200;
+    }
+    Plan p;
+    if (batch <= 8u || batch > 16u || out_dim > 0x40000000u) return 0.0f;
+    return make_plan<kQ4K, 2>(p, cap, in_dim, out_dim, batch) ? p.cost : 0.0f;
 }
 
 // The same for repacked Q8_0 planes (data int8 [out_dim][in_dim], scale f16 [out_dim][in_dim / 32], bias [out_dim] or null).

@@ -53,6 +53,7 @@ __host__ __device__ __forceinline__ Layout layout(uint32_t stages, uint32_t batc
 struct Plan {
     uint32_t split, clusters, rounds, round_tiles, ku, stages;
     size_t smem;
+    float cost;      // the estimate that chose it, in units of one super-block's time in a warp
 };
 
 // S and the number of rounds by an estimate in units of one super-block's time in a warp: the longest warp's units and three
@@ -85,7 +86,7 @@ bool make_plan(Plan& best, const uint32_t* cap, uint32_t in_dim, uint32_t out_di
             const float cost = (float)rounds * (float)(units + 3u) + (float)(batch * ku) / 48.0f + cross;
             if (best.split == 0u || cost < best_cost) {
                 best_cost = cost;
-                best = Plan{s, clusters, rounds, rt, ku, d, layout<F, NT>(d, batch, ku, rt).total};
+                best = Plan{s, clusters, rounds, rt, ku, d, layout<F, NT>(d, batch, ku, rt).total, cost};
             }
             break;     // more rounds only cost more
         }

@@ -16,6 +16,7 @@
 #include <cstdlib>
 
 #include "pdk_common.cuh"
+#include "q4k_runs.cuh"
 
 // kquant_more.cu: Q5_K, Q6_K, Q4_0
 bool pdk_kq_more_has(uint32_t dtype);
@@ -39,6 +40,7 @@ int pdk_q6k_gemv_i8(const void* data, const void* scales, const float* x, float*
 // kq_batch.cu: 1..16 tokens of every format here, f32 or int8 activations; -1 = shape outside its plan
 int pdk_kq_batch(const void* data, const void* scales, const float* x, const int8_t* xq, const float* xq_scale, float* y,
                  uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t dtype, cudaStream_t st);
+float pdk_kq_batch_cost(uint32_t in_dim, uint32_t out_dim, uint32_t batch);   // of its plan for 9..16 tokens; 0 = none
 // q4k_batch_i8.cu: 1..8 tokens, same operands and return convention
 int pdk_q4k_batch_i8(const void* data, const void* scales, const float* x, const int8_t* xq, const float* xq_scale,
                      float* y, uint32_t in_dim, uint32_t out_dim, uint32_t batch, cudaStream_t st);
@@ -271,18 +273,20 @@ bool kq_beats_i8(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
     return (uint64_t)out_dim * (in_dim + 2048u) <= limit;
 }
 
-// 9 and more tokens of Q4_K or Q4_0: both kernels' times in us, fitted to 560 timings (K = 1024 ... 12800, N = 520 ... 25600, 9 ... 32 tokens).
-// tcgen05 takes up to 32 tokens for one price: 4.3 us and 0.75 per super-block of a CTA's run (q4k_tc5.cu: equal runs, or half tiles of 128 rows where
-// the plane has fewer of them than the chip has SMs).  kq_batch pays for weights x tokens, 16 tokens a
-// pass, but fills the chip whatever N is and has exact weights.  Measured (us, kq_batch / tcgen05): Q4_K 9728 x 1100, 9 tokens 11.0 / 31.6,
-// 16 tokens 12.6 / 31.8; 12800 x 5000, 12 tokens 31.8 / 40.7; 5120 x 2560, 16 tokens 12.6 / 12.4; 5120 x 25600, 16 tokens 53.7 / 30.3; 9728 x 520, 32 tokens 20.3 / 30.3.
+// 9 and more tokens of Q4_K or Q4_0, the first 32 of them: both kernels' times in us, fitted to 434 timings (K = 1024 ... 16384, N = 512 ... 27648,
+// 9 ... 32 tokens; the choice is 0.3 % off the faster one on average).  tcgen05 takes up to 32 tokens for one price, the run of its busiest CTA
+// (q4k_runs.cuh).  kq_batch pays for weights x tokens, 16 tokens a pass, but fills the chip whatever N is and has exact weights; where
+// K is so long that the activations leave room for the partial sums of a tile or two, its plan takes many rounds and is the price instead.
+// Measured (us, kq_batch / tcgen05): Q4_K 9728 x 1100, 9 tokens 10.9 / 19.3, 16 tokens 12.5 / 19.6; 9728 x 3000, 9 tokens 17.3 / 19.4; 12800 x 5000, 12 tokens
+// 30.3 / 24.2; 5120 x 2560, 16 tokens 12.4 / 12.2; 9728 x 520, 32 tokens 20.1 / 19.6; Q4_0 14848 x 2112, 16 tokens 55.1 / 26.9 (nine rounds).
 bool kq_beats_tc5(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
-    const uint32_t pairs = in_dim >> 9, tiles = (out_dim + 127u) / 128u, sms = 148u, passes = (batch + 15u) / 16u, take = (batch + passes - 1u) / passes;
-    const float run = tiles >= sms ? ceilf((float)tiles * (float)pairs / (float)sms) : 2u * tiles > sms ? (float)pairs : (float)((pairs + 1u) / 2u);   // of the busiest CTA
-    const float tc5 = (float)((batch + 31u) / 32u) * (4.3f + 1.5f * run);
-    const float kq = (float)passes * (5.0f + (float)in_dim / 3000.0f + 0.1f * ((float)take - 9.0f) +
-                                      (float)out_dim * (float)in_dim * (2.25e-7f + 1.0e-8f * (float)take));
-    return kq < tc5;
+    const uint32_t left = batch < 32u ? batch : 32u, passes = (left + 15u) / 16u, take = (left + passes - 1u) / passes;
+    const float tc5 = q4k_runs::launch_us(in_dim, out_dim, left, (uint32_t)pdk_sm_count());
+    const float kq = 5.0f + (float)in_dim / 3000.0f + 0.1f * ((float)take - 9.0f) +
+                     (float)out_dim * (float)in_dim * (2.25e-7f + 1.0e-8f * (float)take);
+    if ((float)passes * kq >= tc5) return false;
+    const float cost = pdk_kq_batch_cost(in_dim, out_dim, take);
+    return cost != 0.0f && (float)passes * 1.2f * cost < tc5;
 }
 
 // The kernel that a pass over `batch` tokens asks first.  Q4_0 up to 8 tokens: kq_batch against the tcgen05 kernel (which costs the same

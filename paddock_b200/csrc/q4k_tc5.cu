@@ -154,7 +154,8 @@ __device__ __forceinline__ uint32_t h2_dup(float v) {
 // xh f16 [NC][K]: row t = hi term of token t, row NC/2 + t = lo term; tokscale f32 [NC/2] = the
 // power of two the token was divided by (0 for unused columns).  One CTA per token column; the
 // CTAs past the token columns zero y.
-constexpr uint32_t kActThreads = 1024, kZeroCtas = 32;  // kActThreads / 32 == 32: the partial maxima fit one warp
+using q4k_runs::kZeroCtas;
+constexpr uint32_t kActThreads = 1024;  // kActThreads / 32 == 32: the partial maxima fit one warp
 __global__ void __launch_bounds__(kActThreads)
 q4k_act_f16_kernel(const float* __restrict__ x, const int8_t* __restrict__ xq, const float* __restrict__ xq_scale,
                    __half* __restrict__ xh, float* __restrict__ tokscale, float* __restrict__ y, uint32_t in_dim,
@@ -607,7 +608,7 @@ int launch(const void* data, const void* recs, const float* x, const int8_t* xq,
     if (int rc = pdk_launch_pdl(q4k_act_f16_kernel, dim3(NC / 2u + kZeroCtas), dim3(kActThreads), 0, st, x, xq, xq_scale, xh,
                                 tokscale, y, in_dim, out_dim, batch, NC / 2u))
         return rc;
-    const q4k_runs::Runs runs = q4k_runs::pick((out_dim + BM - 1u) / BM, n_unit >> 1, (uint32_t)pdk_sm_count(), NC / 2u + kZeroCtas, NC > 32u);
+    const q4k_runs::Runs runs = q4k_runs::pick((out_dim + BM - 1u) / BM, n_unit >> 1, (uint32_t)pdk_sm_count(), NC / 2u);
     return pdk_launch_pdl(kern, dim3(runs.grid), dim3(kThreads), smem, st, tx, tw, tr, (const float*)tokscale, y, in_dim,
                           out_dim, batch, runs, pdk_error_word());
 }

@@ -77,6 +77,10 @@ def test_routes_of_small_batches():
         assert [route(9728, n, 9, dtype) for n in (1100, 3000, 5000)] == [1, 1, 3]
         assert [route(9728, n, 32, dtype) for n in (520, 2560)] == [3, 3]
         assert [route(5120, n, 16, dtype) for n in (1100, 5000)] == [1, 3]
+        # long K: kq_batch has room for the partial sums of one tile only, nine rounds of them
+        assert route(14848, 2112, 16, dtype) == 3 and route(14848, 704, 16, dtype) == 1
+        # more than 32 tokens: what counts is the first 32, which tcgen05 takes in one launch
+        assert [route(9216, 640, m, dtype) for m in (32, 33, 37, 64)] == [3, 3, 3, 3]
     assert [route(5120, 25600, m, q5_k) for m in (8, 9, 64)] == [2, 1, 1]
     assert [route(5120, 25600, m, q4_0) for m in (2, 8, 9, 64)] == [1, 1, 3, 3]
     assert [route(5120, 25600, m, q6_k) for m in (2, 16, 64)] == [1, 1, 1]

@@ -13,7 +13,7 @@ int main() {
     for (uint32_t sms : {1u, 16u, 132u, 148u})
         for (uint32_t ppt = 1; ppt <= 32u; ++ppt)
             for (uint32_t tiles = 1; tiles <= 700u; ++tiles) {
-                const Runs r = pick(tiles, ppt, sms, tiles & 1u ? 48u : 64u, (tiles & 1u) == 0u);
+                const Runs r = pick(tiles, ppt, sms, tiles & 1u ? 16u : 32u);
                 bool ok = r.grid >= 1u && r.grid <= sms && start(r, 0u, ppt) == 0u && start(r, r.grid, ppt) == tiles * ppt;
                 uint32_t of[700] = {0};
                 for (uint32_t c = 0; c < r.grid && ok; ++c) {
