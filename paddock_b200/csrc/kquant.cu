@@ -249,11 +249,16 @@ bool force_plain() {
 
 enum Route : int { kRouteKq = 1, kRouteI8 = 2, kRouteTc5 = 3 };
 
-// From how many tokens on the tcgen05 kernel takes a Q4_K call (PDK_Q4K_TC5_MIN, read once; 0 = never).
-uint32_t tc5_min_tokens() {
-    static const uint32_t v = [] {
+// From how many tokens on the tcgen05 kernel takes a Q4_K call: 9, where kq_beats_tc5 agrees.  PDK_Q4K_TC5_MIN (read once) sets it by hand, and
+// then no estimate has a say (Q4_0: from 9 tokens); 0 = never.
+struct Tc5Min {
+    uint32_t tokens;
+    bool by_hand;
+};
+const Tc5Min& tc5_min() {
+    static const Tc5Min v = [] {
         const char* e = getenv("PDK_Q4K_TC5_MIN");
-        return e ? (uint32_t)atoi(e) : 9u;
+        return e ? Tc5Min{(uint32_t)atoi(e), true} : Tc5Min{9u, false};
     }();
     return v;
 }
@@ -294,8 +299,9 @@ bool kq_beats_tc5(uint32_t in_dim, uint32_t out_dim, uint32_t batch) {
 // N = 25600: 26.4 / 29.2 us at 4 tokens; N = 9472: 16.2 / 15.2 at 8).  Q5_K from 9 tokens on: two passes of the integer kernel would
 // be faster on wide planes (K = 5120, N = 25600, 16 tokens: 51.6 against 64.5 us), but kq_batch keeps 22 activation bits.
 Route batch_route(uint32_t in_dim, uint32_t out_dim, uint32_t batch, uint32_t dtype) {
-    const uint32_t from = dtype == PDK_KQ_Q4K ? tc5_min_tokens() : dtype == PDK_KQ_Q4_0 && tc5_min_tokens() != 0u ? 9u : 0u;
-    if (from != 0u && batch >= from) return kq_beats_tc5(in_dim, out_dim, batch) ? kRouteKq : kRouteTc5;
+    const Tc5Min& min = tc5_min();
+    const uint32_t from = dtype == PDK_KQ_Q4K ? min.tokens : dtype == PDK_KQ_Q4_0 && min.tokens != 0u ? 9u : 0u;
+    if (from != 0u && batch >= from) return !min.by_hand && kq_beats_tc5(in_dim, out_dim, batch) ? kRouteKq : kRouteTc5;
     if ((dtype == PDK_KQ_Q4K || dtype == PDK_KQ_Q5K) && batch <= 8u && !kq_beats_i8(in_dim, out_dim, batch)) return kRouteI8;
     return kRouteKq;
 }

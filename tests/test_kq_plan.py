@@ -2,6 +2,7 @@
 shared memory fits, the partial sums that a cluster sends fit the ring, the sizes do not wrap at the largest planes; and the rule that gives a call to that kernel or to another."""
 import os
 import subprocess
+import sys
 
 SRC = r"""
 #include <cstdio>
@@ -85,3 +86,12 @@ def test_routes_of_small_batches():
     assert [route(5120, 25600, m, q4_0) for m in (2, 8, 9, 64)] == [1, 1, 3, 3]
     assert [route(5120, 25600, m, q6_k) for m in (2, 16, 64)] == [1, 1, 1]
     assert route(5120, 25600, 4, iq4_xs) == 0
+
+
+def test_the_switch_is_not_overruled():
+    """PDK_Q4K_TC5_MIN by hand: from that many tokens on every Q4_K plane asks tcgen05 first, narrow ones too; 0 = none does."""
+    src = "import paddock_b200; r = paddock_b200.KernelPack.load()._lib.pdk_kquant_gemm_route; print([r(9728, 1100, m, 12) for m in (4, 9, 16)], r(9728, 1100, 9, 2))"
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    for value, want in ((None, "[1, 1, 1] 1"), ("9", "[1, 3, 3] 3"), ("4", "[3, 3, 3] 3"), ("0", "[1, 1, 1] 1")):
+        env = {k: v for k, v in os.environ.items() if k != "PDK_Q4K_TC5_MIN"} | ({"PDK_Q4K_TC5_MIN": value} if value else {})
+        assert subprocess.check_output([sys.executable, "-c", src], cwd=root, env=env, text=True).strip() == want, value
