@@ -422,6 +422,12 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         if (split > 1u) cluster_sync();        // every CTA of the cluster is done with its ring
         const uint32_t rows = nt * kRows, rpo = (rows + split - 1u) / split;
         const uint32_t part = tc5::smem_u32(smem);
+        // Only calls on Q8_0 planes have a bias.  Where the other formats asked for it too it cost them 0.1 to 0.2 us, and 10 % where a cluster
+        // stores many rows (Q4_K 7424 x 5707, 11 tokens 24.8 us with the question, 22.3 without).
+        auto with_bias = [&](float v, uint32_t n) {
+            if constexpr (F == kQ80) return a.bias ? v + a.bias[n] : v;
+            return v;
+        };
         for (uint32_t i = tid; i < rows * a.batch; i += kThreads) {
             const uint32_t tok = i / rows, r = i - tok * rows, tl = r / kRows;
             const uint32_t w_lo = (tl * ku * kWarps + kWarps - 1u) / total, w_hi = ((tl * ku + ku - 1u) * kWarps + kWarps - 1u) / total;
@@ -433,7 +439,7 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 const uint32_t owner = r / rpo;
                 st_cluster(cluster_addr(part, owner) + ((rank * a.batch + tok) * rpo + (r - owner * rpo)) * 4u, v);
             } else if (r0 * kRows + r < a.out_dim) {
-                a.y[(size_t)tok * a.out_dim + r0 * kRows + r] = a.bias ? v + a.bias[r0 * kRows + r] : v;
+                a.y[(size_t)tok * a.out_dim + r0 * kRows + r] = with_bias(v, r0 * kRows + r);
             }
         }
         if (split > 1u) {
@@ -447,7 +453,7 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
                 const uint32_t tok = i / own, r = i - tok * own, n = r0 * kRows + rank * rpo + r;
                 float v = 0.0f;
                 for (uint32_t s = 0; s < split; ++s) v += got[(s * a.batch + tok) * rpo + r];
-                if (n < a.out_dim) a.y[(size_t)tok * a.out_dim + n] = a.bias ? v + a.bias[n] : v;
+                if (n < a.out_dim) a.y[(size_t)tok * a.out_dim + n] = with_bias(v, n);
             }
         }
         if (r0 + a.round_tiles < t_hi) {
