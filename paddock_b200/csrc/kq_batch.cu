@@ -422,10 +422,12 @@ kq_batch_kernel(const __grid_constant__ CUtensorMap tm0, const __grid_constant__
         if (split > 1u) cluster_sync();        // every CTA of the cluster is done with its ring
         const uint32_t rows = nt * kRows, rpo = (rows + split - 1u) / split;
         const uint32_t part = tc5::smem_u32(smem);
-        // Only calls on Q8_0 planes have a bias.  Where the other formats asked for it too it cost them 0.1 to 0.2 us, and 10 % where a cluster
-        // stores many rows (Q4_K 7424 x 5707, 11 tokens 24.8 us with the question, 22.3 without).
+        // Only calls on Q8_0 planes have a bias.  Where the other formats' instances for 5 and more tokens asked for it too it cost them 0.1 to
+        // 0.2 us, and 10 % where a cluster stores many rows (Q4_K 7424 x 5707, 11 tokens 25.0 us, 22.6 without).  Up to four tokens the
+        // question stays: without it the compiler's main loops are 1 to 2 % slower on large planes (Q6_K 17408 x 5003, 3 tokens 25.5 -> 25.8,
+        // Q4_K 17408 x 5120 19.9 -> 20.3), and small ones gain as much (Q5_K 1280 x 2778, 2 tokens 4.48 -> 4.38).
         auto with_bias = [&](float v, uint32_t n) {
-            if constexpr (F == kQ80) return a.bias ? v + a.bias[n] : v;
+            if constexpr (F == kQ80 || HL) return a.bias ? v + a.bias[n] : v;
             return v;
         };
         for (uint32_t i = tid; i < rows * a.batch; i += kThreads) {
