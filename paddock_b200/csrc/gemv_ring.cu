@@ -575,12 +575,18 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
     if constexpr (SPLIT) {
         __syncwarp();
         tc5::cluster_sync();     // every CTA's sums are here
-        for (uint32_t r = tid; r < rpo; r += W * teams * 32u) {
-            const uint32_t at = rank * rpo + r, row = tile_lo * 16u + at;
-            if (at >= rows || row >= out_dim) break;
+        const uint32_t at = rank * rpo, row0 = tile_lo * 16u + at;
+        const uint32_t mine = min(min(rpo, rows - min(rows, at)), out_dim - min(out_dim, row0));
+        auto sum = [&](uint32_t r) {
             float v = 0.0f;
             for (uint32_t s = 0; s < split; ++s) v += recv[s * rpo + r];
-            put(row, v);
+            return v;
+        };
+        // with the peers' store in the one loop, calls without peers took 0.04 to 0.1 us longer (Q6_K 12032 x 832 5.46 -> 5.54)
+        if (peers.n == 0u) {
+            for (uint32_t r = tid; r < mine; r += W * teams * 32u) y[row0 + r] = bias ? sum(r) + bias[row0 + r] : sum(r);
+        } else {
+            for (uint32_t r = tid; r < mine; r += W * teams * 32u) put(row0 + r, sum(r));
         }
     }
     if (peers.n != 0u && peers.signal == 1u) {   // uniform over the grid
