@@ -1,12 +1,14 @@
 """Helpers shared by the -m gpu parity tests: seeded synthetic planes, device
 buffers (torch is only the allocator here) and the two error metrics the
 reference's own GPU tests use."""
+import ctypes
+
 import numpy as np
 import torch
 
 import oracle
 
-TOL = 1e-2  # max relative error for GEMV/GEMM outputs stated by the north star
+TOL = 1e-2  # the largest relative error a GEMV / GEMM output may have; the kernels are held to tighter bounds
 
 
 def dev(a):
@@ -40,3 +42,15 @@ def cond_err(y, ref, abs_sum):
 def rel_l2(y, ref):
     """rel-L2 (tests/gpu_kquant_parity.rs:145-153)."""
     return float(np.linalg.norm(y.astype(np.float64) - ref) / max(np.linalg.norm(ref), 1e-12))
+
+
+def gemv_plan(pack, k, n, dtype):
+    """(warps of a team, teams, CTAs of a cluster, stages) of the ring kernel for a one-token call; all 0: the register kernel."""
+    plan = (ctypes.c_uint32 * 4)()
+    assert pack._lib.pdk_gemv_plan(k, n, dtype, plan) == 0
+    return tuple(plan)
+
+
+def gemm_route(pack, k, n, batch, dtype):
+    """1 kq_batch.cu, 2 the integer kernel, 3 tcgen05 (K a multiple of 512 up to 16384), 0 none of them."""
+    return pack._lib.pdk_kquant_gemm_route(k, n, batch, dtype)

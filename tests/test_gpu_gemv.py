@@ -10,7 +10,7 @@ import pytest
 import torch
 
 import oracle
-from gpu_util import TOL, bf16_activations, cond_err, dev, dev_f32, rel_l2, seed_for
+from gpu_util import TOL, bf16_activations, cond_err, dev, dev_f32, gemm_route, gemv_plan, rel_l2, seed_for
 
 pytestmark = pytest.mark.gpu
 
@@ -126,11 +126,10 @@ def test_q4_k_gemv_shapes(pack, k, n):
     assert rel_l2(y, ref[0]) < 1e-4 < TOL
 
 
-# Shapes chosen for the ring-staged decode GEMV's plans: 8 units per row (the smallest it takes),
-# stages that do not divide the row (18, 22, 68, 108 units), an odd unit count (43: the lanes
-# copy Q4_K's 24-byte records there), fewer than 16
-# rows, a last tile of one row, and more tiles than SMs so that the ring wraps many times.
-RING_SHAPES = [(2048, 7), (2048, 4099), (4608, 33), (5632, 100), (11008, 49), (17408, 161), (27648, 40), (4096, 16 * 148 * 3 + 1)]
+# Shapes chosen for the ring kernel's plans of one team (asserted): 8 units per row, stages that do not divide the row (18, 22, 68, 108
+# units; the longer ones split over a cluster), an odd unit count (43: the lanes copy Q4_K's 24-byte records there), fewer than 16
+# rows, a last tile of three rows, and five tiles per SM so that the ring wraps.  The other plans: test_gpu_gemv_ring.py.
+RING_SHAPES = [(2048, 7), (2048, 2099), (4608, 33), (5632, 100), (11008, 49), (17408, 161), (27648, 40), (4608, 16 * 148 * 4 + 1)]
 
 
 @pytest.mark.parametrize("k,n", RING_SHAPES)
@@ -139,6 +138,7 @@ def test_q4_k_gemv_ring_plans(pack, k, n):
     x = bf16_activations(k, seed_for(2, 3))
     raw, d_data, d_sc = q4k_planes(pack, w, n, k)
     d_y = torch.full((n + 8,), 7.0, dtype=torch.float32, device="cuda")
+    assert gemv_plan(pack, k, n, 12)[1] == 1
     pack.call("kquant_gemv", d_data, d_sc, dev_f32(x), d_y, k, n, 12)
     torch.cuda.synchronize()
     assert pack.device_error() == 0
@@ -156,6 +156,7 @@ def test_q8_0_gemv_ring_plans(pack, k, n):
     raw, d_data, d_scale = q8_planes(pack, w, n, k)
     bias = oracle.fill_normal(n, 9, 0.1)
     d_y = torch.full((n + 8,), 7.0, dtype=torch.float32, device="cuda")
+    assert gemv_plan(pack, k, n, 8)[1] == 1
     pack.call("q8_0_gemv_repacked", d_data, d_scale, dev_f32(bias), dev_f32(x), d_y, k, n)
     torch.cuda.synchronize()
     assert pack.device_error() == 0
@@ -182,10 +183,11 @@ def test_gemv_ring_back_to_back_is_deterministic(pack):
         assert torch.equal(y, ys[0])
 
 
-@pytest.mark.parametrize("batch", [1, 4, 16])
-def test_q4_k_small_batch_k5120_band(pack, batch):
-    """Q4_K K=5120 at 1 / 4 / 16 tokens on a 1536-row band of N=25600."""
-    k, n = 5120, 1536
+@pytest.mark.parametrize("batch,n,route", [(1, 1536, 0), (4, 1536, 1), (16, 1536, 1), (16, 4001, 3)])
+def test_q4_k_small_batch_k5120_band(pack, batch, n, route):
+    """Q4_K K=5120 at 1 / 4 / 16 tokens on bands of N=25600: the GEMV, kq_batch.cu, and tcgen05 from where the band is wide enough."""
+    k = 5120
+    assert gemm_route(pack, k, n, batch, 12) == route
     w = oracle.fill_normal(n * k, seed_for(2, 0), 0.02)
     x = bf16_activations(batch * k, seed_for(2, 100 + batch))
     raw, d_data, d_sc = q4k_planes(pack, w, n, k)
@@ -194,18 +196,19 @@ def test_q4_k_small_batch_k5120_band(pack, batch):
     torch.cuda.synchronize()
     ref, ab = oracle.matmul_f64(oracle.dequant_q4_k(raw), x, k, n, batch, with_abs=True)
     y = d_y.cpu().numpy().reshape(batch, n)
-    # up to 8 tokens: integer tensor path (15-bit activations); from 9 on the f16-weight tcgen05 path
-    assert cond_err(y, ref, ab) < (1e-5 if batch <= 8 else 1e-4)
-    assert rel_l2(y, ref) < (1e-4 if batch <= 8 else 1e-3) < TOL
+    # exact weights; tcgen05 rounds them to f16
+    assert cond_err(y, ref, ab) < (1e-4 if route == 3 else 1e-5)
+    assert rel_l2(y, ref) < (1e-3 if route == 3 else 1e-4) < TOL
 
 
-@pytest.mark.parametrize("k,n,batch", [(5120, 1000, 2), (2048, 130, 8), (1024, 48, 5),      # kq_batch.cu, ragged rows
-                                       (5120, 1000, 9), (2048, 300, 17), (4096, 257, 32),   # tcgen05, K halves
-                                       (1536, 200, 16), (5120, 640, 40),                    # one K part; two launches
-                                       (1280, 64, 16)])                                     # odd super-block count: kq_batch.cu
-def test_q4_k_batch_shapes(pack, k, n, batch):
-    """pdk_kquant_gemm_f32 on f32 activations that are not bf16 values, narrow planes (the integer kernel's wide ones:
-    test_gpu_i8_batch.py)."""
+@pytest.mark.parametrize("k,n,batch,route", [(5120, 1000, 2, 1), (2048, 130, 8, 1), (1024, 48, 5, 1), (5120, 1000, 9, 1),   # kq_batch.cu, ragged rows
+                                             (5120, 4001, 9, 3), (2048, 300, 17, 3), (4096, 257, 32, 3),                 # tcgen05, K halves
+                                             (1536, 9601, 16, 3), (5120, 640, 40, 3),       # whole tiles; a launch and a pass of eight tokens
+                                             (1280, 64, 16, 3)])                            # odd super-block count: tcgen05 declines, kq_batch.cu
+def test_q4_k_batch_shapes(pack, k, n, batch, route):
+    """pdk_kquant_gemm_f32 on f32 activations that are not bf16 values (the integer kernel's wide planes: test_gpu_i8_batch.py)."""
+    assert gemm_route(pack, k, n, batch, 12) == route
+    f16_weights = route == 3 and k % 512 == 0
     w = oracle.fill_normal(n * k, seed_for(2, 900 + k + n), 0.02)
     x = oracle.fill_normal(batch * k, seed_for(2, 901 + batch), 1.0)
     x[:k] *= 1.0e4                       # one token far outside the f16 range, one tiny, one zero
@@ -220,7 +223,7 @@ def test_q4_k_batch_shapes(pack, k, n, batch):
     ref, ab = oracle.matmul_f64(oracle.dequant_q4_k(raw), x, k, n, batch, with_abs=True)
     y = d_y.cpu().numpy().reshape(batch, n)
     for t in range(batch):               # per token: the tokens differ by ten orders of magnitude
-        assert cond_err(y[t:t + 1], ref[t:t + 1], np.maximum(ab[t:t + 1], 1e-30)) < 1e-4, t
+        assert cond_err(y[t:t + 1], ref[t:t + 1], np.maximum(ab[t:t + 1], 1e-30)) < (1e-4 if f16_weights else 1e-5), t
     if batch > 2:
         assert not y[2].any()
 
@@ -251,8 +254,9 @@ def test_q4_k_two_to_eight_tokens(pack, k, n, batch):
 
 
 def test_q4_k_batch_is_deterministic(pack):
-    """The two K halves of a tile add into y in either order: the result must not depend on it."""
-    k, n, batch = 5120, 2048, 16
+    """tcgen05: the two K halves of a tile add into y in either order: the result must not depend on it."""
+    k, n, batch = 5120, 4001, 16
+    assert gemm_route(pack, k, n, batch, 12) == 3
     raw, d_data, d_sc = q4k_planes(pack, oracle.fill_normal(n * k, 77, 0.02), n, k)
     x = dev_f32(oracle.fill_normal(batch * k, 78, 1.0))
     outs = []
@@ -307,9 +311,10 @@ def test_quantize_q8_bit_exact(pack, n):
     assert torch.equal(d_q, d_q2) and torch.equal(d_s, d_s2)
 
 
-@pytest.mark.parametrize("k,n,batch", [(5120, 512, 1), (1024, 96, 1), (5120, 768, 4), (2048, 1000, 16)])
-def test_q4k_w4a8_slots(pack, k, n, batch):
+@pytest.mark.parametrize("k,n,batch,route", [(5120, 512, 1, 0), (1024, 96, 1, 0), (5120, 768, 4, 1), (2048, 1000, 16, 1), (1024, 2561, 16, 3)])
+def test_q4k_w4a8_slots(pack, k, n, batch, route):
     """Slots 217 / 212 / 837 against an f64 matmul of the dequantized weights and q * scale."""
+    assert gemm_route(pack, k, n, batch, 12) == route
     raw, d_data, d_sc = q4k_planes(pack, oracle.fill_normal(n * k, 710 + n, 0.02), n, k)
     x = oracle.fill_normal(batch * k, 711, 1.0)
     q, s, sums = oracle.quantize_q8_act(x)
@@ -329,8 +334,8 @@ def test_q4k_w4a8_slots(pack, k, n, batch):
             pack.call(name, d_data, d_sc, dev(q), dev_f32(s), dev_f32(sums), d_part, d_y, k, n, batch, 12)
         torch.cuda.synchronize()
         y = d_y.cpu().numpy().reshape(batch, n)
-        # up to 8 tokens of these narrow planes run kq_batch.cu, more the f16-weight tcgen05 path
-        assert cond_err(y, ref, ab) < 1e-4 < TOL, name
+        # exact weights; tcgen05 rounds them to f16
+        assert cond_err(y, ref, ab) < (1e-4 if route == 3 else 1e-5) < TOL, name
 
 
 # ---- Q5_K, Q6_K, Q4_0 through the same slots
@@ -380,8 +385,8 @@ def test_more_kquants_dequant_repack_gemv(pack, name, k, n):
             pack.call("pdk_kquant_gemm_f32", d_data, d_sc, dev_f32(x), d_out, k, n, batch, dtype)
         torch.cuda.synchronize()
         ref, ab = oracle.matmul_f64(want, x, k, n, batch, with_abs=True)
-        # Q4_0 from nine tokens on (and K a multiple of 512) runs the f16-weight tcgen05 kernel
-        tol = 1e-4 if (name == "q4_0" and batch >= 4 and k % 512 == 0) else 1e-5
+        # the tcgen05 kernel rounds weights to f16
+        tol = 1e-4 if gemm_route(pack, k, n, batch, dtype) == 3 else 1e-5
         assert cond_err(d_out.cpu().numpy().reshape(batch, n), ref, ab) < tol < TOL
 
 
@@ -415,8 +420,8 @@ def test_q5_k_q6_k_tokens_as_columns(pack, name, batch):
     assert one < 1e-4, ("decode GEMV", one)
 
 
-# (8192, 3200) and (17408, 3200): the ring kernel splits the pairs of a row over a cluster; (1024, 160): the register kernel
-@pytest.mark.parametrize("k,n", [(5120, 512), (8192, 3200), (17408, 3200), (17408, 2560), (1024, 160)])
+# (8192, 3200) and (17408, 3200): the ring kernel splits the pairs of a row over a cluster; (6656, 2501): many warps; (1024, 160): the register kernel
+@pytest.mark.parametrize("k,n", [(5120, 512), (8192, 3200), (17408, 3200), (17408, 2560), (6656, 2501), (15872, 2500), (1024, 160)])
 def test_q4k_gemv_shard_stores_band_into_every_output(pack, k, n):
     """pdk_q4k_gemv_shard and _sync with two destination vectors on one GPU (the multi-GPU case points the
     second at a peer's buffer): both receive the band at row0, bit-identical to kquant_gemv."""

@@ -1,12 +1,13 @@
-"""The ring GEMV (gemv_ring.cu) over its formats and routes: odd super-block counts (the lanes copy the records, the last pair is
-half zeros), one and several teams of warps, rows split over a cluster, row counts from one to more tiles than SMs.
+"""The ring GEMV (gemv_ring.cu) over its formats and instances: odd super-block counts (the lanes copy the records, the last pair is
+half zeros), one and several teams of warps, rows split over a cluster, row counts from one to more tiles than SMs.  test_plans takes shapes
+as they come; test_instances looks for a plan of every instance and asserts it.
 
 Bounds as in test_gpu_gemv.py: 15-bit block floating point activations, exact integer products, f32 folds."""
 import pytest
 import torch
 
 import oracle
-from gpu_util import cond_err, dev, dev_f32, rel_l2
+from gpu_util import cond_err, dev, dev_f32, gemv_plan, rel_l2
 from test_gpu_gemv import KQ, q4k_planes, q8_planes, raw_kquant
 
 pytestmark = pytest.mark.gpu
@@ -31,14 +32,40 @@ def plane(pack, name, k, n, seed):
     return want, lambda x, y, st=0: pack.call("kquant_gemv", data, sc, x, y, k, n, dtype, stream=st)
 
 
+DTYPE = {"q8_0": 8, "q4_k": 12, "q4_0": KQ["q4_0"][0], "q5_k": KQ["q5_k"][0], "q6_k": KQ["q6_k"][0]}
+
+
+@pytest.mark.parametrize("split", [False, True])
+@pytest.mark.parametrize("odd", [False, True])
+@pytest.mark.parametrize("many", [False, True])
+@pytest.mark.parametrize("name", ["q8_0", "q4_k", "q4_0", "q5_k", "q6_k"])
+def test_instances(pack, name, many, odd, split):
+    """Every instance of the kernel - many warps or one team, odd rows, a cluster per row - at the smallest plane of a list that
+    takes it here (clusters of a size that fit the chip differ between parts)."""
+    if many and name == "q8_0":
+        pytest.skip("no instance: two boxes a unit leave no room for the stages")
+    for k, n in sorted(((k, n) for k in range(1536 + 256 * odd, 17408, 512) for n in (523, 1053, 2501, 3203, 4003)), key=lambda s: s[0] * s[1]):
+        warps, teams, ctas, _ = gemv_plan(pack, k, n, DTYPE[name])
+        if warps != 0 and (teams > 1 or warps > 12) == many and (ctas > 1) == split:
+            # the large elements fill whole blocks: in a block with both kinds 15 bits of the largest element alone cost up to 1.2e-5
+            # of sum |w||x| at K = 1536 (the f64 product with x rounded to limbs: 1.21e-5 for Q5_K 1536 x 523)
+            check(pack, name, k, n, 192)
+            return
+    pytest.fail("no shape takes this instance")
+
+
 @pytest.mark.parametrize("name", ["q8_0", "q4_k", "q4_0", "q5_k", "q6_k"])
 @pytest.mark.parametrize("k,n", [(1024, 17), (1536, 1), (1792, 333), (2304, 520), (2560, 2501), (3328, 4749), (5376, 17), (9472, 40),
                                  (17152, 531), (17408, 1040), (27904, 5)])
 def test_plans(pack, name, k, n):
+    check(pack, name, k, n)
+
+
+def check(pack, name, k, n, tail=200):
     want, launch = plane(pack, name, k, n, 40 + k + n)
     x = oracle.fill_normal(k, 41 + k, 1.0)
-    x[k - 200:] *= 100.0                   # the end of the row counts
-    x = oracle.bf16_round(x)               # what 15 bits drop of an f32 value would be the larger error where 200 elements rule the sum
+    x[k - tail:] *= 100.0                  # the end of the row counts
+    x = oracle.bf16_round(x)               # what 15 bits drop of an f32 value would be the larger error where a few elements rule the sum
     outs = []
     for _ in range(2):
         y = torch.full((n,), float("nan"), dtype=torch.float32, device="cuda")

@@ -90,7 +90,9 @@ def test_routes_of_small_batches():
 
 def test_the_switch_is_not_overruled():
     """PDK_Q4K_TC5_MIN by hand: from that many tokens on every Q4_K plane asks tcgen05 first, narrow ones too; 0 = none does."""
-    src = "import paddock_b200; r = paddock_b200.KernelPack.load()._lib.pdk_kquant_gemm_route; print([r(9728, 1100, m, 12) for m in (4, 9, 16)], r(9728, 1100, 9, 2))"
+    src = """import paddock_b200
+route = paddock_b200.KernelPack.load()._lib.pdk_kquant_gemm_route
+print([route(9728, 1100, m, 12) for m in (4, 9, 16)], route(9728, 1100, 9, 2))"""
     root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
     for value, want in ((None, "[1, 1, 1] 1"), ("9", "[1, 3, 3] 3"), ("4", "[3, 3, 3] 3"), ("0", "[1, 1, 1] 1")):
         env = {k: v for k, v in os.environ.items() if k != "PDK_Q4K_TC5_MIN"} | ({"PDK_Q4K_TC5_MIN": value} if value else {})
