@@ -284,7 +284,7 @@ int launch(const void* data, const void* recs, const float* bias, const float* x
 
 }  // namespace
 
-// The register-staged kernel: the route for short rows, where it starts faster than the ring kernel (gemv_ring.cu, make_plan), and for
+// The register-staged kernel: the route for short rows, where it starts faster than the ring kernel (ring_plan.cuh has the line), and for
 // what that one declines.
 // All return 0 / a cudaError_t, or -1 when the shape is outside this kernel's plan too (K not a
 // multiple of 256, fewer than four units per row, or activations too long for shared memory).

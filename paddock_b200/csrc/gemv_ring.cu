@@ -506,7 +506,8 @@ gemv_ring_kernel(const __grid_constant__ CUtensorMap dmap, const __grid_constant
                     Stage st[kSide];
 #pragma unroll
                     for (uint32_t i = 0; i < kSide; ++i)
-                        F::load_ring(st[i], sd + (i0 + i) * kUnitData, sd + kStageHigh + (i0 + i) * kUnitHigh, sr + (i0 + i) * F::kRecBytes, rec8, o0, o1, g, t);
+                        F::load_ring(st[i], sd + (i0 + i) * kUnitData, sd + kStageHigh + (i0 + i) * kUnitHigh, sr + (i0 + i) * F::kRecBytes, rec8, o0,
+                                     o1, g, t);
                     if (MANY || !invariant) load_b(2u * pr + i0);
                     int c[kSide][kPasses][4] = {};
 #pragma unroll
@@ -719,8 +720,8 @@ int shape_plan(uint32_t in_dim, uint32_t out_dim, const RingPlan** plan) {
     return k.ok != 0u ? 0 : -1;
 }
 
-// -1: outside the plan (rows of up to four units: Q6_K 1024 x 618 2.2 us on registers, 2.5 here; planes that do not start on 16 bytes, activations too long), or the
-// register-staged kernel is faster.
+// -1: outside the plan (rows of up to four units: Q6_K 1024 x 618 2.2 us on registers, 2.5 here; planes that do not start on
+// 16 bytes, activations too long), or the register-staged kernel is faster.
 template <class F>
 int launch_ring(const void* data, const void* recs, const float* bias, const float* x, float* y, uint32_t in_dim,
                 uint32_t out_dim, cudaStream_t st, const int8_t* xq = nullptr, const float* xq_scale = nullptr,
@@ -753,7 +754,7 @@ int launch_ring(const void* data, const void* recs, const float* bias, const flo
 // ---------------------------------------------------------------------------
 // Q8_0 with 2..8 tokens on the same ring: the tokens are the mma's eight columns.
 //
-// Plans with one unit pair per warp only (W == K / 512, K = 2048 .. 6144): warp w meets the same
+// Plans with one unit pair per warp only (W == K / 512, K = 2048, 2560 .. 5632): warp w meets the same
 // 512 activations of every token in every tile, so its B operand - two int8 limbs of the 15-bit
 // block floating point, per (token, 32-block) power-of-two steps - is built once from x and stays
 // in 64 registers.  Per 32-weight block: one ldmatrix.x4 takes the 16 rows x 32 int8 out of the
@@ -1033,8 +1034,8 @@ int pdk_q4k_gemv_peers_regs(const void*, const void*, const float*, const gemv_i
 // Decode GEMV entry points of the int8 tensor path.  Each returns 0 / a cudaError_t, or -1 when the
 // shape is outside both kernels' plans (K not a multiple of 256, fewer than four units per row, or
 // activations too long for shared memory) and the caller should take another route.  The ring
-// kernel takes K >= 2048 (even super-block counts for the formats with 24-byte records); the
-// register-staged kernel takes the rest, and Q5_K.
+// kernel takes rows of five units and more where its plan's price is the lower one (ring_plan.cuh);
+// the register-staged kernels take the rest.
 int pdk_q4k_gemv_i8(const void* data, const void* scales, const float* x, float* y, uint32_t in_dim,
                     uint32_t out_dim, cudaStream_t st) {
     const int rc = launch_ring<RQ4K>(data, scales, nullptr, x, y, in_dim, out_dim, st);

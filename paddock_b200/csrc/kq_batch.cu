@@ -20,14 +20,15 @@
 // Split: a cluster of S CTAs shares a run of 16-row tiles, each CTA one part of K - its part of the activations (4 bytes
 // per element and token) has to fit beside the ring, and narrow planes fill the chip that way.  A CTA's (tile, unit)
 // pairs are one sequence, cut into equal runs for its 16 warps whatever the tile count; a warp leaves one partial tile per
-// tile that it touched, and the partials meet once per round (as many tiles as shared memory holds partials of; one, mostly), in a fixed order, across the cluster in distributed
-// shared memory: the same sum whatever the timing, no scratch, no zeroing of y, one launch.
+// tile that it touched, and the partials meet once per round (as many tiles as shared memory holds partials of; one,
+// mostly), in a fixed order, across the cluster in distributed shared memory: the same sum whatever the timing, no
+// scratch, no zeroing of y, one launch.
 //
 // Measured on a B200 (us; up to 4 tokens: terms as two mmas -> as columns).  Q6_K, K = 17408, N = 5003: 28.2 -> 26.0 at 2 tokens, 27.8 -> 25.6 at 3,
 // 28.7 -> 26.5 at 4, 34.1 at 8; K = 5120, N = 25600: 33.2 -> 30.4 at 2, 38 at 8, 76 at 16.  Q4_K, K = 17408, N = 5120: 23.6 -> 20.6 at 2; Q4_0, K = 5120,
-// N = 25600: 25.4 -> 21.5.  Q8_0 (a GEMV per token before): 7424 x 520, 8 tokens 108 -> 6.7; 2816 x 6016, 16 tokens 96 -> 16.  What bounds it from 5 tokens: the shared
-// memory pipe (118 wavefronts per unit, 64 of them the activation fragments: 13 of the 25 us of Q4_K, K = 5120, N = 25600 at 2 tokens with two mmas) and
-// issue slots (450 instructions per unit).  Tiles of 32 rows halve the fragments but double the ring's stages, so that
+// N = 25600: 25.4 -> 21.5.  Q8_0 (a GEMV per token before): 7424 x 520, 8 tokens 108 -> 6.7; 2816 x 6016, 16 tokens 96 -> 16.
+// What bounds it from 5 tokens: the shared memory pipe (118 wavefronts per unit, 64 of them the activation fragments: 13 of
+// the 25 us of Q4_K, K = 5120, N = 25600 at 2 tokens with two mmas) and issue slots (450 instructions per unit).  Tiles of 32 rows halve the fragments but double the ring's stages, so that
 // fewer fit: 24.7 us at 1 token, but 45 at 8 and no plan at all for Q6_K, not kept.
 #include "cluster_caps.cuh"
 #include "kq_plan.cuh"

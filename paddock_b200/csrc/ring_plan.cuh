@@ -7,7 +7,7 @@
 namespace ring {
 
 constexpr uint32_t kMaxWarps = 12;                      // with 168 registers a thread
-constexpr uint32_t kManyWarps = 20, kMaxTeams = 10;     // with 96
+constexpr uint32_t kManyWarps = 20, kMaxTeams = 10;     // with 96: instances spill 8 bytes (Q6_K) to 92
 constexpr uint32_t kMaxDepth = 4;
 constexpr uint32_t kRedBufs = 8;                        // of a team
 constexpr uint32_t kSmemMax = 232448;  // 227 KB per CTA on sm_100
