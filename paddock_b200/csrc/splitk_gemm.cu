@@ -421,7 +421,9 @@ int launch(const void* data, const void* xq, Args& a, uint32_t row_bytes, cudaSt
         //  - for long rows of many tiles: 64 reads each weight twice as often, and L2 paces that (fp8 14592 x 3528, 323 tokens, 19152 slabs in all:
         //    25.2 / 35.2; 15104 x 2424, 283 tokens, 11210: 20.5 / 23.5; 9728 x 2264, 332 tokens, 8208: even);
         //  - above 512 tokens, where 64 was not measured.
-        // Over 67 FP8 and 81 NVFP4 shapes of 65 ... 700 tokens: 0.88 - 0.90 of the time with 128 alone, 3 % longer at worst.
+        // Over 260 shapes of 65 ... 512 tokens: 0.90 of the time with 128 alone, 1 % over the better of the two; longer by more than 3 % on five,
+        // 8 % at worst (fp8 15872 x 3608, 87 tokens 15.1 / 16.3).  More weight on the slabs mends those and loses as much elsewhere
+        // (nvfp4 9216 x 11160, 123 tokens 17.3 / 16.2).
         uint32_t split128 = 1u;
         if (int rc = plan_split<KIND, 128, TO>(a, split128, sms)) return rc;
         const uint64_t tiles = (uint64_t)((a.batch + 63u) / 64u) * ((a.out_dim + BM - 1u) / BM);

@@ -92,16 +92,17 @@ def test_fp8_more_channels_than_a_grid_axis_has_tiles(pack):
 
 
 # The line between tiles of 64 and of 128 tokens, one shape on each side of each of its conditions (296 tiles, 80 tokens on a split
-# row, slabs against tokens, 512 tokens, long rows of many tiles), and second tiles of one and of all but one token.
+# row, 512 tokens; slabs against tokens and, FP8, long rows of many tiles: below), and second tiles of one and of all but one token.
 TILES_64_128 = [(65, 260, 768), (127, 260, 768), (80, 130, 8192), (81, 130, 8192), (129, 300, 5120), (193, 136, 2560), (100, 18944, 256),
                 (100, 18945, 256), (512, 136, 768), (513, 136, 768), (90, 5000, 4096), (120, 5000, 4096)]
 
 
-@pytest.mark.parametrize("m,n,k", TILES_64_128 + [(129, 2700, 16640)])
+# (81, 9500, 2816): a CTA of a 64-token tile has 22 slabs, of a 128-token tile 8, and 3 x 14 + 40 is more than 81 tokens but not than 82
+@pytest.mark.parametrize("m,n,k", TILES_64_128 + [(81, 9500, 2816), (82, 9500, 2816), (128, 2700, 16640), (129, 2700, 16640)])
 def test_fp8_token_tiles(pack, m, n, k):
     test_fp8(pack, m, n, k, "f32")
 
 
-@pytest.mark.parametrize("m,n,k", TILES_64_128)
+@pytest.mark.parametrize("m,n,k", TILES_64_128 + [(81, 9500, 5632), (82, 9500, 5632)])
 def test_nvfp4_token_tiles(pack, m, n, k):
     check_nvf4_gemm_w4a4(pack, m, n, k, "bf16")
