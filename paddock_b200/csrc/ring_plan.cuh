@@ -86,6 +86,7 @@ bool ring_layout(RingPlan& p, uint32_t in_dim, uint32_t out_dim) {
 //   split        1.45 more for two CTAs, 2.18 for more
 //   odd rows     kOddCost more (the lanes copy the records; 4-bit planes, where the register kernel is close)
 //   registers    1.43 + rounds of 64 rows per SM x K / 1024 x kRegsCost, up to 1.32 times that when its four slots are full
+//                (fitted before calls with peers had an instance of their own, which made it 2 to 8 % faster on short rows)
 // Fitted to every split of 973 shapes (K = 1280 ... 17408, N = 520 ... 25600, all formats).  Over every plan of 599 other random shapes
 // (K = 1280 ... 17408, N = 512 ... 27648): 1.9 % over the best plan or the register kernel on average, 26 % at worst (Q4_K 9728 x 4864: 12.0 us, 9.5 with
 // four warps x five teams); without the terms for more pairs a warp and for odd rows 2.3 %, 42 % (Q4_K 6912 x 520: 4.8 us, 3.4 in a cluster of four).
