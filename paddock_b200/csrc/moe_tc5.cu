@@ -12,8 +12,8 @@
 //     ones flush to zero (below 2^-17 of the largest weight block).
 // Activations keep more than 4 bits by being expanded into four NVFP4 terms,
 //   x * 2^-e = t0 + t1/16 + t2/256 + t3/4096,  t_k = nvfp4(16^k * residual_k),
-// which sit side by side in the token dimension of one MMA (8 tokens x 4 terms = N 32,
-// 32 tokens x 4 terms = N 128); the epilogue adds the four column groups.  What is
+// which sit side by side in the token dimension of one MMA (32 columns per group of 8
+// tokens, moe_grouped.cuh); the epilogue adds the four.  What is
 // left of a 16-element group after four terms is below 1e-3 of the group's largest
 // element.  No weight passes through a register: at decode widths the kernel is a
 // pure stream of 4.25 bits per weight.
@@ -24,8 +24,8 @@
 //   (token, slot) rows and multiplied by the routing weight)  ->  pd_moe_slot_combine
 #include <cuda_fp8.h>
 
+#include "moe_grouped.cuh"
 #include "moe_route.cuh"
-#include "nvf4_tc5.cuh"
 
 namespace {
 
@@ -98,23 +98,65 @@ __global__ void nvf4_moe_tile_scales_kernel(const uint8_t* __restrict__ scale, u
 
 // ---------------------------------------------------------------- activations: four NVFP4 terms
 
-__device__ __forceinline__ float e4m3_to_f32(uint32_t b) {
-    const __half_raw h = __nv_cvt_fp8_to_halfraw((__nv_fp8_storage_t)b, __NV_E4M3);
-    return __half2float(*reinterpret_cast<const __half*>(&h));
-}
-// Two f32 -> one byte of two e2m1 codes (RN-even, saturating; low nibble = lo), and the
-// byte's two values back as f32.
-__device__ __forceinline__ uint32_t e2m1x2_rn(float lo, float hi, float& back_lo, float& back_hi) {
+// Two f32 -> one byte of two e2m1 codes (RN-even, saturating; low nibble = lo), and the byte's two values back as f32.
+__device__ __forceinline__ uint32_t e2m1x2_rn(float2 v) {
     uint16_t byte;
-    asm("{\n\t.reg .b8 q;\n\tcvt.rn.satfinite.e2m1x2.f32 q, %1, %2;\n\tmov.b16 %0, {q, 0};\n\t}"
-        : "=h"(byte)
-        : "f"(hi), "f"(lo));
-    uint32_t h2;
-    asm("{\n\t.reg .b8 q, z;\n\tmov.b16 {q, z}, %1;\n\tcvt.rn.f16x2.e2m1x2 %0, q;\n\t}" : "=r"(h2) : "h"(byte));
-    const __half2 v = *reinterpret_cast<const __half2*>(&h2);
-    back_lo = __low2float(v);
-    back_hi = __high2float(v);
+    asm("{\n\t.reg .b8 q;\n\tcvt.rn.satfinite.e2m1x2.f32 q, %1, %2;\n\tmov.b16 %0, {q, 0};\n\t}" : "=h"(byte) : "f"(v.y), "f"(v.x));
     return byte;
+}
+__device__ __forceinline__ float2 e2m1x2_value(uint32_t byte) {
+    uint32_t h2;
+    asm("{\n\t.reg .b8 q, z;\n\tmov.b16 {q, z}, %1;\n\tcvt.rn.f16x2.e2m1x2 %0, q;\n\t}" : "=r"(h2) : "h"((uint16_t)byte));
+    return __half22float2(*reinterpret_cast<const __half2*>(&h2));
+}
+// two f32 operations per instruction
+__device__ __forceinline__ float2 mul2(float2 v, float s) {
+    float2 d;
+    asm("{\n\t.reg .b64 a, b, c;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tmul.rn.f32x2 c, a, b;\n\tmov.b64 {%0, %1}, c;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(v.x), "f"(v.y), "f"(s));
+    return d;
+}
+__device__ __forceinline__ float2 fma2(float2 v, float s, float2 w) {
+    float2 d;
+    asm("{\n\t.reg .b64 a, b, c, e;\n\tmov.b64 a, {%2, %3};\n\tmov.b64 b, {%4, %4};\n\tmov.b64 c, {%5, %6};\n\t"
+        "fma.rn.f32x2 e, a, b, c;\n\tmov.b64 {%0, %1}, e;\n\t}"
+        : "=f"(d.x), "=f"(d.y) : "f"(v.x), "f"(v.y), "f"(s), "f"(w.x), "f"(w.y));
+    return d;
+}
+__device__ __forceinline__ float rcp_approx(float v) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(v));
+    return r;
+}
+
+// One 16-element scale group, r[8] = its pairs in code order (byte i of a term's 8 bytes = pair i), values below 512:
+// the four terms' codes and scale bytes.  The residual stays unscaled; the power 16^k of term k sits in its scale's factor
+// (exact), and the last term leaves none.  The kernel around it is bound by issue: this is half the instructions of the form
+// that scaled 16 residuals up per term, divided by the scale and worked on single floats.
+__device__ __forceinline__ void quantize_group(float2 (&r)[8], uint2 (&codes)[4], uint32_t (&sb)[4]) {
+    float up = 1.0f, down = 1.0f;
+#pragma unroll
+    for (uint32_t term = 0; term < 4u; ++term) {
+        float m = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) m = fmaxf(m, fmaxf(fabsf(r[k].x), fabsf(r[k].y)));
+        uint32_t s = (uint32_t)__nv_cvt_float_to_fp8(m * (up * (1.0f / 6.0f)), __NV_SATFINITE, __NV_E4M3);
+        if (s == 0u) s = 1u;
+        // an e4m3 byte's exponent and mantissa are an f32's, 120 binades lower
+        const float sc = __uint_as_float(s << 20) * (1.329227995784916e36f * down);
+        const float inv = rcp_approx(sc);
+        uint32_t w[2] = {0u, 0u};
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const uint32_t byte = e2m1x2_rn(mul2(r[k], inv));
+            w[k >> 2] |= byte << (8 * (k & 3));
+            if (term < 3u) r[k] = fma2(e2m1x2_value(byte), -sc, r[k]);
+        }
+        codes[term] = make_uint2(w[0], w[1]);
+        sb[term] = m > 0.0f ? s : 0u;
+        up *= 16.0f;
+        down *= 0.0625f;
+    }
 }
 
 struct PrepArgs {
@@ -122,22 +164,44 @@ struct PrepArgs {
     const float* up;             // mode 1: up [positions][dim]
     const uint32_t* sorted_row;  // [positions]; PDK_MOE_PAD = padding (zeros are written)
     const uint32_t* block_expert;  // [blocks]; PDK_MOE_PAD = unused block (its sorted_row entries are not defined; its rows are left as they are)
-    uint8_t* xq;                 // [blocks][4*bm][dim/2]
-    uint8_t* xs;                 // tiled: [blocks][slab][4 cells][512], the weight scale records' layout
+    uint8_t* xq;                 // [groups of 8 positions][32][dim/2]
+    uint8_t* xs;                 // tiled: [records][slab][4 cells][512], the weight scale records' layout
     float* xstep;                // [positions] power of two the row was divided by
     uint32_t dim, bm, mode;  // mode 0 gather, 1 gated (x = gate, up), 2 relu(x)^2 of x [positions][dim],
-                             // 3 one row: position 0 = x, the rest padding; the kernel writes the tables itself
+                             // 3 one row: position 0 = x, the rest padding; the kernel writes the tables itself,
+                             // 4 x [positions][dim] as it is
     uint32_t* tables;        // mode 3: sorted_row[bm], block_expert[1] (written here), then f32 scale2 = table_scale2
     float table_scale2;
     uint32_t natural;        // 0: ggml MXFP4 element order (byte j = elements j, j+16); 1: byte j = elements 2j, 2j+1
     float alpha, limit, up_add;
 };
 
-// One CTA per block position.  Position (block b, token i) writes the four term rows
-// b*4*bm + k*bm + i.  A 16-element scale group of the tensor core's element order is the
+// Where block b's positions keep their scale bytes.  A record holds 128 term rows = four groups of 8 tokens: a 32-token block
+// is a record, and 8-token blocks share one by fours, counted from the first block of their expert (`same(b)`: whether
+// block b belongs to it), at the first block of the four.  Every warp finds the run's start for itself.
+template <class Same>
+__device__ __forceinline__ void record_place(uint32_t pos, uint32_t bm, Same same, uint32_t& rec, uint32_t& col) {
+    const uint32_t b = pos / bm;
+    rec = b;
+    col = (pos >> 3) & 3u;
+    if (bm != 8u) return;
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t first = b;
+    for (;;) {
+        const uint32_t below = lane + 1u;
+        const uint32_t other = __ballot_sync(0xffffffffu, first < below || !same(first - below));
+        const uint32_t n = other ? (uint32_t)__ffs(other) - 1u : 32u;
+        first -= n;
+        if (n < 32u) break;
+    }
+    col = (b - first) & 3u;
+    rec = b - col;
+}
+
+// One CTA per block position.  Position (block b, token i) writes four term rows of its group of 8 tokens,
+// row term * 8 + i % 8 of the group's 32.  A 16-element scale group of the tensor core's element order is the
 // two 8-runs (h*8 .. h*8+7) and (16 + h*8 .. 16 + h*8+7) of a 32-element block.
-__device__ __forceinline__ void prep_position(const PrepArgs& a, uint32_t pos, uint32_t src) {
-    const uint32_t b = pos / a.bm, i = pos % a.bm;
+__device__ __forceinline__ void prep_position(const PrepArgs& a, uint32_t pos, uint32_t src, uint32_t rec, uint32_t col) {
     const uint32_t tid = threadIdx.x;
     const uint32_t groups = a.dim >> 4, kh = a.dim >> 1;
     __shared__ float s_red[8];
@@ -204,87 +268,36 @@ __device__ __forceinline__ void prep_position(const PrepArgs& a, uint32_t pos, u
     if (tid == 0) a.xstep[pos] = live ? __uint_as_float((uint32_t)(127 + (ex - 8)) << 23) : 0.0f;
 
     // ---- four terms per 16-element group
-    const size_t r0 = (size_t)b * 4u * a.bm + i;
-    uint8_t* xs_blk = a.xs + (size_t)b * num_kb * 2048u;
-    if (!live) {
-        // padding (half of the positions when most experts hold a ragged block) and all-zero rows: zero
-        // term rows and scale bytes, none of the term arithmetic
-        for (uint32_t g = tid; g < num_kb * 16u; g += blockDim.x) {
-            uint8_t* xs_g = xs_blk + (size_t)(g >> 4) * 2048u + ((g >> 2) & 3u) * 512u + (g & 3u);
-#pragma unroll
-            for (uint32_t term = 0; term < 4u; ++term) {
-                const uint32_t rr = term * a.bm + i;
-                xs_g[(rr & 31u) * 16u + (rr >> 5) * 4u] = 0;
-                if (g < groups) *reinterpret_cast<uint2*>(a.xq + (r0 + (size_t)term * a.bm) * kh + (size_t)g * 8u) = make_uint2(0u, 0u);
-            }
-        }
-        return;
-    }
+    const uint32_t r0 = pos & 7u;
+    uint8_t* xq_rows = a.xq + ((size_t)(pos >> 3) * 32u + r0) * kh;
+    uint8_t* xs_row = a.xs + (size_t)rec * num_kb * 2048u + r0 * 16u + col * 4u;
     for (uint32_t g = tid; g < num_kb * 16u; g += blockDim.x) {
-        // scale byte of group g and term row r: record g/16, cell (g/4)%4, byte (r%32)*16 + (r/32)*4 + g%4
-        uint8_t* xs_g = xs_blk + (size_t)(g >> 4) * 2048u + ((g >> 2) & 3u) * 512u + (g & 3u);
-        if (g >= groups) {  // past K: the record's cells must read as zero
-#pragma unroll
-            for (uint32_t term = 0; term < 4u; ++term) {
-                const uint32_t r = term * a.bm + i;
-                xs_g[(r & 31u) * 16u + (r >> 5) * 4u] = 0;
+        // scale byte of group g and term row r: record slab g/16, cell (g/4)%4, byte r*16 + col*4 + g%4
+        uint8_t* xs_g = xs_row + (size_t)(g >> 4) * 2048u + ((g >> 2) & 3u) * 512u + (g & 3u);
+        uint2 codes[4] = {};
+        uint32_t sb[4] = {};
+        // padding and all-zero rows: zero term rows and scale bytes, none of the term arithmetic; the record's cells
+        // past K must read as zero too
+        if (live && g < groups) {
+            if (!single) {
+                uint32_t lo_at, hi_at;
+                run_base(g, lo_at, hi_at);
+                load8(lo_at, lo0);
+                load8(hi_at, hi0);
             }
-            continue;
-        }
-        float lo[8], hi[8];
-        if (live && !single) {
-            uint32_t lo_at, hi_at;
-            run_base(g, lo_at, hi_at);
-            load8(lo_at, lo0);
-            load8(hi_at, hi0);
-        }
+            float2 r[8];
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-            lo[k] = live ? lo0[k] * inv_step : 0.0f;
-            hi[k] = live ? hi0[k] * inv_step : 0.0f;
+            for (int k = 0; k < 8; ++k)
+                // ggml order: byte k = (lo run k, hi run k); natural: byte k = lo run (2k, 2k+1), byte 4+k = hi run (2k, 2k+1)
+                r[k] = mul2(!a.natural ? make_float2(lo0[k], hi0[k])
+                            : k < 4    ? make_float2(lo0[2 * (k & 3)], lo0[2 * (k & 3) + 1])
+                                       : make_float2(hi0[2 * (k & 3)], hi0[2 * (k & 3) + 1]), inv_step);
+            quantize_group(r, codes, sb);
         }
 #pragma unroll
         for (uint32_t term = 0; term < 4u; ++term) {
-            float m = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) m = fmaxf(m, fmaxf(fabsf(lo[k]), fabsf(hi[k])));
-            uint32_t sb = 0u;
-            float sc = 0.0f, inv = 0.0f;
-            if (m > 0.0f) {
-                sb = (uint32_t)__nv_cvt_float_to_fp8(m * (1.0f / 6.0f), __NV_SATFINITE, __NV_E4M3);
-                if (sb == 0u) sb = 1u;
-                sc = e4m3_to_f32(sb);
-                inv = 1.0f / sc;
-            }
-            uint32_t w0 = 0u, w1 = 0u;
-#pragma unroll
-            if (!a.natural) {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) {  // byte k = (lo run k, hi run k)
-                    float bl, bh;
-                    const uint32_t byte = e2m1x2_rn(lo[k] * inv, hi[k] * inv, bl, bh);
-                    if (k < 4) w0 |= byte << (8 * k); else w1 |= byte << (8 * (k - 4));
-                    lo[k] = (lo[k] - bl * sc) * 16.0f;
-                    hi[k] = (hi[k] - bh * sc) * 16.0f;
-                }
-            } else {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {  // byte k = lo run (2k, 2k+1); byte 4+k = hi run (2k, 2k+1)
-                    float b0, b1;
-                    uint32_t byte = e2m1x2_rn(lo[2 * k] * inv, lo[2 * k + 1] * inv, b0, b1);
-                    w0 |= byte << (8 * k);
-                    lo[2 * k] = (lo[2 * k] - b0 * sc) * 16.0f;
-                    lo[2 * k + 1] = (lo[2 * k + 1] - b1 * sc) * 16.0f;
-                    byte = e2m1x2_rn(hi[2 * k] * inv, hi[2 * k + 1] * inv, b0, b1);
-                    w1 |= byte << (8 * k);
-                    hi[2 * k] = (hi[2 * k] - b0 * sc) * 16.0f;
-                    hi[2 * k + 1] = (hi[2 * k + 1] - b1 * sc) * 16.0f;
-                }
-            }
-            const size_t r = r0 + (size_t)term * a.bm;
-            *reinterpret_cast<uint2*>(a.xq + r * kh + (size_t)g * 8u) = make_uint2(w0, w1);
-            const uint32_t rr = term * a.bm + i;
-            xs_g[(rr & 31u) * 16u + (rr >> 5) * 4u] = (uint8_t)sb;
+            if (g < groups) *reinterpret_cast<uint2*>(xq_rows + (size_t)(term * 8u) * kh + (size_t)g * 8u) = codes[term];
+            xs_g[term * 128u] = (uint8_t)sb[term];
         }
     }
 }
@@ -293,10 +306,11 @@ __global__ void __launch_bounds__(256) moe_prep_f4_kernel(const PrepArgs a) {
     // dependent launch: may start while the previous kernel of the stream drains; its results are awaited here
     pdk_pdl_launch_dependents();
     pdk_pdl_wait();
-    const uint32_t pos = blockIdx.x;
-    uint32_t src;
+    const uint32_t pos = blockIdx.x, b = pos / a.bm;
+    uint32_t src, rec, col;
     if (a.mode == 3u) {
         src = pos == 0u ? 0u : PDK_MOE_PAD;
+        rec = col = 0u;
         if (threadIdx.x == 0) {
             a.tables[pos] = src;
             if (pos == 0u) {
@@ -305,10 +319,13 @@ __global__ void __launch_bounds__(256) moe_prep_f4_kernel(const PrepArgs a) {
             }
         }
     } else {
-        if (a.block_expert[pos / a.bm] == PDK_MOE_PAD) return;   // an unused block: the GEMMs skip it, nothing reads its rows
+        const uint32_t e = a.block_expert[b];
+        if (e == PDK_MOE_PAD) return;   // an unused block: the GEMMs skip it, nothing reads its rows
         src = a.sorted_row[pos];
+        if (src == PDK_MOE_PAD && a.sorted_row[pos & ~7u] == PDK_MOE_PAD) return;   // nor a group without a token
+        record_place(pos, a.bm, [&](uint32_t q) { return a.block_expert[q] == e; }, rec, col);
     }
-    prep_position(a, pos, src);
+    prep_position(a, pos, src, rec, col);
 }
 
 // Decode widths (rows * k <= 32 pairs): routing, alignment and the first activation preparation in
@@ -368,463 +385,12 @@ __global__ void __launch_bounds__(256) moe_route_prep_f4_kernel(const PrepArgs a
         for (uint32_t p = tid; p < n_pos; p += blockDim.x) { r.sorted_row[p] = s_row[p]; r.sorted_slot[p] = s_slot[p]; }
         if (tid < r.max_blocks) r.block_expert[tid] = s_bexp[tid];
     }
-    const uint32_t pos = blockIdx.x;
-    if (s_bexp[pos / a.bm] == PDK_MOE_PAD) return;   // an unused block
-    prep_position(a, pos, s_row[pos]);
-}
-
-// ---------------------------------------------------------------- grouped GEMM
-
-struct GemmArgs {
-    const uint8_t* w_sf[2];      // tiled UE4M3 weight scales per plane
-    const float* scale2[2];      // per-plane factor (device memory), or per expert when scale2_per_expert
-    const float* bias[2];        // [expert][out_dim] or null
-    float* out[2];               // gate / up: [positions][out_dim]; down: part [(row, slot)][out_dim]
-    const uint8_t* x_sf;         // tiled [blocks][slab][2048]
-    const float* xstep;          // [positions]
-    const uint32_t* block_expert;
-    const uint32_t* sorted_row;
-    const uint32_t* sorted_slot;  // down only
-    const float* topk_w;          // down only
-    uint32_t in_dim, out_dim, max_blocks, n_planes, n_active, scatter, scale2_per_expert;
-    unsigned int* err_word;
-};
-
-// One tile = (block of BN/4 tokens, plane, 128 weight rows of the block's expert), walked
-// by persistent CTAs.  Roles as in the dense NVFP4 GEMM: warp 0 producer (TMA boxes of W
-// and of the block's term rows, bulk copies of both operands' scale records), warp 1 MMA issuer, warps 2..5 epilogue.
-// WG: the weight scales are the row-major plane [rows][in_dim/16] (one expert) and the producer
-// gathers them with 4-byte cp.async copies instead of bulk-copying pre-tiled records - for
-// callers whose slot hands over the checkpoint's own scale plane (the W4A16 decode GEMV).
-template <uint32_t BN, bool WG>
-__global__ void __launch_bounds__(kThreads, 1)
-moe_tc5_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
-                    const __grid_constant__ CUtensorMap tmap_x, const GemmArgs a) {
-    constexpr uint32_t kStages = Cfg<BN>::kStages, kBBytes = Cfg<BN>::kBBytes, kStageBytes = Cfg<BN>::kStageBytes;
-    constexpr uint32_t kSfCol0 = Cfg<BN>::kSfCol0, kIdesc = Cfg<BN>::kIdesc, kSfCols = Cfg<BN>::kSfCols;
-    constexpr uint32_t kOffB = Cfg<BN>::kOffB, kOffSfa = Cfg<BN>::kOffSfa, kOffSfb = Cfg<BN>::kOffSfb;
-    constexpr uint32_t BT = BN / 4u;  // tokens per block
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
-    Shared* sh = reinterpret_cast<Shared*>(tiles + kStages * kStageBytes);
-    uint32_t* s_expert = reinterpret_cast<uint32_t*>(sh + 1);  // block_expert[], read once per tile by every role
-
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t row_tiles = (a.out_dim + BM - 1u) / BM, per_block = a.n_planes * row_tiles;
-    const uint32_t n_tiles = a.max_blocks * per_block;
-    const uint32_t n_mma = a.in_dim >> 6;                 // 64-element MMA steps (in_dim % 64 == 0)
-    const uint32_t num_kb = (n_mma + 3u) >> 2;            // 256-element slabs, the last may be partial
-    const uint32_t num_ks = (num_kb + KS - 1u) / KS;
-
-    if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < kStages; ++s) {
-            tc5::mbar_init(&sh->full[s], WG ? 33 : 1);  // expect_tx arrival (+ 32 lanes' cp.async arrivals)
-            tc5::mbar_init(&sh->empty[s], 1);
-        }
-        for (uint32_t b = 0; b < 2; ++b) {
-            tc5::mbar_init(&sh->tmem_full[b], 1);
-            tc5::mbar_init(&sh->tmem_empty[b], 4);
-        }
-        sh->abort_flag = 0;
-        tc5::mbar_fence_init();
-        tc5::tma_prefetch_desc(&tmap_w0);
-        tc5::tma_prefetch_desc(&tmap_w1);
-        tc5::tma_prefetch_desc(&tmap_x);
-    }
-    if (warp == 1) {
-        tc5::tmem_alloc(&sh->tmem_base, kTmemCols);
-        tc5::tmem_relinquish();
-    }
-    // dependent launch: barriers and tensor memory are set up while the previous kernel drains;
-    // everything below reads what it wrote
-    pdk_pdl_launch_dependents();
-    pdk_pdl_wait();
-    for (uint32_t i = threadIdx.x; i < a.max_blocks; i += kThreads) s_expert[i] = a.block_expert[i];
-    tc5::fence_before_sync();
-    __syncthreads();
-    tc5::fence_after_sync();
-    const uint32_t tmem_base = sh->tmem_base;
-    const tc5::WaitCtx ctx{&sh->abort_flag, a.err_word};
-
-    if (warp == 0) {
-        // ------------------------------------------------------------ producer (whole warp)
-        uint32_t stage = 0, phase = 0;
-        bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            const uint32_t blk = tile / per_block, rem = tile % per_block;
-            const uint32_t plane = rem / row_tiles, rt = rem % row_tiles;
-            const uint32_t expert = s_expert[blk];
-            if (expert == PDK_MOE_PAD) continue;
-            const CUtensorMap* tw = plane ? &tmap_w1 : &tmap_w0;
-            const uint8_t* wsf = a.w_sf[plane] + ((size_t)expert * row_tiles + rt) * num_kb * kSfBytes;
-            const uint8_t* xsf = a.x_sf + (size_t)blk * num_kb * kSfBytes;
-            for (uint32_t ks = 0; ks < num_ks; ++ks) {
-                ok = tc5::mbar_wait(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, stage);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                uint8_t* st = tiles + stage * kStageBytes;
-                const uint32_t kb0 = ks * KS, nsl = min(KS, num_kb - kb0);
-                tc5::mbar_arrive_expect_tx_elect(&sh->full[stage], nsl * (kABytes + kBBytes + (WG ? 1u : 2u) * kSfBytes));
-#pragma unroll
-                for (uint32_t u = 0; u < KS; ++u)
-                    if (u < nsl) {
-                        tc5::tma_load_2d_elect(st + u * kABytes, tw, &sh->full[stage], (int32_t)((kb0 + u) * BKB),
-                                               (int32_t)(expert * a.out_dim + rt * BM));
-                        tc5::tma_load_2d_elect(st + kOffB + u * kBBytes, &tmap_x, &sh->full[stage],
-                                               (int32_t)((kb0 + u) * BKB), (int32_t)(blk * BN));
-                    }
-                if (!WG) {
-                    tc5::bulk_load_elect(st + kOffSfa, wsf + (size_t)kb0 * kSfBytes, nsl * kSfBytes, &sh->full[stage]);
-                } else {
-                    // cell j of slab u: byte l*16 + c*4 + b = scale[rt*128 + c*32 + l][(kb0+u)*16 + j*4 + b]
-                    const uint32_t sf_row = a.in_dim >> 4;
-                    const uint32_t dst0 = tc5::smem_u32(st + kOffSfa) + lane * 16u;
-#pragma unroll
-                    for (uint32_t u = 0; u < KS; ++u)
-                        if (u < nsl)
-#pragma unroll
-                            for (uint32_t j = 0; j < 4u; ++j) {
-                                const uint32_t off = (kb0 + u) * 16u + j * 4u;
-#pragma unroll
-                                for (uint32_t c = 0; c < 4u; ++c) {
-                                    const uint32_t row = rt * BM + c * 32u + lane;
-                                    const uint32_t size = (row < a.out_dim && off < sf_row) ? 4u : 0u;
-                                    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(
-                                                     dst0 + u * kSfBytes + j * 512u + c * 4u),
-                                                 "l"(a.w_sf[plane] + (size ? (size_t)row * sf_row + off : 0u)), "r"(size)
-                                                 : "memory");
-                                }
-                            }
-                    asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];" ::"r"(
-                                     tc5::smem_u32(&sh->full[stage]))
-                                 : "memory");
-                }
-                tc5::bulk_load_elect(st + kOffSfb, xsf + (size_t)kb0 * kSfBytes, nsl * kSfBytes, &sh->full[stage]);
-                if (++stage == kStages) { stage = 0; phase ^= 1u; }
-            }
-        }
-        if (!ok && lane == 0) {
-            for (int i = 0; i < 64; ++i) __nanosleep(1000);
-        }
-    } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer (whole warp, one lane issues)
-        uint32_t stage = 0, phase = 0, iter = 0;
-        bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            if (s_expert[tile / per_block] == PDK_MOE_PAD) continue;
-            const uint32_t buf = iter & 1u, aphase = (iter >> 1) & 1u;
-            ++iter;
-            ok = tc5::mbar_wait(&sh->tmem_empty[buf], aphase ^ 1u, ctx, tc5::kErrTmemEmptyWait, buf);
-            ok = __all_sync(0xffffffffu, ok);
-            if (!ok) break;
-            tc5::fence_after_sync();
-            const uint32_t d_tmem = tmem_base + buf * BN;
-            for (uint32_t ks = 0; ks < num_ks; ++ks) {
-                ok = tc5::mbar_wait(&sh->full[stage], phase, ctx, tc5::kErrFullWait, stage);
-                ok = __all_sync(0xffffffffu, ok);
-                if (!ok) break;
-                tc5::fence_after_sync();
-                if (WG) fence_proxy_async_smem();  // the gathered cells were written through the generic proxy
-                const uint32_t a_addr = tc5::smem_u32(tiles + stage * kStageBytes);
-                const uint32_t nsl = min(KS, num_kb - ks * KS);
-#pragma unroll
-                for (uint32_t u = 0; u < KS; ++u) {
-                    if (u >= nsl) break;
-                    const uint32_t kb = ks * KS + u, steps = min(4u, n_mma - kb * 4u);
-                    const uint32_t sfa_addr = a_addr + kOffSfa + u * kSfBytes, sfb_addr = a_addr + kOffSfb + u * kSfBytes;
-                    const uint32_t sfa_t = tmem_base + kSfCol0 + stage * kSfCols + u * 32u, sfb_t = sfa_t + 16u;
-                    const uint64_t a_desc = tc5::smem_desc_sw128(a_addr + u * kABytes);
-                    const uint64_t b_desc = tc5::smem_desc_sw128(a_addr + kOffB + u * kBBytes);
-                    slab_nvf4<true>(d_tmem, a_desc, b_desc, kIdesc, (ks | u) != 0u, sfa_t, sfb_t, sfa_addr, sfb_addr, steps);
-                }
-                tc5::mma_commit_elect(&sh->empty[stage]);
-                if (++stage == kStages) { stage = 0; phase ^= 1u; }
-            }
-            if (ok) tc5::mma_commit_elect(&sh->tmem_full[buf]);
-        }
-    } else {
-        // ------------------------------------------------------------ epilogue
-        const uint32_t quarter = warp & 3u;
-        uint32_t iter = 0;
-        bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            const uint32_t blk = tile / per_block, rem = tile % per_block;
-            const uint32_t plane = rem / row_tiles, rt = rem % row_tiles;
-            const uint32_t expert = s_expert[blk];
-            if (expert == PDK_MOE_PAD) continue;
-            const uint32_t buf = iter & 1u, aphase = (iter >> 1) & 1u;
-            ++iter;
-            ok = tc5::mbar_wait(&sh->tmem_full[buf], aphase, ctx, tc5::kErrTmemFullWait, buf);
-            if (!ok) break;
-            tc5::fence_after_sync();
-            // lane = weight row; columns = term * BT + token
-            float v[BT];
-            const uint32_t taddr = tmem_base + ((quarter * 32u) << 16) + buf * BN;
-            if (BN == 32u) {
-                uint32_t r[32];
-                tc5::tmem_ld_32x32(taddr, r);
-                tc5::tmem_ld_wait();
-#pragma unroll
-                for (uint32_t i = 0; i < BT; ++i)
-                    v[i] = __uint_as_float(r[i]) + __uint_as_float(r[BT + i]) * 0.0625f +
-                           __uint_as_float(r[2u * BT + i]) * 0.00390625f +
-                           __uint_as_float(r[3u * BT + i]) * 0.000244140625f;
-            } else {
-                float c = 1.0f;
-#pragma unroll
-                for (uint32_t term = 0; term < 4u; ++term) {
-                    uint32_t r[32];
-                    tc5::tmem_ld_32x32(taddr + term * 32u, r);
-                    tc5::tmem_ld_wait();
-#pragma unroll
-                    for (uint32_t i = 0; i < 32u; ++i)
-                        if (i < BT) v[i] = term == 0u ? __uint_as_float(r[i]) : fmaf(__uint_as_float(r[i]), c, v[i]);
-                    c *= 0.0625f;
-                }
-            }
-            tc5::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) tc5::mbar_arrive(&sh->tmem_empty[buf]);  // the accumulator is in registers now
-
-            // lane i < BT fetches token i's routing data once; the loop below broadcasts it
-            const uint32_t my_pos = blk * BT + min(lane, BT - 1u);
-            const uint32_t my_src = a.sorted_row[my_pos];
-            uint32_t my_row = my_pos;  // output row: block position, or the (token, slot) pair
-            float my_wgt = 1.0f;       // routing weight when scattering
-            if (a.scatter && my_src != PDK_MOE_PAD) {
-                my_row = my_src * a.n_active + a.sorted_slot[my_pos];
-                my_wgt = a.topk_w[my_row];
-            }
-            const float my_mul = a.xstep[my_pos] * a.scale2[plane][a.scale2_per_expert ? expert : 0u] * my_wgt;
-            const uint32_t n = rt * BM + quarter * 32u + lane;
-            float bias = 0.0f;
-            if (n < a.out_dim && a.bias[plane]) bias = a.bias[plane][(size_t)expert * a.out_dim + n];
-            float* out = a.out[plane];
-#pragma unroll
-            for (uint32_t i = 0; i < BT; ++i) {
-                const uint32_t src = __shfl_sync(0xffffffffu, my_src, i);
-                const uint32_t row = __shfl_sync(0xffffffffu, my_row, i);
-                const float mul = __shfl_sync(0xffffffffu, my_mul, i);
-                const float wgt = __shfl_sync(0xffffffffu, my_wgt, i);
-                if (src == PDK_MOE_PAD || n >= a.out_dim) continue;
-                // (acc * scale2 * step + bias) * routing weight
-                out[(size_t)row * a.out_dim + n] = fmaf(v[i], mul, bias * wgt);
-            }
-        }
-    }
-
-    tc5::fence_before_sync();
-    __syncthreads();
-    if (warp == 1) {
-        tc5::fence_after_sync();
-        tc5::tmem_dealloc(tmem_base, kTmemCols);
-    }
-}
-
-// Gate and up of blocks of 32 tokens where K is long: the term rows of a block are 128 B rows, as many bytes per K step as
-// the weights.  One 128-row tile at a time brings 36 KB per 256-element slab into shared memory for 32 KB that its four MMAs
-// read and 4 KB of scale cells: 72 KB or 562 cycles of the shared-memory port for 256 of the tensor core, and 415 KB
-// through L2 per 128 x 2880 tile.
-// Here a tile is the gate and the up tile of the same rows under one B.  The accumulators are 2 x 128 columns, so there is
-// one pair of them and not two: the ring (four stages of one slab) keeps filling while the epilogue empties it, but the
-// tensor core waits for the epilogue.  Two tiles take 54 + 64 + 6 KB: 484 port cycles each, and three quarters of the L2 bytes.
-// prefer_dual below has where that pays.
-constexpr uint32_t kDualBN = 128u, kDualStages = 4u;
-constexpr uint32_t kDualB = 2u * kABytes, kDualSfa = kDualB + kDualBN * BKB, kDualSfb = kDualSfa + 2u * kSfBytes;
-constexpr uint32_t kDualStage = kDualSfb + kSfBytes;
-constexpr uint32_t kDualSfCol0 = 2u * kDualBN, kDualSfCols = 48u;      // per stage: the cells of A0, A1 and B
-static_assert(kDualSfCol0 + kDualStages * kDualSfCols <= kTmemCols && kDualStages <= kMaxStages, "tensor memory, barriers");
-
-__global__ void __launch_bounds__(kThreads, 1)
-moe_tc5_dual_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
-                    const __grid_constant__ CUtensorMap tmap_x, const GemmArgs a) {
-    constexpr uint32_t BT = kDualBN / 4u, kIdesc = Cfg<kDualBN>::kIdesc;
-    extern __shared__ uint8_t smem_raw[];
-    uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
-    Shared* sh = reinterpret_cast<Shared*>(tiles + kDualStages * kDualStage);
-    uint32_t* s_expert = reinterpret_cast<uint32_t*>(sh + 1);
-    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
-    const uint32_t row_tiles = (a.out_dim + BM - 1u) / BM, n_tiles = a.max_blocks * row_tiles;
-    const uint32_t n_mma = a.in_dim >> 6, num_kb = (n_mma + 3u) >> 2;
-
-    if (threadIdx.x == 0) {
-        for (uint32_t s = 0; s < kDualStages; ++s) {
-            tc5::mbar_init(&sh->full[s], 1);
-            tc5::mbar_init(&sh->empty[s], 1);
-        }
-        tc5::mbar_init(&sh->tmem_full[0], 1);
-        tc5::mbar_init(&sh->tmem_empty[0], 4);
-        sh->abort_flag = 0;
-        tc5::mbar_fence_init();
-        tc5::tma_prefetch_desc(&tmap_w0);
-        tc5::tma_prefetch_desc(&tmap_w1);
-        tc5::tma_prefetch_desc(&tmap_x);
-    }
-    if (warp == 1) {
-        tc5::tmem_alloc(&sh->tmem_base, kTmemCols);
-        tc5::tmem_relinquish();
-    }
-    pdk_pdl_launch_dependents();
-    pdk_pdl_wait();
-    for (uint32_t i = threadIdx.x; i < a.max_blocks; i += kThreads) s_expert[i] = a.block_expert[i];
-    tc5::fence_before_sync();
-    __syncthreads();
-    tc5::fence_after_sync();
-    const uint32_t tmem_base = sh->tmem_base;
-    const tc5::WaitCtx ctx{&sh->abort_flag, a.err_word};
-
-    if (warp == 0) {
-        // ------------------------------------------------------------ producer (whole warp, one lane issues)
-        uint32_t stage = 0, phase = 0;
-        bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            const uint32_t blk = tile / row_tiles, rt = tile % row_tiles, expert = s_expert[blk];
-            if (expert == PDK_MOE_PAD) continue;
-            const size_t sf = ((size_t)expert * row_tiles + rt) * num_kb * kSfBytes;
-            const uint8_t* xsf = a.x_sf + (size_t)blk * num_kb * kSfBytes;
-            const int32_t row = (int32_t)(expert * a.out_dim + rt * BM);
-            for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, stage));
-                if (!ok) break;
-                uint8_t* st = tiles + stage * kDualStage;
-                uint64_t* full = &sh->full[stage];
-                const size_t kb_sf = (size_t)kb * kSfBytes;
-                const int32_t x = (int32_t)(kb * BKB);
-                tc5::mbar_arrive_expect_tx_elect(full, kDualStage);
-                tc5::tma_load_2d_elect(st, &tmap_w0, full, x, row);
-                tc5::tma_load_2d_elect(st + kABytes, &tmap_w1, full, x, row);
-                tc5::tma_load_2d_elect(st + kDualB, &tmap_x, full, x, (int32_t)(blk * kDualBN));
-                tc5::bulk_load_elect(st + kDualSfa, a.w_sf[0] + sf + kb_sf, kSfBytes, full);
-                tc5::bulk_load_elect(st + kDualSfa + kSfBytes, a.w_sf[1] + sf + kb_sf, kSfBytes, full);
-                tc5::bulk_load_elect(st + kDualSfb, xsf + kb_sf, kSfBytes, full);
-                if (++stage == kDualStages) { stage = 0; phase ^= 1u; }
-            }
-        }
-        if (!ok && lane == 0)
-            for (int i = 0; i < 64; ++i) __nanosleep(1000);
-    } else if (warp == 1) {
-        // ------------------------------------------------------------ MMA issuer (whole warp, one lane issues)
-        uint32_t stage = 0, phase = 0, iter = 0;
-        bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            if (s_expert[tile / row_tiles] == PDK_MOE_PAD) continue;
-            ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->tmem_empty[0], (iter & 1u) ^ 1u, ctx, tc5::kErrTmemEmptyWait, 0u));
-            if (!ok) break;
-            ++iter;
-            tc5::fence_after_sync();
-            for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->full[stage], phase, ctx, tc5::kErrFullWait, stage));
-                if (!ok) break;
-                tc5::fence_after_sync();
-                const uint32_t s_addr = tc5::smem_u32(tiles + stage * kDualStage), steps = min(4u, n_mma - kb * 4u);
-                const uint32_t sf_t = tmem_base + kDualSfCol0 + stage * kDualSfCols, sfb_t = sf_t + 32u;
-                const uint64_t b_desc = tc5::smem_desc_sw128(s_addr + kDualB);
-                slab_nvf4<1u>(tmem_base, tc5::smem_desc_sw128(s_addr), b_desc, kIdesc, kb != 0u, sf_t, sfb_t, s_addr + kDualSfa,
-                              s_addr + kDualSfb, steps);
-                slab_nvf4<2u>(tmem_base + kDualBN, tc5::smem_desc_sw128(s_addr + kABytes), b_desc, kIdesc, kb != 0u, sf_t + 16u,
-                              sfb_t, s_addr + kDualSfa + kSfBytes, s_addr + kDualSfb, steps);
-                tc5::mma_commit_elect(&sh->empty[stage]);
-                if (++stage == kDualStages) { stage = 0; phase ^= 1u; }
-            }
-            if (ok) tc5::mma_commit_elect(&sh->tmem_full[0]);
-        }
-    } else {
-        // ------------------------------------------------------------ epilogue
-        const uint32_t quarter = warp & 3u;
-        uint32_t iter = 0;
-        bool ok = true;
-        for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-            const uint32_t blk = tile / row_tiles, rt = tile % row_tiles, expert = s_expert[blk];
-            if (expert == PDK_MOE_PAD) continue;
-            ok = tc5::mbar_wait(&sh->tmem_full[0], iter & 1u, ctx, tc5::kErrTmemFullWait, 0u);
-            if (!ok) break;
-            ++iter;
-            __syncwarp();
-            tc5::fence_after_sync();
-            // lane = weight row; columns = term * BT + token
-            float v[2][BT];
-#pragma unroll
-            for (uint32_t s = 0; s < 2u; ++s) {
-                float c = 1.0f;
-#pragma unroll
-                for (uint32_t term = 0; term < 4u; ++term) {
-                    uint32_t r[32];
-                    tc5::tmem_ld_32x32(tmem_base + ((quarter * 32u) << 16) + s * kDualBN + term * 32u, r);
-                    tc5::tmem_ld_wait();
-#pragma unroll
-                    for (uint32_t i = 0; i < BT; ++i) v[s][i] = term == 0u ? __uint_as_float(r[i]) : fmaf(__uint_as_float(r[i]), c, v[s][i]);
-                    c *= 0.0625f;
-                }
-            }
-            tc5::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) tc5::mbar_arrive(&sh->tmem_empty[0]);  // the accumulators are in registers now
-
-            // lane i fetches token i's step once; the loop below broadcasts it
-            const uint32_t my_pos = blk * BT + lane;
-            const uint32_t my_src = a.sorted_row[my_pos];
-            const float my_step = a.xstep[my_pos];
-            const uint32_t n = rt * BM + quarter * 32u + lane;
-#pragma unroll
-            for (uint32_t s = 0; s < 2u; ++s) {
-                const float scale2 = a.scale2[s][a.scale2_per_expert ? expert : 0u];
-                float bias = 0.0f;
-                if (n < a.out_dim && a.bias[s]) bias = a.bias[s][(size_t)expert * a.out_dim + n];
-                float* out = a.out[s];
-#pragma unroll
-                for (uint32_t i = 0; i < BT; ++i) {
-                    const uint32_t src = __shfl_sync(0xffffffffu, my_src, i);
-                    const float mul = __shfl_sync(0xffffffffu, my_step, i) * scale2;
-                    if (src == PDK_MOE_PAD || n >= a.out_dim) continue;
-                    out[(size_t)(blk * BT + i) * a.out_dim + n] = fmaf(v[s][i], mul, bias);
-                }
-            }
-        }
-    }
-
-    tc5::fence_before_sync();
-    __syncthreads();
-    if (warp == 1) {
-        tc5::fence_after_sync();
-        tc5::tmem_dealloc(tmem_base, kTmemCols);
-    }
-}
-
-constexpr uint32_t kMaxBlocks = 1024;  // block_expert[] is kept in shared memory
-
-template <uint32_t BN, bool WG = false>
-int launch_gemm(const CUtensorMap& tw0, const CUtensorMap& tw1, const CUtensorMap& tx, const GemmArgs& a,
-                cudaStream_t st) {
-    const size_t smem = (size_t)Cfg<BN>::kStages * Cfg<BN>::kStageBytes + sizeof(Shared) + kMaxBlocks * 4u + 1024u;
-    auto kern = moe_tc5_gemm_kernel<BN, WG>;
-    static const cudaError_t attr_rc =
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (attr_rc != cudaSuccess) return (int)attr_rc;
-    const uint32_t n_tiles = a.max_blocks * a.n_planes * ((a.out_dim + BM - 1u) / BM);
-    uint32_t grid = (uint32_t)pdk_sm_count();
-    if (grid > n_tiles) grid = n_tiles;
-    return pdk_launch_pdl(kern, dim3(grid), dim3(kThreads), smem, st, tw0, tw1, tx, a);
-}
-
-// Whether the two-tile kernel takes a gate | up call of 32-token blocks.  It saves port cycles and L2 bytes per slab and
-// pays an epilogue per tile that nothing overlaps, so it needs long K, and tiles enough that its half as many fill the last round.
-// Measured on a B200 (us, one tile at a time against two; 128 experts and 4 active unless stated): K = 2880, N = 2880: 272 / 251
-// at 1024 tokens, 200 / 199 at 256; K = 2048: 1.02 at 256 tokens (3680 tiles), 0.96 at 1024; K = 1024: 104 / 137 at 1024; K = 2880,
-// N = 768: 0.92 at 64 experts, 8 active, 2048 tokens (3456 tiles) but slower at 512 (1152 tiles).  A single plane (down), two
-// row tiles under one B, gained nothing at any of these sizes (147 / 141 at best, 16.4 / 24.4 at K = 1088, N = 1536).
-bool prefer_dual(const GemmArgs& a) {
-    const uint32_t num_kb = (a.in_dim + 255u) / 256u, row_tiles = (a.out_dim + BM - 1u) / BM;
-    return a.n_planes == 2u && num_kb >= 8u && (uint64_t)a.max_blocks * row_tiles >= 16ull * (uint32_t)pdk_sm_count();
-}
-
-int launch_dual(const CUtensorMap& tw0, const CUtensorMap& tw1, const CUtensorMap& tx, const GemmArgs& a, cudaStream_t st) {
-    const size_t smem = (size_t)kDualStages * kDualStage + sizeof(Shared) + kMaxBlocks * 4u + 1024u;
-    const cudaError_t e = cudaFuncSetAttribute(moe_tc5_dual_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    uint32_t grid = (uint32_t)pdk_sm_count();
-    const uint32_t n_tiles = a.max_blocks * ((a.out_dim + BM - 1u) / BM);
-    if (grid > n_tiles) grid = n_tiles;
-    return pdk_launch_pdl(moe_tc5_dual_kernel, dim3(grid), dim3(kThreads), smem, st, tw0, tw1, tx, a);
+    const uint32_t pos = blockIdx.x, b = pos / a.bm, e = s_bexp[b], src = s_row[pos];
+    if (e == PDK_MOE_PAD) return;   // an unused block
+    if (src == PDK_MOE_PAD && s_row[pos & ~7u] == PDK_MOE_PAD) return;
+    uint32_t rec, col;
+    record_place(pos, a.bm, [&](uint32_t q) { return s_bexp[q] == e; }, rec, col);
+    prep_position(a, pos, src, rec, col);
 }
 
 }  // namespace
@@ -862,7 +428,7 @@ static int prep_impl(const void* x, const void* up, const void* sorted_row, cons
                      void* xstep, uint32_t dim, uint32_t bm, uint32_t max_blocks, uint32_t mode, uint32_t natural,
                      float alpha, float limit, float up_add, void* stream) {
     if (max_blocks == 0) return 0;
-    if (dim == 0 || (dim & 31u) != 0u || (bm != 8u && bm != 32u) || mode > 2u) return cudaErrorInvalidValue;
+    if (dim == 0 || (dim & 31u) != 0u || (bm != 8u && bm != 32u)) return cudaErrorInvalidValue;
     if (!pdk_aligned(x, 16) || !pdk_aligned(xq, 16) || (mode == 1u && !pdk_aligned(up, 16))) return cudaErrorInvalidValue;
     PrepArgs a{};
     a.x = (const float*)x; a.up = (const float*)up; a.sorted_row = (const uint32_t*)sorted_row;
@@ -929,8 +495,17 @@ PDK_EXPORT int pdk_moe_route_prep_f4n(const void* logits, const void* router_bia
 PDK_EXPORT int pdk_moe_prep_act_f4n(const void* x, const void* up, const void* sorted_row, const void* block_expert,
                                     void* xq, void* xs, void* xstep, uint32_t dim, uint32_t bm, uint32_t max_blocks,
                                     uint32_t mode, float alpha, float limit, float up_add, void* stream) {
+    if (mode > 2u) return cudaErrorInvalidValue;
     return prep_impl(x, up, sorted_row, block_expert, xq, xs, xstep, dim, bm, max_blocks, mode, 1u, alpha, limit, up_add,
                      stream);
+}
+
+// The rows a gate|up call left (pdk_*_moe_gate_up_tc5): position p takes row p of h f32 [positions][dim] as it is.
+// natural: 0 the MXFP4 element order, 1 the NVFP4 one.
+PDK_EXPORT int pdk_moe_prep_rows_f4(const void* h, const void* sorted_row, const void* block_expert, void* xq, void* xs,
+                                    void* xstep, uint32_t dim, uint32_t bm, uint32_t max_blocks, uint32_t natural, void* stream) {
+    if (natural > 1u) return cudaErrorInvalidValue;
+    return prep_impl(h, nullptr, sorted_row, block_expert, xq, xs, xstep, dim, bm, max_blocks, 4u, natural, 1.0f, 0.0f, 0.0f, stream);
 }
 
 // No counterpart in the reference (slots 88 / 89 are its mma.sync kernels on int8 activations):
@@ -941,43 +516,51 @@ PDK_EXPORT int pdk_moe_prep_act_f4n(const void* x, const void* up, const void* s
 //              (w1_data NULL = one)
 //   scatter 1: out0 = part f32 [rows*n_active][out_dim], row (sorted_row, sorted_slot), times topk_w
 // in_dim % 64 == 0, max_blocks <= 1024.
-static int gemm_impl(const void* w0_data, const void* w0_sf, const float* w0_scale2, const void* w0_bias, void* out0,
-                     const void* w1_data, const void* w1_sf, const float* w1_scale2, const void* w1_bias, void* out1,
-                     const void* xq, const void* xs, const void* xstep, const void* block_expert, const void* sorted_row,
-                     const void* sorted_slot, const void* topk_w, uint32_t in_dim, uint32_t out_dim, uint32_t n_expert,
-                     uint32_t bm, uint32_t max_blocks, uint32_t n_active, uint32_t scatter, uint32_t scale2_per_expert,
-                     void* stream) {
+namespace {
+struct PlaneArgs { const void *data, *sf, *bias; const float* scale2; };
+struct RowArgs { const void *xq, *xs, *xstep, *block_expert, *sorted_row, *sorted_slot, *topk_w; };
+struct UnitArgs { float alpha, limit, up_add; };
+}  // namespace
+
+static int gemm_impl(const PlaneArgs& w0, const PlaneArgs& w1, void* out0, void* out1, const RowArgs& r, uint32_t in_dim,
+                     uint32_t out_dim, uint32_t n_expert, uint32_t bm, uint32_t max_blocks, uint32_t n_active, uint32_t kind,
+                     uint32_t scale2_per_expert, const UnitArgs& unit, void* stream) {
     if (max_blocks == 0 || out_dim == 0 || n_expert == 0) return 0;
-    if (in_dim == 0 || (in_dim & 63u) != 0u || (bm != 8u && bm != 32u) || max_blocks > kMaxBlocks)
+    if (in_dim == 0 || (in_dim & 63u) != 0u || (bm != 8u && bm != 32u) || max_blocks > moe_gemm::kMaxBlocks)
         return cudaErrorInvalidValue;
-    if (!pdk_aligned(w0_data, 16) || !pdk_aligned(w0_sf, 16) || !pdk_aligned(xq, 16) || !pdk_aligned(xs, 4) ||
-        !pdk_aligned(w0_scale2, 4) || (w1_data && (!pdk_aligned(w1_data, 16) || !pdk_aligned(w1_sf, 16))))
+    if (!pdk_aligned(w0.data, 16) || !pdk_aligned(w0.sf, 16) || !pdk_aligned(r.xq, 16) || !pdk_aligned(r.xs, 4) ||
+        !pdk_aligned(w0.scale2, 4) || (w1.data && (!pdk_aligned(w1.data, 16) || !pdk_aligned(w1.sf, 16))))
         return cudaErrorInvalidValue;
-    if (scatter && (w1_data || !sorted_slot || !topk_w)) return cudaErrorInvalidValue;
-    const uint32_t bn = 4u * bm, kbytes = in_dim >> 1;
+    if (kind == moe_gemm::kScatter && (w1.data || !r.sorted_slot || !r.topk_w)) return cudaErrorInvalidValue;
+    if (kind == moe_gemm::kGated && !w1.data) return cudaErrorInvalidValue;
+    const PlaneArgs& wb = w1.data ? w1 : w0;
+    const uint32_t kbytes = in_dim >> 1;
     CUtensorMap tw0, tw1, tx;
     const uint64_t wrows = (uint64_t)n_expert * out_dim;
-    if (int rc = pdk_make_tmap_2d(&tw0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w0_data, kbytes, wrows, kbytes, BKB, BM)) return rc;
-    if (int rc = pdk_make_tmap_2d(&tw1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w1_data ? w1_data : w0_data, kbytes, wrows,
-                                  kbytes, BKB, BM))
+    if (int rc = pdk_make_tmap_2d(&tw0, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, w0.data, kbytes, wrows, kbytes, BKB, BM)) return rc;
+    if (int rc = pdk_make_tmap_2d(&tw1, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, wb.data, kbytes, wrows, kbytes, BKB, BM)) return rc;
+    if (int rc = pdk_make_tmap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, r.xq, kbytes, (uint64_t)max_blocks * 4u * bm, kbytes,
+                                  BKB, 32u))
         return rc;
-    if (int rc = pdk_make_tmap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, kbytes, (uint64_t)max_blocks * bn, kbytes,
-                                  BKB, bn))
-        return rc;
-    GemmArgs a{};
-    a.w_sf[0] = (const uint8_t*)w0_sf; a.w_sf[1] = (const uint8_t*)(w1_data ? w1_sf : w0_sf);
-    a.scale2[0] = w0_scale2; a.scale2[1] = w1_data ? w1_scale2 : w0_scale2;
+    moe_gemm::Args a{};
+    a.w_sf[0] = (const uint8_t*)w0.sf; a.w_sf[1] = (const uint8_t*)wb.sf;
+    a.scale2[0] = w0.scale2; a.scale2[1] = wb.scale2;
     a.scale2_per_expert = scale2_per_expert;
-    a.bias[0] = (const float*)w0_bias; a.bias[1] = (const float*)w1_bias;
+    a.bias[0] = (const float*)w0.bias; a.bias[1] = (const float*)w1.bias;
     a.out[0] = (float*)out0; a.out[1] = (float*)out1;
-    a.x_sf = (const uint8_t*)xs; a.xstep = (const float*)xstep;
-    a.block_expert = (const uint32_t*)block_expert; a.sorted_row = (const uint32_t*)sorted_row;
-    a.sorted_slot = (const uint32_t*)sorted_slot; a.topk_w = (const float*)topk_w;
-    a.in_dim = in_dim; a.out_dim = out_dim; a.max_blocks = max_blocks; a.n_planes = w1_data ? 2u : 1u;
-    a.n_active = n_active; a.scatter = scatter; a.err_word = pdk_error_word();
+    a.x_sf = (const uint8_t*)r.xs; a.xstep = (const float*)r.xstep;
+    a.block_expert = (const uint32_t*)r.block_expert; a.sorted_row = (const uint32_t*)r.sorted_row;
+    a.sorted_slot = (const uint32_t*)r.sorted_slot; a.topk_w = (const float*)r.topk_w;
+    a.in_dim = in_dim; a.out_dim = out_dim; a.max_blocks = max_blocks; a.n_planes = w1.data ? 2u : 1u;
+    a.n_active = n_active; a.kind = kind; a.block_shift = bm == 32u ? 2u : 0u;
+    a.alpha = unit.alpha; a.limit = unit.limit; a.up_add = unit.up_add; a.err_word = pdk_error_word();
     auto st = (cudaStream_t)stream;
-    if (bm == 8u) return launch_gemm<32>(tw0, tw1, tx, a, st);
-    return prefer_dual(a) ? launch_dual(tw0, tw1, tx, a, st) : launch_gemm<128>(tw0, tw1, tx, a, st);
+    // Gate and up under one B where the unit is computed here (both accumulators have to be in one CTA) and for 32-token blocks,
+    // which bring 24 KB of activations per slab (gate and up of 1024 tokens, 4 of 128 experts, 2880 x 2880: 257 us with a pass per
+    // 32-token block, 220 this way); else one tile at a time.  Tiles of up to six groups where blocks are large: down of
+    // the same block 150 -> 130 us.
+    if (kind == moe_gemm::kGated || (w1.data && bm == 32u)) return moe_gemm::launch<6, 2, 8>(tw0, tw1, tx, a, st);
+    return bm == 32u ? moe_gemm::launch<6, 1, 8>(tw0, tw1, tx, a, st) : moe_gemm::launch<4, 1, 8>(tw0, tw1, tx, a, st);
 }
 
 PDK_EXPORT int pdk_mxfp4_moe_gemm_tc5(const void* w0_data, const void* w0_sf, const void* w0_meta, const void* w0_bias,
@@ -988,9 +571,24 @@ PDK_EXPORT int pdk_mxfp4_moe_gemm_tc5(const void* w0_data, const void* w0_sf, co
                                       uint32_t n_expert, uint32_t bm, uint32_t max_blocks, uint32_t n_active,
                                       uint32_t scatter, void* stream) {
     if (!pdk_aligned(w0_meta, 8) || w0_meta == nullptr || (w1_data && w1_meta == nullptr)) return cudaErrorInvalidValue;
-    return gemm_impl(w0_data, w0_sf, (const float*)w0_meta + 1, w0_bias, out0, w1_data, w1_sf,
-                     w1_meta ? (const float*)w1_meta + 1 : nullptr, w1_bias, out1, xq, xs, xstep, block_expert, sorted_row,
-                     sorted_slot, topk_w, in_dim, out_dim, n_expert, bm, max_blocks, n_active, scatter, 0u, stream);
+    return gemm_impl({w0_data, w0_sf, w0_bias, (const float*)w0_meta + 1},
+                     {w1_data, w1_sf, w1_bias, w1_meta ? (const float*)w1_meta + 1 : nullptr}, out0, out1,
+                     {xq, xs, xstep, block_expert, sorted_row, sorted_slot, topk_w}, in_dim, out_dim, n_expert, bm, max_blocks,
+                     n_active, scatter ? moe_gemm::kScatter : moe_gemm::kPlain, 0u, {}, stream);
+}
+
+// Gate, up and the gated unit (pdk_moe_prep_act_f4n has its formula) in one launch: h f32 [max_blocks*bm][out_dim] in block
+// order, rows of padding left alone.  The raw gate and up rows are never written: at 1024 tokens, 4 experts each, 2880 wide
+// they were 94 MB out and 94 MB back in.
+PDK_EXPORT int pdk_mxfp4_moe_gate_up_tc5(const void* gate_data, const void* gate_sf, const void* gate_meta, const void* gate_bias,
+                                         const void* up_data, const void* up_sf, const void* up_meta, const void* up_bias, void* h,
+                                         const void* xq, const void* xs, const void* xstep, const void* block_expert,
+                                         const void* sorted_row, uint32_t in_dim, uint32_t out_dim, uint32_t n_expert, uint32_t bm,
+                                         uint32_t max_blocks, float alpha, float limit, float up_add, void* stream) {
+    if (!pdk_aligned(gate_meta, 8) || !gate_meta || !up_meta || !up_data) return cudaErrorInvalidValue;
+    return gemm_impl({gate_data, gate_sf, gate_bias, (const float*)gate_meta + 1}, {up_data, up_sf, up_bias, (const float*)up_meta + 1},
+                     h, nullptr, {xq, xs, xstep, block_expert, sorted_row, nullptr, nullptr}, in_dim, out_dim, n_expert, bm, max_blocks,
+                     1u, moe_gemm::kGated, 0u, {alpha, limit, up_add}, stream);
 }
 
 // ---- NVFP4 expert planes (crates/paddock-engine/src/gpu/types.rs:176-226: data [expert*rows][in/2],
@@ -1021,9 +619,20 @@ PDK_EXPORT int pdk_nvf4_moe_gemm_tc5(const void* w0_data, const void* w0_sf, con
                                      uint32_t bm, uint32_t max_blocks, uint32_t n_active, uint32_t scatter,
                                      void* stream) {
     if (w0_scale2 == nullptr || (w1_data && w1_scale2 == nullptr)) return cudaErrorInvalidValue;
-    return gemm_impl(w0_data, w0_sf, (const float*)w0_scale2, w0_bias, out0, w1_data, w1_sf, (const float*)w1_scale2,
-                     w1_bias, out1, xq, xs, xstep, block_expert, sorted_row, sorted_slot, topk_w, in_dim, out_dim,
-                     n_expert, bm, max_blocks, n_active, scatter, 1u, stream);
+    return gemm_impl({w0_data, w0_sf, w0_bias, (const float*)w0_scale2}, {w1_data, w1_sf, w1_bias, (const float*)w1_scale2}, out0,
+                     out1, {xq, xs, xstep, block_expert, sorted_row, sorted_slot, topk_w}, in_dim, out_dim, n_expert, bm, max_blocks,
+                     n_active, scatter ? moe_gemm::kScatter : moe_gemm::kPlain, 1u, {}, stream);
+}
+
+PDK_EXPORT int pdk_nvf4_moe_gate_up_tc5(const void* gate_data, const void* gate_sf, const void* gate_scale2, const void* gate_bias,
+                                        const void* up_data, const void* up_sf, const void* up_scale2, const void* up_bias, void* h,
+                                        const void* xq, const void* xs, const void* xstep, const void* block_expert,
+                                        const void* sorted_row, uint32_t in_dim, uint32_t out_dim, uint32_t n_expert, uint32_t bm,
+                                        uint32_t max_blocks, float alpha, float limit, float up_add, void* stream) {
+    if (!gate_scale2 || !up_scale2 || !up_data) return cudaErrorInvalidValue;
+    return gemm_impl({gate_data, gate_sf, gate_bias, (const float*)gate_scale2}, {up_data, up_sf, up_bias, (const float*)up_scale2}, h,
+                     nullptr, {xq, xs, xstep, block_expert, sorted_row, nullptr, nullptr}, in_dim, out_dim, n_expert, bm, max_blocks, 1u,
+                     moe_gemm::kGated, 1u, {alpha, limit, up_add}, stream);
 }
 
 // ---------------------------------------------------------------- W4A16 decode GEMV on the same kernels
@@ -1068,7 +677,7 @@ int pdk_nvf4_gemv_tc5(const void* data, const void* scale, const void* bias, con
     CUtensorMap tw, tx;
     if (int rc = pdk_make_tmap_2d(&tw, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, data, kbytes, out_dim, kbytes, BKB, BM)) return rc;
     if (int rc = pdk_make_tmap_2d(&tx, CU_TENSOR_MAP_DATA_TYPE_UINT8, 1, xq, kbytes, 32u, kbytes, BKB, 32u)) return rc;
-    GemmArgs a{};
+    moe_gemm::Args a{};
     a.w_sf[0] = a.w_sf[1] = (const uint8_t*)scale;
     a.scale2[0] = a.scale2[1] = reinterpret_cast<const float*>(tables) + 9;
     a.bias[0] = (const float*)bias;
@@ -1077,5 +686,5 @@ int pdk_nvf4_gemv_tc5(const void* data, const void* scale, const void* bias, con
     a.block_expert = tables + 8; a.sorted_row = tables;
     a.in_dim = in_dim; a.out_dim = out_dim; a.max_blocks = 1u; a.n_planes = 1u; a.n_active = 1u;
     a.err_word = pdk_error_word();
-    return launch_gemm<32, true>(tw, tw, tx, a, st);
+    return moe_gemm::launch<4, 1, 4, true>(tw, tw, tx, a, st);
 }

@@ -140,6 +140,9 @@ _EXTRA_SIGS = {
     "pdk_nvf4_moe_tile_scales": "ppuuu",
     "pdk_moe_prep_act_f4n": "pppppppuuuufff",
     "pdk_nvf4_moe_gemm_tc5": "p" * 17 + "u" * 7,
+    "pdk_mxfp4_moe_gate_up_tc5": "p" * 14 + "uuuuufff",
+    "pdk_nvf4_moe_gate_up_tc5": "p" * 14 + "uuuuufff",
+    "pdk_moe_prep_rows_f4": "ppppppuuuu",
 }
 _KIND = {"p": C.c_void_p, "u": C.c_uint32, "U": C.c_uint64, "f": C.c_float}
 
