@@ -13,7 +13,7 @@ namespace moe_gemm {
 
 using namespace nvf4tc5;
 
-enum Kind : uint32_t { kPlain = 0u, kScatter = 1u, kGated = 2u };
+enum Kind : uint32_t { kPlain = 0u, kScatter = 1u, kGated = 2u };   // the kernel of the first two is one (Args::scatter)
 
 struct Args {
     const uint8_t* w_sf[2];      // tiled UE4M3 weight scales per plane
@@ -26,12 +26,14 @@ struct Args {
     const uint32_t* sorted_row;
     const uint32_t* sorted_slot;  // scatter only
     const float* topk_w;          // scatter only
-    uint32_t in_dim, out_dim, max_blocks, n_planes, n_active, kind, scale2_per_expert, block_shift;  // 2: 32-token blocks, 0: 8
+    uint32_t in_dim, out_dim, max_blocks, n_planes, n_active, scatter, scale2_per_expert, block_shift;  // 2: 32-token blocks, 0: 8
     float alpha, limit, up_add;   // gated only
     unsigned int* err_word;
 };
 
-constexpr uint32_t kRing = 216u * 1024u, kMaxSlots = 10u;
+// The ring leaves 16 KB of an SM's shared memory: the kernels in front and behind are dependent launches, and a CTA of theirs
+// that finds no room here starts when this one has left (a ring of 216 KB cost a block of one token 0.4 us).
+constexpr uint32_t kRing = 196u * 1024u, kMaxSlots = 10u;
 constexpr uint32_t kMaxBlocks = 1024;  // block_expert[] and the tile table are kept in shared memory
 constexpr size_t kTableBytes = kMaxBlocks * 9u;   // experts, tiles, live groups
 
@@ -40,7 +42,7 @@ constexpr size_t kTableBytes = kMaxBlocks * 9u;   // experts, tiles, live groups
 // weight tiles, the groups and their scale records; a stage's hand-off costs the issuing warp about as long as half a slab.
 template <uint32_t W, uint32_t NA>
 struct Geo {
-    static constexpr uint32_t kS = NA == 1u && W <= 4u ? 2u : 1u;
+    static constexpr uint32_t kS = NA == 1u && W <= 2u ? 2u : 1u;
     static constexpr uint32_t kN = W * 32u, kGroupBytes = 32u * BKB, kQuads = (W + 3u) / 4u;
     // a stage: weight boxes [tile][slab], groups [slab][group], weight records [tile][slab], activation records [quad][slab]
     static constexpr uint32_t kOffB = kS * NA * kABytes, kOffSfa = kOffB + kS * W * kGroupBytes;
@@ -184,6 +186,16 @@ __device__ __forceinline__ void slab_group(uint32_t d_tmem, uint64_t a_desc, uin
 // uniform register.  Descriptors, tensor-memory addresses and the branches around TMA and tcgen05 instructions depend on it.
 __device__ __forceinline__ uint32_t uniform(uint32_t v) { return __reduce_or_sync(0xffffffffu, v); }
 
+// tc5::mbar_wait with the part that is rarely run out of line.  Two GEMMs and a preparation take turns on the instruction cache of
+// an SM; what a kernel runs once per launch is fetched from L2 each time.
+static __device__ __noinline__ bool wait_longer(uint64_t* bar, uint32_t parity, volatile int* abort_flag, unsigned int* err,
+                                                unsigned int code, unsigned int detail) {
+    return tc5::mbar_wait(bar, parity, tc5::WaitCtx{abort_flag, err}, code, detail);
+}
+__device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity, const tc5::WaitCtx& ctx, unsigned int code, unsigned int detail) {
+    return tc5::mbar_try_wait(bar, parity) || wait_longer(bar, parity, ctx.abort_flag, ctx.err, code, detail);
+}
+
 // What a tile index means: the groups, the weight plane (the first of two, where a tile has both) and the row tile.
 template <uint32_t NA>
 struct TileAt {
@@ -197,12 +209,12 @@ struct TileAt {
 };
 
 // Roles: warp 0 brings the weights (TMA boxes, bulk copies of their scale records), warp 1 issues the MMAs, warp 2 brings the
-// groups' term rows and their records, the others are the epilogue (lane quarter = warp % 4; with eight warps two share a
-// quarter and take the groups in turn).  The geometry is known at compile time and tensor memory is addressed from column 0,
-// where an allocation of all 512 columns starts: descriptors and addresses that come out of memory would be moved into uniform
-// registers before every tcgen05 instruction, which took the issuing warp as long as the stream of weights takes (dual tiles of
-// 2880 x 2880 experts at 1024 tokens: 308 us with a run-time stage size, XXX this way).
-template <uint32_t W, uint32_t NA, uint32_t EPI, bool WG>
+// groups' term rows and their records, the others are the epilogue (lane quarter = warp % 4; the warps of a quarter take the
+// groups in turn).  Tensor memory is addressed from column 0, where an allocation of all 512 columns starts.
+// The code is kept short - one group per turn of the epilogue's loop, one kernel for raw rows and for down: what a launch runs is
+// fetched into the instruction cache anew when another large kernel ran in between (with the epilogue unrolled over a tile's
+// groups a block of one token took 38.2 us instead of 34.8, 512 tokens with 8 of 128 experts of 2048 x 768 180 instead of 166).
+template <uint32_t W, uint32_t NA, uint32_t KIND, uint32_t EPI, bool WG>
 __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensorMap& tmap_w1, const CUtensorMap& tmap_x, const Args& a,
                                       uint8_t* rings, Ctl* sh, const uint32_t* s_expert, const uint32_t* s_tile, uint32_t tiles) {
     using G = Geo<W, NA>;
@@ -227,7 +239,7 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
             const size_t sf0 = ((size_t)expert * row_tiles + t.rt) * num_kb * kSfBytes;
             const uint8_t* wsf = a.w_sf[t.plane] + sf0;
             for (uint32_t kb0 = 0; kb0 < num_kb; kb0 += G::kS) {
-                ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, stage));
+                ok = __all_sync(0xffffffffu, wait_for(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, stage));
                 if (!ok) break;
                 uint8_t* st = rings + stage * G::kSlot;
                 uint64_t* full = &sh->full[stage];
@@ -280,7 +292,7 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
             const size_t rec_bytes = (size_t)num_kb * kSfBytes;
             const uint8_t* xsf = a.x_sf + (size_t)(g0 >> a.block_shift) * rec_bytes;
             for (uint32_t kb0 = 0; kb0 < num_kb; kb0 += G::kS) {
-                ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, stage));
+                ok = __all_sync(0xffffffffu, wait_for(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, stage));
                 if (!ok) break;
                 uint8_t* st = rings + stage * G::kSlot;
                 uint64_t* full = &sh->full[stage];
@@ -314,13 +326,13 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
             const uint32_t buf = kBufs == 2u ? iter & 1u : 0u, aphase = kBufs == 2u ? (iter >> 1) & 1u : iter & 1u;
             // e2m1 x e2m1 (format code 1 in the mxf4 encoding), UE4M3 scales, scale ids 0
             const uint32_t idesc = (1u << 7) | (1u << 10) | ((ng * 4u) << 17) | ((BM >> 4) << 24);
-            ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->tmem_empty[buf], aphase ^ 1u, ctx, tc5::kErrTmemEmptyWait, buf));
+            ok = __all_sync(0xffffffffu, wait_for(&sh->tmem_empty[buf], aphase ^ 1u, ctx, tc5::kErrTmemEmptyWait, buf));
             if (!ok) break;
             ++iter;
             tc5::fence_after_sync();
             const uint32_t d_tmem = buf * G::kN;
             for (uint32_t kb0 = 0; kb0 < num_kb; kb0 += G::kS) {
-                ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->full[stage], phase, ctx, tc5::kErrFullWait, stage));
+                ok = __all_sync(0xffffffffu, wait_for(&sh->full[stage], phase, ctx, tc5::kErrFullWait, stage));
                 if (!ok) break;
                 tc5::fence_after_sync();
                 if (WG) fence_proxy_async_smem();  // the gathered cells were written through the generic proxy
@@ -346,24 +358,24 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
             if (ok) tc5::mma_commit_elect(&sh->tmem_full[buf]);
         }
     } else {
-        // ------------------------------------------------------------ epilogue
-        constexpr uint32_t kHalves = EPI / 4u, kMine = (W + kHalves - 1u) / kHalves;
-        const uint32_t quarter = warp & 3u, half = (warp - 3u) >> 2;
+        // ------------------------------------------------------------ epilogue (one group at a time: the loop stays small)
+        constexpr uint32_t kShare = EPI / 4u;
+        const uint32_t quarter = warp & 3u, share = (warp - 3u) >> 2;
         uint32_t iter = 0;
         bool ok = true;
         for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
             const TileAt<NA> t(s_tile, tile, per_chunk, row_tiles);
-            const uint32_t g0 = tile_group(t.word), ng = tile_ng(t.word), plane = t.plane;
+            const uint32_t g0 = tile_group(t.word), ng = W == 1u ? 1u : tile_ng(t.word);
             const uint32_t expert = s_expert[g0 >> a.block_shift];
             const uint32_t buf = kBufs == 2u ? iter & 1u : 0u, aphase = kBufs == 2u ? (iter >> 1) & 1u : iter & 1u;
             ++iter;
             // lane j * 8 + i: routing data of token i of this warp's j-th group, broadcast below
-            const uint32_t my_g = min(half + kHalves * (lane >> 3), ng - 1u);
+            const uint32_t my_g = min(share + kShare * (lane >> 3), ng - 1u);
             const uint32_t my_pos = (g0 + my_g) * 8u + (lane & 7u);
             const uint32_t my_src = a.sorted_row[my_pos];
             uint32_t my_row = my_pos;  // output row: position, or the (token, slot) pair
             float my_wgt = 1.0f;       // routing weight when scattering
-            if (a.kind == kScatter && my_src != PDK_MOE_PAD) {
+            if (KIND != kGated && a.scatter && my_src != PDK_MOE_PAD) {
                 my_row = my_src * a.n_active + a.sorted_slot[my_pos];
                 my_wgt = a.topk_w[my_row];
             }
@@ -372,68 +384,65 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
             float scale2[NA], bias[NA];
 #pragma unroll
             for (uint32_t s = 0; s < NA; ++s) {
-                const uint32_t p = NA == 2u ? s : plane;
+                const uint32_t p = NA == 2u ? s : t.plane;
                 scale2[s] = a.scale2[p][a.scale2_per_expert ? expert : 0u];
                 bias[s] = (n < a.out_dim && a.bias[p]) ? a.bias[p][(size_t)expert * a.out_dim + n] : 0.0f;
             }
-            ok = tc5::mbar_wait(&sh->tmem_full[buf], aphase, ctx, tc5::kErrTmemFullWait, buf);
+            float* out = a.out[t.plane];
+            ok = wait_for(&sh->tmem_full[buf], aphase, ctx, tc5::kErrTmemFullWait, buf);
             if (!ok) break;
             __syncwarp();
             tc5::fence_after_sync();
-            // tensor-memory lane = weight row; columns of a group = term * 8 + token
-            float v[NA][kMine][8];
+#pragma unroll 1
+            for (uint32_t g = share, from = 0; g < ng; g += kShare, from += 8u) {
+                // tensor-memory lane = weight row; columns of a group = term * 8 + token
+                float v[NA][8];
+                uint32_t r[NA][32];
 #pragma unroll
-            for (uint32_t j = 0; j < kMine; ++j) {
-                const uint32_t g = half + kHalves * j;
-                if (g >= ng) break;
+                for (uint32_t s = 0; s < NA; ++s)
+                    tc5::tmem_ld_32x32(((quarter * 32u) << 16) + (buf + s) * G::kN + g * 32u, r[s]);
+                tc5::tmem_ld_wait();
+                if (g + kShare >= ng) {   // the last of this warp's share: the accumulators are in registers
+                    tc5::fence_before_sync();
+                    __syncwarp();
+                    if (lane == 0) tc5::mbar_arrive(&sh->tmem_empty[buf]);
+                }
 #pragma unroll
-                for (uint32_t s = 0; s < NA; ++s) {
-                    uint32_t r[32];
-                    tc5::tmem_ld_32x32(((quarter * 32u) << 16) + (buf + s) * G::kN + g * 32u, r);
-                    tc5::tmem_ld_wait();
+                for (uint32_t s = 0; s < NA; ++s)
 #pragma unroll
                     for (uint32_t i = 0; i < 8u; ++i)
-                        v[s][j][i] = fmaf(__uint_as_float(r[24u + i]), 0.000244140625f,
-                                          fmaf(__uint_as_float(r[16u + i]), 0.00390625f,
-                                               fmaf(__uint_as_float(r[8u + i]), 0.0625f, __uint_as_float(r[i]))));
-                }
-            }
-            tc5::fence_before_sync();
-            __syncwarp();
-            if (lane == 0) tc5::mbar_arrive(&sh->tmem_empty[buf]);  // the accumulators are in registers now
-#pragma unroll
-            for (uint32_t j = 0; j < kMine; ++j) {
-                if (half + kHalves * j >= ng) break;
+                        v[s][i] = fmaf(__uint_as_float(r[s][24u + i]), 0.000244140625f,
+                                       fmaf(__uint_as_float(r[s][16u + i]), 0.00390625f,
+                                            fmaf(__uint_as_float(r[s][8u + i]), 0.0625f, __uint_as_float(r[s][i]))));
 #pragma unroll
                 for (uint32_t i = 0; i < 8u; ++i) {
-                    const uint32_t from = j * 8u + i;
-                    const uint32_t src = __shfl_sync(0xffffffffu, my_src, from);
-                    const uint32_t row = __shfl_sync(0xffffffffu, my_row, from);
-                    const float step = __shfl_sync(0xffffffffu, my_step, from);
-                    const float wgt = __shfl_sync(0xffffffffu, my_wgt, from);
+                    const uint32_t src = __shfl_sync(0xffffffffu, my_src, from + i);
+                    const uint32_t row = __shfl_sync(0xffffffffu, my_row, from + i);
+                    const float step = __shfl_sync(0xffffffffu, my_step, from + i);
+                    const float wgt = KIND != kGated ? __shfl_sync(0xffffffffu, my_wgt, from + i) : 1.0f;
                     if (src == PDK_MOE_PAD || n >= a.out_dim) continue;
-                    if (NA == 2u && a.kind == kGated) {
-                        const float xg = fminf(fmaf(v[0][j][i], step * scale2[0], bias[0]), a.limit);
-                        const float yu = fminf(fmaxf(fmaf(v[NA - 1u][j][i], step * scale2[NA - 1u], bias[NA - 1u]), -a.limit), a.limit);
-                        a.out[0][(size_t)row * a.out_dim + n] = (xg / (1.0f + __expf(-a.alpha * xg))) * (yu + a.up_add);
-                        continue;
+                    float y;
+                    if (KIND == kGated) {
+                        const float xg = fminf(fmaf(v[0][i], step * scale2[0], bias[0]), a.limit);
+                        const float yu = fminf(fmaxf(fmaf(v[NA - 1u][i], step * scale2[NA - 1u], bias[NA - 1u]), -a.limit), a.limit);
+                        y = (xg / (1.0f + __expf(-a.alpha * xg))) * (yu + a.up_add);
+                    } else {
+                        y = fmaf(v[0][i], step * scale2[0] * wgt, bias[0] * wgt);   // (acc * scale2 * step + bias) * routing weight
                     }
-#pragma unroll
-                    for (uint32_t s = 0; s < NA; ++s)   // (acc * scale2 * step + bias) * routing weight
-                        a.out[NA == 2u ? s : plane][(size_t)row * a.out_dim + n] =
-                            fmaf(v[s][j][i], step * scale2[s] * wgt, bias[s] * wgt);
+                    out[(size_t)row * a.out_dim + n] = y;
                 }
             }
+            if (share >= ng && lane == 0) tc5::mbar_arrive(&sh->tmem_empty[buf]);   // a tile of fewer groups than shares
         }
     }
 }
 
 // MAXG: the most groups of a tile, 4 or 6 (build_tiles); the launch takes the geometry of the widest tile that it has.
-template <uint32_t MAXG, uint32_t NA, uint32_t EPI, bool WG>
+template <uint32_t MAXG, uint32_t NA, uint32_t KIND, uint32_t EPI, bool WG>
 __global__ void __launch_bounds__(96u + 32u * EPI, 1)
 grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
                const __grid_constant__ CUtensorMap tmap_x, const Args a) {
-    static_assert(EPI % 4u == 0u, "whole sets of four lane quarters");
+    static_assert(EPI % 4u == 0u && (KIND == kGated) == (NA == 2u), "whole sets of four lane quarters; gate and up, or one plane");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* rings = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
     Ctl* sh = reinterpret_cast<Ctl*>(rings + kRing);
@@ -491,10 +500,10 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constan
         widest = uniform(sh->widest);
     }
     tc5::fence_after_sync();
-    if (WG || widest <= 1u) roles<1u, NA, EPI, WG>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n);
-    else if (widest <= 2u) roles<2u, NA, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n);
-    else if (widest <= 4u) roles<4u, NA, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n);
-    else if (MAXG > 4u) roles<MAXG, NA, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n);
+    if (WG || widest <= 1u) roles<1u, NA, KIND, EPI, WG>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n);
+    else if (widest <= 2u) roles<2u, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n);
+    else if (widest <= 4u) roles<4u, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n);
+    else if (MAXG > 4u) roles<MAXG, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n);
 
     tc5::fence_before_sync();
     __syncthreads();
@@ -504,11 +513,11 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constan
     }
 }
 
-template <uint32_t MAXG, uint32_t NA, uint32_t EPI, bool WG = false>
+template <uint32_t MAXG, uint32_t NA, uint32_t KIND, uint32_t EPI, bool WG = false>
 int launch(const CUtensorMap& tw0, const CUtensorMap& tw1, const CUtensorMap& tx, const Args& a, cudaStream_t st) {
     constexpr size_t smem = (size_t)kRing + sizeof(Ctl) + kTableBytes + 1024u;
     static_assert(smem <= 227u * 1024u, "shared memory of an SM");
-    auto kern = grouped_kernel<MAXG, NA, EPI, WG>;
+    auto kern = grouped_kernel<MAXG, NA, KIND, EPI, WG>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const uint32_t row_tiles = (a.out_dim + BM - 1u) / BM;

@@ -552,15 +552,14 @@ static int gemm_impl(const PlaneArgs& w0, const PlaneArgs& w1, void* out0, void*
     a.block_expert = (const uint32_t*)r.block_expert; a.sorted_row = (const uint32_t*)r.sorted_row;
     a.sorted_slot = (const uint32_t*)r.sorted_slot; a.topk_w = (const float*)r.topk_w;
     a.in_dim = in_dim; a.out_dim = out_dim; a.max_blocks = max_blocks; a.n_planes = w1.data ? 2u : 1u;
-    a.n_active = n_active; a.kind = kind; a.block_shift = bm == 32u ? 2u : 0u;
+    a.n_active = n_active; a.scatter = kind == moe_gemm::kScatter; a.block_shift = bm == 32u ? 2u : 0u;
     a.alpha = unit.alpha; a.limit = unit.limit; a.up_add = unit.up_add; a.err_word = pdk_error_word();
     auto st = (cudaStream_t)stream;
-    // Gate and up under one B where the unit is computed here (both accumulators have to be in one CTA) and for 32-token blocks,
-    // which bring 24 KB of activations per slab (gate and up of 1024 tokens, 4 of 128 experts, 2880 x 2880: 257 us with a pass per
-    // 32-token block, 220 this way); else one tile at a time.  Tiles of up to six groups where blocks are large: down of
-    // the same block 150 -> 130 us.
-    if (kind == moe_gemm::kGated || (w1.data && bm == 32u)) return moe_gemm::launch<6, 2, 8>(tw0, tw1, tx, a, st);
-    return bm == 32u ? moe_gemm::launch<6, 1, 8>(tw0, tw1, tx, a, st) : moe_gemm::launch<4, 1, 8>(tw0, tw1, tx, a, st);
+    // The gated unit needs gate and up in one CTA.  Tiles of up to six groups where blocks are large (1024 tokens, 4 of 128 experts,
+    // 2880 x 2880: down 150 -> 130 us).
+    using namespace moe_gemm;
+    if (kind == kGated) return launch<6, 2, kGated, 12>(tw0, tw1, tx, a, st);
+    return bm == 32u ? launch<6, 1, kPlain, 8>(tw0, tw1, tx, a, st) : launch<4, 1, kPlain, 8>(tw0, tw1, tx, a, st);
 }
 
 PDK_EXPORT int pdk_mxfp4_moe_gemm_tc5(const void* w0_data, const void* w0_sf, const void* w0_meta, const void* w0_bias,
@@ -686,5 +685,5 @@ int pdk_nvf4_gemv_tc5(const void* data, const void* scale, const void* bias, con
     a.block_expert = tables + 8; a.sorted_row = tables;
     a.in_dim = in_dim; a.out_dim = out_dim; a.max_blocks = 1u; a.n_planes = 1u; a.n_active = 1u;
     a.err_word = pdk_error_word();
-    return moe_gemm::launch<4, 1, 4, true>(tw, tw, tx, a, st);
+    return moe_gemm::launch<4, 1, moe_gemm::kPlain, 4, true>(tw, tw, tx, a, st);
 }

@@ -139,7 +139,7 @@ def _unit_in_gemm(bm, max_blocks):
     instead of two: with 32-token blocks that saves 94 MB each way at 1024 tokens (gate|up + second preparation 313 -> 250 us),
     and with a few blocks a launch's end (one token 16.2 -> 13.9 us); in between two accumulators per tile overlap
     better and the raw planes stay in L2 (60 tokens: 172 against 174 us; 128 tokens on 32 experts of 1024 x 768: 20 against 23)."""
-    return bm == 32 or max_blocks <= 32
+    return bm == 32
 
 
 class MoeWorkspace:
