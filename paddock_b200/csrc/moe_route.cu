@@ -87,87 +87,142 @@ moe_align_kernel(const uint32_t* __restrict__ idx, uint32_t* __restrict__ sorted
     }
 }
 
-// Same layout, linear work: the pair list is walked in chunks of one pair per thread; a
-// pair's place among its expert's entries is (entries of earlier chunks) + (entries of
-// earlier warps of this chunk) + (earlier lanes of its warp with the same expert, from
-// __match_any_sync).  Needs a [warps][n_expert] table in shared memory.
-__global__ void __launch_bounds__(1024)
-moe_align_rank_kernel(const uint32_t* __restrict__ idx, uint32_t* __restrict__ sorted_row,
-                      uint32_t* __restrict__ sorted_slot, uint32_t* __restrict__ block_expert, uint32_t rows,
-                      uint32_t n_active, uint32_t n_expert, uint32_t bm, uint32_t max_blocks) {
+// Same layout, linear work, one CTA: every warp owns a run of consecutive pairs.  It counts them per expert, one thread per
+// expert turns the warps' counts into first places, and a second walk over the same pairs, held in registers, places them - in
+// shared memory, from where the tables go out in whole lines.  The lanes with the same expert come from one vote per bit of the expert's number: __match_any_sync takes as many turns as there
+// are different values.  Needs a [warps][n_expert] table in shared memory.
+// pair_pos (may be null): position of pair p | its group's place in a scale record << 30, PDK_MOE_PAD for a pair that has none.
+// (With a chunk of 1024 pairs at a time, its table cleared and summed up for each: 16.5 us at 4096 pairs of 128 experts, bound
+// by barriers and the serial sums; this way XXX.)
+struct AlignArgs {
+    const uint32_t* idx;
+    uint32_t *sorted_row, *sorted_slot, *block_expert, *pair_pos;
+    uint32_t rows, n_active, n_expert, bm, max_blocks, staged;   // staged: positions in shared memory first
+};
+constexpr uint32_t kAlignHeld = 4u;   // chunks of 32 pairs a warp keeps in registers
+
+__device__ __forceinline__ void align_cta(const AlignArgs& a, uint32_t* ash) {
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nwarp = blockDim.x >> 5, ne = a.n_expert;
+    uint32_t* count = ash;                // [ne] entries per expert
+    uint32_t* boff = count + ne;          // [ne + 1] first block of each expert
+    uint32_t* table = boff + ne + 1u;     // [nwarp][ne] entries, then the warp's next place among its expert's
+    uint32_t* sums = table + nwarp * ne;  // [64] blocks of 32 experts each (up to 2048 experts)
+    uint32_t* mine = table + warp * ne;
+    const uint32_t npairs = a.rows * a.n_active, cap = a.max_blocks * a.bm;
+    const uint32_t chunks = (npairs + 32u * nwarp - 1u) / (32u * nwarp), p0 = warp * chunks * 32u + lane;
+    uint32_t held[kAlignHeld];
+#pragma unroll
+    for (uint32_t c = 0; c < kAlignHeld; ++c)
+        held[c] = c < chunks && p0 + c * 32u < npairs ? a.idx[p0 + c * 32u] : 0xFFFFFFFFu;
+    for (uint32_t e = lane; e < ne; e += 32u) mine[e] = 0u;
+    __syncwarp();
+    const uint32_t bits = 32u - __clz(ne);   // ne itself stands for every number that is no expert's
+    auto peers_of = [&](uint32_t e) {
+        const uint32_t v = min(e, ne);
+        uint32_t m = 0xffffffffu;
+        for (uint32_t i = 0; i < bits; ++i) {
+            const uint32_t b = (v >> i) & 1u, ones = __ballot_sync(0xffffffffu, b);
+            m &= b ? ones : ~ones;
+        }
+        return m;
+    };
+    uint32_t peers_held[kAlignHeld];
+    auto add = [&](uint32_t e, uint32_t peers) {
+        if (e < ne && (peers & ((1u << lane) - 1u)) == 0u) mine[e] += __popc(peers);
+        __syncwarp();
+    };
+#pragma unroll
+    for (uint32_t c = 0; c < kAlignHeld; ++c)
+        if (c < chunks) { peers_held[c] = peers_of(held[c]); add(held[c], peers_held[c]); }
+    for (uint32_t c = kAlignHeld; c < chunks; ++c) {
+        const uint32_t e = p0 + c * 32u < npairs ? a.idx[p0 + c * 32u] : 0xFFFFFFFFu;
+        add(e, peers_of(e));
+    }
+    __syncthreads();
+    for (uint32_t e = tid; e < ne; e += blockDim.x) {   // per expert: places before each warp's
+        uint32_t run = 0;
+        for (uint32_t w = 0; w < nwarp; w += 8u) {
+            uint32_t t[8];
+#pragma unroll
+            for (uint32_t k = 0; k < 8u; ++k) t[k] = w + k < nwarp ? table[(w + k) * ne + e] : 0u;
+#pragma unroll
+            for (uint32_t k = 0; k < 8u; ++k)
+                if (w + k < nwarp) { table[(w + k) * ne + e] = run; run += t[k]; }
+        }
+        count[e] = run;
+    }
+    __syncthreads();
+    // exclusive scan of the block counts: a warp per 32 experts, then the sums of the warps before
+    const uint32_t turns = (ne + 31u) >> 5;
+    for (uint32_t t = warp; t < turns; t += nwarp) {
+        const uint32_t e = t * 32u + lane;
+        const uint32_t nb = e < ne ? (count[e] + a.bm - 1u) / a.bm : 0u;
+        uint32_t inc = nb;
+#pragma unroll
+        for (uint32_t d = 1; d < 32u; d <<= 1) {
+            const uint32_t up = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += up;
+        }
+        if (e < ne) boff[e] = inc - nb;
+        if (lane == 31u) sums[t] = inc;
+    }
+    uint32_t* place_of = sums + 64u;      // [cap] when staged: the pair at a position
+    if (a.staged)
+        for (uint32_t at = tid; at < cap; at += blockDim.x) place_of[at] = PDK_MOE_PAD;
+    __syncthreads();
+    for (uint32_t e = tid; e <= ne; e += blockDim.x) {
+        uint32_t before = 0;
+        for (uint32_t t = 0; t < (e == ne ? turns : e >> 5); ++t) before += sums[t];
+        boff[e] = e == ne ? before : boff[e] + before;
+    }
+    __syncthreads();
+    const uint32_t used = min(boff[ne], a.max_blocks);
+    auto put = [&](uint32_t p, uint32_t e, uint32_t peers) {
+        const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
+        const bool live = e < ne;
+        const uint32_t place = live ? mine[e] + rank : 0u;
+        __syncwarp();
+        if (live && rank == 0u) mine[e] = place + __popc(peers);
+        __syncwarp();
+        if (p >= npairs) return;
+        const uint32_t at = live ? boff[e] * a.bm + place : cap;
+        if (at < cap) {
+            if (a.staged) place_of[at] = p;
+            else { a.sorted_row[at] = p / a.n_active; a.sorted_slot[at] = p % a.n_active; }
+        }
+        if (a.pair_pos) a.pair_pos[p] = at < cap ? at | ((a.bm == 8u ? place >> 3 : at >> 3) & 3u) << 30 : PDK_MOE_PAD;
+    };
+#pragma unroll
+    for (uint32_t c = 0; c < kAlignHeld; ++c)
+        if (c < chunks) put(p0 + c * 32u, held[c], peers_held[c]);
+    for (uint32_t c = kAlignHeld; c < chunks; ++c) {
+        const uint32_t p = p0 + c * 32u, e = p < npairs ? a.idx[p] : 0xFFFFFFFFu;
+        put(p, e, peers_of(e));
+    }
+    for (uint32_t b = used + tid; b < a.max_blocks; b += blockDim.x) a.block_expert[b] = PDK_MOE_PAD;
+    for (uint32_t e = tid; e < ne; e += blockDim.x) {
+        for (uint32_t b = boff[e]; b < boff[e + 1u] && b < a.max_blocks; ++b) a.block_expert[b] = e;
+        if (!a.staged)   // padding of the expert's last block
+            for (uint32_t at = boff[e] * a.bm + count[e]; at < boff[e + 1u] * a.bm && at < cap; ++at) {
+                a.sorted_row[at] = PDK_MOE_PAD;
+                a.sorted_slot[at] = 0;
+            }
+    }
+    if (!a.staged) return;
+    __syncthreads();
+    for (uint32_t at = tid; at < used * a.bm; at += blockDim.x) {
+        const uint32_t p = place_of[at];
+        a.sorted_row[at] = p == PDK_MOE_PAD ? PDK_MOE_PAD : p / a.n_active;
+        a.sorted_slot[at] = p == PDK_MOE_PAD ? 0u : p % a.n_active;
+    }
+}
+
+__global__ void __launch_bounds__(1024) moe_align_rank_kernel(const AlignArgs a) {
     extern __shared__ uint32_t ash[];
-    uint32_t* count = ash;                    // [n_expert] entries per expert
-    uint32_t* boff = count + n_expert;        // [n_expert + 1] first block of each expert
-    uint32_t* cursor = boff + n_expert + 1u;  // [n_expert] entries placed by earlier chunks
-    uint32_t* table = cursor + n_expert;      // [nwarp][n_expert]
-    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, nwarp = blockDim.x >> 5;
-    const uint32_t npairs = rows * n_active, cap = max_blocks * bm;
     // dependent launch: may start while the previous kernel of the stream drains; its results are awaited here
     pdk_pdl_launch_dependents();
     pdk_pdl_wait();
-    for (uint32_t e = tid; e < n_expert; e += blockDim.x) { count[e] = 0; cursor[e] = 0; }
-    __syncthreads();
-    for (uint32_t p = tid; p < npairs; p += blockDim.x) {
-        const uint32_t e = idx[p];
-        if (e < n_expert) atomicAdd(&count[e], 1u);
-    }
-    __syncthreads();
-    if (warp == 0) {  // exclusive scan of the block counts, 32 experts at a time
-        uint32_t carry = 0;
-        for (uint32_t e0 = 0; e0 < n_expert; e0 += 32u) {
-            const uint32_t e = e0 + lane;
-            const uint32_t nb = e < n_expert ? (count[e] + bm - 1u) / bm : 0u;
-            uint32_t inc = nb;
-#pragma unroll
-            for (uint32_t d = 1; d < 32u; d <<= 1) {
-                const uint32_t up = __shfl_up_sync(0xffffffffu, inc, d);
-                if (lane >= d) inc += up;
-            }
-            if (e < n_expert) boff[e] = carry + inc - nb;
-            carry += __shfl_sync(0xffffffffu, inc, 31);
-        }
-        if (lane == 0) boff[n_expert] = carry;
-    }
-    __syncthreads();
-    const uint32_t used = min(boff[n_expert], max_blocks);
-    for (uint32_t b = used + tid; b < max_blocks; b += blockDim.x) block_expert[b] = PDK_MOE_PAD;
-    for (uint32_t e = tid; e < n_expert; e += blockDim.x) {
-        for (uint32_t b = boff[e]; b < boff[e + 1] && b < max_blocks; ++b) block_expert[b] = e;
-        // padding of the expert's last block
-        for (uint32_t at = boff[e] * bm + count[e]; at < boff[e + 1] * bm && at < cap; ++at) {
-            sorted_row[at] = PDK_MOE_PAD;
-            sorted_slot[at] = 0;
-        }
-    }
-    for (uint32_t base = 0; base < npairs; base += blockDim.x) {
-        for (uint32_t i = tid; i < nwarp * n_expert; i += blockDim.x) table[i] = 0;
-        __syncthreads();
-        const uint32_t p = base + tid;
-        const uint32_t e = p < npairs ? idx[p] : 0xFFFFFFFFu;
-        const bool live = e < n_expert;
-        const uint32_t peers = __match_any_sync(0xffffffffu, live ? e : 0xFFFFFFFFu);
-        const uint32_t rank = __popc(peers & ((1u << lane) - 1u));
-        if (live && rank == 0u) table[warp * n_expert + e] = __popc(peers);
-        __syncthreads();
-        for (uint32_t x = tid; x < n_expert; x += blockDim.x) {  // per expert: prefix over the warps
-            uint32_t run = cursor[x];
-            for (uint32_t w = 0; w < nwarp; ++w) {
-                const uint32_t t = table[w * n_expert + x];
-                table[w * n_expert + x] = run;
-                run += t;
-            }
-            cursor[x] = run;
-        }
-        __syncthreads();
-        if (live) {
-            const uint32_t at = boff[e] * bm + table[warp * n_expert + e] + rank;
-            if (at < cap) {
-                sorted_row[at] = p / n_active;
-                sorted_slot[at] = p % n_active;
-            }
-        }
-        __syncthreads();
-    }
+    align_cta(a, ash);
 }
 
 // ---------------------------------------------------------------- activation prep
@@ -219,22 +274,31 @@ moe_prep_act_kernel(const float* __restrict__ x, uint8_t* __restrict__ xq, float
 }
 
 // ---------------------------------------------------------------- slot combine
-__global__ void moe_slot_combine_kernel(const float4* __restrict__ part, float4* __restrict__ residual,
-                                        uint32_t embd4, uint32_t n_active, uint32_t rows) {
+// A thread per four columns of a row (grid y); the slots' loads of a thread are in flight together, four at a time.
+__global__ void __launch_bounds__(256)
+moe_slot_combine_kernel(const float4* __restrict__ part, float4* __restrict__ residual, uint32_t embd4, uint32_t n_active,
+                        uint32_t rows) {
     // dependent launch: may start while the previous kernel of the stream drains; its results are awaited here
     pdk_pdl_launch_dependents();
     pdk_pdl_wait();
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)rows * embd4) return;
-    const size_t t = i / embd4, r = i % embd4;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (uint32_t k = 0; k < n_active; ++k) {  // fixed slot order: bit-reproducible
-        const float4 p = part[(t * n_active + k) * embd4 + r];
-        acc.x += p.x; acc.y += p.y; acc.z += p.z; acc.w += p.w;
+    const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= embd4) return;
+    for (size_t t = blockIdx.y; t < rows; t += gridDim.y) {
+        const float4* p = part + t * n_active * embd4 + r;
+        float4 d = residual[t * embd4 + r];
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        for (uint32_t k = 0; k < n_active; k += 4u) {  // fixed slot order: bit-reproducible
+            float4 v[4];
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; ++j)
+                if (k + j < n_active) v[j] = __ldcs(p + (size_t)(k + j) * embd4);
+#pragma unroll
+            for (uint32_t j = 0; j < 4u; ++j)
+                if (k + j < n_active) { acc.x += v[j].x; acc.y += v[j].y; acc.z += v[j].z; acc.w += v[j].w; }
+        }
+        d.x += acc.x; d.y += acc.y; d.z += acc.z; d.w += acc.w;
+        residual[t * embd4 + r] = d;
     }
-    float4 d = residual[i];
-    d.x += acc.x; d.y += acc.y; d.z += acc.z; d.w += acc.w;
-    residual[i] = d;
 }
 
 }  // namespace
@@ -249,19 +313,26 @@ PDK_EXPORT int pd_moe_topk_batch(const void* logits, const void* bias, uint32_t 
 }
 
 // slot 146, packs/cuda/src/gemm/f32_qkv.cuh:1269-1279 (kernel attn/decode.cuh:2316-2396)
-PDK_EXPORT int pd_moe_align_bm(const void* idx, void* sorted_row, void* sorted_slot, void* block_expert,
-                               uint32_t rows, uint32_t n_active, uint32_t n_expert, uint32_t bm, uint32_t max_blocks,
-                               void* stream) {
+// shared memory of align_cta without and with the staged positions
+static size_t align_smem(uint32_t n_expert, uint32_t warps) { return ((size_t)(warps + 2u) * n_expert + 65u) * sizeof(uint32_t); }
+
+static int align_impl(const void* idx, void* sorted_row, void* sorted_slot, void* block_expert, void* pair_pos, uint32_t rows,
+                      uint32_t n_active, uint32_t n_expert, uint32_t bm, uint32_t max_blocks, void* stream) {
     if (rows == 0 || n_expert == 0) return 0;
     if (bm == 0 || (bm & (bm - 1u)) || n_expert > 4096u) return cudaErrorInvalidValue;
     static const cudaError_t attr_rank =
         cudaFuncSetAttribute(moe_align_rank_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    const size_t rank_smem = ((size_t)3u * n_expert + 1u + (size_t)32u * n_expert) * sizeof(uint32_t);
-    if (attr_rank == cudaSuccess && rank_smem <= 200u * 1024u) {
-        return pdk_launch_pdl(moe_align_rank_kernel, dim3(1), dim3(1024), rank_smem, (cudaStream_t)stream,
-                              (const uint32_t*)idx, (uint32_t*)sorted_row, (uint32_t*)sorted_slot,
-                              (uint32_t*)block_expert, rows, n_active, n_expert, bm, max_blocks);
+    // a warp per 32 pairs, up to 32 warps: with few pairs the counts of the idle ones would only be cleared and summed
+    const uint64_t pairs = (uint64_t)rows * n_active;
+    const uint32_t warps = pairs >= 1024u ? 32u : pairs <= 128u ? 4u : (uint32_t)((pairs + 31u) / 32u);
+    const size_t base = align_smem(n_expert, warps), places = (size_t)max_blocks * bm * sizeof(uint32_t);
+    const uint32_t in_smem = base + places <= 200u * 1024u ? 1u : 0u;
+    if (attr_rank == cudaSuccess && base <= 200u * 1024u && n_expert <= 2048u) {
+        const AlignArgs a{(const uint32_t*)idx, (uint32_t*)sorted_row, (uint32_t*)sorted_slot, (uint32_t*)block_expert,
+                          (uint32_t*)pair_pos, rows, n_active, n_expert, bm, max_blocks, in_smem};
+        return pdk_launch_pdl(moe_align_rank_kernel, dim3(1), dim3(32u * warps), base + (in_smem ? places : 0u), (cudaStream_t)stream, a);
     }
+    if (pair_pos) return cudaErrorInvalidValue;
     // many experts: the scan kernel, one warp per expert
     size_t shmem = (size_t)(2u * n_expert + 1u) * sizeof(uint32_t);
     // the pick list is staged in shared memory when it fits (up to 200 KB)
@@ -275,6 +346,23 @@ PDK_EXPORT int pd_moe_align_bm(const void* idx, void* sorted_row, void* sorted_s
                                                                (uint32_t*)sorted_slot, (uint32_t*)block_expert, rows,
                                                                n_active, n_expert, bm, max_blocks, staged);
     return pdk_launch_status();
+}
+
+PDK_EXPORT int pd_moe_align_bm(const void* idx, void* sorted_row, void* sorted_slot, void* block_expert,
+                               uint32_t rows, uint32_t n_active, uint32_t n_expert, uint32_t bm, uint32_t max_blocks,
+                               void* stream) {
+    return align_impl(idx, sorted_row, sorted_slot, block_expert, nullptr, rows, n_active, n_expert, bm, max_blocks, stream);
+}
+
+// No slot: moe_align_bm that also leaves every pair's position for pdk_moe_prep_tokens_f4, u32[rows * n_active]: the position |
+// its group's place in a scale record << 30, or PDK_MOE_PAD where the pair has no expert or no room.  bm 8 or 32, up to 1500
+// experts, positions below 2^30.
+PDK_EXPORT int pdk_moe_align_pos(const void* idx, void* sorted_row, void* sorted_slot, void* block_expert, void* pair_pos,
+                                 uint32_t rows, uint32_t n_active, uint32_t n_expert, uint32_t bm, uint32_t max_blocks,
+                                 void* stream) {
+    if (rows == 0 || n_expert == 0) return 0;
+    if ((bm != 8u && bm != 32u) || n_expert > 1500u || !pair_pos || max_blocks >= (1u << 25)) return cudaErrorInvalidValue;
+    return align_impl(idx, sorted_row, sorted_slot, block_expert, pair_pos, rows, n_active, n_expert, bm, max_blocks, stream);
 }
 
 // slot 34, packs/cuda/src/attn/decode.cuh:2316-2396: blocks of 32 entries
@@ -299,7 +387,7 @@ PDK_EXPORT int pd_moe_slot_combine(const void* part, void* residual, uint32_t em
                                    void* stream) {
     if (rows == 0 || embd == 0) return 0;
     if ((embd & 3u) != 0u || !pdk_aligned(part, 16) || !pdk_aligned(residual, 16)) return cudaErrorInvalidValue;
-    const size_t total = (size_t)rows * (embd >> 2);
-    return pdk_launch_pdl(moe_slot_combine_kernel, dim3((uint32_t)((total + 255u) / 256u)), dim3(256), 0,
-                          (cudaStream_t)stream, (const float4*)part, (float4*)residual, embd >> 2, n_active, rows);
+    const uint32_t embd4 = embd >> 2, threads = embd4 < 256u ? (embd4 + 31u) & ~31u : 256u;
+    return pdk_launch_pdl(moe_slot_combine_kernel, dim3((embd4 + threads - 1u) / threads, rows < 65535u ? rows : 65535u), dim3(threads),
+                          0, (cudaStream_t)stream, (const float4*)part, (float4*)residual, embd4, n_active, rows);
 }

@@ -198,6 +198,16 @@ __device__ __forceinline__ void record_place(uint32_t pos, uint32_t bm, Same sam
     rec = b - col;
 }
 
+// Four lanes' scale bytes of the four terms, transposed: lane j of the four gets term j's, groups in byte order.
+__device__ __forceinline__ uint32_t scale_word(const uint32_t (&sb)[4]) {
+    const uint32_t lane = threadIdx.x & 31u;
+    uint32_t v = sb[0] | sb[1] << 8 | sb[2] << 16 | sb[3] << 24;
+    const uint32_t a = __shfl_xor_sync(0xffffffffu, v, 1);
+    v = lane & 1u ? __byte_perm(v, a, 0x3715) : __byte_perm(v, a, 0x6240);   // even lane: terms 0 and 2 of both, odd: 1 and 3
+    const uint32_t b = __shfl_xor_sync(0xffffffffu, v, 2);
+    return lane & 2u ? __byte_perm(v, b, 0x3276) : __byte_perm(v, b, 0x5410);
+}
+
 // One CTA per block position.  Position (block b, token i) writes four term rows of its group of 8 tokens,
 // row term * 8 + i % 8 of the group's 32.  A 16-element scale group of the tensor core's element order is the
 // two 8-runs (h*8 .. h*8+7) and (16 + h*8 .. 16 + h*8+7) of a 32-element block.
@@ -271,9 +281,11 @@ __device__ __forceinline__ void prep_position(const PrepArgs& a, uint32_t pos, u
     const uint32_t r0 = pos & 7u;
     uint8_t* xq_rows = a.xq + ((size_t)(pos >> 3) * 32u + r0) * kh;
     uint8_t* xs_row = a.xs + (size_t)rec * num_kb * 2048u + r0 * 16u + col * 4u;
-    for (uint32_t g = tid; g < num_kb * 16u; g += blockDim.x) {
+    for (uint32_t base = 0; base < num_kb * 16u; base += blockDim.x) {   // whole warps: scale_word shuffles
+        const uint32_t g = base + tid;
         // scale byte of group g and term row r: record slab g/16, cell (g/4)%4, byte r*16 + col*4 + g%4
-        uint8_t* xs_g = xs_row + (size_t)(g >> 4) * 2048u + ((g >> 2) & 3u) * 512u + (g & 3u);
+        // (four threads write their groups' bytes of a term as one word)
+        uint8_t* xs_g = xs_row + (size_t)(g >> 4) * 2048u + ((g >> 2) & 3u) * 512u;
         uint2 codes[4] = {};
         uint32_t sb[4] = {};
         // padding and all-zero rows: zero term rows and scale bytes, none of the term arithmetic; the record's cells
@@ -294,11 +306,12 @@ __device__ __forceinline__ void prep_position(const PrepArgs& a, uint32_t pos, u
                                        : make_float2(hi0[2 * (k & 3)], hi0[2 * (k & 3) + 1]), inv_step);
             quantize_group(r, codes, sb);
         }
+        if (g < groups)
 #pragma unroll
-        for (uint32_t term = 0; term < 4u; ++term) {
-            if (g < groups) *reinterpret_cast<uint2*>(xq_rows + (size_t)(term * 8u) * kh + (size_t)g * 8u) = codes[term];
-            xs_g[term * 128u] = (uint8_t)sb[term];
-        }
+            for (uint32_t term = 0; term < 4u; ++term)
+                *reinterpret_cast<uint2*>(xq_rows + (size_t)(term * 8u) * kh + (size_t)g * 8u) = codes[term];
+        const uint32_t word = scale_word(sb);
+        if (g < num_kb * 16u) *reinterpret_cast<uint32_t*>(xs_g + (g & 3u) * 128u) = word;
     }
 }
 
@@ -326,6 +339,81 @@ __global__ void __launch_bounds__(256) moe_prep_f4_kernel(const PrepArgs a) {
         record_place(pos, a.bm, [&](uint32_t q) { return a.block_expert[q] == e; }, rec, col);
     }
     prep_position(a, pos, src, rec, col);
+}
+
+// One CTA per token: its row is quantized once and written to the positions of all its k pairs (pair_pos, moe_route.cu), where
+// a CTA per position read and quantized it k times.  Positions without a pair are left as they are: their columns of the
+// GEMM are never read.  (1024 tokens of 2880, 4 of 128 experts: 26.2 us -> XXX.)
+struct TokenArgs {
+    const float* x;             // [rows][dim]
+    const uint32_t* pair_pos;   // [rows][k]
+    uint8_t *xq, *xs;
+    float* xstep;
+    uint32_t dim, k, bm, natural;
+};
+
+__global__ void __launch_bounds__(256) moe_prep_tokens_kernel(const TokenArgs a) {
+    __shared__ float s_red[8];
+    pdk_pdl_launch_dependents();
+    pdk_pdl_wait();
+    const uint32_t tid = threadIdx.x, token = blockIdx.x, groups = a.dim >> 4, kh = a.dim >> 1, num_kb = (a.dim + 255u) >> 8;
+    const float* row = a.x + (size_t)token * a.dim;
+    auto load = [&](uint32_t g, float2 (&r)[8]) {   // in code order, as prep_position
+        const uint32_t lo_at = a.natural ? g * 16u : (g >> 1) * 32u + (g & 1u) * 8u, hi_at = lo_at + (a.natural ? 8u : 16u);
+        const float4 p = *reinterpret_cast<const float4*>(row + lo_at), q = *reinterpret_cast<const float4*>(row + lo_at + 4u);
+        const float4 u = *reinterpret_cast<const float4*>(row + hi_at), v = *reinterpret_cast<const float4*>(row + hi_at + 4u);
+        if (a.natural) {
+            r[0] = make_float2(p.x, p.y); r[1] = make_float2(p.z, p.w); r[2] = make_float2(q.x, q.y); r[3] = make_float2(q.z, q.w);
+            r[4] = make_float2(u.x, u.y); r[5] = make_float2(u.z, u.w); r[6] = make_float2(v.x, v.y); r[7] = make_float2(v.z, v.w);
+        } else {
+            r[0] = make_float2(p.x, u.x); r[1] = make_float2(p.y, u.y); r[2] = make_float2(p.z, u.z); r[3] = make_float2(p.w, u.w);
+            r[4] = make_float2(q.x, v.x); r[5] = make_float2(q.y, v.y); r[6] = make_float2(q.z, v.z); r[7] = make_float2(q.w, v.w);
+        }
+    };
+    float2 r[8] = {};
+    float amax = 0.0f;
+    for (uint32_t g = tid; g < groups; g += blockDim.x) {
+        load(g, r);
+#pragma unroll
+        for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fmaxf(fabsf(r[k].x), fabsf(r[k].y)));
+    }
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, off));
+    if ((tid & 31u) == 0u) s_red[tid >> 5] = amax;
+    __syncthreads();
+    amax = 0.0f;
+    for (uint32_t w = 0; w < (blockDim.x >> 5); ++w) amax = fmaxf(amax, s_red[w]);
+    const int ex = (int)((__float_as_uint(amax) >> 23) & 0xffu) - 127;
+    const bool live = amax > 0.0f && ex > -110 && ex < 120;
+    const float inv_step = live ? __uint_as_float((uint32_t)(127 - (ex - 8)) << 23) : 0.0f;
+    const float step = live ? __uint_as_float((uint32_t)(127 + (ex - 8)) << 23) : 0.0f;
+    const bool single = num_kb * 16u <= blockDim.x;
+    for (uint32_t base = 0; base < num_kb * 16u; base += blockDim.x) {   // whole warps: scale_word shuffles
+        const uint32_t g = base + tid;
+        uint2 codes[4] = {};
+        uint32_t sb[4] = {};
+        if (live && g < groups) {
+            if (!single) load(g, r);
+#pragma unroll
+            for (int k = 0; k < 8; ++k) r[k] = mul2(r[k], inv_step);
+            quantize_group(r, codes, sb);
+        }
+        const uint32_t word = scale_word(sb);
+        if (g >= num_kb * 16u) continue;
+        for (uint32_t s = 0; s < a.k; ++s) {
+            const uint32_t at = a.pair_pos[(size_t)token * a.k + s];
+            if (at == PDK_MOE_PAD) continue;
+            const uint32_t pos = at & 0x3FFFFFFFu, col = at >> 30, r0 = pos & 7u, b = pos / a.bm, rec = a.bm == 8u ? b - col : b;
+            uint8_t* xq_rows = a.xq + ((size_t)(pos >> 3) * 32u + r0) * kh + (size_t)g * 8u;
+            if (g < groups)
+#pragma unroll
+                for (uint32_t term = 0; term < 4u; ++term)
+                    *reinterpret_cast<uint2*>(xq_rows + (size_t)(term * 8u) * kh) = codes[term];
+            *reinterpret_cast<uint32_t*>(a.xs + ((size_t)rec * num_kb + (g >> 4)) * 2048u + ((g >> 2) & 3u) * 512u + r0 * 16u +
+                                         col * 4u + (g & 3u) * 128u) = word;
+            if (g == 0u) a.xstep[pos] = step;
+        }
+    }
 }
 
 // Decode widths (rows * k <= 32 pairs): routing, alignment and the first activation preparation in
@@ -429,7 +517,8 @@ static int prep_impl(const void* x, const void* up, const void* sorted_row, cons
                      float alpha, float limit, float up_add, void* stream) {
     if (max_blocks == 0) return 0;
     if (dim == 0 || (dim & 31u) != 0u || (bm != 8u && bm != 32u)) return cudaErrorInvalidValue;
-    if (!pdk_aligned(x, 16) || !pdk_aligned(xq, 16) || (mode == 1u && !pdk_aligned(up, 16))) return cudaErrorInvalidValue;
+    if (!pdk_aligned(x, 16) || !pdk_aligned(xq, 16) || !pdk_aligned(xs, 4) || (mode == 1u && !pdk_aligned(up, 16)))
+        return cudaErrorInvalidValue;
     PrepArgs a{};
     a.x = (const float*)x; a.up = (const float*)up; a.sorted_row = (const uint32_t*)sorted_row;
     a.block_expert = (const uint32_t*)block_expert;
@@ -446,6 +535,20 @@ PDK_EXPORT int pdk_moe_prep_act_f4(const void* x, const void* up, const void* so
     if (mode > 1u) return cudaErrorInvalidValue;
     return prep_impl(x, up, sorted_row, block_expert, xq, xs, xstep, dim, bm, max_blocks, mode, 0u, alpha, limit, 1.0f,
                      stream);
+}
+
+// The rows of x f32 [rows][dim] to the positions of their pairs (pair_pos u32 [rows][k], pdk_moe_align_pos):
+// the same term rows, scale records and steps there as pdk_moe_prep_act_f4 (natural 0) or ..._f4n (1) in mode 0; positions of padding
+// are left alone.
+PDK_EXPORT int pdk_moe_prep_tokens_f4(const void* x, const void* pair_pos, void* xq, void* xs, void* xstep, uint32_t dim, uint32_t k,
+                                      uint32_t rows, uint32_t bm, uint32_t natural, void* stream) {
+    if (rows == 0 || k == 0) return 0;
+    if (dim == 0 || (dim & 31u) != 0u || (bm != 8u && bm != 32u) || natural > 1u) return cudaErrorInvalidValue;
+    if (!pdk_aligned(x, 16) || !pdk_aligned(xq, 16) || !pdk_aligned(xs, 16)) return cudaErrorInvalidValue;
+    const TokenArgs a{(const float*)x, (const uint32_t*)pair_pos, (uint8_t*)xq, (uint8_t*)xs, (float*)xstep, dim, k, bm, natural};
+    const uint32_t per_row = ((dim + 255u) >> 8) * 16u;
+    return pdk_launch_pdl(moe_prep_tokens_kernel, dim3(rows), dim3(per_row <= 256u ? (per_row + 31u) & ~31u : 256u), 0,
+                          (cudaStream_t)stream, a);
 }
 
 // No counterpart in the reference.  moe_topk_batch + moe_align_bm + pdk_moe_prep_act_f4 (mode 0) in one

@@ -143,6 +143,8 @@ _EXTRA_SIGS = {
     "pdk_mxfp4_moe_gate_up_tc5": "p" * 14 + "uuuuufff",
     "pdk_nvf4_moe_gate_up_tc5": "p" * 14 + "uuuuufff",
     "pdk_moe_prep_rows_f4": "ppppppuuuu",
+    "pdk_moe_align_pos": "pppppuuuuu",
+    "pdk_moe_prep_tokens_f4": "pppppuuuuu",
 }
 _KIND = {"p": C.c_void_p, "u": C.c_uint32, "U": C.c_uint64, "f": C.c_float}
 

@@ -156,6 +156,7 @@ class MoeWorkspace:
         self.sorted_row = torch.empty(nb, dtype=u32, device=dev)
         self.sorted_slot = torch.empty(nb, dtype=u32, device=dev)
         self.block_expert = torch.empty(self.max_blocks, dtype=u32, device=dev)
+        self.pair_pos = torch.empty(pairs, dtype=u32, device=dev)      # where each (token, slot) pair went
         self.xq = torch.empty(tokens * planes.embd * 2, dtype=torch.uint8, device=dev)
         self.xscale = torch.empty(tokens, dtype=f32, device=dev)
         self.h = torch.zeros(nb * planes.ff, dtype=f32, device=dev)
@@ -193,11 +194,33 @@ def moe_mxfp4_experts(ex, planes, ws, x, rows, alpha=1.702, limit=7.0):
     return 5
 
 
-def moe_mxfp4_experts_tc5(ex, planes, ws, x, rows, alpha=1.702, limit=7.0, route=None):
+def _route_and_prepare(ex, ws, x, rows, embd, n_expert, max_blocks, natural, logits=None, router_bias=None):
+    """Positions and term rows of x: top-k (with logits; else ws.idx / ws.w hold the choices already), alignment, one preparation
+    per token.  Returns the number of launches."""
+    st = _stream()
+    c = ex.pack.call
+    k, bm = ws.n_active, ws.bm
+    n = 2
+    if logits is not None:
+        c("moe_topk_batch", logits, router_bias, n_expert, k, ws.idx, ws.w, rows, stream=st)
+        n = 3
+    if n_expert > 1500:       # beyond the alignment that knows the pairs' positions
+        c("moe_align_bm", ws.idx, ws.sorted_row, ws.sorted_slot, ws.block_expert, rows, k, n_expert, bm, max_blocks, stream=st)
+        args = x, None, ws.sorted_row, ws.block_expert, ws.x4q, ws.x4s, ws.x4step, embd, bm, max_blocks, 0, 1.0, 0.0
+        c(*(("pdk_moe_prep_act_f4n", *args, 0.0) if natural else ("pdk_moe_prep_act_f4", *args)), stream=st)
+        return n
+    c("pdk_moe_align_pos", ws.idx, ws.sorted_row, ws.sorted_slot, ws.block_expert, ws.pair_pos, rows, k, n_expert, bm, max_blocks,
+      stream=st)
+    c("pdk_moe_prep_tokens_f4", x, ws.pair_pos, ws.x4q, ws.x4s, ws.x4step, embd, k, rows, bm, int(natural), stream=st)
+    return n
+
+
+def moe_mxfp4_experts_tc5(ex, planes, ws, x, rows, alpha=1.702, limit=7.0, route=None, routed=False):
     """moe_mxfp4_experts on the block-scaled tensor-core path (planes prepared with prepare_tc5):
     align -> term rows of x -> gate and up GEMM -> SwiGLU + term rows of h -> down GEMM scattered
     into ws.part.  Five launches; with route = (router_logits, router_bias) at decode widths the
-    top-k, the alignment and the first preparation are one launch (four in all)."""
+    top-k, the alignment and the first preparation are one launch (four in all); routed: they are
+    done already (_route_and_prepare), three launches."""
     st = _stream()
     c = ex.pack.call
     k, bm, t = ws.n_active, ws.bm, planes.tc5
@@ -205,11 +228,8 @@ def moe_mxfp4_experts_tc5(ex, planes, ws, x, rows, alpha=1.702, limit=7.0, route
     if route is not None:
         c("pdk_moe_route_prep_f4", route[0], route[1], x, ws.idx, ws.w, ws.sorted_row, ws.sorted_slot, ws.block_expert,
           ws.x4q, ws.x4s, ws.x4step, planes.n_expert, k, rows, planes.embd, bm, max_blocks, stream=st)
-    else:
-        c("moe_align_bm", ws.idx, ws.sorted_row, ws.sorted_slot, ws.block_expert, rows, k, planes.n_expert, bm,
-          max_blocks, stream=st)
-        c("pdk_moe_prep_act_f4", x, None, ws.sorted_row, ws.block_expert, ws.x4q, ws.x4s, ws.x4step, planes.embd, bm,
-          max_blocks, 0, alpha, limit, stream=st)
+    elif not routed:
+        _route_and_prepare(ex, ws, x, rows, planes.embd, planes.n_expert, max_blocks, False)
     if not _unit_in_gemm(bm, max_blocks):
         c("pdk_mxfp4_moe_gemm_tc5", planes.gate.data, t["gate"][0], t["gate"][1], planes.gate_bias, ws.g_raw,
           planes.up.data, t["up"][0], t["up"][1], planes.up_bias, ws.u_raw, ws.x4q, ws.x4s, ws.x4step,
@@ -241,13 +261,15 @@ def moe_mxfp4_forward(ex, planes, ws, x, router_logits, out, alpha=1.702, limit=
         moe_mxfp4_experts_tc5(ex, planes, ws, x, T, alpha, limit, route=(router_logits, router_bias))
         c("moe_slot_combine", ws.part, out, planes.embd, k, T, stream=st)
         return 5
-    c("moe_topk_batch", router_logits, router_bias, planes.n_expert, k, ws.idx, ws.w, T, stream=st)
     if planes.tc5 is not None:
-        moe_mxfp4_experts_tc5(ex, planes, ws, x, T, alpha, limit)
-    else:
-        moe_mxfp4_experts(ex, planes, ws, x, T, alpha, limit)
+        n = _route_and_prepare(ex, ws, x, T, planes.embd, planes.n_expert, ws.max_blocks, False, router_logits, router_bias)
+        moe_mxfp4_experts_tc5(ex, planes, ws, x, T, alpha, limit, routed=True)
+        c("moe_slot_combine", ws.part, out, planes.embd, k, T, stream=st)
+        return n + 4  # launches
+    c("moe_topk_batch", router_logits, router_bias, planes.n_expert, k, ws.idx, ws.w, T, stream=st)
+    moe_mxfp4_experts(ex, planes, ws, x, T, alpha, limit)
     c("moe_slot_combine", ws.part, out, planes.embd, k, T, stream=st)
-    return 7  # launches
+    return 7
 
 
 # ---- NVFP4 expert planes (gpu/types.rs:176-226, Row order) on the same grouped GEMM
@@ -287,11 +309,9 @@ def moe_nvf4_forward(ex, gate, up, down, ws, x, router_logits, out, gated=True, 
     if fused:      # decode widths: routing, alignment and the first activation preparation in one launch
         c("pdk_moe_route_prep_f4n", router_logits, router_bias, x, ws.idx, ws.w, ws.sorted_row, ws.sorted_slot, ws.block_expert,
           ws.x4q, ws.x4s, ws.x4step, n_expert, k, T, embd, bm, max_blocks, stream=st)
+        n = 1
     else:
-        c("moe_topk_batch", router_logits, router_bias, n_expert, k, ws.idx, ws.w, T, stream=st)
-        c("moe_align_bm", ws.idx, ws.sorted_row, ws.sorted_slot, ws.block_expert, T, k, n_expert, bm, max_blocks, stream=st)
-        c("pdk_moe_prep_act_f4n", x, None, ws.sorted_row, ws.block_expert, ws.x4q, ws.x4s, ws.x4step, embd, bm, max_blocks, 0,
-          alpha, limit, up_add, stream=st)
+        n = _route_and_prepare(ex, ws, x, T, embd, n_expert, max_blocks, True, router_logits, router_bias)
     if gated and _unit_in_gemm(bm, max_blocks):
         c("pdk_nvf4_moe_gate_up_tc5", gate.data, gate.tiled, gate.scale2, None, up.data, up.tiled, up.scale2, None, ws.h,
           ws.x4q, ws.x4s, ws.x4step, ws.block_expert, ws.sorted_row, embd, ff, n_expert, bm, max_blocks, alpha, limit, up_add,
@@ -314,4 +334,4 @@ def moe_nvf4_forward(ex, gate, up, down, ws, x, router_logits, out, gated=True, 
       ws.h4s, ws.h4step, ws.block_expert, ws.sorted_row, ws.sorted_slot, ws.w, ff, embd, n_expert, bm, max_blocks, k, 1,
       stream=st)
     c("moe_slot_combine", ws.part, out, embd, k, T, stream=st)
-    return 5 if fused else 7
+    return n + 4

@@ -59,3 +59,64 @@ def test_tiles_over_runs_of_blocks(pack, tokens, n_expert, k, embd, ff, bm, gate
     # every row by itself: a tile that took another expert's weights, or missed a group, is a whole row wrong
     rows = np.linalg.norm(y - ref, axis=1) / np.linalg.norm(ref, axis=1)
     assert rows.max() < 1e-2
+
+
+@pytest.mark.parametrize("tokens,n_expert,k,embd,bm,skew", [
+    (9, 8, 2, 128, 8, 0.0),
+    (64, 128, 4, 512, 8, 0.0),
+    (128, 5, 4, 288, 8, 2.0),         # half a warp in the last slab; runs of a dozen blocks
+    (300, 16, 4, 4352, 32, 1.0),      # a row of more groups than threads
+    (700, 128, 8, 256, 32, 0.0),      # 5600 pairs: more chunks per warp than it holds in registers
+    (1, 512, 16, 64, 8, 0.0),
+    (3000, 64, 1, 64, 32, 4.0),       # one token of 64 per expert at best, a thousand blocks; positions staged in shared memory
+    (9000, 16, 8, 32, 8, 0.0),        # too many positions for that: written where they go
+])
+@pytest.mark.parametrize("natural", [False, True])
+def test_positions_and_token_rows_equal_the_gathered_ones(pack, tokens, n_expert, k, embd, bm, skew, natural):
+    """pdk_moe_align_pos leaves moe_align_bm's tables and, per pair, its position;
+    pdk_moe_prep_tokens_f4 then writes, byte for byte, the rows that pdk_moe_prep_act_f4(n) gathers for these positions."""
+    c = P.GpuExecutor(pack).pack.call
+    pairs = tokens * k
+    max_blocks = min(pairs, pairs // bm + n_expert)
+    nb = max_blocks * bm
+    x = dev_f32(oracle.bf16_round(oracle.fill_normal(tokens * embd, 7, 1.0)))
+    logits = oracle.fill_normal(tokens * n_expert, 8, 1.0).reshape(tokens, n_expert)
+    logits = dev_f32((logits - skew * np.arange(n_expert, dtype=np.float32)).reshape(-1))
+    i32, u8 = torch.int32, torch.uint8
+    new = lambda n, dt: torch.zeros(n, dtype=dt, device="cuda")
+    t = [dict(idx=new(pairs, i32), w=new(pairs, torch.float32), row=new(nb, i32), slot=new(nb, i32), blk=new(max_blocks, i32),
+              q=new(nb * 4 * embd // 2, u8), s=new(max_blocks * ((embd + 255) // 256) * 2048, u8), step=new(nb, torch.float32))
+         for _ in range(2)]
+    a, b = t
+    pos = new(pairs, i32)
+    c("moe_topk_batch", logits, None, n_expert, k, a["idx"], a["w"], tokens)
+    c("moe_align_bm", a["idx"], a["row"], a["slot"], a["blk"], tokens, k, n_expert, bm, max_blocks)
+    args = x, None, a["row"], a["blk"], a["q"], a["s"], a["step"], embd, bm, max_blocks, 0, 1.0, 7.0
+    c(*(("pdk_moe_prep_act_f4n", *args, 0.0) if natural else ("pdk_moe_prep_act_f4", *args)))
+    b["idx"], b["w"] = a["idx"], a["w"]
+    c("pdk_moe_align_pos", b["idx"], b["row"], b["slot"], b["blk"], pos, tokens, k, n_expert, bm, max_blocks)
+    c("pdk_moe_prep_tokens_f4", x, pos, b["q"], b["s"], b["step"], embd, k, tokens, bm, int(natural))
+    torch.cuda.synchronize()
+    assert pack.device_error() == 0
+    # unused blocks keep what they had in every table
+    for name in a:
+        assert torch.equal(a[name].view(u8), b[name].view(u8)), name
+    p = torch.arange(pairs, device="cuda")
+    at = (pos.long() & 0x3FFFFFFF)
+    assert torch.equal(b["row"][at].long(), p // k) and torch.equal(b["slot"][at].long(), p % k)
+    # the positions follow the oracle's grouping: expert of the block a pair landed in, pairs of an expert in order
+    idx = torch.from_numpy(oracle.moe_topk(logits.cpu().numpy(), n_expert, k)[0].astype(np.int64)).cuda().view(-1)
+    assert torch.equal(b["blk"][at // bm].long(), idx)
+    order = torch.argsort(idx * pairs + p)
+    assert (at[order][1:] > at[order][:-1]).all()
+
+
+def test_pairs_without_an_expert_have_no_position(pack):
+    c = P.GpuExecutor(pack).pack.call
+    idx = torch.tensor([0, -1, 1, 5, 0, 1], dtype=torch.int32, device="cuda")     # two of them outside [0, 2)
+    new = lambda n: torch.full((n,), -7, dtype=torch.int32, device="cuda")
+    row, slot, blk, pos = new(16), new(16), new(2), new(6)
+    c("pdk_moe_align_pos", idx, row, slot, blk, pos, 6, 1, 2, 8, 2)
+    torch.cuda.synchronize()
+    assert pos.tolist() == [0, -1, 8, -1, 1, 9] and blk.tolist() == [0, 1]
+    assert row.tolist() == [0, 4] + [-1] * 6 + [2, 5] + [-1] * 6
