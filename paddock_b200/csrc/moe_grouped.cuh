@@ -472,8 +472,7 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constan
     }
     // dependent launch: barriers and tensor memory are set up while the previous kernel drains;
     // everything below reads what it wrote
-    pdk_pdl_launch_dependents();
-    pdk_pdl_wait();
+    pdk_pdl_wait_then_launch();
     uint32_t n, widest;
     if (a.max_blocks <= 32u) {
         s_tile = s_expert + 64u * warp;

@@ -129,21 +129,24 @@ __device__ __forceinline__ float rcp_approx(float v) {
     return r;
 }
 
-// One 16-element scale group, r[8] = its pairs in code order (byte i of a term's 8 bytes = pair i), values below 512:
-// the four terms' codes and scale bytes.  The residual stays unscaled; the power 16^k of term k sits in its scale's factor
-// (exact), and the last term leaves none.  The kernel around it is bound by issue: this is half the instructions of the form
-// that scaled 16 residuals up per term, divided by the scale and worked on single floats.
-__device__ __forceinline__ void quantize_group(float2 (&r)[8], uint2 (&codes)[4], uint32_t (&sb)[4]) {
-    float up = 1.0f, down = 1.0f;
-#pragma unroll
+// One 16-element scale group, r[8] = its pairs in code order (byte i of a term's 8 bytes = pair i), values below 512: the four
+// terms' codes, handed to put(term, codes), and the four scale bytes as one word.  The residual stays unscaled; the power 16^k of term k sits
+// in its scale's factor (exact), and the last term leaves none.  The kernels around it are bound by issue: this is half the
+// instructions of the form that scaled 16 residuals up per term, divided by the scale and worked on single floats.  One copy of a
+// term's code: what a launch runs once per thread it fetches into the instruction cache first.
+template <class Put>
+__device__ __forceinline__ uint32_t quantize_group(float2 (&r)[8], Put&& put) {
+    float up = 1.0f / 6.0f, down = 1.329227995784916e36f;   // 2^120
+    uint32_t word = 0u;
+#pragma unroll 1
     for (uint32_t term = 0; term < 4u; ++term) {
         float m = 0.0f;
 #pragma unroll
         for (int k = 0; k < 8; ++k) m = fmaxf(m, fmaxf(fabsf(r[k].x), fabsf(r[k].y)));
-        uint32_t s = (uint32_t)__nv_cvt_float_to_fp8(m * (up * (1.0f / 6.0f)), __NV_SATFINITE, __NV_E4M3);
+        uint32_t s = (uint32_t)__nv_cvt_float_to_fp8(m * up, __NV_SATFINITE, __NV_E4M3);
         if (s == 0u) s = 1u;
         // an e4m3 byte's exponent and mantissa are an f32's, 120 binades lower
-        const float sc = __uint_as_float(s << 20) * (1.329227995784916e36f * down);
+        const float sc = __uint_as_float(s << 20) * down;
         const float inv = rcp_approx(sc);
         uint32_t w[2] = {0u, 0u};
 #pragma unroll
@@ -152,11 +155,12 @@ __device__ __forceinline__ void quantize_group(float2 (&r)[8], uint2 (&codes)[4]
             w[k >> 2] |= byte << (8 * (k & 3));
             if (term < 3u) r[k] = fma2(e2m1x2_value(byte), -sc, r[k]);
         }
-        codes[term] = make_uint2(w[0], w[1]);
-        sb[term] = m > 0.0f ? s : 0u;
+        put(term, make_uint2(w[0], w[1]));
+        word |= (m > 0.0f ? s : 0u) << (8u * term);
         up *= 16.0f;
         down *= 0.0625f;
     }
+    return word;
 }
 
 struct PrepArgs {
@@ -199,9 +203,8 @@ __device__ __forceinline__ void record_place(uint32_t pos, uint32_t bm, Same sam
 }
 
 // Four lanes' scale bytes of the four terms, transposed: lane j of the four gets term j's, groups in byte order.
-__device__ __forceinline__ uint32_t scale_word(const uint32_t (&sb)[4]) {
+__device__ __forceinline__ uint32_t scale_word(uint32_t v) {
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t v = sb[0] | sb[1] << 8 | sb[2] << 16 | sb[3] << 24;
     const uint32_t a = __shfl_xor_sync(0xffffffffu, v, 1);
     v = lane & 1u ? __byte_perm(v, a, 0x3715) : __byte_perm(v, a, 0x6240);   // even lane: terms 0 and 2 of both, odd: 1 and 3
     const uint32_t b = __shfl_xor_sync(0xffffffffu, v, 2);
@@ -286,8 +289,10 @@ __device__ __forceinline__ void prep_position(const PrepArgs& a, uint32_t pos, u
         // scale byte of group g and term row r: record slab g/16, cell (g/4)%4, byte r*16 + col*4 + g%4
         // (four threads write their groups' bytes of a term as one word)
         uint8_t* xs_g = xs_row + (size_t)(g >> 4) * 2048u + ((g >> 2) & 3u) * 512u;
-        uint2 codes[4] = {};
-        uint32_t sb[4] = {};
+        uint32_t sb = 0u;
+        auto put = [&](uint32_t term, uint2 codes) {
+            *reinterpret_cast<uint2*>(xq_rows + (size_t)(term * 8u) * kh + (size_t)g * 8u) = codes;
+        };
         // padding and all-zero rows: zero term rows and scale bytes, none of the term arithmetic; the record's cells
         // past K must read as zero too
         if (live && g < groups) {
@@ -304,21 +309,18 @@ __device__ __forceinline__ void prep_position(const PrepArgs& a, uint32_t pos, u
                 r[k] = mul2(!a.natural ? make_float2(lo0[k], hi0[k])
                             : k < 4    ? make_float2(lo0[2 * (k & 3)], lo0[2 * (k & 3) + 1])
                                        : make_float2(hi0[2 * (k & 3)], hi0[2 * (k & 3) + 1]), inv_step);
-            quantize_group(r, codes, sb);
+            sb = quantize_group(r, put);
+        } else if (g < groups) {
+#pragma unroll 1
+            for (uint32_t term = 0; term < 4u; ++term) put(term, make_uint2(0u, 0u));
         }
-        if (g < groups)
-#pragma unroll
-            for (uint32_t term = 0; term < 4u; ++term)
-                *reinterpret_cast<uint2*>(xq_rows + (size_t)(term * 8u) * kh + (size_t)g * 8u) = codes[term];
         const uint32_t word = scale_word(sb);
         if (g < num_kb * 16u) *reinterpret_cast<uint32_t*>(xs_g + (g & 3u) * 128u) = word;
     }
 }
 
 __global__ void __launch_bounds__(256) moe_prep_f4_kernel(const PrepArgs a) {
-    // dependent launch: may start while the previous kernel of the stream drains; its results are awaited here
-    pdk_pdl_launch_dependents();
-    pdk_pdl_wait();
+    pdk_pdl_wait_then_launch();   // dependent launch: may start while the previous kernel of the stream drains
     const uint32_t pos = blockIdx.x, b = pos / a.bm;
     uint32_t src, rec, col;
     if (a.mode == 3u) {
@@ -343,7 +345,7 @@ __global__ void __launch_bounds__(256) moe_prep_f4_kernel(const PrepArgs a) {
 
 // One CTA per token: its row is quantized once and written to the positions of all its k pairs (pair_pos, moe_route.cu), where
 // a CTA per position read and quantized it k times.  Positions without a pair are left as they are: their columns of the
-// GEMM are never read.  (1024 tokens of 2880, 4 of 128 experts: 26.2 us -> XXX.)
+// GEMM are never read.  (1024 tokens of 2880, 4 of 128 experts: 26.2 -> 12.4 us.)
 struct TokenArgs {
     const float* x;             // [rows][dim]
     const uint32_t* pair_pos;   // [rows][k]
@@ -354,8 +356,9 @@ struct TokenArgs {
 
 __global__ void __launch_bounds__(256) moe_prep_tokens_kernel(const TokenArgs a) {
     __shared__ float s_red[8];
-    pdk_pdl_launch_dependents();
-    pdk_pdl_wait();
+    __shared__ uint32_t s_pos[16];
+    pdk_pdl_wait_then_launch();
+    if (threadIdx.x < a.k) s_pos[threadIdx.x] = a.pair_pos[(size_t)blockIdx.x * a.k + threadIdx.x];
     const uint32_t tid = threadIdx.x, token = blockIdx.x, groups = a.dim >> 4, kh = a.dim >> 1, num_kb = (a.dim + 255u) >> 8;
     const float* row = a.x + (size_t)token * a.dim;
     auto load = [&](uint32_t g, float2 (&r)[8]) {   // in code order, as prep_position
@@ -390,25 +393,30 @@ __global__ void __launch_bounds__(256) moe_prep_tokens_kernel(const TokenArgs a)
     const bool single = num_kb * 16u <= blockDim.x;
     for (uint32_t base = 0; base < num_kb * 16u; base += blockDim.x) {   // whole warps: scale_word shuffles
         const uint32_t g = base + tid;
-        uint2 codes[4] = {};
-        uint32_t sb[4] = {};
+        uint32_t sb = 0u;
+        auto put = [&](uint32_t term, uint2 codes) {
+            for (uint32_t s = 0; s < a.k; ++s) {
+                const uint32_t at = s_pos[s];
+                if (at == PDK_MOE_PAD) continue;
+                const uint32_t pos = at & 0x3FFFFFFFu;
+                *reinterpret_cast<uint2*>(a.xq + ((size_t)(pos >> 3) * 32u + (pos & 7u) + term * 8u) * kh + (size_t)g * 8u) = codes;
+            }
+        };
         if (live && g < groups) {
             if (!single) load(g, r);
 #pragma unroll
             for (int k = 0; k < 8; ++k) r[k] = mul2(r[k], inv_step);
-            quantize_group(r, codes, sb);
+            sb = quantize_group(r, put);
+        } else if (g < groups) {
+#pragma unroll 1
+            for (uint32_t term = 0; term < 4u; ++term) put(term, make_uint2(0u, 0u));
         }
         const uint32_t word = scale_word(sb);
         if (g >= num_kb * 16u) continue;
         for (uint32_t s = 0; s < a.k; ++s) {
-            const uint32_t at = a.pair_pos[(size_t)token * a.k + s];
+            const uint32_t at = s_pos[s];
             if (at == PDK_MOE_PAD) continue;
             const uint32_t pos = at & 0x3FFFFFFFu, col = at >> 30, r0 = pos & 7u, b = pos / a.bm, rec = a.bm == 8u ? b - col : b;
-            uint8_t* xq_rows = a.xq + ((size_t)(pos >> 3) * 32u + r0) * kh + (size_t)g * 8u;
-            if (g < groups)
-#pragma unroll
-                for (uint32_t term = 0; term < 4u; ++term)
-                    *reinterpret_cast<uint2*>(xq_rows + (size_t)(term * 8u) * kh) = codes[term];
             *reinterpret_cast<uint32_t*>(a.xs + ((size_t)rec * num_kb + (g >> 4)) * 2048u + ((g >> 2) & 3u) * 512u + r0 * 16u +
                                          col * 4u + (g & 3u) * 128u) = word;
             if (g == 0u) a.xstep[pos] = step;
@@ -439,8 +447,7 @@ __global__ void __launch_bounds__(256) moe_route_prep_f4_kernel(const PrepArgs a
     __shared__ uint32_t s_idx[32];
     __shared__ float s_w[32];
     __shared__ uint32_t s_row[kRouteMaxPos], s_slot[kRouteMaxPos], s_bexp[32];
-    pdk_pdl_launch_dependents();
-    pdk_pdl_wait();
+    pdk_pdl_wait_then_launch();
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
     const uint32_t npairs = r.rows * r.k, n_pos = r.max_blocks * a.bm;
     if (warp < r.rows) moe_route::topk_warp(r.logits + (size_t)warp * r.n_expert, r.bias, r.n_expert, r.k, lane, s_idx + warp * r.k, s_w + warp * r.k);
@@ -543,7 +550,7 @@ PDK_EXPORT int pdk_moe_prep_act_f4(const void* x, const void* up, const void* so
 PDK_EXPORT int pdk_moe_prep_tokens_f4(const void* x, const void* pair_pos, void* xq, void* xs, void* xstep, uint32_t dim, uint32_t k,
                                       uint32_t rows, uint32_t bm, uint32_t natural, void* stream) {
     if (rows == 0 || k == 0) return 0;
-    if (dim == 0 || (dim & 31u) != 0u || (bm != 8u && bm != 32u) || natural > 1u) return cudaErrorInvalidValue;
+    if (dim == 0 || (dim & 31u) != 0u || (bm != 8u && bm != 32u) || natural > 1u || k > 16u) return cudaErrorInvalidValue;
     if (!pdk_aligned(x, 16) || !pdk_aligned(xq, 16) || !pdk_aligned(xs, 16)) return cudaErrorInvalidValue;
     const TokenArgs a{(const float*)x, (const uint32_t*)pair_pos, (uint8_t*)xq, (uint8_t*)xs, (float*)xstep, dim, k, bm, natural};
     const uint32_t per_row = ((dim + 255u) >> 8) * 16u;

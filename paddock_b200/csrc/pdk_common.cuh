@@ -52,6 +52,14 @@ __device__ __forceinline__ void pdk_pdl_launch_dependents() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 __device__ __forceinline__ void pdk_pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// The order for chains of several short kernels: the next one's CTAs come in when this one may run, not when it is resident.
+// Released before the wait, each kernel of a chain releases the one behind it, and CTAs of launches far ahead sit on the SMs
+// that the next ones need (a mixture-of-experts block of seven launches, 12 tokens on 32 experts of 2880 x 2880: 70.0 us, in this
+// order 62.9, without dependent launches 66.8).
+__device__ __forceinline__ void pdk_pdl_wait_then_launch() {
+    pdk_pdl_wait();
+    pdk_pdl_launch_dependents();
+}
 
 __device__ __forceinline__ float pdk_warp_sum(float v) {
 #pragma unroll
