@@ -26,7 +26,7 @@ struct Args {
     const uint32_t* sorted_row;
     const uint32_t* sorted_slot;  // scatter only
     const float* topk_w;          // scatter only
-    uint32_t in_dim, out_dim, max_blocks, n_planes, n_active, scatter, scale2_per_expert, block_shift;  // 2: 32-token blocks, 0: 8
+    uint32_t in_dim, out_dim, max_blocks, n_planes, n_active, scatter, ahead, scale2_per_expert, block_shift;  // 2: 32-token blocks, 0: 8
     float alpha, limit, up_add;   // gated only
     unsigned int* err_word;
 };
@@ -285,6 +285,7 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
             for (int i = 0; i < 64; ++i) __nanosleep(1000);
     } else if (warp == 2) {
         // ------------------------------------------------------------ activations (whole warp, one lane issues)
+        if (a.ahead) pdk_pdl_wait_then_launch();
         uint32_t stage = 0, phase = 0;
         bool ok = true;
         for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
@@ -361,6 +362,7 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
         // ------------------------------------------------------------ epilogue (one group at a time: the loop stays small)
         constexpr uint32_t kShare = EPI / 4u;
         const uint32_t quarter = warp & 3u, share = (warp - 3u) >> 2;
+        if (a.ahead) pdk_pdl_wait();
         uint32_t iter = 0;
         bool ok = true;
         for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
@@ -470,9 +472,10 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constan
         tc5::tmem_alloc(&sh->tmem_base, kTmemCols);
         tc5::tmem_relinquish();
     }
-    // dependent launch: barriers and tensor memory are set up while the previous kernel drains;
-    // everything below reads what it wrote
-    pdk_pdl_wait_then_launch();
+    // dependent launch: barriers and tensor memory are set up while the previous kernel drains.  ahead: the routing tables are
+    // older than the kernel in front, so the tiles are laid out and the first weights requested under that kernel as well; only
+    // what reads its rows, or writes where it may still read, waits for it.
+    if (!a.ahead) pdk_pdl_wait_then_launch();
     uint32_t n, widest;
     if (a.max_blocks <= 32u) {
         s_tile = s_expert + 64u * warp;

@@ -443,48 +443,66 @@ struct RouteArgs {
 };
 constexpr uint32_t kRouteMaxPos = 32u * 32u;
 
-__global__ void __launch_bounds__(256) moe_route_prep_f4_kernel(const PrepArgs a, const RouteArgs r) {
-    __shared__ uint32_t s_idx[32];
-    __shared__ float s_w[32];
-    __shared__ uint32_t s_row[kRouteMaxPos], s_slot[kRouteMaxPos], s_bexp[32];
-    pdk_pdl_wait_then_launch();
+// The tables of the few tokens, in shared memory (256 threads).
+struct RouteTables {
+    uint32_t idx[32], row[kRouteMaxPos], slot[kRouteMaxPos], bexp[32], pos[32];   // pos: pair -> position
+    float w[32];
+};
+__device__ __forceinline__ void route_few(const RouteArgs& r, uint32_t bm, RouteTables& s) {
     const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-    const uint32_t npairs = r.rows * r.k, n_pos = r.max_blocks * a.bm;
-    if (warp < r.rows) moe_route::topk_warp(r.logits + (size_t)warp * r.n_expert, r.bias, r.n_expert, r.k, lane, s_idx + warp * r.k, s_w + warp * r.k);
-    for (uint32_t p = tid; p < n_pos; p += blockDim.x) { s_row[p] = PDK_MOE_PAD; s_slot[p] = 0u; }
-    if (tid < 32u) s_bexp[tid] = PDK_MOE_PAD;
+    const uint32_t npairs = r.rows * r.k, n_pos = r.max_blocks * bm;
+    if (warp < r.rows) moe_route::topk_warp(r.logits + (size_t)warp * r.n_expert, r.bias, r.n_expert, r.k, lane, s.idx + warp * r.k, s.w + warp * r.k);
+    for (uint32_t p = tid; p < n_pos; p += blockDim.x) { s.row[p] = PDK_MOE_PAD; s.slot[p] = 0u; }
+    if (tid < 32u) { s.bexp[tid] = PDK_MOE_PAD; s.pos[tid] = PDK_MOE_PAD; }
     __syncthreads();
     if (warp == 0u) {
         const bool valid = lane < npairs;
-        const uint32_t e = valid ? s_idx[lane] : 0x80000000u + lane;     // idle lanes: distinct keys that match nobody
+        const uint32_t e = valid ? s.idx[lane] : 0x80000000u + lane;     // idle lanes: distinct keys that match nobody
         const uint32_t grp = __match_any_sync(0xffffffffu, e);
         const uint32_t rank = __popc(grp & ((1u << lane) - 1u)), cnt = __popc(grp);
-        const uint32_t nblk = (valid && rank == 0u) ? (cnt + a.bm - 1u) / a.bm : 0u;   // counted once, by the group's first lane
+        const uint32_t nblk = (valid && rank == 0u) ? (cnt + bm - 1u) / bm : 0u;   // counted once, by the group's first lane
         uint32_t first = 0u;
         for (uint32_t q = 0; q < 32u; ++q) {
             const uint32_t eq = __shfl_sync(0xffffffffu, e, q), nq = __shfl_sync(0xffffffffu, nblk, q);
             if (eq < e) first += nq;
         }
         if (valid) {
-            const uint32_t blk = first + rank / a.bm, at = blk * a.bm + rank % a.bm;
+            const uint32_t blk = first + rank / bm, at = blk * bm + rank % bm;
             if (blk < r.max_blocks) {
-                s_row[at] = lane / r.k;
-                s_slot[at] = lane % r.k;
-                if (rank % a.bm == 0u) s_bexp[blk] = e;
+                s.row[at] = lane / r.k;
+                s.slot[at] = lane % r.k;
+                s.pos[lane] = at | ((bm == 8u ? rank >> 3 : at >> 3) & 3u) << 30;
+                if (rank % bm == 0u) s.bexp[blk] = e;
             }
         }
     }
     __syncthreads();
-    if (blockIdx.x == 0u) {
-        if (tid < npairs) { r.idx[tid] = s_idx[tid]; r.w[tid] = s_w[tid]; }
-        for (uint32_t p = tid; p < n_pos; p += blockDim.x) { r.sorted_row[p] = s_row[p]; r.sorted_slot[p] = s_slot[p]; }
-        if (tid < r.max_blocks) r.block_expert[tid] = s_bexp[tid];
-    }
-    const uint32_t pos = blockIdx.x, b = pos / a.bm, e = s_bexp[b], src = s_row[pos];
+}
+__device__ __forceinline__ void route_store(const RouteArgs& r, uint32_t bm, const RouteTables& s) {
+    const uint32_t tid = threadIdx.x, npairs = r.rows * r.k;
+    if (tid < npairs) { r.idx[tid] = s.idx[tid]; r.w[tid] = s.w[tid]; }
+    for (uint32_t p = tid; p < r.max_blocks * bm; p += blockDim.x) { r.sorted_row[p] = s.row[p]; r.sorted_slot[p] = s.slot[p]; }
+    if (tid < r.max_blocks) r.block_expert[tid] = s.bexp[tid];
+}
+
+__global__ void __launch_bounds__(256) moe_route_few_kernel(const RouteArgs r, uint32_t* __restrict__ pair_pos, uint32_t bm) {
+    __shared__ RouteTables s;
+    pdk_pdl_wait_then_launch();
+    route_few(r, bm, s);
+    route_store(r, bm, s);
+    if (threadIdx.x < r.rows * r.k) pair_pos[threadIdx.x] = s.pos[threadIdx.x];
+}
+
+__global__ void __launch_bounds__(256) moe_route_prep_f4_kernel(const PrepArgs a, const RouteArgs r) {
+    __shared__ RouteTables s;
+    pdk_pdl_wait_then_launch();
+    route_few(r, a.bm, s);
+    if (blockIdx.x == 0u) route_store(r, a.bm, s);
+    const uint32_t pos = blockIdx.x, b = pos / a.bm, e = s.bexp[b], src = s.row[pos];
     if (e == PDK_MOE_PAD) return;   // an unused block
-    if (src == PDK_MOE_PAD && s_row[pos & ~7u] == PDK_MOE_PAD) return;
+    if (src == PDK_MOE_PAD && s.row[pos & ~7u] == PDK_MOE_PAD) return;
     uint32_t rec, col;
-    record_place(pos, a.bm, [&](uint32_t q) { return s_bexp[q] == e; }, rec, col);
+    record_place(pos, a.bm, [&](uint32_t q) { return s.bexp[q] == e; }, rec, col);
     prep_position(a, pos, src, rec, col);
 }
 
@@ -581,6 +599,23 @@ static int route_prep_impl(const void* logits, const void* router_bias, const vo
     return pdk_launch_pdl(moe_route_prep_f4_kernel, dim3(max_blocks * bm), dim3(256), 0, (cudaStream_t)stream, a, r);
 }
 
+// moe_topk_batch + pdk_moe_align_pos in one small launch, with pdk_moe_route_prep_f4's limits.  Unlike that call it leaves the
+// preparation to pdk_moe_prep_tokens_f4, under which the expert GEMM behind it requests its weights already.
+PDK_EXPORT int pdk_moe_route_few(const void* logits, const void* router_bias, void* idx, void* w, void* sorted_row, void* sorted_slot,
+                                 void* block_expert, void* pair_pos, uint32_t n_expert, uint32_t k, uint32_t rows, uint32_t bm,
+                                 uint32_t max_blocks, void* stream) {
+    if (rows == 0 || max_blocks == 0) return 0;
+    if (rows > 8u || k == 0 || k > 16u || rows * k > 32u || n_expert == 0 || n_expert > 512u || k > n_expert ||
+        max_blocks > 32u || (bm != 8u && bm != 32u) || max_blocks * bm > kRouteMaxPos)
+        return cudaErrorInvalidValue;
+    RouteArgs r{};
+    r.logits = (const float*)logits; r.bias = (const float*)router_bias;
+    r.idx = (uint32_t*)idx; r.w = (float*)w;
+    r.sorted_row = (uint32_t*)sorted_row; r.sorted_slot = (uint32_t*)sorted_slot; r.block_expert = (uint32_t*)block_expert;
+    r.rows = rows; r.k = k; r.n_expert = n_expert; r.max_blocks = max_blocks;
+    return pdk_launch_pdl(moe_route_few_kernel, dim3(1), dim3(256), 0, (cudaStream_t)stream, r, (uint32_t*)pair_pos, bm);
+}
+
 PDK_EXPORT int pdk_moe_route_prep_f4(const void* logits, const void* router_bias, const void* x, void* idx, void* w,
                                      void* sorted_row, void* sorted_slot, void* block_expert, void* xq, void* xs, void* xstep,
                                      uint32_t n_expert, uint32_t k, uint32_t rows, uint32_t dim, uint32_t bm,
@@ -630,6 +665,7 @@ namespace {
 struct PlaneArgs { const void *data, *sf, *bias; const float* scale2; };
 struct RowArgs { const void *xq, *xs, *xstep, *block_expert, *sorted_row, *sorted_slot, *topk_w; };
 struct UnitArgs { float alpha, limit, up_add; };
+constexpr uint32_t kAhead = 0x10000u;   // beside a kind: moe_gemm::Args::ahead
 }  // namespace
 
 static int gemm_impl(const PlaneArgs& w0, const PlaneArgs& w1, void* out0, void* out1, const RowArgs& r, uint32_t in_dim,
@@ -641,6 +677,8 @@ static int gemm_impl(const PlaneArgs& w0, const PlaneArgs& w1, void* out0, void*
     if (!pdk_aligned(w0.data, 16) || !pdk_aligned(w0.sf, 16) || !pdk_aligned(r.xq, 16) || !pdk_aligned(r.xs, 4) ||
         !pdk_aligned(w0.scale2, 4) || (w1.data && (!pdk_aligned(w1.data, 16) || !pdk_aligned(w1.sf, 16))))
         return cudaErrorInvalidValue;
+    const uint32_t ahead = kind & kAhead ? 1u : 0u;
+    kind &= ~kAhead;
     if (kind == moe_gemm::kScatter && (w1.data || !r.sorted_slot || !r.topk_w)) return cudaErrorInvalidValue;
     if (kind == moe_gemm::kGated && !w1.data) return cudaErrorInvalidValue;
     const PlaneArgs& wb = w1.data ? w1 : w0;
@@ -662,7 +700,7 @@ static int gemm_impl(const PlaneArgs& w0, const PlaneArgs& w1, void* out0, void*
     a.block_expert = (const uint32_t*)r.block_expert; a.sorted_row = (const uint32_t*)r.sorted_row;
     a.sorted_slot = (const uint32_t*)r.sorted_slot; a.topk_w = (const float*)r.topk_w;
     a.in_dim = in_dim; a.out_dim = out_dim; a.max_blocks = max_blocks; a.n_planes = w1.data ? 2u : 1u;
-    a.n_active = n_active; a.scatter = kind == moe_gemm::kScatter; a.block_shift = bm == 32u ? 2u : 0u;
+    a.n_active = n_active; a.scatter = kind == moe_gemm::kScatter; a.ahead = ahead; a.block_shift = bm == 32u ? 2u : 0u;
     a.alpha = unit.alpha; a.limit = unit.limit; a.up_add = unit.up_add; a.err_word = pdk_error_word();
     auto st = (cudaStream_t)stream;
     // The gated unit needs gate and up in one CTA.  Tiles of up to six groups where blocks are large (1024 tokens, 4 of 128 experts,
@@ -686,8 +724,26 @@ PDK_EXPORT int pdk_mxfp4_moe_gemm_tc5(const void* w0_data, const void* w0_sf, co
                      n_active, scatter ? moe_gemm::kScatter : moe_gemm::kPlain, 0u, {}, stream);
 }
 
+// The same where block_expert, sorted_row and sorted_slot were written before the launch in front of this one in the stream began (as
+// they are behind pdk_moe_prep_*: the preparations release the next launch only when everything before them is complete): the
+// tiles are laid out and the first weights requested while that launch runs.
+PDK_EXPORT int pdk_mxfp4_moe_gemm_tc5_ahead(const void* w0_data, const void* w0_sf, const void* w0_meta, const void* w0_bias,
+                                      void* out0, const void* w1_data, const void* w1_sf, const void* w1_meta,
+                                      const void* w1_bias, void* out1, const void* xq, const void* xs,
+                                      const void* xstep, const void* block_expert, const void* sorted_row,
+                                      const void* sorted_slot, const void* topk_w, uint32_t in_dim, uint32_t out_dim,
+                                      uint32_t n_expert, uint32_t bm, uint32_t max_blocks, uint32_t n_active,
+                                      uint32_t scatter, void* stream) {
+    if (!pdk_aligned(w0_meta, 8) || w0_meta == nullptr || (w1_data && w1_meta == nullptr)) return cudaErrorInvalidValue;
+    return gemm_impl({w0_data, w0_sf, w0_bias, (const float*)w0_meta + 1},
+                     {w1_data, w1_sf, w1_bias, w1_meta ? (const float*)w1_meta + 1 : nullptr}, out0, out1,
+                     {xq, xs, xstep, block_expert, sorted_row, sorted_slot, topk_w}, in_dim, out_dim, n_expert, bm, max_blocks,
+                     n_active, (scatter ? moe_gemm::kScatter : moe_gemm::kPlain) | kAhead, 0u, {}, stream);
+}
+
 // Gate, up and the gated unit (pdk_moe_prep_act_f4n has its formula) in one launch: h f32 [max_blocks*bm][out_dim] in block
-// order, rows of padding left alone.  The raw gate and up rows are never written: at 1024 tokens, 4 experts each, 2880 wide
+// order, rows of padding left alone.  The tables are older than the launch in front
+// (pdk_mxfp4_moe_gemm_tc5_ahead).  The raw gate and up rows are never written: at 1024 tokens, 4 experts each, 2880 wide
 // they were 94 MB out and 94 MB back in.
 PDK_EXPORT int pdk_mxfp4_moe_gate_up_tc5(const void* gate_data, const void* gate_sf, const void* gate_meta, const void* gate_bias,
                                          const void* up_data, const void* up_sf, const void* up_meta, const void* up_bias, void* h,
@@ -697,7 +753,7 @@ PDK_EXPORT int pdk_mxfp4_moe_gate_up_tc5(const void* gate_data, const void* gate
     if (!pdk_aligned(gate_meta, 8) || !gate_meta || !up_meta || !up_data) return cudaErrorInvalidValue;
     return gemm_impl({gate_data, gate_sf, gate_bias, (const float*)gate_meta + 1}, {up_data, up_sf, up_bias, (const float*)up_meta + 1},
                      h, nullptr, {xq, xs, xstep, block_expert, sorted_row, nullptr, nullptr}, in_dim, out_dim, n_expert, bm, max_blocks,
-                     1u, moe_gemm::kGated, 0u, {alpha, limit, up_add}, stream);
+                     1u, moe_gemm::kGated | kAhead, 0u, {alpha, limit, up_add}, stream);
 }
 
 // ---- NVFP4 expert planes (crates/paddock-engine/src/gpu/types.rs:176-226: data [expert*rows][in/2],
@@ -733,6 +789,19 @@ PDK_EXPORT int pdk_nvf4_moe_gemm_tc5(const void* w0_data, const void* w0_sf, con
                      n_active, scatter ? moe_gemm::kScatter : moe_gemm::kPlain, 1u, {}, stream);
 }
 
+PDK_EXPORT int pdk_nvf4_moe_gemm_tc5_ahead(const void* w0_data, const void* w0_sf, const void* w0_scale2, const void* w0_bias,
+                                     void* out0, const void* w1_data, const void* w1_sf, const void* w1_scale2,
+                                     const void* w1_bias, void* out1, const void* xq, const void* xs, const void* xstep,
+                                     const void* block_expert, const void* sorted_row, const void* sorted_slot,
+                                     const void* topk_w, uint32_t in_dim, uint32_t out_dim, uint32_t n_expert,
+                                     uint32_t bm, uint32_t max_blocks, uint32_t n_active, uint32_t scatter,
+                                     void* stream) {
+    if (w0_scale2 == nullptr || (w1_data && w1_scale2 == nullptr)) return cudaErrorInvalidValue;
+    return gemm_impl({w0_data, w0_sf, w0_bias, (const float*)w0_scale2}, {w1_data, w1_sf, w1_bias, (const float*)w1_scale2}, out0,
+                     out1, {xq, xs, xstep, block_expert, sorted_row, sorted_slot, topk_w}, in_dim, out_dim, n_expert, bm, max_blocks,
+                     n_active, (scatter ? moe_gemm::kScatter : moe_gemm::kPlain) | kAhead, 1u, {}, stream);
+}
+
 PDK_EXPORT int pdk_nvf4_moe_gate_up_tc5(const void* gate_data, const void* gate_sf, const void* gate_scale2, const void* gate_bias,
                                         const void* up_data, const void* up_sf, const void* up_scale2, const void* up_bias, void* h,
                                         const void* xq, const void* xs, const void* xstep, const void* block_expert,
@@ -741,7 +810,7 @@ PDK_EXPORT int pdk_nvf4_moe_gate_up_tc5(const void* gate_data, const void* gate_
     if (!gate_scale2 || !up_scale2 || !up_data) return cudaErrorInvalidValue;
     return gemm_impl({gate_data, gate_sf, gate_bias, (const float*)gate_scale2}, {up_data, up_sf, up_bias, (const float*)up_scale2}, h,
                      nullptr, {xq, xs, xstep, block_expert, sorted_row, nullptr, nullptr}, in_dim, out_dim, n_expert, bm, max_blocks, 1u,
-                     moe_gemm::kGated, 1u, {alpha, limit, up_add}, stream);
+                     moe_gemm::kGated | kAhead, 1u, {alpha, limit, up_add}, stream);
 }
 
 // ---------------------------------------------------------------- W4A16 decode GEMV on the same kernels

@@ -134,12 +134,14 @@ def repack_mxfp4(ex, raw_dev):
     return RepackedMxfp4(data, scale)
 
 
-def _unit_in_gemm(bm, max_blocks):
+def _unit_in_gemm(ws, max_blocks, ff):
     """Whether the gate|up GEMM applies the gated unit itself.  It then keeps both accumulators in one CTA and writes one plane
-    instead of two: with 32-token blocks that saves 94 MB each way at 1024 tokens (gate|up + second preparation 313 -> 250 us),
-    and with a few blocks a launch's end (one token 16.2 -> 13.9 us); in between two accumulators per tile overlap
-    better and the raw planes stay in L2 (60 tokens: 172 against 174 us; 128 tokens on 32 experts of 1024 x 768: 20 against 23)."""
-    return bm == 32
+    instead of two: with 32-token blocks that saves 94 MB each way at 1024 tokens (gate|up + second preparation 313 -> 250 us).
+    With 8-token blocks two accumulators per tile overlap better and the raw planes stay in L2 (60 tokens: 172 against 174 us; 128
+    tokens on 32 experts of 1024 x 768: 20 against 23), but where tiles of one plane would just need a second round over the SMs
+    (one token of 4 experts of 2880 x 2880: 31.9 us a block against 30.3)."""
+    tiles = max_blocks * ((ff + 127) // 128)
+    return ws.bm == 32 or tiles <= ws.sms < 2 * tiles
 
 
 class MoeWorkspace:
@@ -150,6 +152,7 @@ class MoeWorkspace:
         pairs = tokens * n_active
         self.bm, self.tokens, self.n_active = bm, tokens, n_active
         self.max_blocks = min(pairs, pairs // bm + planes.n_expert)
+        self.sms = torch.cuda.get_device_properties(dev).multi_processor_count if torch.device(dev).type == "cuda" else 148
         nb = self.max_blocks * bm
         self.idx = torch.empty(pairs, dtype=u32, device=dev)
         self.w = torch.empty(pairs, dtype=f32, device=dev)
@@ -200,6 +203,13 @@ def _route_and_prepare(ex, ws, x, rows, embd, n_expert, max_blocks, natural, log
     st = _stream()
     c = ex.pack.call
     k, bm = ws.n_active, ws.bm
+    tokens = x, ws.pair_pos, ws.x4q, ws.x4s, ws.x4step, embd, k, rows, bm, int(natural)
+    if logits is not None and rows <= 8 and rows * k <= 32 and n_expert <= 512 and max_blocks <= 32:
+        # decode widths: top-k and alignment in one launch
+        c("pdk_moe_route_few", logits, router_bias, ws.idx, ws.w, ws.sorted_row, ws.sorted_slot, ws.block_expert, ws.pair_pos,
+          n_expert, k, rows, bm, max_blocks, stream=st)
+        c("pdk_moe_prep_tokens_f4", *tokens, stream=st)
+        return 2
     n = 2
     if logits is not None:
         c("moe_topk_batch", logits, router_bias, n_expert, k, ws.idx, ws.w, rows, stream=st)
@@ -211,27 +221,21 @@ def _route_and_prepare(ex, ws, x, rows, embd, n_expert, max_blocks, natural, log
         return n
     c("pdk_moe_align_pos", ws.idx, ws.sorted_row, ws.sorted_slot, ws.block_expert, ws.pair_pos, rows, k, n_expert, bm, max_blocks,
       stream=st)
-    c("pdk_moe_prep_tokens_f4", x, ws.pair_pos, ws.x4q, ws.x4s, ws.x4step, embd, k, rows, bm, int(natural), stream=st)
+    c("pdk_moe_prep_tokens_f4", *tokens, stream=st)
     return n
 
 
-def moe_mxfp4_experts_tc5(ex, planes, ws, x, rows, alpha=1.702, limit=7.0, route=None, routed=False):
+def moe_mxfp4_experts_tc5(ex, planes, ws, x, rows, alpha=1.702, limit=7.0, route=None):
     """moe_mxfp4_experts on the block-scaled tensor-core path (planes prepared with prepare_tc5):
     align -> term rows of x -> gate and up GEMM -> SwiGLU + term rows of h -> down GEMM scattered
-    into ws.part.  Five launches; with route = (router_logits, router_bias) at decode widths the
-    top-k, the alignment and the first preparation are one launch (four in all); routed: they are
-    done already (_route_and_prepare), three launches."""
+    into ws.part.  Five launches; route = (router_logits, router_bias) has the experts chosen here too."""
     st = _stream()
     c = ex.pack.call
     k, bm, t = ws.n_active, ws.bm, planes.tc5
     max_blocks = min(ws.max_blocks, min(rows * k, rows * k // bm + planes.n_expert))
-    if route is not None:
-        c("pdk_moe_route_prep_f4", route[0], route[1], x, ws.idx, ws.w, ws.sorted_row, ws.sorted_slot, ws.block_expert,
-          ws.x4q, ws.x4s, ws.x4step, planes.n_expert, k, rows, planes.embd, bm, max_blocks, stream=st)
-    elif not routed:
-        _route_and_prepare(ex, ws, x, rows, planes.embd, planes.n_expert, max_blocks, False)
-    if not _unit_in_gemm(bm, max_blocks):
-        c("pdk_mxfp4_moe_gemm_tc5", planes.gate.data, t["gate"][0], t["gate"][1], planes.gate_bias, ws.g_raw,
+    n = _route_and_prepare(ex, ws, x, rows, planes.embd, planes.n_expert, max_blocks, False, *(route or ()))
+    if not _unit_in_gemm(ws, max_blocks, planes.ff):
+        c("pdk_mxfp4_moe_gemm_tc5_ahead", planes.gate.data, t["gate"][0], t["gate"][1], planes.gate_bias, ws.g_raw,
           planes.up.data, t["up"][0], t["up"][1], planes.up_bias, ws.u_raw, ws.x4q, ws.x4s, ws.x4step,
           ws.block_expert, ws.sorted_row, None, None, planes.embd, planes.ff, planes.n_expert, bm, max_blocks, k, 0,
           stream=st)
@@ -243,10 +247,10 @@ def moe_mxfp4_experts_tc5(ex, planes, ws, x, rows, alpha=1.702, limit=7.0, route
           ws.sorted_row, planes.embd, planes.ff, planes.n_expert, bm, max_blocks, alpha, limit, 1.0, stream=st)
         c("pdk_moe_prep_rows_f4", ws.h, ws.sorted_row, ws.block_expert, ws.h4q, ws.h4s, ws.h4step, planes.ff, bm,
           max_blocks, 0, stream=st)
-    c("pdk_mxfp4_moe_gemm_tc5", planes.down.data, t["down"][0], t["down"][1], planes.down_bias, ws.part,
+    c("pdk_mxfp4_moe_gemm_tc5_ahead", planes.down.data, t["down"][0], t["down"][1], planes.down_bias, ws.part,
       None, None, None, None, None, ws.h4q, ws.h4s, ws.h4step, ws.block_expert, ws.sorted_row, ws.sorted_slot,
       ws.w, planes.ff, planes.embd, planes.n_expert, bm, max_blocks, k, 1, stream=st)
-    return 5
+    return n + 3
 
 
 def moe_mxfp4_forward(ex, planes, ws, x, router_logits, out, alpha=1.702, limit=7.0, router_bias=None):
@@ -256,16 +260,10 @@ def moe_mxfp4_forward(ex, planes, ws, x, router_logits, out, alpha=1.702, limit=
     st = _stream()
     c = ex.pack.call
     T, k = ws.tokens, ws.n_active
-    if planes.tc5 is not None and T <= 8 and T * k <= 32 and planes.n_expert <= 512 and ws.max_blocks <= 32:
-        # decode widths: routing, alignment and the first activation preparation in one launch
-        moe_mxfp4_experts_tc5(ex, planes, ws, x, T, alpha, limit, route=(router_logits, router_bias))
-        c("moe_slot_combine", ws.part, out, planes.embd, k, T, stream=st)
-        return 5
     if planes.tc5 is not None:
-        n = _route_and_prepare(ex, ws, x, T, planes.embd, planes.n_expert, ws.max_blocks, False, router_logits, router_bias)
-        moe_mxfp4_experts_tc5(ex, planes, ws, x, T, alpha, limit, routed=True)
+        n = moe_mxfp4_experts_tc5(ex, planes, ws, x, T, alpha, limit, route=(router_logits, router_bias))
         c("moe_slot_combine", ws.part, out, planes.embd, k, T, stream=st)
-        return n + 4  # launches
+        return n + 1  # launches
     c("moe_topk_batch", router_logits, router_bias, planes.n_expert, k, ws.idx, ws.w, T, stream=st)
     moe_mxfp4_experts(ex, planes, ws, x, T, alpha, limit)
     c("moe_slot_combine", ws.part, out, planes.embd, k, T, stream=st)
@@ -305,33 +303,27 @@ def moe_nvf4_forward(ex, gate, up, down, ws, x, router_logits, out, gated=True, 
     T, k, bm = ws.tokens, ws.n_active, ws.bm
     n_expert, embd, ff = up.n_expert, up.in_dim, up.rows
     max_blocks = min(ws.max_blocks, min(T * k, T * k // bm + n_expert))
-    fused = T <= 8 and T * k <= 32 and n_expert <= 512 and max_blocks <= 32
-    if fused:      # decode widths: routing, alignment and the first activation preparation in one launch
-        c("pdk_moe_route_prep_f4n", router_logits, router_bias, x, ws.idx, ws.w, ws.sorted_row, ws.sorted_slot, ws.block_expert,
-          ws.x4q, ws.x4s, ws.x4step, n_expert, k, T, embd, bm, max_blocks, stream=st)
-        n = 1
-    else:
-        n = _route_and_prepare(ex, ws, x, T, embd, n_expert, max_blocks, True, router_logits, router_bias)
-    if gated and _unit_in_gemm(bm, max_blocks):
+    n = _route_and_prepare(ex, ws, x, T, embd, n_expert, max_blocks, True, router_logits, router_bias)
+    if gated and _unit_in_gemm(ws, max_blocks, ff):
         c("pdk_nvf4_moe_gate_up_tc5", gate.data, gate.tiled, gate.scale2, None, up.data, up.tiled, up.scale2, None, ws.h,
           ws.x4q, ws.x4s, ws.x4step, ws.block_expert, ws.sorted_row, embd, ff, n_expert, bm, max_blocks, alpha, limit, up_add,
           stream=st)
         c("pdk_moe_prep_rows_f4", ws.h, ws.sorted_row, ws.block_expert, ws.h4q, ws.h4s, ws.h4step, ff, bm, max_blocks, 1,
           stream=st)
     elif gated:
-        c("pdk_nvf4_moe_gemm_tc5", gate.data, gate.tiled, gate.scale2, None, ws.g_raw, up.data, up.tiled, up.scale2, None,
+        c("pdk_nvf4_moe_gemm_tc5_ahead", gate.data, gate.tiled, gate.scale2, None, ws.g_raw, up.data, up.tiled, up.scale2, None,
           ws.u_raw, ws.x4q, ws.x4s, ws.x4step, ws.block_expert, ws.sorted_row, None, None, embd, ff, n_expert, bm,
           max_blocks, k, 0, stream=st)
         c("pdk_moe_prep_act_f4n", ws.g_raw, ws.u_raw, ws.sorted_row, ws.block_expert, ws.h4q, ws.h4s, ws.h4step, ff, bm,
           max_blocks, 1, alpha, limit, up_add, stream=st)
     else:
-        c("pdk_nvf4_moe_gemm_tc5", up.data, up.tiled, up.scale2, None, ws.u_raw, None, None, None, None, None, ws.x4q,
+        c("pdk_nvf4_moe_gemm_tc5_ahead", up.data, up.tiled, up.scale2, None, ws.u_raw, None, None, None, None, None, ws.x4q,
           ws.x4s, ws.x4step, ws.block_expert, ws.sorted_row, None, None, embd, ff, n_expert, bm, max_blocks, k, 0,
           stream=st)
         c("pdk_moe_prep_act_f4n", ws.u_raw, None, ws.sorted_row, ws.block_expert, ws.h4q, ws.h4s, ws.h4step, ff, bm,
           max_blocks, 2, alpha, limit, up_add, stream=st)
-    c("pdk_nvf4_moe_gemm_tc5", down.data, down.tiled, down.scale2, None, ws.part, None, None, None, None, None, ws.h4q,
+    c("pdk_nvf4_moe_gemm_tc5_ahead", down.data, down.tiled, down.scale2, None, ws.part, None, None, None, None, None, ws.h4q,
       ws.h4s, ws.h4step, ws.block_expert, ws.sorted_row, ws.sorted_slot, ws.w, ff, embd, n_expert, bm, max_blocks, k, 1,
       stream=st)
     c("moe_slot_combine", ws.part, out, embd, k, T, stream=st)
-    return n + 4
+    return n + 4  # launches

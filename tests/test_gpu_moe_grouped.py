@@ -68,6 +68,9 @@ def test_tiles_over_runs_of_blocks(pack, tokens, n_expert, k, embd, ff, bm, gate
     (300, 16, 4, 4352, 32, 1.0),      # a row of more groups than threads
     (700, 128, 8, 256, 32, 0.0),      # 5600 pairs: more chunks per warp than it holds in registers
     (1, 512, 16, 64, 8, 0.0),
+    (8, 128, 4, 2880, 8, 0.0),        # the widest pdk_moe_route_few takes
+    (8, 2, 2, 256, 8, 0.0),
+    (2, 512, 8, 256, 32, 0.0),
     (3000, 64, 1, 64, 32, 4.0),       # one token of 64 per expert at best, a thousand blocks; positions staged in shared memory
     (9000, 16, 8, 32, 8, 0.0),        # too many positions for that: written where they go
 ])
@@ -95,6 +98,16 @@ def test_positions_and_token_rows_equal_the_gathered_ones(pack, tokens, n_expert
     c(*(("pdk_moe_prep_act_f4n", *args, 0.0) if natural else ("pdk_moe_prep_act_f4", *args)))
     b["idx"], b["w"] = a["idx"], a["w"]
     c("pdk_moe_align_pos", b["idx"], b["row"], b["slot"], b["blk"], pos, tokens, k, n_expert, bm, max_blocks)
+    if tokens <= 8 and pairs <= 32 and max_blocks <= 32:
+        few = {n: torch.full_like(b[n], 3) for n in ("idx", "w", "row", "slot", "blk")}
+        few_pos = new(pairs, i32)
+        c("pdk_moe_route_few", logits, None, few["idx"], few["w"], few["row"], few["slot"], few["blk"], few_pos, n_expert, k, tokens,
+          bm, max_blocks)
+        used = (b["blk"] != -1).repeat_interleave(bm)
+        for n in few:
+            ta, tb = (few[n][used], b[n][used]) if n in ("row", "slot") else (few[n], b[n])
+            assert torch.equal(ta.view(u8), tb.view(u8)), n
+        assert torch.equal(few_pos, pos)
     c("pdk_moe_prep_tokens_f4", x, pos, b["q"], b["s"], b["step"], embd, k, tokens, bm, int(natural))
     torch.cuda.synchronize()
     assert pack.device_error() == 0
