@@ -115,7 +115,7 @@ __device__ __forceinline__ void build_tiles(const Args& a, const uint32_t* s_exp
 // The same for calls of up to 32 blocks: every warp for itself, from global memory straight into a table of its own, so
 // nothing waits for another warp (1.1 us of a call of one token's).
 template <uint32_t MAXG>
-__device__ __forceinline__ uint32_t build_tiles_warp(const Args& a, uint32_t* s_expert, uint32_t* s_tile, uint32_t& widest) {
+__device__ __forceinline__ uint32_t build_tiles_warp(const Args& a, uint32_t* s_expert, uint32_t* s_tile, uint32_t& widest, bool& once) {
     const uint32_t lane = threadIdx.x & 31u, shift = a.block_shift;
     const uint32_t e = lane < a.max_blocks ? a.block_expert[lane] : PDK_MOE_PAD;
     const bool used = e != PDK_MOE_PAD;
@@ -144,6 +144,7 @@ __device__ __forceinline__ uint32_t build_tiles_warp(const Args& a, uint32_t* s_
     s_expert[lane] = e;
     if (ng) s_tile[__popc(tiles & ((1u << lane) - 1u))] = (lane << shift) | (ng << 13);
     widest = __reduce_max_sync(0xffffffffu, ng);
+    once = __popc(tiles) == __popc(starts & __ballot_sync(0xffffffffu, used));
     __syncwarp();
     return __popc(tiles);
 }
@@ -196,6 +197,19 @@ __device__ __forceinline__ bool wait_for(uint64_t* bar, uint32_t parity, const t
     return tc5::mbar_try_wait(bar, parity) || wait_longer(bar, parity, ctx.abort_flag, ctx.err, code, detail);
 }
 
+__device__ __forceinline__ uint64_t l2_policy_normal() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(p));
+    return p;
+}
+__device__ __forceinline__ void bulk_load_hint_elect(void* smem_dst, const void* gmem, uint32_t bytes, uint64_t* bar, uint64_t policy) {
+    asm volatile(TC5_ELECT
+                 "@e cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;\n\t}" ::"r"(
+                     tc5::smem_u32(smem_dst)),
+                 "l"(gmem), "r"(bytes), "r"(tc5::smem_u32(bar)), "l"(policy)
+                 : "memory");
+}
+
 // What a tile index means: the groups, the weight plane (the first of two, where a tile has both) and the row tile.
 template <uint32_t NA>
 struct TileAt {
@@ -216,7 +230,7 @@ struct TileAt {
 // groups a block of one token took 38.2 us instead of 34.8, 512 tokens with 8 of 128 experts of 2048 x 768 180 instead of 166).
 template <uint32_t W, uint32_t NA, uint32_t KIND, uint32_t EPI, bool WG>
 __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensorMap& tmap_w1, const CUtensorMap& tmap_x, const Args& a,
-                                      uint8_t* rings, Ctl* sh, const uint32_t* s_expert, const uint32_t* s_tile, uint32_t tiles) {
+                                      uint8_t* rings, Ctl* sh, const uint32_t* s_expert, const uint32_t* s_tile, uint32_t tiles, bool once) {
     using G = Geo<W, NA>;
     constexpr uint32_t kBufs = NA == 2u ? 1u : 2u;
     const uint32_t warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31u;
@@ -229,6 +243,10 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
 
     if (warp == 0) {
         // ------------------------------------------------------------ weights (whole warp, one lane issues)
+        // Weights that a small call reads once leave L2 first, so the rows that the launches around this one hand on stay there (128
+        // experts of 2880 x 2880, 1 / 4 / 8 tokens: 27.3 / 54.5 / 84.3 -> 26.0 / 50.9 / 80.4 us a block).  In calls of most experts
+        // it is slower (60 tokens 273 -> 293: the rest of a 256-byte line that the next slab wants has left by then).
+        const uint64_t policy = once ? tc5::l2_policy_evict_first() : l2_policy_normal();
         uint32_t stage = 0, phase = 0;
         bool ok = true;
         for (uint32_t tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
@@ -250,12 +268,12 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
                 for (uint32_t u = 0; u < G::kS; ++u)
                     if (u < nsl) {
                         const int32_t x = (int32_t)((kb0 + u) * BKB);
-                        tc5::tma_load_2d_elect(st + u * kABytes, tw, full, x, row);
-                        if (NA == 2u) tc5::tma_load_2d_elect(st + (G::kS + u) * kABytes, &tmap_w1, full, x, row);
+                        tc5::tma_load_2d_hint_elect(st + u * kABytes, tw, full, x, row, policy);
+                        if (NA == 2u) tc5::tma_load_2d_hint_elect(st + (G::kS + u) * kABytes, &tmap_w1, full, x, row, policy);
                     }
                 if (!WG) {
-                    tc5::bulk_load_elect(st + G::kOffSfa, wsf + kb_sf, nsl * kSfBytes, full);
-                    if (NA == 2u) tc5::bulk_load_elect(st + G::kOffSfa + G::kS * kSfBytes, a.w_sf[1] + sf0 + kb_sf, nsl * kSfBytes, full);
+                    bulk_load_hint_elect(st + G::kOffSfa, wsf + kb_sf, nsl * kSfBytes, full, policy);
+                    if (NA == 2u) bulk_load_hint_elect(st + G::kOffSfa + G::kS * kSfBytes, a.w_sf[1] + sf0 + kb_sf, nsl * kSfBytes, full, policy);
                 } else {
                     // cell j of slab u: byte l*16 + c*4 + b = scale[rt*128 + c*32 + l][(kb0+u)*16 + j*4 + b]
                     const uint32_t sf_row = a.in_dim >> 4;
@@ -477,10 +495,11 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constan
     // what reads its rows, or writes where it may still read, waits for it.
     if (!a.ahead) pdk_pdl_wait_then_launch();
     uint32_t n, widest;
+    bool once = false;   // every expert has one tile per row tile
     if (a.max_blocks <= 32u) {
         s_tile = s_expert + 64u * warp;
         s_expert = s_tile + 32u;
-        n = build_tiles_warp<MAXG>(a, s_expert, s_tile, widest);
+        n = build_tiles_warp<MAXG>(a, s_expert, s_tile, widest, once);
         tc5::fence_before_sync();
         __syncthreads();
     } else {
@@ -502,10 +521,10 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constan
         widest = uniform(sh->widest);
     }
     tc5::fence_after_sync();
-    if (WG || widest <= 1u) roles<1u, NA, KIND, EPI, WG>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n);
-    else if (widest <= 2u) roles<2u, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n);
-    else if (widest <= 4u) roles<4u, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n);
-    else if (MAXG > 4u) roles<MAXG, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n);
+    if (WG || widest <= 1u) roles<1u, NA, KIND, EPI, WG>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
+    else if (widest <= 2u) roles<2u, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
+    else if (widest <= 4u) roles<4u, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
+    else if (MAXG > 4u) roles<MAXG, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
 
     tc5::fence_before_sync();
     __syncthreads();
