@@ -172,8 +172,7 @@ struct PrepArgs {
     uint8_t* xs;                 // tiled: [records][slab][4 cells][512], the weight scale records' layout
     float* xstep;                // [positions] power of two the row was divided by
     uint32_t dim, bm, mode;  // mode 0 gather, 1 gated (x = gate, up), 2 relu(x)^2 of x [positions][dim],
-                             // 3 one row: position 0 = x, the rest padding; the kernel writes the tables itself,
-                             // 4 x [positions][dim] as it is
+                             // 3 one row: position 0 = x, the rest padding; the kernel writes the tables itself
     uint32_t* tables;        // mode 3: sorted_row[bm], block_expert[1] (written here), then f32 scale2 = table_scale2
     float table_scale2;
     uint32_t natural;        // 0: ggml MXFP4 element order (byte j = elements j, j+16); 1: byte j = elements 2j, 2j+1
@@ -343,28 +342,61 @@ __global__ void __launch_bounds__(256) moe_prep_f4_kernel(const PrepArgs a) {
     prep_position(a, pos, src, rec, col);
 }
 
-// One CTA per token: its row is quantized once and written to the positions of all its k pairs (pair_pos, moe_route.cu), where
-// a CTA per position read and quantized it k times.  Positions without a pair are left as they are: their columns of the
-// GEMM are never read.  (1024 tokens of 2880, 4 of 128 experts: 26.2 -> 12.4 us.)
+// The preparations by pair: one CTA per row that has a token, none for padding.
+//   kTokens  a token's row is quantized once and written to the positions of all its k pairs, where a CTA per position read and
+//            quantized it k times (1024 tokens of 2880, 4 of 128 experts: 26.2 -> 12.4 us);
+//   the others: the row at pair p's own position, as it is, gate and up through the gated unit, or relu^2.  A CTA per position
+//            meets as many empty ones as live ones where experts hold ragged blocks (the same call's second preparation: XXX).
+// Positions without a pair are left as they are: their columns of the GEMM are never read.
+enum PrepKind : uint32_t { kTokens = 0u, kRows = 1u, kGatedRows = 2u, kSquaredRows = 3u };
 struct TokenArgs {
-    const float* x;             // [rows][dim]
+    const float *x, *up;        // kTokens: [rows][dim]; else [positions][dim] (x = gate with kGatedRows)
     const uint32_t* pair_pos;   // [rows][k]
     uint8_t *xq, *xs;
     float* xstep;
     uint32_t dim, k, bm, natural;
+    float alpha, limit, up_add;
 };
 
-__global__ void __launch_bounds__(256) moe_prep_tokens_kernel(const TokenArgs a) {
+template <uint32_t KIND>
+__global__ void __launch_bounds__(256) moe_prep_pairs_kernel(const TokenArgs a) {
     __shared__ float s_red[8];
     __shared__ uint32_t s_pos[16];
     pdk_pdl_wait_then_launch();
-    if (threadIdx.x < a.k) s_pos[threadIdx.x] = a.pair_pos[(size_t)blockIdx.x * a.k + threadIdx.x];
-    const uint32_t tid = threadIdx.x, token = blockIdx.x, groups = a.dim >> 4, kh = a.dim >> 1, num_kb = (a.dim + 255u) >> 8;
-    const float* row = a.x + (size_t)token * a.dim;
+    const uint32_t tid = threadIdx.x, groups = a.dim >> 4, kh = a.dim >> 1, num_kb = (a.dim + 255u) >> 8;
+    size_t row = blockIdx.x;
+    const uint32_t k = KIND == kTokens ? a.k : 1u;
+    if (KIND == kTokens) {
+        if (tid < k) s_pos[tid] = a.pair_pos[row * k + tid];
+    } else {
+        const uint32_t at = a.pair_pos[row];
+        if (at == PDK_MOE_PAD) return;
+        if (tid == 0u) s_pos[0] = at;
+        row = at & 0x3FFFFFFFu;
+    }
+    const float* x = a.x + row * a.dim;
+    const float* up = a.up + row * a.dim;
+    auto load4 = [&](uint32_t at) {
+        float4 v = *reinterpret_cast<const float4*>(x + at);
+        if (KIND == kGatedRows) {
+            const float4 u = *reinterpret_cast<const float4*>(up + at);
+            // gated unit: (xg * sigmoid(alpha * xg)) * (yu + up_add); OpenAI variant (reference/ops.rs:27-36) = alpha 1.702, limit 7,
+            // up_add 1; plain SwiGLU = alpha 1, limit inf, up_add 0
+            auto unit = [&](float g, float w) {
+                const float xg = fminf(g, a.limit), yu = fminf(fmaxf(w, -a.limit), a.limit);
+                return (xg / (1.0f + __expf(-a.alpha * xg))) * (yu + a.up_add);
+            };
+            v = make_float4(unit(v.x, u.x), unit(v.y, u.y), unit(v.z, u.z), unit(v.w, u.w));
+        }
+        if (KIND == kSquaredRows) {
+            auto sq = [](float g) { const float r = fmaxf(g, 0.0f); return r * r; };
+            v = make_float4(sq(v.x), sq(v.y), sq(v.z), sq(v.w));
+        }
+        return v;
+    };
     auto load = [&](uint32_t g, float2 (&r)[8]) {   // in code order, as prep_position
         const uint32_t lo_at = a.natural ? g * 16u : (g >> 1) * 32u + (g & 1u) * 8u, hi_at = lo_at + (a.natural ? 8u : 16u);
-        const float4 p = *reinterpret_cast<const float4*>(row + lo_at), q = *reinterpret_cast<const float4*>(row + lo_at + 4u);
-        const float4 u = *reinterpret_cast<const float4*>(row + hi_at), v = *reinterpret_cast<const float4*>(row + hi_at + 4u);
+        const float4 p = load4(lo_at), q = load4(lo_at + 4u), u = load4(hi_at), v = load4(hi_at + 4u);
         if (a.natural) {
             r[0] = make_float2(p.x, p.y); r[1] = make_float2(p.z, p.w); r[2] = make_float2(q.x, q.y); r[3] = make_float2(q.z, q.w);
             r[4] = make_float2(u.x, u.y); r[5] = make_float2(u.z, u.w); r[6] = make_float2(v.x, v.y); r[7] = make_float2(v.z, v.w);
@@ -395,7 +427,7 @@ __global__ void __launch_bounds__(256) moe_prep_tokens_kernel(const TokenArgs a)
         const uint32_t g = base + tid;
         uint32_t sb = 0u;
         auto put = [&](uint32_t term, uint2 codes) {
-            for (uint32_t s = 0; s < a.k; ++s) {
+            for (uint32_t s = 0; s < k; ++s) {
                 const uint32_t at = s_pos[s];
                 if (at == PDK_MOE_PAD) continue;
                 const uint32_t pos = at & 0x3FFFFFFFu;
@@ -413,7 +445,7 @@ __global__ void __launch_bounds__(256) moe_prep_tokens_kernel(const TokenArgs a)
         }
         const uint32_t word = scale_word(sb);
         if (g >= num_kb * 16u) continue;
-        for (uint32_t s = 0; s < a.k; ++s) {
+        for (uint32_t s = 0; s < k; ++s) {
             const uint32_t at = s_pos[s];
             if (at == PDK_MOE_PAD) continue;
             const uint32_t pos = at & 0x3FFFFFFFu, col = at >> 30, r0 = pos & 7u, b = pos / a.bm, rec = a.bm == 8u ? b - col : b;
@@ -537,6 +569,10 @@ PDK_EXPORT int pdk_mxfp4_tc5_tile_scales(const void* scale, void* tiled, void* m
 // Writes xq u8 [max_blocks*4*bm][dim/2], xs u8 [max_blocks][ceil(dim/256)][2048] (scale records in the
 // weight scale records' layout; bytes of term rows a block does not have are left alone), xstep f32 [max_blocks*bm].
 // dim % 32 == 0, bm 8 or 32.
+static uint32_t prep_threads(uint32_t dim) {
+    const uint32_t per_row = ((dim + 255u) >> 8) * 16u;  // scale groups incl. the zero tail of the last record
+    return per_row <= 256u ? (per_row + 31u) & ~31u : 256u;
+}
 static int prep_impl(const void* x, const void* up, const void* sorted_row, const void* block_expert, void* xq, void* xs,
                      void* xstep, uint32_t dim, uint32_t bm, uint32_t max_blocks, uint32_t mode, uint32_t natural,
                      float alpha, float limit, float up_add, void* stream) {
@@ -549,9 +585,7 @@ static int prep_impl(const void* x, const void* up, const void* sorted_row, cons
     a.block_expert = (const uint32_t*)block_expert;
     a.xq = (uint8_t*)xq; a.xs = (uint8_t*)xs; a.xstep = (float*)xstep;
     a.dim = dim; a.bm = bm; a.mode = mode; a.natural = natural; a.alpha = alpha; a.limit = limit; a.up_add = up_add;
-    const uint32_t per_row = ((dim + 255u) >> 8) * 16u;  // scale groups incl. the zero tail of the last record
-    return pdk_launch_pdl(moe_prep_f4_kernel, dim3(max_blocks * bm),
-                          dim3(per_row <= 256u ? (per_row + 31u) & ~31u : 256u), 0, (cudaStream_t)stream, a);
+    return pdk_launch_pdl(moe_prep_f4_kernel, dim3(max_blocks * bm), dim3(prep_threads(dim)), 0, (cudaStream_t)stream, a);
 }
 
 PDK_EXPORT int pdk_moe_prep_act_f4(const void* x, const void* up, const void* sorted_row, const void* block_expert,
@@ -570,12 +604,29 @@ PDK_EXPORT int pdk_moe_prep_tokens_f4(const void* x, const void* pair_pos, void*
     if (rows == 0 || k == 0) return 0;
     if (dim == 0 || (dim & 31u) != 0u || (bm != 8u && bm != 32u) || natural > 1u || k > 16u) return cudaErrorInvalidValue;
     if (!pdk_aligned(x, 16) || !pdk_aligned(xq, 16) || !pdk_aligned(xs, 16)) return cudaErrorInvalidValue;
-    const TokenArgs a{(const float*)x, (const uint32_t*)pair_pos, (uint8_t*)xq, (uint8_t*)xs, (float*)xstep, dim, k, bm, natural};
-    const uint32_t per_row = ((dim + 255u) >> 8) * 16u;
-    return pdk_launch_pdl(moe_prep_tokens_kernel, dim3(rows), dim3(per_row <= 256u ? (per_row + 31u) & ~31u : 256u), 0,
-                          (cudaStream_t)stream, a);
+    TokenArgs a{};
+    a.x = (const float*)x; a.pair_pos = (const uint32_t*)pair_pos; a.xq = (uint8_t*)xq; a.xs = (uint8_t*)xs; a.xstep = (float*)xstep;
+    a.dim = dim; a.k = k; a.bm = bm; a.natural = natural;
+    return pdk_launch_pdl(moe_prep_pairs_kernel<kTokens>, dim3(rows), dim3(prep_threads(dim)), 0, (cudaStream_t)stream, a);
 }
 
+// Position rows to term rows for the pairs' positions only: x f32 [positions][dim] as it is (mode 0, the rows of
+// pdk_*_moe_gate_up_tc5), gate = x and up through the gated unit (mode 1) or relu(x)^2 (mode 2).  pair_pos u32 [pairs] as above;
+// natural, alpha, limit and up_add as in pdk_moe_prep_act_f4 / ..._f4n, and the same rows, records and steps at these positions.
+PDK_EXPORT int pdk_moe_prep_pairs_f4(const void* x, const void* up, const void* pair_pos, void* xq, void* xs, void* xstep, uint32_t dim,
+                                     uint32_t bm, uint32_t pairs, uint32_t mode, uint32_t natural, float alpha, float limit, float up_add,
+                                     void* stream) {
+    if (pairs == 0) return 0;
+    if (dim == 0 || (dim & 31u) != 0u || (bm != 8u && bm != 32u) || natural > 1u || mode > 2u) return cudaErrorInvalidValue;
+    if (!pdk_aligned(x, 16) || !pdk_aligned(xq, 16) || !pdk_aligned(xs, 16) || (mode == 1u && (!up || !pdk_aligned(up, 16))))
+        return cudaErrorInvalidValue;
+    TokenArgs a{};
+    a.x = (const float*)x; a.up = (const float*)up; a.pair_pos = (const uint32_t*)pair_pos;
+    a.xq = (uint8_t*)xq; a.xs = (uint8_t*)xs; a.xstep = (float*)xstep;
+    a.dim = dim; a.bm = bm; a.natural = natural; a.alpha = alpha; a.limit = limit; a.up_add = up_add;
+    auto kern = mode == 0u ? moe_prep_pairs_kernel<kRows> : mode == 1u ? moe_prep_pairs_kernel<kGatedRows> : moe_prep_pairs_kernel<kSquaredRows>;
+    return pdk_launch_pdl(kern, dim3(pairs), dim3(prep_threads(dim)), 0, (cudaStream_t)stream, a);
+}
 // No counterpart in the reference.  moe_topk_batch + moe_align_bm + pdk_moe_prep_act_f4 (mode 0) in one
 // launch for decode widths: rows * k <= 32 pairs, rows <= 8, n_expert <= 512, max_blocks <= 32.  Writes
 // the same idx / w / sorted_row / sorted_slot / block_expert the three calls would, and the term rows.
@@ -643,14 +694,6 @@ PDK_EXPORT int pdk_moe_prep_act_f4n(const void* x, const void* up, const void* s
     if (mode > 2u) return cudaErrorInvalidValue;
     return prep_impl(x, up, sorted_row, block_expert, xq, xs, xstep, dim, bm, max_blocks, mode, 1u, alpha, limit, up_add,
                      stream);
-}
-
-// The rows a gate|up call left (pdk_*_moe_gate_up_tc5): position p takes row p of h f32 [positions][dim] as it is.
-// natural: 0 the MXFP4 element order, 1 the NVFP4 one.
-PDK_EXPORT int pdk_moe_prep_rows_f4(const void* h, const void* sorted_row, const void* block_expert, void* xq, void* xs,
-                                    void* xstep, uint32_t dim, uint32_t bm, uint32_t max_blocks, uint32_t natural, void* stream) {
-    if (natural > 1u) return cudaErrorInvalidValue;
-    return prep_impl(h, nullptr, sorted_row, block_expert, xq, xs, xstep, dim, bm, max_blocks, 4u, natural, 1.0f, 0.0f, 0.0f, stream);
 }
 
 // No counterpart in the reference (slots 88 / 89 are its mma.sync kernels on int8 activations):
@@ -847,9 +890,7 @@ int pdk_nvf4_gemv_tc5(const void* data, const void* scale, const void* bias, con
     PrepArgs pa{};
     pa.x = (const float*)x; pa.xq = xq; pa.xs = xs; pa.xstep = xstep;
     pa.dim = in_dim; pa.bm = 8u; pa.mode = 3u; pa.natural = 1u; pa.tables = tables; pa.table_scale2 = scale2;
-    const uint32_t per_row = ((in_dim + 255u) >> 8) * 16u;
-    if (int rc = pdk_launch_pdl(moe_prep_f4_kernel, dim3(8), dim3(per_row <= 256u ? (per_row + 31u) & ~31u : 256u), 0,
-                                st, pa))
+    if (int rc = pdk_launch_pdl(moe_prep_f4_kernel, dim3(8), dim3(prep_threads(in_dim)), 0, st, pa))
         return rc;
     const uint32_t kbytes = in_dim >> 1;
     CUtensorMap tw, tx;

@@ -74,7 +74,7 @@ const SigRow kSigs[] = {
     PDK_SIG("ppppppfuuu"), PDK_SIG("pppppppppppuuuuff"), PDK_SIG("ppppppppppuuuuu"), PDK_SIG("ppppppppppuuuuuu"),
     PDK_SIG("ppppppuuuuuu"), PDK_SIG("puuu"), PDK_SIG("up"), PDK_SIG("uup"), PDK_SIG("pppuuu"),
     PDK_SIG("pppppppuuuuff"), PDK_SIG("pppppppppppuuuuuu"), PDK_SIG("pppppppppppppppppuuuuuuu"),
-    PDK_SIG("pppppppuuuufff"), PDK_SIG("ppppppppppppppuuuuufff"), PDK_SIG("ppppppuuuu"),
+    PDK_SIG("pppppppuuuufff"), PDK_SIG("ppppppppppppppuuuuufff"), PDK_SIG("ppppppuuuuufff"),
     PDK_SIG("pppppuuuuu"), PDK_SIG("ppppppppuuuuu"),
 };
 #undef PDK_SIG

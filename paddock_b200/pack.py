@@ -142,7 +142,7 @@ _EXTRA_SIGS = {
     "pdk_nvf4_moe_gemm_tc5": "p" * 17 + "u" * 7,
     "pdk_mxfp4_moe_gate_up_tc5": "p" * 14 + "uuuuufff",
     "pdk_nvf4_moe_gate_up_tc5": "p" * 14 + "uuuuufff",
-    "pdk_moe_prep_rows_f4": "ppppppuuuu",
+    "pdk_moe_prep_pairs_f4": "ppppppuuuuufff",
     "pdk_moe_route_few": "ppppppppuuuuu",
     "pdk_mxfp4_moe_gemm_tc5_ahead": "p" * 17 + "u" * 7,
     "pdk_nvf4_moe_gemm_tc5_ahead": "p" * 17 + "u" * 7,

@@ -134,14 +134,14 @@ def repack_mxfp4(ex, raw_dev):
     return RepackedMxfp4(data, scale)
 
 
-def _unit_in_gemm(ws, max_blocks, ff):
+def _unit_in_gemm(ws, max_blocks, ff, n_expert):
     """Whether the gate|up GEMM applies the gated unit itself.  It then keeps both accumulators in one CTA and writes one plane
     instead of two: with 32-token blocks that saves 94 MB each way at 1024 tokens (gate|up + second preparation 313 -> 250 us).
     With 8-token blocks two accumulators per tile overlap better and the raw planes stay in L2 (60 tokens: 172 against 174 us; 128
     tokens on 32 experts of 1024 x 768: 20 against 23), but where tiles of one plane would just need a second round over the SMs
     (one token of 4 experts of 2880 x 2880: 31.9 us a block against 30.3)."""
     tiles = max_blocks * ((ff + 127) // 128)
-    return ws.bm == 32 or tiles <= ws.sms < 2 * tiles
+    return n_expert <= _PAIR_EXPERTS and (ws.bm == 32 or tiles <= ws.sms < 2 * tiles)
 
 
 class MoeWorkspace:
@@ -197,6 +197,9 @@ def moe_mxfp4_experts(ex, planes, ws, x, rows, alpha=1.702, limit=7.0):
     return 5
 
 
+_PAIR_EXPERTS = 1500      # the most that pdk_moe_align_pos, which knows the pairs' positions, takes
+
+
 def _route_and_prepare(ex, ws, x, rows, embd, n_expert, max_blocks, natural, logits=None, router_bias=None):
     """Positions and term rows of x: top-k (with logits; else ws.idx / ws.w hold the choices already), alignment, one preparation
     per token.  Returns the number of launches."""
@@ -214,7 +217,7 @@ def _route_and_prepare(ex, ws, x, rows, embd, n_expert, max_blocks, natural, log
     if logits is not None:
         c("moe_topk_batch", logits, router_bias, n_expert, k, ws.idx, ws.w, rows, stream=st)
         n = 3
-    if n_expert > 1500:       # beyond the alignment that knows the pairs' positions
+    if n_expert > _PAIR_EXPERTS:
         c("moe_align_bm", ws.idx, ws.sorted_row, ws.sorted_slot, ws.block_expert, rows, k, n_expert, bm, max_blocks, stream=st)
         args = x, None, ws.sorted_row, ws.block_expert, ws.x4q, ws.x4s, ws.x4step, embd, bm, max_blocks, 0, 1.0, 0.0
         c(*(("pdk_moe_prep_act_f4n", *args, 0.0) if natural else ("pdk_moe_prep_act_f4", *args)), stream=st)
@@ -223,6 +226,17 @@ def _route_and_prepare(ex, ws, x, rows, embd, n_expert, max_blocks, natural, log
       stream=st)
     c("pdk_moe_prep_tokens_f4", *tokens, stream=st)
     return n
+
+
+def _prepare_unit(ex, ws, x, up, rows, ff, n_expert, max_blocks, mode, natural, alpha, limit, up_add):
+    """Term rows for down from what gate|up left: mode 0 the unit's own rows, 1 raw gate and up rows, 2 relu(x)^2."""
+    st = _stream()
+    if n_expert <= _PAIR_EXPERTS:
+        ex.pack.call("pdk_moe_prep_pairs_f4", x, up, ws.pair_pos, ws.h4q, ws.h4s, ws.h4step, ff, ws.bm, rows * ws.n_active, mode,
+                     int(natural), alpha, limit, up_add, stream=st)
+        return
+    args = x, up, ws.sorted_row, ws.block_expert, ws.h4q, ws.h4s, ws.h4step, ff, ws.bm, max_blocks, mode, alpha, limit
+    ex.pack.call(*(("pdk_moe_prep_act_f4n", *args, up_add) if natural else ("pdk_moe_prep_act_f4", *args)), stream=st)
 
 
 def moe_mxfp4_experts_tc5(ex, planes, ws, x, rows, alpha=1.702, limit=7.0, route=None):
@@ -234,19 +248,18 @@ def moe_mxfp4_experts_tc5(ex, planes, ws, x, rows, alpha=1.702, limit=7.0, route
     k, bm, t = ws.n_active, ws.bm, planes.tc5
     max_blocks = min(ws.max_blocks, min(rows * k, rows * k // bm + planes.n_expert))
     n = _route_and_prepare(ex, ws, x, rows, planes.embd, planes.n_expert, max_blocks, False, *(route or ()))
-    if not _unit_in_gemm(ws, max_blocks, planes.ff):
+    if not _unit_in_gemm(ws, max_blocks, planes.ff, planes.n_expert):
         c("pdk_mxfp4_moe_gemm_tc5_ahead", planes.gate.data, t["gate"][0], t["gate"][1], planes.gate_bias, ws.g_raw,
           planes.up.data, t["up"][0], t["up"][1], planes.up_bias, ws.u_raw, ws.x4q, ws.x4s, ws.x4step,
           ws.block_expert, ws.sorted_row, None, None, planes.embd, planes.ff, planes.n_expert, bm, max_blocks, k, 0,
           stream=st)
-        c("pdk_moe_prep_act_f4", ws.g_raw, ws.u_raw, ws.sorted_row, ws.block_expert, ws.h4q, ws.h4s, ws.h4step, planes.ff, bm,
-          max_blocks, 1, alpha, limit, stream=st)
+        x2, up2, mode = ws.g_raw, ws.u_raw, 1
     else:
         c("pdk_mxfp4_moe_gate_up_tc5", planes.gate.data, t["gate"][0], t["gate"][1], planes.gate_bias,
           planes.up.data, t["up"][0], t["up"][1], planes.up_bias, ws.h, ws.x4q, ws.x4s, ws.x4step, ws.block_expert,
           ws.sorted_row, planes.embd, planes.ff, planes.n_expert, bm, max_blocks, alpha, limit, 1.0, stream=st)
-        c("pdk_moe_prep_rows_f4", ws.h, ws.sorted_row, ws.block_expert, ws.h4q, ws.h4s, ws.h4step, planes.ff, bm,
-          max_blocks, 0, stream=st)
+        x2, up2, mode = ws.h, None, 0
+    _prepare_unit(ex, ws, x2, up2, rows, planes.ff, planes.n_expert, max_blocks, mode, False, alpha, limit, 1.0)
     c("pdk_mxfp4_moe_gemm_tc5_ahead", planes.down.data, t["down"][0], t["down"][1], planes.down_bias, ws.part,
       None, None, None, None, None, ws.h4q, ws.h4s, ws.h4step, ws.block_expert, ws.sorted_row, ws.sorted_slot,
       ws.w, planes.ff, planes.embd, planes.n_expert, bm, max_blocks, k, 1, stream=st)
@@ -304,24 +317,22 @@ def moe_nvf4_forward(ex, gate, up, down, ws, x, router_logits, out, gated=True, 
     n_expert, embd, ff = up.n_expert, up.in_dim, up.rows
     max_blocks = min(ws.max_blocks, min(T * k, T * k // bm + n_expert))
     n = _route_and_prepare(ex, ws, x, T, embd, n_expert, max_blocks, True, router_logits, router_bias)
-    if gated and _unit_in_gemm(ws, max_blocks, ff):
+    if gated and _unit_in_gemm(ws, max_blocks, ff, n_expert):
         c("pdk_nvf4_moe_gate_up_tc5", gate.data, gate.tiled, gate.scale2, None, up.data, up.tiled, up.scale2, None, ws.h,
           ws.x4q, ws.x4s, ws.x4step, ws.block_expert, ws.sorted_row, embd, ff, n_expert, bm, max_blocks, alpha, limit, up_add,
           stream=st)
-        c("pdk_moe_prep_rows_f4", ws.h, ws.sorted_row, ws.block_expert, ws.h4q, ws.h4s, ws.h4step, ff, bm, max_blocks, 1,
-          stream=st)
+        x2, up2, mode = ws.h, None, 0
     elif gated:
         c("pdk_nvf4_moe_gemm_tc5_ahead", gate.data, gate.tiled, gate.scale2, None, ws.g_raw, up.data, up.tiled, up.scale2, None,
           ws.u_raw, ws.x4q, ws.x4s, ws.x4step, ws.block_expert, ws.sorted_row, None, None, embd, ff, n_expert, bm,
           max_blocks, k, 0, stream=st)
-        c("pdk_moe_prep_act_f4n", ws.g_raw, ws.u_raw, ws.sorted_row, ws.block_expert, ws.h4q, ws.h4s, ws.h4step, ff, bm,
-          max_blocks, 1, alpha, limit, up_add, stream=st)
+        x2, up2, mode = ws.g_raw, ws.u_raw, 1
     else:
         c("pdk_nvf4_moe_gemm_tc5_ahead", up.data, up.tiled, up.scale2, None, ws.u_raw, None, None, None, None, None, ws.x4q,
           ws.x4s, ws.x4step, ws.block_expert, ws.sorted_row, None, None, embd, ff, n_expert, bm, max_blocks, k, 0,
           stream=st)
-        c("pdk_moe_prep_act_f4n", ws.u_raw, None, ws.sorted_row, ws.block_expert, ws.h4q, ws.h4s, ws.h4step, ff, bm,
-          max_blocks, 2, alpha, limit, up_add, stream=st)
+        x2, up2, mode = ws.u_raw, None, 2
+    _prepare_unit(ex, ws, x2, up2, T, ff, n_expert, max_blocks, mode, True, alpha, limit, up_add)
     c("pdk_nvf4_moe_gemm_tc5_ahead", down.data, down.tiled, down.scale2, None, ws.part, None, None, None, None, None, ws.h4q,
       ws.h4s, ws.h4step, ws.block_expert, ws.sorted_row, ws.sorted_slot, ws.w, ff, embd, n_expert, bm, max_blocks, k, 1,
       stream=st)

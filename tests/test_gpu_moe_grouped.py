@@ -114,6 +114,25 @@ def test_positions_and_token_rows_equal_the_gathered_ones(pack, tokens, n_expert
     # unused blocks keep what they had in every table
     for name in a:
         assert torch.equal(a[name].view(u8), b[name].view(u8)), name
+    # what the by-pair preparation of position rows leaves, against the call that walks every position; bytes of padding aside
+    h, u = (torch.randn(nb * embd, device="cuda", generator=torch.Generator(device="cuda").manual_seed(s)) for s in (5, 6))
+    for mode in ((0, 1, 2) if natural else (0, 1)):
+        u1 = u if mode == 1 else None
+        both = []
+        for by_pair in (False, True):
+            q, sc, st = torch.zeros_like(a["q"]), torch.zeros_like(a["s"]), torch.zeros_like(a["step"])
+            if by_pair:
+                c("pdk_moe_prep_pairs_f4", h, u1, pos, q, sc, st, embd, bm, pairs, mode, int(natural), 1.7, 7.0, 1.0)
+            elif mode == 0:     # as a gather of each position's own row
+                own = torch.where(a["row"] == -1, a["row"], torch.arange(nb, dtype=i32, device="cuda"))
+                args = h, None, own, a["blk"], q, sc, st, embd, bm, max_blocks, 0, 1.0, 7.0
+                c(*(("pdk_moe_prep_act_f4n", *args, 0.0) if natural else ("pdk_moe_prep_act_f4", *args)))
+            else:
+                args = h, u1, a["row"], a["blk"], q, sc, st, embd, bm, max_blocks, mode, 1.7, 7.0
+                c(*(("pdk_moe_prep_act_f4n", *args, 1.0) if natural else ("pdk_moe_prep_act_f4", *args)))
+            both.append((q, sc, st))
+        for v, w in zip(*both):
+            assert torch.equal(v.view(u8), w.view(u8)), mode
     p = torch.arange(pairs, device="cuda")
     at = (pos.long() & 0x3FFFFFFF)
     assert torch.equal(b["row"][at].long(), p // k) and torch.equal(b["slot"][at].long(), p % k)
