@@ -346,7 +346,7 @@ __global__ void __launch_bounds__(256) moe_prep_f4_kernel(const PrepArgs a) {
 //   kTokens  a token's row is quantized once and written to the positions of all its k pairs, where a CTA per position read and
 //            quantized it k times (1024 tokens of 2880, 4 of 128 experts: 26.2 -> 12.4 us);
 //   the others: the row at pair p's own position, as it is, gate and up through the gated unit, or relu^2.  A CTA per position
-//            meets as many empty ones as live ones where experts hold ragged blocks (the same call's second preparation: XXX).
+//            meets as many empty ones as live ones where experts hold ragged blocks (the same call: 31 -> 28 us; 60 tokens, 240 rows at 1264 positions: 7.7 -> 4).
 // Positions without a pair are left as they are: their columns of the GEMM are never read.
 enum PrepKind : uint32_t { kTokens = 0u, kRows = 1u, kGatedRows = 2u, kSquaredRows = 3u };
 struct TokenArgs {
