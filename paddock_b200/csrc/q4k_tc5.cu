@@ -79,6 +79,7 @@ struct Cfg {
 struct Shared {
     uint64_t raw_full[kRawStages];
     uint64_t raw_empty[kRawStages];
+    uint64_t act_full[kRawStages];    // BRAW: a box's activation tiles, which the dequantizing warps do not wait for
     uint64_t full[kMaxStages];
     uint64_t empty[kMaxStages];
     uint64_t tmem_full[2];
@@ -344,6 +345,7 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         for (uint32_t s = 0; s < kRawStages; ++s) {
             tc5::mbar_init(&sh->raw_full[s], 1);
             tc5::mbar_init(&sh->raw_empty[s], C::kRawEmptyCount);
+            tc5::mbar_init(&sh->act_full[s], 1);
         }
         for (uint32_t s = 0; s < kStages; ++s) {
             tc5::mbar_init(&sh->full[s], C::kFullCount);  // one arrival per producer warp (+ the activation loader's)
@@ -470,34 +472,52 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
         }
     } else if (warp == kRawWarp) {
         // ------------------------------------------------------------ packed weights and scale records (TMA)
-        // Weights depend on nothing the previous kernel in the stream writes: no wait for it.
-        uint32_t rs = 0, rphase = 0;
+        // Weights depend on nothing the previous kernel in the stream writes: no wait for it.  With BRAW the activation tiles of a box
+        // come behind its weights on a barrier of their own, and the first ring of boxes is requested (and dequantized) before the
+        // wait for the f16 rows, which are the previous kernel's output.
+        uint32_t rs = 0, rphase = 0, ready = 0;
         bool ok = true, waited = false;
+        uint32_t held[kRawStages];       // first unit in K of the boxes whose activation tiles are still to be requested
+        auto issue_act = [&](uint32_t at, uint32_t u) {
+            tc5::mbar_arrive_expect_tx_elect(&sh->act_full[at], 4u * C::kBBytes);
+#pragma unroll
+            for (uint32_t j = 0; j < 8u; ++j)  // 4 half units x 2 k-slabs of 64
+                tc5::tma_load_2d_elect(ring + at * C::kRawBytes + kRawStageBytes + j * C::kBSlab, &tmap_x, &sh->act_full[at],
+                                       (int32_t)(u * 256u + j * 64u), 0);
+        };
+        auto flush = [&]() {
+            pdk_pdl_wait();
+            waited = true;
+#pragma unroll
+            for (uint32_t i = 0; i < kRawStages; ++i)
+                if (i < ready) issue_act(i, held[i]);
+        };
         for (uint32_t at = p_lo, tile = tile_lo; at < p_hi && ok; ++tile) {
             const uint32_t row0 = tile * BM, u0 = 2u * (at - tile * ppt), upi = 2u * (min(p_hi, (tile + 1u) * ppt) - at);
             at += upi >> 1;
             for (uint32_t u = 0; u < upi; u += 2u) {
+                if (C::BRAW && !waited && ready == kRawStages) flush();
                 ok = mbar_wait_park(&sh->raw_empty[rs], rphase ^ 1u, ctx, tc5::kErrEmptyWait, 0x20u + rs);
                 ok = __all_sync(0xffffffffu, ok);
                 if (!ok) break;
                 uint8_t* raw = ring + rs * C::kRawBytes;
-                tc5::mbar_arrive_expect_tx_elect(&sh->raw_full[rs], C::kRawBytes);
+                tc5::mbar_arrive_expect_tx_elect(&sh->raw_full[rs], kRawStageBytes);
                 tc5::tma_load_2d_elect(raw, &tmap_w, &sh->raw_full[rs], (int32_t)((u0 + u) * 128u), (int32_t)row0);
                 tc5::tma_load_2d_elect(raw + kRawData, &tmap_w, &sh->raw_full[rs], (int32_t)((u0 + u + 1u) * 128u), (int32_t)row0);
                 tc5::tma_load_2d_elect(raw + 2u * kRawData, &tmap_r, &sh->raw_full[rs], (int32_t)((u0 + u) * 24u), (int32_t)row0);
                 if (C::BRAW) {
-                    if (!waited) {  // the f16 rows are the previous kernel's output; the weights above are not
-                        pdk_pdl_wait();
-                        waited = true;
-                    }
+                    if (waited) issue_act(rs, u0 + u);
+                    else {
 #pragma unroll
-                    for (uint32_t j = 0; j < 8u; ++j)  // 4 half units x 2 k-slabs of 64
-                        tc5::tma_load_2d_elect(raw + kRawStageBytes + j * C::kBSlab, &tmap_x, &sh->raw_full[rs],
-                                               (int32_t)((u0 + u) * 256u + j * 64u), 0);
+                        for (uint32_t i = 0; i < kRawStages; ++i)
+                            if (i == ready) held[i] = u0 + u;
+                        ++ready;
+                    }
                 }
                 if (++rs == kRawStages) { rs = 0; rphase ^= 1u; }
             }
         }
+        if (C::BRAW && !waited) flush();     // fewer boxes than the ring holds
         if (!ok && lane == 0)
             for (int i = 0; i < 64; ++i) __nanosleep(1000);  // copies in flight still land in this CTA's shared memory
     } else if (warp == kActWarp) {
@@ -539,7 +559,7 @@ q4k_tc5_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constant
             const uint32_t d_tmem = tmem_base + buf * NC;
             for (uint32_t u = 0; u < upi; ++u) {
                 if (C::BRAW && (u & 1u) == 0u) {  // the activation tiles of this pair of units are in the weight box
-                    ok = mbar_wait_park(&sh->raw_full[rs], rphase, ctx, tc5::kErrFullWait, 0x30u + rs);
+                    ok = mbar_wait_park(&sh->act_full[rs], rphase, ctx, tc5::kErrFullWait, 0x30u + rs);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                 }
