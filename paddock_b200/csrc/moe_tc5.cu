@@ -19,9 +19,12 @@
 // pure stream of 4.25 bits per weight.
 //
 // Launch order of one MoE block (host side in planes.py):
-//   pdk_moe_prep_act_f4 (gather by sorted_row)  ->  pdk_mxfp4_moe_gemm_tc5 (gate and up, raw)
-//   pdk_moe_prep_act_f4 (SwiGLU of gate/up)     ->  pdk_mxfp4_moe_gemm_tc5 (down, scattered to
-//   (token, slot) rows and multiplied by the routing weight)  ->  pd_moe_slot_combine
+//   pd_moe_topk_batch, pdk_moe_align_pos (decode widths: pdk_moe_route_few for both)
+//   pdk_moe_prep_tokens_f4 (each token's term rows to its pairs' positions)
+//   pdk_*_moe_gate_up_tc5 (gate, up and the unit)  or  pdk_*_moe_gemm_tc5_ahead (gate and up, raw)
+//   pdk_moe_prep_pairs_f4 (the unit where it is still to do, term rows)
+//   pdk_*_moe_gemm_tc5_ahead (down, scattered to (token, slot) rows and multiplied by the routing weight)
+//   pd_moe_slot_combine
 #include <cuda_fp8.h>
 
 #include "moe_grouped.cuh"
@@ -566,8 +569,9 @@ PDK_EXPORT int pdk_mxfp4_tc5_tile_scales(const void* scale, void* tiled, void* m
 // No counterpart in the reference: block positions -> four NVFP4 term rows each.
 //   mode 0: position p takes row sorted_row[p] of x f32 [rows][dim]            (`up` unused)
 //   mode 1: position p takes swiglu(x[p], up[p]) of the raw gate / up outputs f32 [positions][dim]
-// Writes xq u8 [max_blocks*4*bm][dim/2], xs u8 [max_blocks][ceil(dim/256)][2048] (scale records in the
-// weight scale records' layout; bytes of term rows a block does not have are left alone), xstep f32 [max_blocks*bm].
+// Writes xq u8 [max_blocks*4*bm][dim/2] (term t of position p in row p/8*32 + t*8 + p%8), xs u8 [max_blocks][ceil(dim/256)][2048]
+// (scale records in the weight scale records' layout, one for the 128 term rows of four groups of eight: with bm 8 four blocks of
+// a run share the first one's; bytes of term rows that are not there are left alone), xstep f32 [max_blocks*bm].
 // dim % 32 == 0, bm 8 or 32.
 static uint32_t prep_threads(uint32_t dim) {
     const uint32_t per_row = ((dim + 255u) >> 8) * 16u;  // scale groups incl. the zero tail of the last record
@@ -627,6 +631,7 @@ PDK_EXPORT int pdk_moe_prep_pairs_f4(const void* x, const void* up, const void* 
     auto kern = mode == 0u ? moe_prep_pairs_kernel<kRows> : mode == 1u ? moe_prep_pairs_kernel<kGatedRows> : moe_prep_pairs_kernel<kSquaredRows>;
     return pdk_launch_pdl(kern, dim3(pairs), dim3(prep_threads(dim)), 0, (cudaStream_t)stream, a);
 }
+
 // No counterpart in the reference.  moe_topk_batch + moe_align_bm + pdk_moe_prep_act_f4 (mode 0) in one
 // launch for decode widths: rows * k <= 32 pairs, rows <= 8, n_expert <= 512, max_blocks <= 32.  Writes
 // the same idx / w / sorted_row / sorted_slot / block_expert the three calls would, and the term rows.

@@ -63,7 +63,7 @@ tc5_issue_probe_kernel(uint32_t n_mma, unsigned int* err, unsigned long long* cy
         constexpr uint32_t n_cols = kKind >= 2 ? 128u : 256u;
         constexpr uint32_t idesc = kKind == 0   ? tc5::idesc_f32acc(1u, 1u, 128u, 256u)
                                    : kKind == 1 ? tc5::idesc_f32acc(0u, 0u, 128u, 256u)
-                                                : nvf4tc5::Cfg<128>::kIdesc;
+                                                : nvf4tc5::idesc(128u);
         const uint32_t sfa_t = tmem + 256u, sfb_t = sfa_t + 16u;
         if (kKind >= 2)
             for (uint32_t j = 0; j < 4u; ++j) {
