@@ -421,11 +421,29 @@ int pdk_mxfp4_tc5_tile_scales(const void* scale, void* tiled, void* meta, uint32
  * swiglu_oai(x[p], up[p]) of raw gate / up outputs f32[positions][dim].
  * Padding positions of used blocks become zero rows; the rows of unused blocks (block_expert = PDK_MOE_PAD),
  * which the GEMMs skip, are left as they are.
- * xq u8[max_blocks*4*bm][dim/2], xs u8[max_blocks][ceil(dim/256)][2048] (scale records, the layout
- * of the tiled weight scales; zero the buffer once), xstep f32[max_blocks*bm]. */
+ * xq u8[max_blocks*4*bm][dim/2], term t of position p in row p/8*32 + t*8 + p%8; xs
+ * u8[max_blocks][ceil(dim/256)][2048] (scale records, the layout of the tiled weight scales; a record holds
+ * four groups of eight positions: one block of 32, or four consecutive blocks of 8 of one expert, counted from
+ * the expert's first, in the first one's record; zero the buffer once); xstep f32[max_blocks*bm]. */
 int pdk_moe_prep_act_f4(const void* x, const void* up, const void* sorted_row, const void* block_expert, void* xq,
                         void* xs, void* xstep, uint32_t dim, uint32_t bm, uint32_t max_blocks, uint32_t mode, float alpha, float limit,
                         void* stream);
+/* moe_align_bm that also leaves where each (row, slot) pair went, pair_pos u32[rows*n_active]: its position |
+ * its group's place in a scale record << 30, PDK_MOE_PAD for a pair without an expert.  bm 8 or 32, at most 1500 experts. */
+int pdk_moe_align_pos(const void* idx, void* sorted_row, void* sorted_slot, void* block_expert, void* pair_pos,
+                      uint32_t rows, uint32_t n_active, uint32_t n_expert, uint32_t bm, uint32_t max_blocks, void* stream);
+/* pd_moe_topk_batch + pdk_moe_align_pos in one launch: rows * k <= 32, rows <= 8, k <= 16, n_expert <= 512, max_blocks <= 32. */
+int pdk_moe_route_few(const void* logits, const void* router_bias, void* idx, void* w, void* sorted_row, void* sorted_slot,
+                      void* block_expert, void* pair_pos, uint32_t n_expert, uint32_t k, uint32_t rows, uint32_t bm,
+                      uint32_t max_blocks, void* stream);
+/* pdk_moe_prep_act_f4 (natural 0) or ..._f4n (1) in mode 0, each token quantized once for its k <= 16 pairs; padding is left alone. */
+int pdk_moe_prep_tokens_f4(const void* x, const void* pair_pos, void* xq, void* xs, void* xstep, uint32_t dim, uint32_t k,
+                           uint32_t rows, uint32_t bm, uint32_t natural, void* stream);
+/* Term rows of position rows, the pairs' positions only: x f32[positions][dim] as it is (mode 0), through the gated unit with up
+ * (mode 1), relu(x)^2 (mode 2); natural, alpha, limit, up_add as in pdk_moe_prep_act_f4 / ..._f4n. */
+int pdk_moe_prep_pairs_f4(const void* x, const void* up, const void* pair_pos, void* xq, void* xs, void* xstep, uint32_t dim,
+                          uint32_t bm, uint32_t pairs, uint32_t mode, uint32_t natural, float alpha, float limit, float up_add,
+                          void* stream);
 /* Grouped GEMM of one or two planes (w1_data NULL = one) over the term rows.  scatter 0: out_p
  * f32[max_blocks*bm][out_dim], block order, bias added, no activation function; scatter 1 (one
  * plane): out0 = part f32[rows*n_active][out_dim] at row (sorted_row, sorted_slot), times topk_w.
@@ -436,6 +454,21 @@ int pdk_mxfp4_moe_gemm_tc5(const void* w0_data, const void* w0_sf, const void* w
                            const void* sorted_row, const void* sorted_slot, const void* topk_w, uint32_t in_dim,
                            uint32_t out_dim, uint32_t n_expert, uint32_t bm, uint32_t max_blocks, uint32_t n_active,
                            uint32_t scatter, void* stream);
+/* The same directly behind a pdk_moe_prep_* call that came after the launch which wrote the tables: they, and the weights,
+ * are read while the preparation still runs.  Not behind a kernel that writes block_expert, sorted_row or sorted_slot. */
+int pdk_mxfp4_moe_gemm_tc5_ahead(const void* w0_data, const void* w0_sf, const void* w0_meta, const void* w0_bias, void* out0,
+                                 const void* w1_data, const void* w1_sf, const void* w1_meta, const void* w1_bias, void* out1,
+                                 const void* xq, const void* xs, const void* xstep, const void* block_expert,
+                                 const void* sorted_row, const void* sorted_slot, const void* topk_w, uint32_t in_dim,
+                                 uint32_t out_dim, uint32_t n_expert, uint32_t bm, uint32_t max_blocks, uint32_t n_active,
+                                 uint32_t scatter, void* stream);
+/* Gate, up and the gated unit in one launch, h f32[max_blocks*bm][out_dim] in block order (padding left alone); to be called
+ * where pdk_mxfp4_moe_gemm_tc5_ahead may be. */
+int pdk_mxfp4_moe_gate_up_tc5(const void* gate_data, const void* gate_sf, const void* gate_meta, const void* gate_bias,
+                              const void* up_data, const void* up_sf, const void* up_meta, const void* up_bias, void* h,
+                              const void* xq, const void* xs, const void* xstep, const void* block_expert,
+                              const void* sorted_row, uint32_t in_dim, uint32_t out_dim, uint32_t n_expert, uint32_t bm,
+                              uint32_t max_blocks, float alpha, float limit, float up_add, void* stream);
 
 /* ---- NVFP4 expert planes on the same grouped GEMM (plane layout of
  * crates/paddock-engine/src/gpu/types.rs:176-226, Row order: data [expert*rows][in/2], scale e4m3
@@ -468,6 +501,18 @@ int pdk_nvf4_moe_gemm_tc5(const void* w0_data, const void* w0_sf, const void* w0
                           const void* sorted_row, const void* sorted_slot, const void* topk_w, uint32_t in_dim,
                           uint32_t out_dim, uint32_t n_expert, uint32_t bm, uint32_t max_blocks, uint32_t n_active,
                           uint32_t scatter, void* stream);
+/* as pdk_mxfp4_moe_gemm_tc5_ahead and pdk_mxfp4_moe_gate_up_tc5 */
+int pdk_nvf4_moe_gemm_tc5_ahead(const void* w0_data, const void* w0_sf, const void* w0_scale2, const void* w0_bias, void* out0,
+                                const void* w1_data, const void* w1_sf, const void* w1_scale2, const void* w1_bias, void* out1,
+                                const void* xq, const void* xs, const void* xstep, const void* block_expert,
+                                const void* sorted_row, const void* sorted_slot, const void* topk_w, uint32_t in_dim,
+                                uint32_t out_dim, uint32_t n_expert, uint32_t bm, uint32_t max_blocks, uint32_t n_active,
+                                uint32_t scatter, void* stream);
+int pdk_nvf4_moe_gate_up_tc5(const void* gate_data, const void* gate_sf, const void* gate_scale2, const void* gate_bias,
+                             const void* up_data, const void* up_sf, const void* up_scale2, const void* up_bias, void* h,
+                             const void* xq, const void* xs, const void* xstep, const void* block_expert, const void* sorted_row,
+                             uint32_t in_dim, uint32_t out_dim, uint32_t n_expert, uint32_t bm, uint32_t max_blocks, float alpha,
+                             float limit, float up_add, void* stream);
 
 /* No counterpart in the reference.  pdk_mxfp4_moe_down + pd_moe_slot_combine for callers that may
  * not allocate device memory (a serving loop that must stay off the allocator, a plug-in handed
