@@ -60,6 +60,28 @@ def test_quantize_e4m3_row_single_pass_route(pack, rows, n):
     assert np.array_equal(d_q.cpu().numpy().reshape(rows, n), q_ref)
 
 
+@pytest.mark.parametrize("field", [0, 1, 2, 8, 19, 20, 21, 126, 127, 135, 253, 254])
+def test_row_scale_from_the_exponent_field(pack, field):
+    """Row maxima around 0.875 * 2^e (mantissa 0x600000) in every class of exponent: both ways to the scale, down to subnormal rows."""
+    n, rng = 256, np.random.default_rng(field)
+    rows = []
+    for m in (0, 1, 0x5FFFFF, 0x600000, 0x600001, 0x7FFFFF):
+        top = np.uint32(max((field << 23) | m, 1)).view(np.float32)
+        row = (rng.uniform(0.05, 1.0, n) * top * rng.choice([-1.0, 1.0], n)).astype(np.float32)
+        row[row == 0.0] = top
+        row[rng.integers(n)] = -top
+        rows.append(row)
+    rows.append(np.zeros(n, np.float32))
+    x = np.concatenate(rows)
+    q_ref, s_ref = oracle.quantize_e4m3_row_pow2(x, len(rows), n)
+    d_q = torch.zeros(x.size, dtype=torch.uint8, device="cuda")
+    d_s = torch.zeros(len(rows), dtype=torch.float32, device="cuda")
+    pack.call("quantize_e4m3_row", dev_f32(x), d_q, d_s, n, len(rows))
+    torch.cuda.synchronize()
+    assert np.array_equal(d_s.cpu().numpy().view(np.uint32), s_ref.view(np.uint32))
+    assert np.array_equal(d_q.cpu().numpy().reshape(len(rows), n), q_ref)
+
+
 @pytest.mark.parametrize("rows,n", [(1, 64), (5, 5120), (80, 17408)])
 def test_swiglu_quant_e4m3_row(pack, rows, n):
     """Slot 511: silu(gate) * up, then the row quantizer."""
