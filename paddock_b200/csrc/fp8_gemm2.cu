@@ -127,24 +127,17 @@ f8row_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
         // ------------------------------------------------------------ TMA producer (both CTAs)
         uint32_t stage = 0, phase = 0;
         bool ok = true;
-        auto issue_w = [&](uint32_t at, uint32_t kb, uint32_t n0) {
-            if (leader) tc5::mbar_arrive_expect_tx_elect(&sh->full[at], 2u * kStageBytes);
-            tma_load_2d_pair_elect(tiles + at * kStageBytes + kABytes, &tmap_w, &sh->full[at], (int32_t)(kb * BK), (int32_t)n0);
-        };
-        // The weights depend on nothing that the launch in front writes: the first tile's first stages are requested under it.
-        const uint32_t pre = pair < n_tiles ? min(num_kb, kStages) : 0u;
-        for (uint32_t kb = 0; kb < pre; ++kb) issue_w(kb, kb, (pair / tiles_m) * BN + rank * BNH);
         pdk_pdl_wait();
         for (uint32_t tile = pair; tile < n_tiles && ok; tile += n_pairs) {
             const uint32_t m0 = (tile % tiles_m) * 2u * BM + rank * BM, n0 = (tile / tiles_m) * BN + rank * BNH;
             for (uint32_t kb = 0; kb < num_kb; ++kb) {
-                if (tile != pair || kb >= pre) {
-                    ok = tc5::mbar_wait(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, stage);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    issue_w(stage, kb, n0);
-                }
-                tma_load_2d_pair_elect(tiles + stage * kStageBytes, &tmap_x, &sh->full[stage], (int32_t)(kb * BK), (int32_t)m0);
+                ok = tc5::mbar_wait(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, stage);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
+                uint8_t* a = tiles + stage * kStageBytes;
+                if (leader) tc5::mbar_arrive_expect_tx_elect(&sh->full[stage], 2u * kStageBytes);
+                tma_load_2d_pair_elect(a, &tmap_x, &sh->full[stage], (int32_t)(kb * BK), (int32_t)m0);
+                tma_load_2d_pair_elect(a + kABytes, &tmap_w, &sh->full[stage], (int32_t)(kb * BK), (int32_t)n0);
                 if (++stage == kStages) { stage = 0; phase ^= 1u; }
             }
         }

@@ -185,40 +185,29 @@ nvf4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
         // ------------------------------------------------------------ producer (both CTAs)
         uint32_t stage = 0, phase = 0;
         bool ok = true;
-        // one stage's boxes; the scale boxes always span kSlabs records (rows past the plane read as zero and count)
-        auto issue_w = [&](uint32_t at, uint32_t tile_a, uint32_t kb0, uint32_t nsl) {
-            uint8_t* a = tiles + at * kStageBytes;
-            if (leader)
-                tc5::mbar_arrive_expect_tx_elect(&sh->full[at],
-                                                 2u * (nsl * (kABytes + C::kBHalf) + (1u + C::kRec) * kSlabs * kSfBytes));
-#pragma unroll
-            for (uint32_t u = 0; u < kSlabs; ++u)
-                if (u < nsl)
-                    tma_load_2d_pair_elect(a + u * kABytes, &tmap_w, &sh->full[at], (int32_t)((kb0 + u) * BKB), (int32_t)(tile_a * BM));
-            tma_load_2d_pair_elect(a + C::kOffSfa, &tmap_wsf, &sh->full[at], 0, (int32_t)((tile_a * num_kb + kb0) * 8u));
-        };
-        // The weights depend on nothing that the launch in front writes: the first tile's first stages are requested under it.
-        const uint32_t pre = pair < n_tiles ? min(num_ks, kStages) : 0u;
-        for (uint32_t ks = 0; ks < pre; ++ks)
-            issue_w(ks, (pair / tiles_b) * 2u + rank, ks * kSlabs, min(kSlabs, num_kb - ks * kSlabs));
         pdk_pdl_wait();
         for (uint32_t tile = pair; tile < n_tiles && ok; tile += n_pairs) {
             // B tile fastest: the pairs of a wave share a few A tiles
             const uint32_t tile_a = (tile / tiles_b) * 2u + rank, tile_b = tile % tiles_b;
             for (uint32_t ks = 0; ks < num_ks; ++ks) {
+                ok = tc5::mbar_wait(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, stage);
+                ok = __all_sync(0xffffffffu, ok);
+                if (!ok) break;
                 uint8_t* a = tiles + stage * kStageBytes;
                 const uint32_t kb0 = ks * kSlabs, nsl = min(kSlabs, num_kb - kb0);
-                if (tile != pair || ks >= pre) {
-                    ok = tc5::mbar_wait(&sh->empty[stage], phase ^ 1u, ctx, tc5::kErrEmptyWait, stage);
-                    ok = __all_sync(0xffffffffu, ok);
-                    if (!ok) break;
-                    issue_w(stage, tile_a, kb0, nsl);
-                }
+                // the scale boxes always span kSlabs records (rows past the plane read as zero and count)
+                if (leader)
+                    tc5::mbar_arrive_expect_tx_elect(&sh->full[stage],
+                                                     2u * (nsl * (kABytes + C::kBHalf) + (1u + C::kRec) * kSlabs * kSfBytes));
 #pragma unroll
                 for (uint32_t u = 0; u < kSlabs; ++u)
-                    if (u < nsl)
+                    if (u < nsl) {
+                        tma_load_2d_pair_elect(a + u * kABytes, &tmap_w, &sh->full[stage], (int32_t)((kb0 + u) * BKB),
+                                               (int32_t)(tile_a * BM));
                         tma_load_2d_pair_elect(a + C::kOffB + u * C::kBHalf, &tmap_x, &sh->full[stage], (int32_t)((kb0 + u) * BKB),
                                                (int32_t)(tile_b * BN + rank * C::BNH));
+                    }
+                tma_load_2d_pair_elect(a + C::kOffSfa, &tmap_wsf, &sh->full[stage], 0, (int32_t)((tile_a * num_kb + kb0) * 8u));
 #pragma unroll
                 for (uint32_t j = 0; j < C::kRec; ++j)   // one box of kSlabs records per 128 tokens
                     tma_load_2d_pair_elect(a + C::kOffSfb + j * kSlabs * kSfBytes, &tmap_xsf, &sh->full[stage], 0,
