@@ -21,8 +21,10 @@ enum RowMode : int {
 };
 
 __device__ __forceinline__ uint32_t e4m3x4(const float4& v, float inv) {
-    return (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(v.x * inv, v.y * inv), __NV_SATFINITE, __NV_E4M3) |
-           (uint32_t)__nv_cvt_float2_to_fp8x2(make_float2(v.z * inv, v.w * inv), __NV_SATFINITE, __NV_E4M3) << 16;
+    return (uint32_t)__nv_cvt_float_to_fp8(v.x * inv, __NV_SATFINITE, __NV_E4M3) |
+           (uint32_t)__nv_cvt_float_to_fp8(v.y * inv, __NV_SATFINITE, __NV_E4M3) << 8 |
+           (uint32_t)__nv_cvt_float_to_fp8(v.z * inv, __NV_SATFINITE, __NV_E4M3) << 16 |
+           (uint32_t)__nv_cvt_float_to_fp8(v.w * inv, __NV_SATFINITE, __NV_E4M3) << 24;
 }
 __device__ __forceinline__ float silu_mul(float g, float u) { return (g / (1.0f + expf(-g))) * u; }
 
@@ -33,7 +35,7 @@ f8_row_producer_kernel(float* __restrict__ a, const float* __restrict__ b, const
                        float* __restrict__ xn, uint8_t* __restrict__ q, float* __restrict__ rscale, uint32_t n, float eps,
                        float pscale) {
     __shared__ double warp_sq[32];
-    __shared__ uint32_t warp_max[32];
+    __shared__ float warp_max[32];
     const uint32_t t = threadIdx.x, width = blockDim.x, n4 = n >> 2, lane = t & 31u, warp = t >> 5;
     const size_t row4 = (size_t)blockIdx.x * n4;
     pdk_pdl_launch_dependents();
@@ -87,29 +89,20 @@ f8_row_producer_kernel(float* __restrict__ a, const float* __restrict__ b, const
 #pragma unroll
     for (int c = 0; c < kChunks; ++c)
         amax = fmaxf(amax, fmaxf(fmaxf(fabsf(held[c].x), fabsf(held[c].y)), fmaxf(fabsf(held[c].z), fabsf(held[c].w))));
-    // no NaN gets into amax, and non-negative floats order as their bits: one reduction instruction per warp, one over the warps
-    const uint32_t warp_bits = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
-    if (lane == 0u) warp_max[warp] = warp_bits;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, d));
+    if (lane == 0u) warp_max[warp] = amax;
     __syncthreads();
-    const uint32_t bits = __reduce_max_sync(0xffffffffu, lane < (width >> 5) ? warp_max[lane] : 0u);
-    float scale, inv;
-    if (bits >= (20u << 23) && bits < (255u << 23)) {
-        // m = fr * 2^ex with ex = exponent field - 126 and fr > 0.875 where the mantissa is above 0x600000; 2^e and 2^-e are normal
-        const uint32_t e127 = (bits >> 23) - 126u - 9u + 127u + ((bits & 0x7FFFFFu) > 0x600000u ? 1u : 0u);
-        scale = __uint_as_float(e127 << 23);
-        inv = __uint_as_float((254u - e127) << 23);
-    } else {
-        const float m = __uint_as_float(bits);
-        int e = 0;
-        if (m > 0.0f) {
-            int ex;
-            const float fr = frexpf(m, &ex);
-            e = ex - 9 + (fr > 0.875f ? 1 : 0);
-        }
-        scale = ldexpf(1.0f, e);
-        inv = ldexpf(1.0f, -e);
+    float m = 0.0f;
+    for (uint32_t i = 0; i < (width >> 5); ++i) m = fmaxf(m, warp_max[i]);
+    int e = 0;
+    if (m > 0.0f) {
+        int ex;
+        const float fr = frexpf(m, &ex);
+        e = ex - 9 + (fr > 0.875f ? 1 : 0);
     }
-    if (t == 0u) rscale[blockIdx.x] = scale;
+    if (t == 0u) rscale[blockIdx.x] = ldexpf(1.0f, e);
+    const float inv = ldexpf(1.0f, -e);
     uint32_t* qrow = reinterpret_cast<uint32_t*>(q + (size_t)blockIdx.x * n);
 #pragma unroll
     for (int c = 0; c < kChunks; ++c) {

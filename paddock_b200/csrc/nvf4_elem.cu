@@ -196,7 +196,6 @@ __global__ void nvf4_dequant_kernel(const uint8_t* __restrict__ data, const uint
 // (rows past out_dim read as 0).  One thread per 4-byte word of the output.
 __global__ void nvf4_tile_scales_kernel(const uint8_t* __restrict__ scale, uint32_t* __restrict__ tiled,
                                         uint32_t in_dim, uint32_t out_dim, uint64_t n_words, bool plane) {
-    if (!plane) pdk_pdl_wait_then_launch();   // a call's activation scales: between a quantizer and a GEMM, both dependent launches
     const uint64_t w = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= n_words) return;
     const uint32_t n_slab = in_dim >> 8, kb16 = in_dim >> 4;
@@ -342,9 +341,6 @@ int pdk_nvf4_tile_scales(const void* scale, void* tiled, uint32_t in_dim, uint32
     const uint64_t n_words = (uint64_t)((out_dim + 127u) / 128u) * (in_dim >> 8) * 512u;
     const uint64_t blocks = (n_words + 255u) / 256u;
     if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
-    if (!plane)
-        return pdk_launch_pdl(nvf4_tile_scales_kernel, dim3((uint32_t)blocks), dim3(256), 0, st, (const uint8_t*)scale, (uint32_t*)tiled,
-                              in_dim, out_dim, n_words, plane);
     nvf4_tile_scales_kernel<<<(uint32_t)blocks, 256, 0, st>>>((const uint8_t*)scale, (uint32_t*)tiled, in_dim, out_dim, n_words, plane);
     return pdk_launch_status();
 }
