@@ -61,8 +61,8 @@ def test_quantize_e4m3_row_single_pass_route(pack, rows, n):
 
 
 @pytest.mark.parametrize("field", [0, 1, 2, 8, 19, 20, 21, 126, 127, 135, 253, 254])
-def test_row_scale_from_the_exponent_field(pack, field):
-    """Row maxima around 0.875 * 2^e (mantissa 0x600000) in every class of exponent: both ways to the scale, down to subnormal rows."""
+def test_row_scale_around_every_class_of_exponent(pack, field):
+    """Row maxima around 0.875 * 2^e (mantissa 0x600000) in every class of exponent, down to subnormal rows."""
     n, rng = 256, np.random.default_rng(field)
     rows = []
     for m in (0, 1, 0x5FFFFF, 0x600000, 0x600001, 0x7FFFFF):
