@@ -141,7 +141,7 @@ def _unit_in_gemm(ws, max_blocks, ff, n_expert):
     tokens on 32 experts of 1024 x 768: 20 against 23), but where tiles of one plane would just need a second round over the SMs
     (one token of 4 experts of 2880 x 2880: 31.9 us a block against 30.3)."""
     tiles = max_blocks * ((ff + 127) // 128)
-    return n_expert <= _PAIR_EXPERTS and (ws.bm == 32 or tiles <= ws.sms < 2 * tiles)
+    return _by_pair(ws, n_expert) and (ws.bm == 32 or tiles <= ws.sms < 2 * tiles)
 
 
 class MoeWorkspace:
@@ -197,7 +197,10 @@ def moe_mxfp4_experts(ex, planes, ws, x, rows, alpha=1.702, limit=7.0):
     return 5
 
 
-_PAIR_EXPERTS = 1500      # the most that pdk_moe_align_pos, which knows the pairs' positions, takes
+def _by_pair(ws, n_expert):
+    """Whether the preparations go by (token, slot) pair: pdk_moe_align_pos, which knows the pairs' positions, takes up to 1500
+    experts, pdk_moe_prep_tokens_f4 up to 16 pairs of a token.  Other blocks go by position, through calls without these limits."""
+    return n_expert <= 1500 and ws.n_active <= 16
 
 
 def _route_and_prepare(ex, ws, x, rows, embd, n_expert, max_blocks, natural, logits=None, router_bias=None):
@@ -217,7 +220,7 @@ def _route_and_prepare(ex, ws, x, rows, embd, n_expert, max_blocks, natural, log
     if logits is not None:
         c("moe_topk_batch", logits, router_bias, n_expert, k, ws.idx, ws.w, rows, stream=st)
         n = 3
-    if n_expert > _PAIR_EXPERTS:
+    if not _by_pair(ws, n_expert):
         c("moe_align_bm", ws.idx, ws.sorted_row, ws.sorted_slot, ws.block_expert, rows, k, n_expert, bm, max_blocks, stream=st)
         args = x, None, ws.sorted_row, ws.block_expert, ws.x4q, ws.x4s, ws.x4step, embd, bm, max_blocks, 0, 1.0, 0.0
         c(*(("pdk_moe_prep_act_f4n", *args, 0.0) if natural else ("pdk_moe_prep_act_f4", *args)), stream=st)
@@ -231,7 +234,7 @@ def _route_and_prepare(ex, ws, x, rows, embd, n_expert, max_blocks, natural, log
 def _prepare_unit(ex, ws, x, up, rows, ff, n_expert, max_blocks, mode, natural, alpha, limit, up_add):
     """Term rows for down from what gate|up left: mode 0 the unit's own rows, 1 raw gate and up rows, 2 relu(x)^2."""
     st = _stream()
-    if n_expert <= _PAIR_EXPERTS:
+    if _by_pair(ws, n_expert):
         ex.pack.call("pdk_moe_prep_pairs_f4", x, up, ws.pair_pos, ws.h4q, ws.h4s, ws.h4step, ff, ws.bm, rows * ws.n_active, mode,
                      int(natural), alpha, limit, up_add, stream=st)
         return

@@ -10,8 +10,8 @@ import torch
 
 import oracle
 from paddock_b200 import planes as P
-from gpu_util import dev_f32, rel_l2
-from test_gpu_moe import nvf4_expert_plane
+from gpu_util import dev, dev_f32, rel_l2
+from test_gpu_moe import make_layer, nvf4_expert_plane
 
 pytestmark = pytest.mark.gpu
 
@@ -152,3 +152,25 @@ def test_pairs_without_an_expert_have_no_position(pack):
     torch.cuda.synchronize()
     assert pos.tolist() == [0, -1, 8, -1, 1, 9] and blk.tolist() == [0, 1]
     assert row.tolist() == [0, 4] + [-1] * 6 + [2, 5] + [-1] * 6
+
+
+@pytest.mark.parametrize("bm", [8, 32])
+def test_more_than_sixteen_choices_of_a_token(pack, bm):
+    """The caller's own choices may be more than the by-pair preparation takes of a token: the block then goes by position."""
+    tokens, n_expert, k, embd, ff = 5, 24, 20, 128, 192
+    ex = P.GpuExecutor(pack)
+    raw, _ = make_layer(n_expert, embd, ff, 1500, False)
+    planes = P.prepare_tc5(ex, P.MoeMxfp4Planes(*(P.repack_mxfp4(ex, dev(raw[n])) for n in ("gate", "up", "down")), n_expert, embd, ff))
+    x = oracle.bf16_round(oracle.fill_normal(tokens * embd, 1501, 1.0))
+    rng = np.random.default_rng(1502)
+    idx = np.stack([rng.permutation(n_expert)[:k] for _ in range(tokens)]).astype(np.uint32)
+    w = (rng.random((tokens, k)) / k).astype(np.float32)
+    ws = P.MoeWorkspace(ex, planes, tokens, k, bm)
+    ws.idx.view(torch.uint8).copy_(dev(idx))
+    ws.w.copy_(dev_f32(w).view(-1))
+    P.moe_mxfp4_experts_tc5(ex, planes, ws, dev_f32(x), tokens)
+    torch.cuda.synchronize()
+    assert pack.device_error() == 0
+    ref = oracle.moe_mxfp4_layer(raw["gate"], raw["up"], raw["down"], x, idx, w, tokens, k, embd, ff, None, None, None)
+    y = ws.part.cpu().numpy().reshape(tokens, k, embd).astype(np.float64).sum(axis=1)
+    assert rel_l2(y, ref) < 2e-3
