@@ -424,7 +424,8 @@ int pdk_mxfp4_tc5_tile_scales(const void* scale, void* tiled, void* meta, uint32
  * xq u8[max_blocks*4*bm][dim/2], term t of position p in row p/8*32 + t*8 + p%8; xs
  * u8[max_blocks][ceil(dim/256)][2048] (scale records, the layout of the tiled weight scales; a record holds
  * four groups of eight positions: one block of 32, or four consecutive blocks of 8 of one expert, counted from
- * the expert's first, in the first one's record; zero the buffer once); xstep f32[max_blocks*bm]. */
+ * the expert's first, in the first one's record; zero the buffer once); xstep f32[max_blocks*bm].
+ * The GEMMs want xq and xs on 16-byte boundaries. */
 int pdk_moe_prep_act_f4(const void* x, const void* up, const void* sorted_row, const void* block_expert, void* xq,
                         void* xs, void* xstep, uint32_t dim, uint32_t bm, uint32_t max_blocks, uint32_t mode, float alpha, float limit,
                         void* stream);

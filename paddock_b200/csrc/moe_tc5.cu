@@ -722,7 +722,7 @@ static int gemm_impl(const PlaneArgs& w0, const PlaneArgs& w1, void* out0, void*
     if (max_blocks == 0 || out_dim == 0 || n_expert == 0) return 0;
     if (in_dim == 0 || (in_dim & 63u) != 0u || (bm != 8u && bm != 32u) || max_blocks > moe_gemm::kMaxBlocks)
         return cudaErrorInvalidValue;
-    if (!pdk_aligned(w0.data, 16) || !pdk_aligned(w0.sf, 16) || !pdk_aligned(r.xq, 16) || !pdk_aligned(r.xs, 4) ||
+    if (!pdk_aligned(w0.data, 16) || !pdk_aligned(w0.sf, 16) || !pdk_aligned(r.xq, 16) || !pdk_aligned(r.xs, 16) ||
         !pdk_aligned(w0.scale2, 4) || (w1.data && (!pdk_aligned(w1.data, 16) || !pdk_aligned(w1.sf, 16))))
         return cudaErrorInvalidValue;
     const uint32_t ahead = kind & kAhead ? 1u : 0u;
