@@ -606,7 +606,7 @@ PDK_EXPORT int pdk_moe_prep_act_f4(const void* x, const void* up, const void* so
 PDK_EXPORT int pdk_moe_prep_tokens_f4(const void* x, const void* pair_pos, void* xq, void* xs, void* xstep, uint32_t dim, uint32_t k,
                                       uint32_t rows, uint32_t bm, uint32_t natural, void* stream) {
     if (rows == 0 || k == 0) return 0;
-    if (dim == 0 || (dim & 31u) != 0u || (bm != 8u && bm != 32u) || natural > 1u || k > 16u) return cudaErrorInvalidValue;
+    if (dim == 0 || (dim & 31u) != 0u || (bm != 8u && bm != 32u) || natural > 1u || k > 16u || !pair_pos) return cudaErrorInvalidValue;
     if (!pdk_aligned(x, 16) || !pdk_aligned(xq, 16) || !pdk_aligned(xs, 16)) return cudaErrorInvalidValue;
     TokenArgs a{};
     a.x = (const float*)x; a.pair_pos = (const uint32_t*)pair_pos; a.xq = (uint8_t*)xq; a.xs = (uint8_t*)xs; a.xstep = (float*)xstep;
@@ -621,7 +621,7 @@ PDK_EXPORT int pdk_moe_prep_pairs_f4(const void* x, const void* up, const void* 
                                      uint32_t bm, uint32_t pairs, uint32_t mode, uint32_t natural, float alpha, float limit, float up_add,
                                      void* stream) {
     if (pairs == 0) return 0;
-    if (dim == 0 || (dim & 31u) != 0u || (bm != 8u && bm != 32u) || natural > 1u || mode > 2u) return cudaErrorInvalidValue;
+    if (dim == 0 || (dim & 31u) != 0u || (bm != 8u && bm != 32u) || natural > 1u || mode > 2u || !pair_pos) return cudaErrorInvalidValue;
     if (!pdk_aligned(x, 16) || !pdk_aligned(xq, 16) || !pdk_aligned(xs, 16) || (mode == 1u && (!up || !pdk_aligned(up, 16))))
         return cudaErrorInvalidValue;
     TokenArgs a{};
@@ -662,7 +662,7 @@ PDK_EXPORT int pdk_moe_route_few(const void* logits, const void* router_bias, vo
                                  uint32_t max_blocks, void* stream) {
     if (rows == 0 || max_blocks == 0) return 0;
     if (rows > 8u || k == 0 || k > 16u || rows * k > 32u || n_expert == 0 || n_expert > 512u || k > n_expert ||
-        max_blocks > 32u || (bm != 8u && bm != 32u) || max_blocks * bm > kRouteMaxPos)
+        max_blocks > 32u || (bm != 8u && bm != 32u) || max_blocks * bm > kRouteMaxPos || !pair_pos)
         return cudaErrorInvalidValue;
     RouteArgs r{};
     r.logits = (const float*)logits; r.bias = (const float*)router_bias;

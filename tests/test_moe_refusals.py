@@ -31,3 +31,11 @@ def test_gemm_refuses_scale_records_that_bulk_copies_cannot_read(name, off):
     else:
         args = (A, A, A, None, A) + (None,) * 5 + rows + (None, None, 256, 128, 4, 8, 4, 2, 0)
     assert status(name, *args) == INVALID
+
+
+def test_by_pair_calls_refuse_a_missing_position_table():
+    """pdk_moe_align_pos refuses it too; the launches would read or write at address 0."""
+    assert status("pdk_moe_align_pos", A, A, A, A, None, 4, 2, 8, 8, 8) == INVALID
+    assert status("pdk_moe_route_few", A, None, A, A, A, A, A, None, 8, 2, 4, 8, 8) == INVALID
+    assert status("pdk_moe_prep_tokens_f4", A, None, A, A, A, 256, 2, 4, 8, 0) == INVALID
+    assert status("pdk_moe_prep_pairs_f4", A, None, None, A, A, A, 256, 8, 8, 0, 0, 1.0, 7.0, 0.0) == INVALID
