@@ -456,7 +456,9 @@ int pdk_mxfp4_moe_gemm_tc5(const void* w0_data, const void* w0_sf, const void* w
                            uint32_t out_dim, uint32_t n_expert, uint32_t bm, uint32_t max_blocks, uint32_t n_active,
                            uint32_t scatter, void* stream);
 /* The same directly behind a pdk_moe_prep_* call that came after the launch which wrote the tables: they, and the weights,
- * are read while the preparation still runs.  Not behind a kernel that writes block_expert, sorted_row or sorted_slot. */
+ * are read while the preparation still runs.  That is sound because a preparation lets the next launch begin only when everything
+ * in front of itself is complete, and the tables are read past the first-level cache.  Not behind a kernel that writes
+ * block_expert, sorted_row, sorted_slot or a weight plane. */
 int pdk_mxfp4_moe_gemm_tc5_ahead(const void* w0_data, const void* w0_sf, const void* w0_meta, const void* w0_bias, void* out0,
                                  const void* w1_data, const void* w1_sf, const void* w1_meta, const void* w1_bias, void* out1,
                                  const void* xq, const void* xs, const void* xstep, const void* block_expert,

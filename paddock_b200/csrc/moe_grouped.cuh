@@ -112,17 +112,22 @@ __device__ __forceinline__ void build_tiles(const Args& a, const uint32_t* s_exp
     if (lane == 0u) { sh->tiles = count; sh->widest = widest; }
 }
 
+// The routing tables past the first-level cache.  With `ahead` they are read before this kernel's own griddepcontrol.wait: the
+// kernel in front began only when the one that wrote them was complete (it waits before it lets this one in), so L2 has them, but
+// nothing clears a line that an earlier launch left in this SM's first level before that wait.
+__device__ __forceinline__ uint32_t table_word(const uint32_t* p) { return __ldcg(p); }
+
 // The same for calls of up to 32 blocks: every warp for itself, from global memory straight into a table of its own, so
 // nothing waits for another warp (1.1 us of a call of one token's).
 template <uint32_t MAXG>
 __device__ __forceinline__ uint32_t build_tiles_warp(const Args& a, uint32_t* s_expert, uint32_t* s_tile, uint32_t& widest, bool& once) {
     const uint32_t lane = threadIdx.x & 31u, shift = a.block_shift;
-    const uint32_t e = lane < a.max_blocks ? a.block_expert[lane] : PDK_MOE_PAD;
+    const uint32_t e = lane < a.max_blocks ? table_word(a.block_expert + lane) : PDK_MOE_PAD;
     const bool used = e != PDK_MOE_PAD;
     uint32_t live = 1;
     if (shift && used) {
 #pragma unroll
-        for (uint32_t g = 1; g < 4u; ++g) live += a.sorted_row[lane * 32u + g * 8u] != PDK_MOE_PAD;
+        for (uint32_t g = 1; g < 4u; ++g) live += table_word(a.sorted_row + lane * 32u + g * 8u) != PDK_MOE_PAD;
     }
     const uint32_t prev = __shfl_up_sync(0xffffffffu, e, 1);
     const uint32_t starts = __ballot_sync(0xffffffffu, lane == 0u || e != prev);
@@ -504,12 +509,12 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constan
         __syncthreads();
     } else {
         for (uint32_t i = threadIdx.x; i < a.max_blocks; i += blockDim.x) {
-            const uint32_t e = a.block_expert[i];
+            const uint32_t e = table_word(a.block_expert + i);
             s_expert[i] = e;
             if (a.block_shift && e != PDK_MOE_PAD) {   // a 32-token block's padding is at its end
                 uint32_t live = 1;
 #pragma unroll
-                for (uint32_t g = 1; g < 4u; ++g) live += a.sorted_row[i * 32u + g * 8u] != PDK_MOE_PAD;
+                for (uint32_t g = 1; g < 4u; ++g) live += table_word(a.sorted_row + i * 32u + g * 8u) != PDK_MOE_PAD;
                 s_live[i] = (uint8_t)live;
             }
         }

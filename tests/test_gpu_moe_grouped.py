@@ -174,3 +174,49 @@ def test_more_than_sixteen_choices_of_a_token(pack, bm):
     ref = oracle.moe_mxfp4_layer(raw["gate"], raw["up"], raw["down"], x, idx, w, tokens, k, embd, ff, None, None, None)
     y = ws.part.cpu().numpy().reshape(tokens, k, embd).astype(np.float64).sum(axis=1)
     assert rel_l2(y, ref) < 2e-3
+
+
+@pytest.mark.parametrize("tokens,n_expert,k,embd,ff,bm,fmt", [
+    (1, 64, 4, 512, 384, 8, "mxfp4"),        # up to 32 blocks: every warp builds the tile table; top-k and alignment in one launch
+    (8, 16, 4, 256, 192, 8, "nvfp4"),
+    (40, 4, 2, 256, 192, 32, "nvfp4"),       # up to 32 blocks of 32
+    (60, 32, 4, 320, 256, 8, "mxfp4"),       # more than 32 blocks: one warp builds it
+    (300, 16, 4, 256, 320, 32, "nvfp4"),
+])
+@pytest.mark.parametrize("graph", [False, True])
+def test_blocks_of_different_routing_in_a_row(pack, tokens, n_expert, k, embd, ff, bm, fmt, graph):
+    """Calls on one workspace with other logits each time and nothing between them give the bits of calls by themselves: the GEMMs
+    read the routing tables before their own wait for the kernel in front, on SMs that read the call before's."""
+    ex = P.GpuExecutor(pack)
+    shape = P.MoeMxfp4Planes(None, None, None, n_expert, embd, ff)
+    if fmt == "nvfp4":
+        planes = tuple(nvf4_expert_plane(ex, n_expert, r, c, s)[0] for r, c, s in ((ff, embd, 1000), (ff, embd, 2000), (embd, ff, 3000)))
+        forward = lambda *a: P.moe_nvf4_forward(ex, *planes, *a)
+    else:
+        raw, _ = make_layer(n_expert, embd, ff, 1600, False)
+        shape = P.prepare_tc5(ex, P.MoeMxfp4Planes(*(P.repack_mxfp4(ex, dev(raw[n])) for n in ("gate", "up", "down")), n_expert, embd, ff))
+        forward = lambda *a: P.moe_mxfp4_forward(ex, shape, *a)
+    calls = 12
+    # skewed one way and the other, so that runs and tiles change from call to call
+    tilt = np.linspace(-2.0, 2.0, n_expert, dtype=np.float32)
+    logits = [dev_f32(oracle.fill_normal(tokens * n_expert, 1700 + i, 1.0).reshape(tokens, n_expert) + tilt * (i % 3 - 1)).view(-1)
+              for i in range(calls)]
+    xs = [dev_f32(oracle.bf16_round(oracle.fill_normal(tokens * embd, 1800 + i, 1.0))) for i in range(calls)]
+    alone, row = (torch.zeros(calls, tokens * embd, device="cuda") for _ in range(2))
+    for i in range(calls):
+        forward(P.MoeWorkspace(ex, shape, tokens, k, bm), xs[i], logits[i], alone[i])
+        torch.cuda.synchronize()
+    ws = P.MoeWorkspace(ex, shape, tokens, k, bm)
+    every = lambda: [forward(ws, xs[i], logits[i], row[i]) for i in range(calls)]
+    every()
+    torch.cuda.synchronize()
+    if graph:
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            every()
+        for _ in range(3):
+            row.zero_()
+            g.replay()
+        torch.cuda.synchronize()
+    assert pack.device_error() == 0
+    assert bool(alone.any(dim=1).all()) and torch.equal(row, alone)
