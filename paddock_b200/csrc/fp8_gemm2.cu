@@ -180,7 +180,7 @@ f8row_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_
         for (uint32_t tile = pair; tile < n_tiles && ok; tile += n_pairs, ++iter) {
             const uint32_t buf = iter & 1u, aphase = (iter >> 1) & 1u;
             const uint32_t m0 = (tile % tiles_m) * 2u * BM + rank * BM, n0 = (tile / tiles_m) * BN;
-            ok = tc5::mbar_wait(&sh->tmem_full[buf], aphase, ctx, tc5::kErrTmemFullWait, buf);
+            ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->tmem_full[buf], aphase, ctx, tc5::kErrTmemFullWait, buf));
             if (!ok) break;
             tc5::fence_after_sync();
             const uint32_t t = m0 + quarter * 32u + lane;

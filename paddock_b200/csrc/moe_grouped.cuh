@@ -414,9 +414,8 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
                 bias[s] = (n < a.out_dim && a.bias[p]) ? a.bias[p][(size_t)expert * a.out_dim + n] : 0.0f;
             }
             float* out = a.out[t.plane];
-            ok = wait_for(&sh->tmem_full[buf], aphase, ctx, tc5::kErrTmemFullWait, buf);
+            ok = __all_sync(0xffffffffu, wait_for(&sh->tmem_full[buf], aphase, ctx, tc5::kErrTmemFullWait, buf));
             if (!ok) break;
-            __syncwarp();
             tc5::fence_after_sync();
 #pragma unroll 1
             for (uint32_t g = share, from = 0; g < ng; g += kShare, from += 8u) {
@@ -468,6 +467,7 @@ __global__ void __launch_bounds__(96u + 32u * EPI, 1)
 grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
                const __grid_constant__ CUtensorMap tmap_x, const Args a) {
     static_assert(EPI % 4u == 0u && (KIND == kGated) == (NA == 2u), "whole sets of four lane quarters; gate and up, or one plane");
+    static_assert(MAXG <= EPI, "a warp's lanes hold the routing data of four groups: EPI / 4 shares of up to four");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* rings = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
     Ctl* sh = reinterpret_cast<Ctl*>(rings + kRing);

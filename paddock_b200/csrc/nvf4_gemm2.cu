@@ -277,7 +277,7 @@ nvf4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                 if (threadIdx.x == 64u) tc5::tma_store_wait_read();
                 asm volatile("bar.sync 2, 256;" ::: "memory");
             }
-            ok = tc5::mbar_wait(&sh->tmem_full[buf], aphase, ctx, tc5::kErrTmemFullWait, buf);
+            ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->tmem_full[buf], aphase, ctx, tc5::kErrTmemFullWait, buf));
             if (!ok) break;
             tc5::fence_after_sync();
             auto put_group = [&](uint32_t g, const uint32_t (&ra)[32], const uint32_t (&rb)[32]) {
