@@ -278,7 +278,12 @@ nvf4_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_c
                 asm volatile("bar.sync 2, 256;" ::: "memory");
             }
             ok = __all_sync(0xffffffffu, tc5::mbar_wait(&sh->tmem_full[buf], aphase, ctx, tc5::kErrTmemFullWait, buf));
-            if (!ok) break;
+            if (!ok) {
+                // the other warps go on to barrier 2, which waits without a limit: come to every meeting that is left
+                if (tma_out)
+                    for (uint32_t left = 2u * ((n_tiles - 1u - tile) / n_pairs) + 1u; left; --left) asm volatile("bar.sync 2, 256;" ::: "memory");
+                break;
+            }
             tc5::fence_after_sync();
             auto put_group = [&](uint32_t g, const uint32_t (&ra)[32], const uint32_t (&rb)[32]) {
                 if (tma_out) {

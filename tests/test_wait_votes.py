@@ -40,3 +40,20 @@ def test_the_waits_are_found():
     for name, least in (("moe_grouped.cuh", 5), ("q4k_tc5.cu", 8), ("fp8_gemm2.cu", 4), ("nvf4_gemm2.cu", 4), ("splitk_gemm.cu", 4),
                         ("gemv_ring.cu", 6), ("kq_batch.cu", 1), ("q4k_batch_i8.cu", 1)):
         assert count[name] >= least, (name, count)
+
+
+def test_a_warp_that_gave_up_still_comes_to_the_named_barriers():
+    """The NVFP4 pair kernel's eight epilogue warps meet at a named barrier before and after they fill the output box, and bar.sync
+    has no limit: a warp whose accumulator never came must come to all meetings that are left before it leaves the loop."""
+    text = open(os.path.join(CSRC, "nvf4_gemm2.cu")).read()
+    body = text[text.index("epilogue (both CTAs"):text.index("tma_store_wait_all()")]
+    assert [body.count(c) for c in ("bar.sync 2, 256;", "break;")] == [3, 1]
+    gave_up = body[body.index("if (!ok) {"):body.index("break;")]
+    left = re.search(r"for \(uint32_t left = ([^;]*); left; --left\) asm volatile\(\"bar.sync 2, 256;\"", gave_up).group(1)
+    left = left.replace("u ", " ").replace("u;", "").replace("1u", "1").replace("/", "//")
+    for n_pairs in (1, 3, 74):
+        for n_tiles in (1, 2, 74, 75, 300):
+            for pair in range(min(n_pairs, n_tiles)):
+                tiles = list(range(pair, n_tiles, n_pairs))
+                for i, tile in enumerate(tiles):      # gave up in tile i, between its two meetings
+                    assert eval(left, {}, {"n_tiles": n_tiles, "tile": tile, "n_pairs": n_pairs}) == 1 + 2 * (len(tiles) - 1 - i)
