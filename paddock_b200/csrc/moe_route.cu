@@ -270,14 +270,20 @@ moe_prep_act_kernel(const float* __restrict__ x, uint8_t* __restrict__ xq, float
 }
 
 // ---------------------------------------------------------------- slot combine
-// A thread per four columns of a row (grid y); the slots' loads of a thread are in flight together, four at a time.
+// A thread per four columns of a row; the slots' loads of a thread are in flight together, four at a time.  Bound by memory where
+// rows are many.  Where they are narrow too, a block takes several (NARROW, up to 512 columns and from 1024 rows on), and no call
+// has more than 16 blocks per SM: a block per row starts blocks and does little else (70000 rows of 32 columns 68 -> 4.1 us, 5000 of
+// 64, 8 slots, 5.7 -> 2.4, 5000 of 516 5.85 -> 4.8; 1024 of 2880, 4 slots, 5.5 either way; several rows a block cost 64 rows of
+// 128 columns 1.4 -> 1.56).
+template <bool NARROW>
 __global__ void __launch_bounds__(256)
 moe_slot_combine_kernel(const float4* __restrict__ part, float4* __restrict__ residual, uint32_t embd4, uint32_t n_active,
                         uint32_t rows) {
     pdk_pdl_wait_then_launch();   // dependent launch: may start while the previous kernel of the stream drains
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= embd4) return;
-    for (size_t t = blockIdx.y; t < rows; t += gridDim.y) {
+    const uint32_t step = NARROW ? gridDim.y * blockDim.y : gridDim.y;
+    for (size_t t = NARROW ? blockIdx.y * blockDim.y + threadIdx.y : blockIdx.y; t < rows; t += step) {
         const float4* p = part + t * n_active * embd4 + r;
         float4 d = residual[t * embd4 + r];
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
@@ -381,7 +387,12 @@ PDK_EXPORT int pd_moe_slot_combine(const void* part, void* residual, uint32_t em
                                    void* stream) {
     if (rows == 0 || embd == 0) return 0;
     if ((embd & 3u) != 0u || !pdk_aligned(part, 16) || !pdk_aligned(residual, 16)) return cudaErrorInvalidValue;
-    const uint32_t embd4 = embd >> 2, threads = embd4 < 256u ? (embd4 + 31u) & ~31u : 256u;
-    return pdk_launch_pdl(moe_slot_combine_kernel, dim3((embd4 + threads - 1u) / threads, rows < 65535u ? rows : 65535u), dim3(threads),
-                          0, (cudaStream_t)stream, (const float4*)part, (float4*)residual, embd4, n_active, rows);
+    const uint32_t embd4 = embd >> 2, nx = (embd4 + 255u) / 256u;
+    const bool narrow = embd4 <= 128u && rows >= 1024u;
+    const uint32_t cols = narrow ? embd4 : ((embd4 + nx - 1u) / nx + 31u) & ~31u, rows_per_block = narrow ? 256u / cols : 1u;
+    const uint64_t blocks = ((uint64_t)rows + rows_per_block - 1u) / rows_per_block;
+    const uint32_t cap = (16u * (uint32_t)pdk_sm_count() + nx - 1u) / nx;
+    return pdk_launch_pdl(narrow ? moe_slot_combine_kernel<true> : moe_slot_combine_kernel<false>,
+                          dim3(nx, (uint32_t)(blocks < cap ? blocks : cap)), dim3(cols, rows_per_block), 0, (cudaStream_t)stream,
+                          (const float4*)part, (float4*)residual, embd4, n_active, rows);
 }

@@ -220,3 +220,25 @@ def test_blocks_of_different_routing_in_a_row(pack, tokens, n_expert, k, embd, f
         torch.cuda.synchronize()
     assert pack.device_error() == 0
     assert bool(alone.any(dim=1).all()) and torch.equal(row, alone)
+
+
+@pytest.mark.parametrize("rows,k,embd", [
+    (1, 1, 4), (5, 3, 1020), (1023, 4, 512),
+    (1024, 4, 512), (1024, 5, 516),           # both sides of several rows a block; the last of them has none left over
+    (3001, 9, 36), (20001, 2, 4),             # rows of no whole number of warps; a row of four columns
+    (2500, 1, 1028), (5000, 2, 640),          # more rows than blocks
+    (2400, 4, 260),
+])
+def test_slot_combine_adds_every_row_once(pack, rows, k, embd):
+    """residual += the slots' rows, added up in slot order: bit for bit, and nothing behind the last row."""
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    part = torch.randn(rows, k, embd, device="cuda", generator=g)
+    res = torch.randn(rows + 3, embd, device="cuda", generator=g)
+    acc = torch.zeros(rows, embd, device="cuda")
+    for s in range(k):
+        acc = acc + part[:, s]
+    want = res.clone()
+    want[:rows] += acc
+    pack.call("moe_slot_combine", part, res, embd, k, rows)
+    torch.cuda.synchronize()
+    assert pack.device_error() == 0 and torch.equal(res, want)
