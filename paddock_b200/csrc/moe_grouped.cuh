@@ -35,7 +35,7 @@ struct Args {
 // that finds no room here starts when this one has left (a ring of 216 KB cost a block of one token 0.4 us).
 constexpr uint32_t kRing = 196u * 1024u, kMaxSlots = 10u;
 constexpr uint32_t kMaxBlocks = 1024;  // block_expert[] and the tile table are kept in shared memory
-constexpr size_t kTableBytes = kMaxBlocks * 9u;   // experts, tiles, live groups
+constexpr size_t kTableBytes = kMaxBlocks * 8u;   // experts, tiles, groups by block, live groups
 
 // W groups per tile at most, NA weight tiles of 128 rows under one B.  NA = 2 (gate and up): one pair of accumulators.  NA = 1:
 // two accumulators, the next tile's MMAs run under this one's epilogue.  A stage of the ring is KS slabs (256 elements) of the
@@ -59,68 +59,89 @@ struct Ctl {
     uint64_t full[kMaxSlots], empty[kMaxSlots], tmem_full[2], tmem_empty[2];
     uint32_t tmem_base;
     int abort_flag;
-    uint32_t tiles, widest;   // of the call: how many, and the most groups of one
+    uint32_t starts[kMaxBlocks / 32u], counts[kMaxBlocks / 32u], widths[kMaxBlocks / 32u];   // of 32 blocks each, for the tile table
 };
 
 // tile word: first group | live groups << 13
 __device__ __forceinline__ uint32_t tile_group(uint32_t t) { return t & 0x1FFFu; }
 __device__ __forceinline__ uint32_t tile_ng(uint32_t t) { return t >> 13; }
 
-// The tiles of a call, one warp.  A run = the consecutive blocks of one expert.  Every four groups are a tile; with MAXG = 6 the
-// last one takes a rest of up to six (a rest of one or two groups is not worth a pass over the weights).  Tiles start at a scale
-// record's first group: an MMA takes its scales from an even tensor-memory column, an odd one is a misaligned address.
-template <uint32_t MAXG>
-__device__ __forceinline__ void build_tiles(const Args& a, const uint32_t* s_expert, const uint8_t* s_live, uint32_t* s_tile, Ctl* sh) {
-    static_assert(MAXG == 4u || MAXG == 6u, "tiles start at whole records");
-    const uint32_t lane = threadIdx.x & 31u, nb = a.max_blocks, shift = a.block_shift;
-    uint32_t count = 0, widest = 0, carry_e = PDK_MOE_PAD, carry_s = 0;
-    for (uint32_t c = 0; c < nb; c += 32u) {
-        const uint32_t b = c + lane;
-        const uint32_t e = b < nb ? s_expert[b] : PDK_MOE_PAD;
-        uint32_t prev = __shfl_up_sync(0xffffffffu, e, 1);
-        if (lane == 0u) prev = carry_e;
-        const uint32_t starts = __ballot_sync(0xffffffffu, e != prev);
-        const uint32_t mine = starts & (0xffffffffu >> (31u - lane));
-        const uint32_t first = mine ? c + 31u - __clz(mine) : carry_s;   // the run's first block
-        carry_e = __shfl_sync(0xffffffffu, e, 31);
-        carry_s = __shfl_sync(0xffffffffu, first, 31);
-        uint32_t ng = 0;
-        if (e != PDK_MOE_PAD) {
-            auto same = [&](uint32_t bb) { return bb < nb && s_expert[bb] == e; };
-            if (shift == 0u) {
-                uint32_t r = 1;                                          // groups of the run from here on, up to MAXG + 1
-                while (r <= MAXG && same(b + r)) ++r;
-                if (((b - first) & 3u) == 0u) ng = MAXG > 4u && b != first && r <= MAXG - 4u ? 0u : r <= MAXG ? r : 4u;
-            } else {
-                // live groups of a block: all four, but for the run's last one
-                auto live = [&](uint32_t bb) { return same(bb + 1u) ? 4u : (uint32_t)s_live[bb]; };
-                ng = live(b);
-                if (MAXG > 4u) {
-                    if (b != first && !same(b + 1u) && ng <= MAXG - 4u) ng = 0u;
-                    else if (same(b + 1u) && !same(b + 2u)) {
-                        const uint32_t next = live(b + 1u);
-                        if (next <= MAXG - 4u) ng = 4u + next;
-                    }
-                }
-            }
-        }
-        const uint32_t tiles = __ballot_sync(0xffffffffu, ng != 0u);
-        if (ng) s_tile[count + __popc(tiles & ((1u << lane) - 1u))] = (b << shift) | (ng << 13);
-        count += __popc(tiles);
-        widest = max(widest, __reduce_max_sync(0xffffffffu, ng));
-    }
-    if (lane == 0u) { sh->tiles = count; sh->widest = widest; }
-}
-
 // The routing tables past the first-level cache.  With `ahead` they are read before this kernel's own griddepcontrol.wait: the
 // kernel in front began only when the one that wrote them was complete (it waits before it lets this one in), so L2 has them, but
 // nothing clears a line that an earlier launch left in this SM's first level before that wait.
 __device__ __forceinline__ uint32_t table_word(const uint32_t* p) { return __ldcg(p); }
 
+// Groups of the tile that starts at block b, 0 where none does; r: blocks of the run from b on (counted up to MAXG + 1), from_first:
+// blocks of the run before b, live / next_live: live groups of b and of the block behind it.  A run = the consecutive blocks of one
+// expert.  Every four groups are a tile; with MAXG = 6 the last one takes a rest of up to six (a rest of one or two groups is not
+// worth a pass over the weights).  Tiles start at a scale record's first group: an MMA takes its scales from an even tensor-memory
+// column, an odd one is a misaligned address.
+template <uint32_t MAXG>
+__device__ __forceinline__ uint32_t tile_groups(uint32_t shift, uint32_t from_first, uint32_t r, uint32_t live, uint32_t next_live) {
+    static_assert(MAXG == 4u || MAXG == 6u, "tiles start at whole records");
+    if (shift == 0u) return (from_first & 3u) != 0u || (MAXG > 4u && from_first && r <= MAXG - 4u) ? 0u : r <= MAXG ? r : 4u;
+    if (MAXG > 4u && from_first && r == 1u && live <= MAXG - 4u) return 0u;
+    if (MAXG > 4u && r == 2u && next_live <= MAXG - 4u) return 4u + next_live;
+    return r > 1u ? 4u : live;
+}
+
+// The tile table of a call, the whole CTA; a warp takes 32 blocks at a time.  (One warp for all of them took 0.33 us per 32 blocks, all
+// of it in front of the first MMA where nothing hides it: down at K = 512, N = 384, 32 experts, 12800 pairs on 430 blocks 24.9 us, in
+// this form 20.8.)
+template <uint32_t MAXG>
+__device__ __forceinline__ uint32_t build_tiles(const Args& a, uint32_t* s_expert, uint16_t* s_tile, uint8_t* s_ng, uint8_t* s_live,
+                                                Ctl* sh, uint32_t& widest) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5, nb = a.max_blocks, shift = a.block_shift;
+    const uint32_t chunks = (nb + 31u) >> 5;
+    for (uint32_t b = threadIdx.x; b < nb; b += blockDim.x) {
+        const uint32_t e = table_word(a.block_expert + b);
+        s_expert[b] = e;
+        if (shift && e != PDK_MOE_PAD) {   // a 32-token block's padding is at its end
+            uint32_t live = 1;
+#pragma unroll
+            for (uint32_t g = 1; g < 4u; ++g) live += table_word(a.sorted_row + b * 32u + g * 8u) != PDK_MOE_PAD;
+            s_live[b] = (uint8_t)live;
+        }
+    }
+    __syncthreads();
+    auto expert_at = [&](uint32_t b) { return b < nb ? s_expert[b] : PDK_MOE_PAD; };
+    for (uint32_t c = warp; c < chunks; c += nwarp) {
+        const uint32_t b = c * 32u + lane;
+        const uint32_t starts = __ballot_sync(0xffffffffu, b == 0u || expert_at(b) != expert_at(b - 1u));
+        if (lane == 0u) sh->starts[c] = starts;
+    }
+    __syncthreads();
+    auto groups_at = [&](uint32_t c) {
+        const uint32_t b = c * 32u + lane, e = expert_at(b);
+        if (e == PDK_MOE_PAD) return 0u;
+        uint32_t q = c, mine = sh->starts[c] & (0xffffffffu >> (31u - lane));
+        while (mine == 0u) mine = sh->starts[--q];     // bit 0 of the first word is set
+        const uint32_t from_first = b - (q * 32u + 31u - __clz(mine));
+        uint32_t r = 1;
+        while (r <= MAXG && expert_at(b + r) == e) ++r;
+        const uint32_t live = shift ? s_live[b] : 1u, next_live = shift && r > 1u ? s_live[b + 1u] : 1u;
+        return tile_groups<MAXG>(shift, from_first, r, live, next_live);
+    };
+    for (uint32_t c = warp; c < chunks; c += nwarp) {
+        const uint32_t ng = groups_at(c), tiles = __ballot_sync(0xffffffffu, ng != 0u), most = __reduce_max_sync(0xffffffffu, ng);
+        if (c * 32u + lane < nb) s_ng[c * 32u + lane] = (uint8_t)ng;
+        if (lane == 0u) { sh->counts[c] = __popc(tiles); sh->widths[c] = most; }
+    }
+    __syncthreads();
+    const uint32_t count = lane < chunks ? sh->counts[lane] : 0u;
+    widest = __reduce_max_sync(0xffffffffu, lane < chunks ? sh->widths[lane] : 0u);
+    for (uint32_t c = warp; c < chunks; c += nwarp) {
+        const uint32_t b = c * 32u + lane, ng = b < nb ? s_ng[b] : 0u, before = __reduce_add_sync(0xffffffffu, lane < c ? count : 0u);
+        const uint32_t tiles = __ballot_sync(0xffffffffu, ng != 0u);
+        if (ng) s_tile[before + __popc(tiles & ((1u << lane) - 1u))] = (uint16_t)((b << shift) | (ng << 13));
+    }
+    return __reduce_add_sync(0xffffffffu, count);
+}
+
 // The same for calls of up to 32 blocks: every warp for itself, from global memory straight into a table of its own, so
 // nothing waits for another warp (1.1 us of a call of one token's).
 template <uint32_t MAXG>
-__device__ __forceinline__ uint32_t build_tiles_warp(const Args& a, uint32_t* s_expert, uint32_t* s_tile, uint32_t& widest, bool& once) {
+__device__ __forceinline__ uint32_t build_tiles_warp(const Args& a, uint32_t* s_expert, uint16_t* s_tile, uint32_t& widest, bool& once) {
     const uint32_t lane = threadIdx.x & 31u, shift = a.block_shift;
     const uint32_t e = lane < a.max_blocks ? table_word(a.block_expert + lane) : PDK_MOE_PAD;
     const bool used = e != PDK_MOE_PAD;
@@ -135,19 +156,10 @@ __device__ __forceinline__ uint32_t build_tiles_warp(const Args& a, uint32_t* s_
     const uint32_t later = lane == 31u ? 0u : starts >> (lane + 1u);               // runs that start behind this block
     const uint32_t r = later ? (uint32_t)__ffs(later) : 32u - lane;                // blocks of the run from here on
     const uint32_t next_live = __shfl_down_sync(0xffffffffu, live, 1);
-    uint32_t ng = 0;
-    if (used && shift == 0u) {
-        if (((lane - first) & 3u) == 0u) ng = MAXG > 4u && lane != first && r <= MAXG - 4u ? 0u : r <= MAXG ? r : 4u;
-    } else if (used) {
-        ng = r > 1u ? 4u : live;
-        if (MAXG > 4u) {
-            if (lane != first && r == 1u && ng <= MAXG - 4u) ng = 0u;
-            else if (r == 2u && next_live <= MAXG - 4u) ng = 4u + next_live;
-        }
-    }
+    const uint32_t ng = used ? tile_groups<MAXG>(shift, lane - first, r, live, next_live) : 0u;
     const uint32_t tiles = __ballot_sync(0xffffffffu, ng != 0u);
     s_expert[lane] = e;
-    if (ng) s_tile[__popc(tiles & ((1u << lane) - 1u))] = (lane << shift) | (ng << 13);
+    if (ng) s_tile[__popc(tiles & ((1u << lane) - 1u))] = (uint16_t)((lane << shift) | (ng << 13));
     widest = __reduce_max_sync(0xffffffffu, ng);
     once = __popc(tiles) == __popc(starts & __ballot_sync(0xffffffffu, used));
     __syncwarp();
@@ -219,7 +231,7 @@ __device__ __forceinline__ void bulk_load_hint_elect(void* smem_dst, const void*
 template <uint32_t NA>
 struct TileAt {
     uint32_t word, plane, rt;
-    __device__ __forceinline__ TileAt(const uint32_t* s_tile, uint32_t tile, uint32_t per_chunk, uint32_t row_tiles) {
+    __device__ __forceinline__ TileAt(const uint16_t* s_tile, uint32_t tile, uint32_t per_chunk, uint32_t row_tiles) {
         const uint32_t rem = tile % per_chunk;
         word = uniform(s_tile[tile / per_chunk]);
         plane = NA == 1u ? rem / row_tiles : 0u;
@@ -235,7 +247,7 @@ struct TileAt {
 // groups a block of one token took 38.2 us instead of 34.8, 512 tokens with 8 of 128 experts of 2048 x 768 180 instead of 166).
 template <uint32_t W, uint32_t NA, uint32_t KIND, uint32_t EPI, bool WG>
 __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensorMap& tmap_w1, const CUtensorMap& tmap_x, const Args& a,
-                                      uint8_t* rings, Ctl* sh, const uint32_t* s_expert, const uint32_t* s_tile, uint32_t tiles, bool once) {
+                                      uint8_t* rings, Ctl* sh, const uint32_t* s_expert, const uint16_t* s_tile, uint32_t tiles, bool once) {
     using G = Geo<W, NA>;
     constexpr uint32_t kBufs = NA == 2u ? 1u : 2u;
     const uint32_t warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31u;
@@ -472,8 +484,7 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constan
     uint8_t* rings = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
     Ctl* sh = reinterpret_cast<Ctl*>(rings + kRing);
     uint32_t* s_expert = reinterpret_cast<uint32_t*>(sh + 1);
-    uint32_t* s_tile = s_expert + kMaxBlocks;
-    uint8_t* s_live = reinterpret_cast<uint8_t*>(s_tile + kMaxBlocks);
+    uint16_t* s_tile = reinterpret_cast<uint16_t*>(s_expert + kMaxBlocks);
     const uint32_t warp = threadIdx.x >> 5;
 
     if (threadIdx.x == 0) {
@@ -502,29 +513,15 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constan
     uint32_t n, widest;
     bool once = false;   // every expert has one tile per row tile
     if (a.max_blocks <= 32u) {
-        s_tile = s_expert + 64u * warp;
-        s_expert = s_tile + 32u;
+        s_expert += 64u * warp;
+        s_tile = reinterpret_cast<uint16_t*>(s_expert + 32u);
         n = build_tiles_warp<MAXG>(a, s_expert, s_tile, widest, once);
-        tc5::fence_before_sync();
-        __syncthreads();
     } else {
-        for (uint32_t i = threadIdx.x; i < a.max_blocks; i += blockDim.x) {
-            const uint32_t e = table_word(a.block_expert + i);
-            s_expert[i] = e;
-            if (a.block_shift && e != PDK_MOE_PAD) {   // a 32-token block's padding is at its end
-                uint32_t live = 1;
-#pragma unroll
-                for (uint32_t g = 1; g < 4u; ++g) live += table_word(a.sorted_row + i * 32u + g * 8u) != PDK_MOE_PAD;
-                s_live[i] = (uint8_t)live;
-            }
-        }
-        __syncthreads();
-        if (warp == 0) build_tiles<MAXG>(a, s_expert, s_live, s_tile, sh);
-        tc5::fence_before_sync();
-        __syncthreads();
-        n = uniform(sh->tiles);
-        widest = uniform(sh->widest);
+        uint8_t* s_ng = reinterpret_cast<uint8_t*>(s_tile + kMaxBlocks);
+        n = build_tiles<MAXG>(a, s_expert, s_tile, s_ng, s_ng + kMaxBlocks, sh, widest);
     }
+    tc5::fence_before_sync();
+    __syncthreads();
     tc5::fence_after_sync();
     if (WG || widest <= 1u) roles<1u, NA, KIND, EPI, WG>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
     else if (widest <= 2u) roles<2u, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);

@@ -24,6 +24,11 @@ pytestmark = pytest.mark.gpu
     (500, 8, 2, 192, 320, 32, True, 2.0),     # runs of one block and of a dozen, rests of one to four groups
     (130, 4, 2, 256, 192, 32, False, 0.5),    # 12 blocks: every warp builds the table
     (37, 2, 1, 256, 128, 32, True, 0.0),      # two runs, each with a rest beside a whole block or less than one
+    (3000, 5, 2, 128, 64, 8, True, 0.7),      # 755 blocks: runs that span many of a warp's 32 blocks
+    (2600, 40, 3, 64, 64, 8, False, 0.0),     # 1015 blocks
+    (6000, 7, 4, 64, 128, 32, False, 0.5),    # 757 blocks of 32
+    (300, 16, 4, 1600, 1088, 32, True, 1.0),  # long K: the ring turns inside a tile, tiles alternate between accumulators
+    (200, 4, 2, 2112, 640, 8, True, 1.0),     # the same with runs of a dozen groups of 8
 ])
 def test_tiles_over_runs_of_blocks(pack, tokens, n_expert, k, embd, ff, bm, gated, skew):
     ex = P.GpuExecutor(pack)
