@@ -425,6 +425,7 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
                 scale2[s] = a.scale2[p][a.scale2_per_expert ? expert : 0u];
                 bias[s] = (n < a.out_dim && a.bias[p]) ? a.bias[p][(size_t)expert * a.out_dim + n] : 0.0f;
             }
+            const uint32_t live = __ballot_sync(0xffffffffu, my_src != PDK_MOE_PAD);
             float* out = a.out[t.plane];
             ok = __all_sync(0xffffffffu, wait_for(&sh->tmem_full[buf], aphase, ctx, tc5::kErrTmemFullWait, buf));
             if (!ok) break;
@@ -450,13 +451,15 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
                         v[s][i] = fmaf(__uint_as_float(r[s][24u + i]), 0.000244140625f,
                                        fmaf(__uint_as_float(r[s][16u + i]), 0.00390625f,
                                             fmaf(__uint_as_float(r[s][8u + i]), 0.0625f, __uint_as_float(r[s][i]))));
+                // plain rows are computed for padding too and the store is predicated: with a branch around each row a tile of 32
+                // tokens held the epilogue for 2500 cycles, and with short K it is what a tile costs (this form 1800)
 #pragma unroll
                 for (uint32_t i = 0; i < 8u; ++i) {
-                    const uint32_t src = __shfl_sync(0xffffffffu, my_src, from + i);
+                    const bool is_live = (live >> (from + i)) & 1u;
+                    if (KIND == kGated && !is_live) continue;   // a token of a decode step has seven of padding beside it
                     const uint32_t row = __shfl_sync(0xffffffffu, my_row, from + i);
                     const float step = __shfl_sync(0xffffffffu, my_step, from + i);
                     const float wgt = KIND != kGated ? __shfl_sync(0xffffffffu, my_wgt, from + i) : 1.0f;
-                    if (src == PDK_MOE_PAD || n >= a.out_dim) continue;
                     float y;
                     if (KIND == kGated) {
                         const float xg = fminf(fmaf(v[0][i], step * scale2[0], bias[0]), a.limit);
@@ -465,7 +468,7 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
                     } else {
                         y = fmaf(v[0][i], step * scale2[0] * wgt, bias[0] * wgt);   // (acc * scale2 * step + bias) * routing weight
                     }
-                    out[(size_t)row * a.out_dim + n] = y;
+                    if (is_live && n < a.out_dim) out[(size_t)row * a.out_dim + n] = y;
                 }
             }
             if (share >= ng && lane == 0) tc5::mbar_arrive(&sh->tmem_empty[buf]);   // a tile of fewer groups than shares
