@@ -451,12 +451,14 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
                         v[s][i] = fmaf(__uint_as_float(r[s][24u + i]), 0.000244140625f,
                                        fmaf(__uint_as_float(r[s][16u + i]), 0.00390625f,
                                             fmaf(__uint_as_float(r[s][8u + i]), 0.0625f, __uint_as_float(r[s][i]))));
-                // plain rows are computed for padding too and the store is predicated: with a branch around each row a tile of 32
-                // tokens held the epilogue for 2500 cycles, and with short K it is what a tile costs (this form 1800)
+                // Padding is computed too and the store is predicated: with a branch around each row a tile of 32 tokens held the
+                // epilogue for 2500 cycles, and with short K it is what a tile costs (this form 1800).  The gated unit costs more a row,
+                // and a group of a decode step has one or two tokens: it may stop at two points.
+                const uint32_t rows = KIND == kGated ? 32u - __clz((live >> from) & 0xFFu) : 8u;
 #pragma unroll
                 for (uint32_t i = 0; i < 8u; ++i) {
+                    if (KIND == kGated && (i == 2u || i == 4u) && rows <= i) break;
                     const bool is_live = (live >> (from + i)) & 1u;
-                    if (KIND == kGated && !is_live) continue;   // a token of a decode step has seven of padding beside it
                     const uint32_t row = __shfl_sync(0xffffffffu, my_row, from + i);
                     const float step = __shfl_sync(0xffffffffu, my_step, from + i);
                     const float wgt = KIND != kGated ? __shfl_sync(0xffffffffu, my_wgt, from + i) : 1.0f;
