@@ -32,22 +32,24 @@ struct Args {
 };
 
 // The ring leaves 16 KB of an SM's shared memory: the kernels in front and behind are dependent launches, and a CTA of theirs
-// that finds no room here starts when this one has left (a ring of 216 KB cost a block of one token 0.4 us).
-constexpr uint32_t kRing = 196u * 1024u, kMaxSlots = 10u;
+// that finds no room here starts when this one has left (a ring of 216 KB cost a block of one token 0.4 us).  The ring of LONG runs
+// takes it all: three stages of two slabs.
+constexpr uint32_t kRing = 196u * 1024u, kRingLong = 216u * 1024u, kMaxSlots = 10u;
 constexpr uint32_t kMaxBlocks = 1024;  // block_expert[] and the tile table are kept in shared memory
 constexpr size_t kTableBytes = kMaxBlocks * 8u;   // experts, tiles, groups by block, live groups
 
 // W groups per tile at most, NA weight tiles of 128 rows under one B.  NA = 2 (gate and up): one pair of accumulators.  NA = 1:
 // two accumulators, the next tile's MMAs run under this one's epilogue.  A stage of the ring is KS slabs (256 elements) of the
-// weight tiles, the groups and their scale records; a stage's hand-off costs the issuing warp about as long as half a slab.
-template <uint32_t W, uint32_t NA>
+// weight tiles, the groups and their scale records; a stage's hand-off costs the issuing warp about as long as half a slab (its
+// busy cycles per slab of four groups: 530 in stages of two slabs, 615 in stages of one, 660 with the second scale cell of six groups).
+template <uint32_t W, uint32_t NA, bool LONG>
 struct Geo {
-    static constexpr uint32_t kS = NA == 1u && W <= 2u ? 2u : 1u;
+    static constexpr uint32_t kS = NA == 1u && W <= (LONG ? 4u : 2u) ? 2u : 1u;
     static constexpr uint32_t kN = W * 32u, kGroupBytes = 32u * BKB, kQuads = (W + 3u) / 4u;
     // a stage: weight boxes [tile][slab], groups [slab][group], weight records [tile][slab], activation records [quad][slab]
     static constexpr uint32_t kOffB = kS * NA * kABytes, kOffSfa = kOffB + kS * W * kGroupBytes;
     static constexpr uint32_t kOffSfb = kOffSfa + kS * NA * kSfBytes, kSlot = kOffSfb + kS * kQuads * kSfBytes;
-    static constexpr uint32_t kFit = kRing / kSlot, kSlots = kFit < kMaxSlots ? kFit : kMaxSlots;
+    static constexpr uint32_t kFit = (LONG ? kRingLong : kRing) / kSlot, kSlots = kFit < kMaxSlots ? kFit : kMaxSlots;
     // tensor memory: two accumulators, then the scale cells of a slab; copies and MMAs of one thread execute in order, two
     // sets or more let a slab's copies run under the MMAs of the one before
     static constexpr uint32_t kSfStep = 4u * kQuads, kSfSlab = NA * 16u + 4u * kSfStep, kSfCol0 = 2u * kN;
@@ -245,10 +247,10 @@ struct TileAt {
 // The code is kept short - one group per turn of the epilogue's loop, one kernel for raw rows and for down: what a launch runs is
 // fetched into the instruction cache anew when another large kernel ran in between (with the epilogue unrolled over a tile's
 // groups a block of one token took 38.2 us instead of 34.8, 512 tokens with 8 of 128 experts of 2048 x 768 180 instead of 166).
-template <uint32_t W, uint32_t NA, uint32_t KIND, uint32_t EPI, bool WG>
+template <uint32_t W, uint32_t NA, uint32_t KIND, uint32_t EPI, bool WG, bool LONG>
 __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensorMap& tmap_w1, const CUtensorMap& tmap_x, const Args& a,
                                       uint8_t* rings, Ctl* sh, const uint32_t* s_expert, const uint16_t* s_tile, uint32_t tiles, bool once) {
-    using G = Geo<W, NA>;
+    using G = Geo<W, NA, LONG>;
     constexpr uint32_t kBufs = NA == 2u ? 1u : 2u;
     const uint32_t warp = uniform(threadIdx.x >> 5), lane = threadIdx.x & 31u;
     const uint32_t row_tiles = (a.out_dim + BM - 1u) / BM;
@@ -479,7 +481,7 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
 }
 
 // MAXG: the most groups of a tile, 4 or 6 (build_tiles); the launch takes the geometry of the widest tile that it has.
-template <uint32_t MAXG, uint32_t NA, uint32_t KIND, uint32_t EPI, bool WG>
+template <uint32_t MAXG, uint32_t NA, uint32_t KIND, uint32_t EPI, bool WG, bool LONG>
 __global__ void __launch_bounds__(96u + 32u * EPI, 1)
 grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constant__ CUtensorMap tmap_w1,
                const __grid_constant__ CUtensorMap tmap_x, const Args a) {
@@ -487,7 +489,7 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constan
     static_assert(MAXG <= EPI, "a warp's lanes hold the routing data of four groups: EPI / 4 shares of up to four");
     extern __shared__ uint8_t smem_raw[];
     uint8_t* rings = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023u) & ~(uintptr_t)1023u);
-    Ctl* sh = reinterpret_cast<Ctl*>(rings + kRing);
+    Ctl* sh = reinterpret_cast<Ctl*>(rings + (LONG ? kRingLong : kRing));
     uint32_t* s_expert = reinterpret_cast<uint32_t*>(sh + 1);
     uint16_t* s_tile = reinterpret_cast<uint16_t*>(s_expert + kMaxBlocks);
     const uint32_t warp = threadIdx.x >> 5;
@@ -528,10 +530,10 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constan
     tc5::fence_before_sync();
     __syncthreads();
     tc5::fence_after_sync();
-    if (WG || widest <= 1u) roles<1u, NA, KIND, EPI, WG>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
-    else if (widest <= 2u) roles<2u, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
-    else if (widest <= 4u) roles<4u, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
-    else if (MAXG > 4u) roles<MAXG, NA, KIND, EPI, false>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
+    if (WG || widest <= 1u) roles<1u, NA, KIND, EPI, WG, LONG>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
+    else if (widest <= 2u) roles<2u, NA, KIND, EPI, false, LONG>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
+    else if (widest <= 4u) roles<4u, NA, KIND, EPI, false, LONG>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
+    else if (MAXG > 4u) roles<MAXG, NA, KIND, EPI, false, LONG>(tmap_w0, tmap_w1, tmap_x, a, rings, sh, s_expert, s_tile, n, once);
 
     tc5::fence_before_sync();
     __syncthreads();
@@ -541,11 +543,11 @@ grouped_kernel(const __grid_constant__ CUtensorMap tmap_w0, const __grid_constan
     }
 }
 
-template <uint32_t MAXG, uint32_t NA, uint32_t KIND, uint32_t EPI, bool WG = false>
+template <uint32_t MAXG, uint32_t NA, uint32_t KIND, uint32_t EPI, bool WG = false, bool LONG = false>
 int launch(const CUtensorMap& tw0, const CUtensorMap& tw1, const CUtensorMap& tx, const Args& a, cudaStream_t st) {
-    constexpr size_t smem = (size_t)kRing + sizeof(Ctl) + kTableBytes + 1024u;
+    constexpr size_t smem = (size_t)(LONG ? kRingLong : kRing) + sizeof(Ctl) + kTableBytes + 1024u;
     static_assert(smem <= 227u * 1024u, "shared memory of an SM");
-    auto kern = grouped_kernel<MAXG, NA, KIND, EPI, WG>;
+    auto kern = grouped_kernel<MAXG, NA, KIND, EPI, WG, LONG>;
     const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return (int)e;
     const uint32_t row_tiles = (a.out_dim + BM - 1u) / BM;

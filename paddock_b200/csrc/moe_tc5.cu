@@ -751,11 +751,19 @@ static int gemm_impl(const PlaneArgs& w0, const PlaneArgs& w1, void* out0, void*
     a.n_active = n_active; a.scatter = kind == moe_gemm::kScatter; a.ahead = ahead; a.block_shift = bm == 32u ? 2u : 0u;
     a.alpha = unit.alpha; a.limit = unit.limit; a.up_add = unit.up_add; a.err_word = pdk_error_word();
     auto st = (cudaStream_t)stream;
-    // The gated unit needs gate and up in one CTA.  Tiles of up to six groups where blocks are large (1024 tokens, 4 of 128 experts,
-    // 2880 x 2880: down 150 -> 130 us).
+    // The gated unit needs gate and up in one CTA.  One plane, blocks of 32: where an expert has a block or a little more on average,
+    // half of the experts spill a few tokens into the next one, and tiles of up to six groups save that pass over the weights
+    // (1024 tokens, 4 of 128 experts, 2880 x 2880: down 150 -> 130 us).  From 48 tokens an expert on, runs are long and the tensor core is what
+    // they wait for: tiles of four groups in stages of two slabs (down of 1000 tokens an expert, 2048 x 2048: 54.2 -> 42.8 us, of 256,
+    // 2880 x 768: 126 -> 104; but of 44, 1664 x 2176: 78 -> 85).  Blocks of 8: six groups instead of four 0.97 to 1.08 times
+    // the time over 40 shapes, 1.00 on average.
     using namespace moe_gemm;
     if (kind == kGated) return launch<6, 2, kGated, 12>(tw0, tw1, tx, a, st);
-    return bm == 32u ? launch<6, 1, kPlain, 8>(tw0, tw1, tx, a, st) : launch<4, 1, kPlain, 8>(tw0, tw1, tx, a, st);
+    if (bm == 8u) return launch<4, 1, kPlain, 8>(tw0, tw1, tx, a, st);
+    // max_blocks has room for a partly filled block of every expert
+    const uint64_t tokens = max_blocks > n_expert ? (uint64_t)(max_blocks - n_expert) * bm : 0u;
+    return tokens > 48ull * n_expert ? launch<4, 1, kPlain, 8, false, true>(tw0, tw1, tx, a, st)
+                                     : launch<6, 1, kPlain, 8>(tw0, tw1, tx, a, st);
 }
 
 PDK_EXPORT int pdk_mxfp4_moe_gemm_tc5(const void* w0_data, const void* w0_sf, const void* w0_meta, const void* w0_bias,
