@@ -136,12 +136,14 @@ def repack_mxfp4(ex, raw_dev):
 
 def _unit_in_gemm(ws, max_blocks, ff, n_expert):
     """Whether the gate|up GEMM applies the gated unit itself.  It then keeps both accumulators in one CTA and writes one plane
-    instead of two: with 32-token blocks that saves 94 MB each way at 1024 tokens (gate|up + second preparation 313 -> 250 us).
-    With 8-token blocks two accumulators per tile overlap better and the raw planes stay in L2 (60 tokens: 172 against 174 us; 128
-    tokens on 32 experts of 1024 x 768: 20 against 23), but where tiles of one plane would just need a second round over the SMs
-    (one token of 4 experts of 2880 x 2880: 31.9 us a block against 30.3)."""
+    instead of two, but no tile's epilogue runs under the next tile's MMAs.  With 32-token blocks that pays where a CTA has ten
+    tiles or more: 1024 tokens, 4 of 128 experts, 2880 x 2880 (40 tiles each) 0.91 of the raw planes' time, 64 experts of 2432 x 1408, 913
+    tokens (22) 0.91; 32 experts of 1920 x 896, 130 tokens (3) 1.11, 64 of 1024 x 960, 1547 tokens (6) 1.17; the line
+    loses 0.2 % over 70 shapes, 3 % at worst (always the unit 2.7 and 17 %).  With 8-token blocks the raw planes stay in L2 (60
+    tokens: 172 against 174 us; 128 tokens on 32 experts of 1024 x 768: 20 against 23), but where tiles of one plane would just need
+    a second round over the SMs (one token of 4 experts of 2880 x 2880: 31.9 us a block against 30.3)."""
     tiles = max_blocks * ((ff + 127) // 128)
-    return _by_pair(ws, n_expert) and (ws.bm == 32 or tiles <= ws.sms < 2 * tiles)
+    return _by_pair(ws, n_expert) and (tiles >= 10 * ws.sms if ws.bm == 32 else tiles <= ws.sms < 2 * tiles)
 
 
 class MoeWorkspace:
