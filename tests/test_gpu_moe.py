@@ -272,16 +272,16 @@ def test_nvf4_moe_block_matches_f64(pack, tokens, n_expert, k, embd, ff, bm, gat
     assert rel_l2(y, ref) < 2e-3 < TOL
 
 
-@pytest.mark.parametrize("in_dim,dual", [(1792, False), (2048, True), (2624, True)])
-def test_gate_and_up_in_one_tile_equal_one_plane_calls(pack, in_dim, dual):
-    """32-token blocks, both sides of prefer_dual's line (8 slabs of K; a whole and a ragged last slab, a ragged last row tile):
-    gate and up in one call give the bits of one call per plane, which always takes one tile at a time."""
+@pytest.mark.parametrize("in_dim", [1792, 2048, 2624])
+def test_two_planes_in_one_call_equal_one_plane_calls(pack, in_dim):
+    """Raw gate and up of 32-token blocks in one launch (a whole and a ragged last slab, a ragged last row tile): every tile takes its
+    own plane, so the bits are those of one launch per plane.  (The kernel with both planes under one B is
+    test_gpu_moe_grouped.py's.)"""
     n_expert, tokens, k, bm, out_dim = 8, 1024, 4, 32, 2400
     gen = torch.Generator(device="cuda").manual_seed(in_dim)
     rand = lambda lo, hi, n: torch.randint(lo, hi, (n,), dtype=torch.uint8, device="cuda", generator=gen)
     max_blocks = tokens * k // bm + n_expert
     slabs, row_tiles = (in_dim + 255) // 256, (out_dim + 127) // 128
-    assert (slabs >= 8 and max_blocks * row_tiles >= 16 * torch.cuda.get_device_properties(0).multi_processor_count) == dual
     i32 = lambda n: torch.zeros(n, dtype=torch.int32, device="cuda")
     idx, wgt, row, slot, blk = i32(tokens * k), torch.zeros(tokens * k, device="cuda"), i32(max_blocks * bm), i32(max_blocks * bm), i32(max_blocks)
     pack.call("moe_topk_batch", torch.randn(tokens * n_expert, device="cuda", generator=gen), None, n_expert, k, idx, wgt, tokens)

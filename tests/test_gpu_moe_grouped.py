@@ -247,3 +247,79 @@ def test_slot_combine_adds_every_row_once(pack, rows, k, embd):
     pack.call("moe_slot_combine", part, res, embd, k, rows)
     torch.cuda.synchronize()
     assert pack.device_error() == 0 and torch.equal(res, want)
+
+
+UNITS = {"clamped": (1.702, 7.0, 1.0), "swiglu": (1.0, float("inf"), 0.0), "tight": (1.2, 0.5, 0.25)}   # tight: most values reach the limit
+
+
+@pytest.mark.parametrize("tokens,n_expert,k,in_dim,out_dim,bm,skew,unit", [
+    (1, 8, 4, 320, 384, 8, 0.0, "clamped"),       # tiles of one group, one token in it
+    (37, 2, 1, 256, 128, 32, 0.0, "swiglu"),      # a run of one block and a rest
+    (150, 8, 2, 448, 320, 8, 3.0, "tight"),       # runs of a dozen groups of 8, a ragged last row tile
+    (60, 32, 4, 2112, 136, 8, 0.0, "clamped"),    # long K: the ring turns inside a tile; eight rows in the last row tile
+    (300, 16, 4, 1600, 200, 32, 1.0, "swiglu"),   # runs of one to many blocks, tiles of one to six groups
+    (700, 64, 2, 256, 256, 32, 0.0, "tight"),     # more than 32 blocks, 22 tokens an expert
+    (2000, 24, 2, 576, 256, 32, 0.3, "clamped"),  # several tiles a CTA under its one pair of accumulators
+])
+@pytest.mark.parametrize("fmt", ["mxfp4", "nvf4"])
+def test_gate_and_up_under_one_operand_equal_raw_planes_and_the_unit(pack, tokens, n_expert, k, in_dim, out_dim, bm, skew, unit, fmt):
+    """pdk_*_moe_gate_up_tc5 against the unit, in f64, of the raw rows that one-plane calls leave.  Both kernels sum a row in the
+    same order, so what may differ is the unit's f32 arithmetic: __expf is within 2 + 1.173 |x| ulp (CUDA's bound), the sigmoid takes
+    over at most that, and the sum, the quotient, the two products and the second factor's sum round once each."""
+    c = P.GpuExecutor(pack).pack.call
+    alpha, limit, up_add = UNITS[unit]
+    gen = torch.Generator(device="cuda").manual_seed(tokens + out_dim)
+    rand = lambda lo, hi, n: torch.randint(lo, hi, (n,), dtype=torch.uint8, device="cuda", generator=gen)
+    norm = lambda *n: torch.randn(*n, device="cuda", generator=gen)
+    new = lambda n, dt=torch.int32: torch.zeros(n, dtype=dt, device="cuda")
+    pairs, slabs, row_tiles, u8 = tokens * k, (in_dim + 255) // 256, (out_dim + 127) // 128, torch.uint8
+    max_blocks = min(pairs, pairs // bm + n_expert)
+    nb = max_blocks * bm
+    logits = norm(tokens, n_expert) - skew * torch.arange(n_expert, device="cuda")
+    idx, w, row, slot, blk = new(pairs), new(pairs, torch.float32), new(nb), new(nb), new(max_blocks)
+    c("moe_topk_batch", logits.view(-1), None, n_expert, k, idx, w, tokens)
+    c("moe_align_bm", idx, row, slot, blk, tokens, k, n_expert, bm, max_blocks)
+    planes = []
+    for _ in range(2):
+        data, tiled = rand(0, 256, n_expert * out_dim * in_dim // 2), new(n_expert * row_tiles * slabs * 2048, u8)
+        if fmt == "mxfp4":
+            factor = new(2)
+            c("pdk_mxfp4_tc5_tile_scales", rand(117, 122, n_expert * out_dim * in_dim // 32), tiled, factor, out_dim, in_dim, n_expert)
+        else:
+            factor = (torch.rand(n_expert, device="cuda", generator=gen) + 0.5) * 0.02
+            c("pdk_nvf4_moe_tile_scales", rand(0x20, 0x40, n_expert * out_dim * in_dim // 16), tiled, out_dim, in_dim, n_expert)
+        planes.append((data, tiled, factor, norm(n_expert * out_dim)))
+    x = norm(tokens * in_dim)
+    xq, xs, step = new(nb * 4 * in_dim // 2, u8), new(max_blocks * slabs * 2048, u8), new(nb, torch.float32)
+    prep_args = x, None, row, blk, xq, xs, step, in_dim, bm, max_blocks, 0, 1.0, 7.0
+    prepare = lambda: c(*(("pdk_moe_prep_act_f4", *prep_args) if fmt == "mxfp4" else ("pdk_moe_prep_act_f4n", *prep_args, 0.0)))
+    rows = xq, xs, step, blk, row
+    dims = in_dim, out_dim, n_expert, bm, max_blocks
+    one = (None,) * 5
+    gemm = f"pdk_{'mxfp4' if fmt == 'mxfp4' else 'nvf4'}_moe_gemm_tc5"
+    raw = [torch.full((nb, out_dim), -7.5, device="cuda") for _ in range(6)]
+    part = [torch.zeros(pairs, out_dim, device="cuda") for _ in range(2)]
+    prepare()
+    for p in range(2):
+        c(gemm, *planes[p], raw[p], *one, *rows, None, None, *dims, k, 0)
+    c(gemm, *planes[0], part[0], *one, *rows, slot, w, *dims, k, 1)
+    # the calls that begin under a preparation in front of them
+    prepare()
+    c(gemm + "_ahead", *planes[0], raw[2], *planes[1], raw[3], *rows, None, None, *dims, k, 0)
+    prepare()
+    c(gemm + "_ahead", *planes[0], part[1], *one, *rows, slot, w, *dims, k, 1)
+    prepare()
+    c(gemm.replace("gemm", "gate_up"), *planes[0], *planes[1], raw[4], *rows, *dims, alpha, limit, up_add)
+    torch.cuda.synchronize()
+    assert pack.device_error() == 0
+    assert torch.equal(raw[0], raw[2]) and torch.equal(raw[1], raw[3]) and torch.equal(part[0], part[1]) and bool(part[0].any())
+    used = (blk != -1).repeat_interleave(bm) & (row != -1)
+    assert int(used.sum()) == pairs
+    assert bool((raw[4][~used] == -7.5).all())                       # rows of padding are left alone
+    g, u = raw[0][used].double(), raw[1][used].double()
+    xg, yu = g.clamp(max=limit), u.clamp(-limit, limit)
+    ref = xg / (1.0 + torch.exp(-alpha * xg)) * (yu + up_add)
+    if np.isfinite(limit):
+        assert 0.0 < float((g > limit).double().mean()) < 1.0 or unit == "clamped"
+    bound = ((2.0 + 1.173 * (alpha * xg).abs() + 6.0) * 2.0 ** -23) * ref.abs() + 1e-30
+    assert bool(((raw[4][used].double() - ref).abs() <= bound).all())
