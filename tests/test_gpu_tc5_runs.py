@@ -1,5 +1,8 @@
 """The runs of q4k_tc5.cu: equal runs of unit pairs that cut tiles anywhere (a tile per SM and more), half tiles of even and odd pair counts, one
-pair to a tile, ragged rows.  Bound: weights rounded to f16, 1e-4 of sum |w||x| as in test_gpu_gemv.py."""
+pair to a tile, ragged rows.  Up to 16 tokens a CTA requests and dequantizes a ring of three boxes (pairs) before it waits for the
+activation rows: runs of fewer boxes, of three, of four and of more, with tiles that change inside the ring and without.
+Bound: weights rounded to f16, 1e-4 of sum |w||x| as in test_gpu_gemv.py (a weight's rounding is at most 2^-11 of it and a row's add up
+like a random walk: the bound is 5 deviations at K = 512, where half a million results of one call reach 1.2e-4)."""
 import numpy as np
 import pytest
 import torch
@@ -12,7 +15,10 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("k,n,batch,name", [(512, 6001, 9, "q4_k"), (512, 19000, 16, "q4_0"), (1024, 2561, 16, "q4_k"), (1024, 19001, 20, "q4_k"),
-                                            (1536, 9001, 12, "q4_k"), (1536, 20000, 9, "q4_0"), (2560, 19100, 33, "q4_k"), (3584, 12000, 16, "q4_0")])
+                                            (1536, 9001, 12, "q4_k"), (1536, 20000, 9, "q4_0"), (2560, 19100, 33, "q4_k"), (3584, 12000, 16, "q4_0"),
+                                            (1536, 12000, 16, "q4_k"),      # a tile of three boxes a CTA: the ring
+                                            (2048, 12000, 9, "q4_0"),       # of four: one more
+                                            (1024, 33001, 12, "q4_k")])     # three or four, two to a tile
 def test_runs(pack, k, n, batch, name):
     dtype = 12 if name == "q4_k" else 2
     assert pack._lib.pdk_kquant_gemm_route(k, n, batch, dtype) == 3
