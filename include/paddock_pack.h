@@ -419,7 +419,8 @@ int pdk_mxfp4_tc5_tile_scales(const void* scale, void* tiled, void* meta, uint32
 /* Block positions (pd_moe_align_bm order) -> four NVFP4 term rows each:
  * mode 0: position p = row sorted_row[p] of x f32[rows][dim];  mode 1: position p =
  * swiglu_oai(x[p], up[p]) of raw gate / up outputs f32[positions][dim].
- * Padding positions of used blocks become zero rows; the rows of unused blocks (block_expert = PDK_MOE_PAD),
+ * The entries of a block are at its front, as moe_align_bm leaves them.  Padding positions become zero rows where their
+ * group of eight positions has an entry; the rows of groups without one and of unused blocks (block_expert = PDK_MOE_PAD),
  * which the GEMMs skip, are left as they are.
  * xq u8[max_blocks*4*bm][dim/2], term t of position p in row p/8*32 + t*8 + p%8; xs
  * u8[max_blocks][ceil(dim/256)][2048] (scale records, the layout of the tiled weight scales; a record holds

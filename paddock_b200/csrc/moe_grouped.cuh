@@ -263,8 +263,10 @@ __device__ __forceinline__ void roles(const CUtensorMap& tmap_w0, const CUtensor
     if (warp == 0) {
         // ------------------------------------------------------------ weights (whole warp, one lane issues)
         // Weights that a small call reads once leave L2 first, so the rows that the launches around this one hand on stay there (128
-        // experts of 2880 x 2880, 1 / 4 / 8 tokens: 27.3 / 54.5 / 84.3 -> 26.0 / 50.9 / 80.4 us a block).  In calls of most experts
-        // it is slower (60 tokens 273 -> 293: the rest of a 256-byte line that the next slab wants has left by then).
+        // experts of 2880 x 2880, 1 / 4 / 8 tokens: 27.3 / 54.5 / 84.3 -> 26.0 / 50.9 / 80.4 us a block; over 24 shapes of up to 32
+        // blocks 1.006 to 1.08 times faster, 1.04 on average).  Calls of most experts keep the normal policy: 60 tokens of that block
+        // take 1.04 times as long with the other (the rest of a 256-byte line that the next slab wants has left by then), though of
+        // 16 shapes with 37 to 160 blocks most would gain 1 to 6 %.
         const uint64_t policy = once ? tc5::l2_policy_evict_first() : l2_policy_normal();
         uint32_t stage = 0, phase = 0;
         bool ok = true;

@@ -312,7 +312,6 @@ PDK_EXPORT int pd_moe_topk_batch(const void* logits, const void* bias, uint32_t 
                           (const float*)logits, (const float*)bias, n_expert, k, (uint32_t*)out_idx, (float*)out_w, batch);
 }
 
-// slot 146, packs/cuda/src/gemm/f32_qkv.cuh:1269-1279 (kernel attn/decode.cuh:2316-2396)
 // shared memory of align_cta without and with the staged positions
 static size_t align_smem(uint32_t n_expert, uint32_t warps) { return ((size_t)(warps + 2u) * n_expert + 65u) * sizeof(uint32_t); }
 
@@ -348,6 +347,7 @@ static int align_impl(const void* idx, void* sorted_row, void* sorted_slot, void
     return pdk_launch_status();
 }
 
+// slot 146, packs/cuda/src/gemm/f32_qkv.cuh:1269-1279 (kernel attn/decode.cuh:2316-2396)
 PDK_EXPORT int pd_moe_align_bm(const void* idx, void* sorted_row, void* sorted_slot, void* block_expert,
                                uint32_t rows, uint32_t n_active, uint32_t n_expert, uint32_t bm, uint32_t max_blocks,
                                void* stream) {

@@ -136,7 +136,8 @@ __device__ __forceinline__ float rcp_approx(float v) {
 // terms' codes, handed to put(term, codes), and the four scale bytes as one word.  The residual stays unscaled; the power 16^k of term k sits
 // in its scale's factor (exact), and the last term leaves none.  The kernels around it are bound by issue: this is half the
 // instructions of the form that scaled 16 residuals up per term, divided by the scale and worked on single floats.  One copy of a
-// term's code: what a launch runs once per thread it fetches into the instruction cache first.
+// term's code: what a launch runs once per thread it fetches into the instruction cache first.  The reciprocal is the approximate
+// instruction, but of a value with three bits of mantissa: for every scale byte and term it is the rounded quotient's bits.
 template <class Put>
 __device__ __forceinline__ uint32_t quantize_group(float2 (&r)[8], Put&& put) {
     float up = 1.0f / 6.0f, down = 1.329227995784916e36f;   // 2^120
@@ -213,7 +214,7 @@ __device__ __forceinline__ uint32_t scale_word(uint32_t v) {
     return lane & 2u ? __byte_perm(v, b, 0x3276) : __byte_perm(v, b, 0x5410);
 }
 
-// One CTA per block position.  Position (block b, token i) writes four term rows of its group of 8 tokens,
+// One CTA per block position; groups of eight without a token return before this.  Position (block b, token i) writes four term rows of its group of 8 tokens,
 // row term * 8 + i % 8 of the group's 32.  A 16-element scale group of the tensor core's element order is the
 // two 8-runs (h*8 .. h*8+7) and (16 + h*8 .. 16 + h*8+7) of a 32-element block.
 __device__ __forceinline__ void prep_position(const PrepArgs& a, uint32_t pos, uint32_t src, uint32_t rec, uint32_t col) {

@@ -247,7 +247,8 @@ def _prepare_unit(ex, ws, x, up, rows, ff, n_expert, max_blocks, mode, natural, 
 def moe_mxfp4_experts_tc5(ex, planes, ws, x, rows, alpha=1.702, limit=7.0, route=None):
     """moe_mxfp4_experts on the block-scaled tensor-core path (planes prepared with prepare_tc5):
     align -> term rows of x -> gate and up GEMM -> SwiGLU + term rows of h -> down GEMM scattered
-    into ws.part.  Five launches; route = (router_logits, router_bias) has the experts chosen here too."""
+    into ws.part.  Returns the number of launches: five, and one more (none at decode widths) with route = (router_logits,
+    router_bias), which has the experts chosen here too."""
     st = _stream()
     c = ex.pack.call
     k, bm, t = ws.n_active, ws.bm, planes.tc5
